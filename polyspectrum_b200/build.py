@@ -30,8 +30,8 @@ DRIVER = os.path.join(PKG, "ps_run")
 KBENCH = os.path.join(PKG, "ps_kbench")
 CREATE_INI_SRC = os.path.join(PKG, "driver", "ps_create_ini.c")
 CREATE_INI = os.path.join(PKG, "ps_create_ini")
-SOURCES = ["ps_api.cu", "ps_inst_f32.cu", "ps_inst_f64.cu", "ps_inst_f32_mixed.cu", "ps_inst_f64_mixed.cu",
-           "ps_noalloc.cu"]
+SOURCES = ["ps_inst_f32_a.cu", "ps_inst_f32_b.cu", "ps_inst_f32_mixed.cu", "ps_inst_f64_mixed.cu", "ps_inst_f64_a.cu",
+           "ps_api.cu", "ps_inst_f32_c.cu", "ps_inst_f64_b.cu", "ps_inst_f64_c.cu", "ps_noalloc.cu"]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-ffp-contract=off"]
@@ -47,6 +47,17 @@ def nvcc() -> str:
 def _deps() -> list[str]:
     return (glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh"))
             + glob.glob(os.path.join(ROOT, "include", "*.h")))
+
+
+def _stale(obj: str) -> bool:
+    """Whether an object is older than a file it was compiled from (nvcc's own dependency list)."""
+    dep = obj + ".d"
+    if not os.path.exists(obj) or not os.path.exists(dep):
+        return True
+    with open(dep) as f:
+        files = f.read().split(":", 1)[1].replace("\\\n", " ").split()
+    t = os.path.getmtime(obj)
+    return any(not os.path.exists(p) or os.path.getmtime(p) > t for p in files)
 
 
 def up_to_date() -> bool:
@@ -91,7 +102,9 @@ def build(force: bool = False, ptxas_verbose: bool = False, quiet: bool = False)
     for src in SOURCES:
         obj = os.path.join(OUT_DIR, src.replace(".cu", ".o"))
         objs.append(obj)
-        cmd = [exe, *FLAGS, "-c", os.path.join(CSRC, src), "-o", obj]
+        if not force and not ptxas_verbose and not _stale(obj):
+            continue
+        cmd = [exe, *FLAGS, "-MD", "-MF", obj + ".d", "-c", os.path.join(CSRC, src), "-o", obj]
         if ptxas_verbose:
             cmd += ["-Xptxas", "-v"]
         procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT,

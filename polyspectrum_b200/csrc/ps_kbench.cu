@@ -16,7 +16,7 @@
 #include <vector>
 #include <cmath>
 #include <algorithm>
-#include "ps_launch.cuh"
+#include "ps_launch_impl.cuh"
 #include "ps_counts.cuh"
 
 namespace ps {
