@@ -24,6 +24,7 @@
 #include "../../include/ps_gpu.h"
 #include "ps_launch.cuh"
 #include "ps_counts.cuh"
+#include "ps_pair2.cuh"
 
 namespace ps {
 PS_EXTERN_L3(float)
@@ -1863,11 +1864,28 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
             table.push_back(host_shell_of(s));
         }
     }
-    struct P2Chunk {
-        int ofs, cnt, band, lut_size, idx_ofs;
-        bool lut_ok;
+    // n = 2: lists whose shells are all r^2 intervals take one sweep over the
+    // field spectrum (ps_pair2.cuh), the others (WATKINSON) one pass per 16
+    struct P2Pass {
+        int ofs, cnt, band, idx_ofs;
     };
-    std::vector<P2Chunk> p2;
+    std::vector<P2Pass> p2;
+    std::vector<P2Range> iv;   // sorted by lo
+    std::vector<int> iv_cfg;
+    {
+        std::vector<int> other;
+        for (int q : pairs2) {
+            const Shell &sa = host_shell_of(lid[q][0]), &sb = host_shell_of(lid[q][1]);
+            (sa.kind <= SHELL_RANGE && sb.kind <= SHELL_RANGE ? iv_cfg : other).push_back(q);
+        }
+        pairs2.swap(other);
+        auto range_of = [&](int q) {
+            const Shell &sa = host_shell_of(lid[q][0]), &sb = host_shell_of(lid[q][1]);
+            return P2Range{std::max(sa.r2lo, sb.r2lo), std::min(sa.r2hi, sb.r2hi)};
+        };
+        std::stable_sort(iv_cfg.begin(), iv_cfg.end(), [&](int x, int y) { return range_of(x).lo < range_of(y).lo; });
+        for (int q : iv_cfg) iv.push_back(range_of(q));
+    }
     std::vector<int> idx_all;  // scatter indices (groups, then n=2 chunks)
     std::vector<int> gidx_ofs(groups.size());
     for (size_t g = 0; g < groups.size(); g++) {
@@ -1875,31 +1893,26 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
         for (int q : groups[g].cfg) idx_all.push_back(q);
     }
     for (size_t q0 = 0; q0 < pairs2.size(); q0 += MAX_DOT_SHELLS) {
-        P2Chunk ch;
+        P2Pass ch;
         ch.cnt = (int)std::min<size_t>(MAX_DOT_SHELLS, pairs2.size() - q0);
         ch.ofs = (int)table.size();
-        ch.lut_ok = true;
         ch.band = 0;
-        ch.lut_size = 0;
         for (int x = 0; x < ch.cnt; x++) {
             const Shell& sa = host_shell_of(lid[pairs2[q0 + x]][0]);
             const Shell& sb = host_shell_of(lid[pairs2[q0 + x]][1]);
             table.push_back(sa);
             table.push_back(sb);
             ch.band = std::max(ch.band, std::min(sa.band, sb.band));
-            if (sa.kind > SHELL_RANGE || sb.kind > SHELL_RANGE) ch.lut_ok = false;
-        }
-        for (int x = 0; x < ch.cnt && ch.lut_ok; x++) {
-            Shell iv = table[ch.ofs + 2 * x];
-            iv.r2lo = std::max(table[ch.ofs + 2 * x].r2lo, table[ch.ofs + 2 * x + 1].r2lo);
-            iv.r2hi = std::min(table[ch.ofs + 2 * x].r2hi, table[ch.ofs + 2 * x + 1].r2hi);
-            ch.lut_size = std::max(ch.lut_size, iv.r2hi + 1);
-            table.push_back(iv);
         }
         ch.idx_ofs = (int)idx_all.size();
         for (int x = 0; x < ch.cnt; x++) idx_all.push_back(pairs2[q0 + x]);
         p2.push_back(ch);
     }
+    int p2_lut = 0, p2_blocks = 0;
+    const std::vector<P2Chunk> chunks = pair2_chunks(iv, N, 148 * 9 * 2, &p2_lut);
+    if (!chunks.empty()) p2_blocks = chunks.back().block0 + chunks.back().nblocks;
+    const int iv_ofs = (int)idx_all.size();
+    for (int q : iv_cfg) idx_all.push_back(q);
 
     // ---- device buffers of the plan, scratch of the context sized up front
     Shell* dtable = nullptr;
@@ -1926,6 +1939,16 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
     for (int q = 0; q < nconf; q++) coef[q] = norm_coef(L, N, cfgs[q].n);
     double* dcoef = nullptr;
     PS_TRY(plan_upload(P, &dcoef, coef));
+    P2Chunk* dchunks = nullptr;
+    unsigned short* dp2lut = nullptr;
+    if (!chunks.empty()) {
+        P2Range* div = nullptr;
+        PS_TRY(plan_upload(P, &dchunks, chunks));
+        PS_TRY(plan_upload(P, &div, iv));
+        PS_TRY(plan_alloc(P, &dp2lut, (size_t)std::max(p2_lut, 1)));
+        k_pair2_lut<<<dim3(16, (unsigned)chunks.size()), 256, 0, c->stream>>>(dchunks, div, dp2lut);
+        PS_CK(launch_status());
+    }
     const size_t gs = std::max<size_t>(nconf, 2 * MAX_DOT_SHELLS);
     double *sumD = nullptr, *sumI = nullptr, *sumA = nullptr, *gD = nullptr;  // gD: n = 2 chunk sums
     PS_TRY(plan_alloc(P, &sumD, nconf));
@@ -1952,7 +1975,7 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
     {
         const size_t pen32 = (size_t)N * (c->f.S / pw<float>(N)), pen64 = (size_t)N * (c->d.S / pw<double>(N));
         const size_t np = std::max({(size_t)N * N, pen32 * MAX_DOT_SHELLS, pen64 * MAX_DOT_SHELLS,
-                                    (size_t)148 * 8 * 2 * MAX_DOT_SHELLS});
+                                    (size_t)148 * 8 * 2 * MAX_DOT_SHELLS, (size_t)p2_blocks * 2 * kP2Shells});
         PS_TRY(ensure_partials(c, np));
         PS_TRY(ensure_lut(c, (size_t)3 * (N / 2) * (N / 2) + 2));
         if (!groups.empty()) {
@@ -2202,25 +2225,34 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
         });
     }
     auto& tail = P->ops_tail;
-    // ---- n = 2 (Parseval): one k-space pass per chunk
-    for (const P2Chunk ch : p2) {
+    // ---- n = 2 (Parseval)
+    if (!chunks.empty()) {
+        const int nch = (int)chunks.size();
+        double modes = 0.0;
+        for (const P2Chunk& ch : chunks)  // half-spectrum modes of the chunk's radius range
+            modes += 2.0 / 3.0 * 3.14159 * (pow((double)std::max(ch.hi, 0), 1.5) - pow((double)ch.lo, 1.5));
         tail.push_back([=]() {
-            const unsigned short* lut = nullptr;
-            if (ch.lut_ok) {
+            {
                 Prof pf(c);
-                if (ch.lut_size > 0)
-                    k_shell_lut<<<(ch.lut_size + 255) / 256, 256, 0, c->stream>>>(dtable + ch.ofs + 2 * ch.cnt, ch.cnt,
-                                                                                   ch.lut_size, c->dlut);
-                pf.end(KF_LUT, 2.0 * ch.lut_size);
-                lut = c->dlut;
+                k_pair2_sweep<float><<<p2_blocks, kP2Threads, 0, c->stream>>>(N, c->f.spec, c->f.S, dchunks, nch, dp2lut,
+                                                                              c->partials);
+                pf.end(KF_PAIR2, modes * sizeof(V2<float>));
             }
+            Prof pf(c);
+            k_pair2_finish<<<nch, 256, 0, c->stream>>>(dchunks, c->partials, didx + iv_ofs, n3, sumD, sumI);
+            pf.end(KF_SUM, 16.0 * p2_blocks * kP2Shells);
+            return PS_OK;
+        });
+    }
+    for (const P2Pass ch : p2) {  // shells that are no r^2 intervals: one k-space pass per 16
+        tail.push_back([=]() {
             const int b = std::min(ch.band, N / 2);
             const long long modes = (long long)(2 * b + 1) * (2 * b + 1) * (b + 1);
             const int blocks = (int)std::max<long long>(1, std::min<long long>((modes + 255) / 256, 148 * 8));
             {
                 Prof pf(c);
-                k_pair2_sums<float><<<blocks, 256, 0, c->stream>>>(N, c->f.spec, c->f.S, lut, ch.lut_size, dtable + ch.ofs,
-                                                                   ch.cnt, b, c->partials);
+                k_pair2_sums<float><<<blocks, 256, 0, c->stream>>>(N, c->f.spec, c->f.S, dtable + ch.ofs, ch.cnt, b,
+                                                                   c->partials);
                 pf.end(KF_PAIR2, (double)modes * sizeof(V2<float>));
             }
             PS_TRY(sum_partials_n(c, blocks, 2 * MAX_DOT_SHELLS, gD));

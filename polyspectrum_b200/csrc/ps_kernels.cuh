@@ -1054,13 +1054,14 @@ __global__ void k_scale_out(const T* __restrict__ in, O* __restrict__ out, size_
 // ------------------------------------------------------------------ n = 2 (Parseval)
 // Per configuration c (legs a, b): S_D = N^3 sum_half w(h) F_a F_b |dk|^2 and
 // the count sum_half w(h) F_a F_b (exact), over the band cube |m| <= band.
-// The per-mode configuration bitmask comes from lut[r2] (interval shells) or
-// from the shell pairs legs[2c], legs[2c+1].  Per-thread FP64 sums, one
-// fixed-order reduction: partials[c] (sums) and partials[MAX + c] (counts).
+// For shells that are no r^2 intervals (those take k_pair2_sweep): the per-mode
+// configuration bitmask comes from the shell pairs legs[2c], legs[2c+1].
+// Per-thread FP64 sums, one fixed-order reduction: partials[c] (sums) and
+// partials[MAX + c] (counts).
 template <typename T>
 __global__ void __launch_bounds__(256)
-    k_pair2_sums(int n, const V2<T>* __restrict__ dk, int dks, const unsigned short* __restrict__ lut, int lut_size,
-                 const Shell* __restrict__ legs, int ncfg, int band, double* __restrict__ partials)
+    k_pair2_sums(int n, const V2<T>* __restrict__ dk, int dks, const Shell* __restrict__ legs, int ncfg, int band,
+                 double* __restrict__ partials)
 {
     double acc[MAX_DOT_SHELLS], cnt[MAX_DOT_SHELLS];
 #pragma unroll
@@ -1077,17 +1078,12 @@ __global__ void __launch_bounds__(256)
         if (mx >= n / 2 || my >= n / 2) continue;  // +N/2 is the index of -N/2, visited as such
         const int mz = h == n / 2 ? -(n / 2) : h;
         unsigned bits = 0u;
-        if (lut) {
-            const int r2 = mx * mx + my * my + mz * mz;
-            bits = r2 < lut_size ? (unsigned)__ldg(lut + r2) : 0u;
-        } else {
-            for (int c = 0; c < ncfg; c++) {
-                const Shell& sa = legs[2 * c];
-                const Shell& sb = legs[2 * c + 1];
-                if (in_band(sa, mx, my, mz) && shell_bit(sa, mx, my, mz) && in_band(sb, mx, my, mz) &&
-                    shell_bit(sb, mx, my, mz))
-                    bits |= 1u << c;
-            }
+        for (int c = 0; c < ncfg; c++) {
+            const Shell& sa = legs[2 * c];
+            const Shell& sb = legs[2 * c + 1];
+            if (in_band(sa, mx, my, mz) && shell_bit(sa, mx, my, mz) && in_band(sb, mx, my, mz) &&
+                shell_bit(sb, mx, my, mz))
+                bits |= 1u << c;
         }
         if (!bits) continue;
         const int i = mx < 0 ? mx + n : mx, j = my < 0 ? my + n : my;

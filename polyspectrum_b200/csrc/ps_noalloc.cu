@@ -22,14 +22,17 @@
 //   * the first call on each device looks up the array's device address
 //     (cudaGetSymbolAddress) with that device current; make that first call
 //     before any stream capture begins.
+#include <algorithm>
 #include <cmath>
+#include <exception>
 #include <mutex>
+#include <vector>
 
 #include "ps_launch.cuh"
+#include "ps_pair2.cuh"
 
 namespace ps {
 PS_EXTERN_L3(float)
-PS_EXTERN_L3(double)
 }  // namespace ps
 
 using namespace ps;
@@ -67,14 +70,14 @@ int noalloc_scratch_ptr(int dev, unsigned char** out)
 
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-// B = coef * sumD / (N^3 * count), Npoly = count = rint(sumI / N^3): the
-// batched method's normalisation of leg-by-leg configurations.
+// B = coef * sumD / (N^3 * count), Npoly = count: the batched method's
+// normalisation.
 __global__ void k_noalloc_finalize(int ns, double coef, double n3, const double* __restrict__ sums,
                                    double* __restrict__ out)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= ns) return;
-    const double cnt = rint(sums[ns + s] / n3);
+    const double cnt = sums[ns + s];
     out[2 * s] = __ddiv_rn(__dmul_rn(coef, sums[s]), __dmul_rn(cnt, n3));
     out[2 * s + 1] = cnt;
 }
@@ -84,10 +87,45 @@ int run_noalloc(cudaStream_t st, unsigned char* base, double L, const float* fie
                 const double* k, double bw, double* P, double* Npoly)
 {
     using V32 = float2;
-    using V64 = double2;
-    constexpr int W32 = PencilGeom<float, N>::W, W64 = PencilGeom<double, N>::W;
+    constexpr int W32 = PencilGeom<float, N>::W;
     constexpr int S32 = (N / 2 + 1 + W32 - 1) / W32 * W32;
-    constexpr int S64 = (N / 2 + 1 + W64 - 1) / W64 * W64;
+    // host values of what the call copies in, one block: the twiddle tables (the
+    // context's expressions, made once per size) and the sorted shells
+    struct Head {
+        V32 tw[N], twp[N], twr[N / 2];
+        P2Chunk chunks[(PS_NOALLOC_MAX_SHELLS + kP2Shells - 1) / kP2Shells];
+        P2Range iv[PS_NOALLOC_MAX_SHELLS];
+        int idx[PS_NOALLOC_MAX_SHELLS];
+    };
+    static thread_local Head h;
+    static thread_local bool tables = false;
+    if (!tables) {
+        const long double two_pi = 6.283185307179586476925286766559005768L;
+        for (int m = 0; m < N; m++) {
+            const long double a = two_pi * (long double)m / (long double)N;
+            h.tw[m] = V32{(float)cosl(a), (float)(-sinl(a))};
+        }
+        L3<float, N>::host_tables(h.twp, h.twr);
+        tables = true;
+    }
+    std::vector<P2Range> iv(ns);
+    std::vector<int> order(ns);
+    std::vector<P2Range> by_cfg(ns);
+    for (int s = 0; s < ns; s++) {
+        const Shell sh = host_shell(SHELL_DEFAULT, k[s], 0.0, 0.0, bw, L, N);
+        by_cfg[s] = P2Range{sh.r2lo, sh.r2hi};
+        order[s] = s;
+    }
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return by_cfg[x].lo < by_cfg[y].lo; });
+    for (int s = 0; s < ns; s++) {
+        h.iv[s] = iv[s] = by_cfg[order[s]];
+        h.idx[s] = order[s];
+    }
+    int lut_size = 0;
+    const std::vector<P2Chunk> chunks = pair2_chunks(iv, N, 148 * 4, &lut_size);
+    std::copy(chunks.begin(), chunks.end(), h.chunks);
+    const int nch = (int)chunks.size(), blocks = chunks.back().block0 + chunks.back().nblocks;
+
     size_t off = 0;
     auto carve = [&](size_t bytes) {
         unsigned char* p = base + off;
@@ -95,65 +133,27 @@ int run_noalloc(cudaStream_t st, unsigned char* base, double L, const float* fie
         return p;
     };
     V32* spec32 = (V32*)carve(sizeof(V32) * (size_t)N * N * S32);
-    V32* work32 = (V32*)carve(sizeof(V32) * (size_t)N * N * S32);
-    V64* work64 = (V64*)carve(sizeof(V64) * (size_t)N * N * S64);
-    V32* tw32 = (V32*)carve(sizeof(V32) * N);
-    V64* tw64 = (V64*)carve(sizeof(V64) * N);
-    V32* twp32 = (V32*)carve(sizeof(V32) * N);
-    V32* twr32 = (V32*)carve(sizeof(V32) * N / 2);
-    V64* twp64 = (V64*)carve(sizeof(V64) * N);
-    V64* twr64 = (V64*)carve(sizeof(V64) * N / 2);
-    const Tables<float> tb32{twp32, twr32, tw32};
-    const Tables<double> tb64{twp64, twr64, tw64};
-    double* partials = (double*)carve(sizeof(double) * (size_t)N * N);
+    Head* d = (Head*)carve(sizeof(Head));
+    unsigned short* lut = (unsigned short*)carve(sizeof(unsigned short) * (size_t)(lut_size + 1));
+    double* partials = (double*)carve(sizeof(double) * (size_t)blocks * 2 * kP2Shells);
     double* sums = (double*)carve(sizeof(double) * 2 * PS_NOALLOC_MAX_SHELLS);
     double* out = (double*)carve(sizeof(double) * 2 * PS_NOALLOC_MAX_SHELLS);
-    Shell* shells = (Shell*)carve(sizeof(Shell) * PS_NOALLOC_MAX_SHELLS);
     if (off > PS_NOALLOC_SCRATCH_BYTES) return report_error(PS_ERR_ARG, "no-alloc scratch too small");
-
-    // twiddles and shells: host values (same expressions as the context's), copied in
-    V32 h32[N];
-    V64 h64[N];
-    const long double two_pi = 6.283185307179586476925286766559005768L;
-    for (int m = 0; m < N; m++) {
-        const long double a = two_pi * (long double)m / (long double)N;
-        h64[m] = V64{(double)cosl(a), (double)(-sinl(a))};
-        h32[m] = V32{(float)cosl(a), (float)(-sinl(a))};
-    }
-    static thread_local Shell hs[PS_NOALLOC_MAX_SHELLS];
-    for (int s = 0; s < ns; s++) hs[s] = host_shell(SHELL_DEFAULT, k[s], 0.0, 0.0, bw, L, N);
-    V32 hp32[N], hr32[N / 2];
-    V64 hp64[N], hr64[N / 2];
-    L3<float, N>::host_tables(hp32, hr32);
-    L3<double, N>::host_tables(hp64, hr64);
-    PS_LCK(cudaMemcpyAsync(tw32, h32, sizeof(h32), cudaMemcpyHostToDevice, st));
-    PS_LCK(cudaMemcpyAsync(tw64, h64, sizeof(h64), cudaMemcpyHostToDevice, st));
-    PS_LCK(cudaMemcpyAsync(twp32, hp32, sizeof(hp32), cudaMemcpyHostToDevice, st));
-    PS_LCK(cudaMemcpyAsync(twr32, hr32, sizeof(hr32), cudaMemcpyHostToDevice, st));
-    PS_LCK(cudaMemcpyAsync(twp64, hp64, sizeof(hp64), cudaMemcpyHostToDevice, st));
-    PS_LCK(cudaMemcpyAsync(twr64, hr64, sizeof(hr64), cudaMemcpyHostToDevice, st));
-    PS_LCK(cudaMemcpyAsync(shells, hs, sizeof(Shell) * ns, cudaMemcpyHostToDevice, st));
+    PS_LCK(cudaMemcpyAsync(d, &h, sizeof(Head), cudaMemcpyHostToDevice, st));
+    const Tables<float> tb32{d->twp, d->twr, d->tw};
 
     // forward transform of the field (get_FT_field + optional phase normalisation)
     PS_LTRY((L3<float, N>::fwd_z(st, SRC_F32, field, nullptr, spec32, S32, N / 2 + 1, tb32)));
     PS_LTRY((L3<float, N>::pass_y(st, spec32, S32, false, tb32)));
     PS_LTRY((L3<float, N>::fwd_x(st, spec32, S32, N / 2 + 1, phase == 1 ? SPEC_STORE_PHASE : SPEC_STORE,
                                  spec32, S32, nullptr, 0, nullptr, 0, nullptr, 0, nullptr, tb32, nullptr)));
-    // per shell: sum_x D^2 (FP32 transform, FP64 sum) and sum_x I^2 (FP64)
-    for (int s = 0; s < ns; s++) {
-        const int hb = (hs[s].band < N / 2 ? hs[s].band : N / 2) + 1;
-        const int Sd = (hb + W32 - 1) / W32 * W32, Si = (hb + W64 - 1) / W64 * W64;
-        int nb = 0;
-        PS_LTRY((L3<float, N>::inv_x(st, spec32, S32, work32, Sd, LOAD_MASKED, shells + s, N / 2 + 1, tb32)));
-        PS_LTRY((L3<float, N>::pass_y(st, work32, Sd, true, tb32)));
-        PS_LTRY((L3<float, N>::inv_z(st, work32, Sd, hb, nullptr, nullptr, EPI_REDUCE, 2, partials, tb32, &nb)));
-        k_sum_partials<<<1, 1024, 0, st>>>(partials, nb, sums + s, 1, nullptr);
-        PS_LTRY((L3<double, N>::inv_x(st, nullptr, S64, work64, Si, LOAD_UNIT, shells + s, N / 2 + 1, tb64)));
-        PS_LTRY((L3<double, N>::pass_y(st, work64, Si, true, tb64)));
-        PS_LTRY((L3<double, N>::inv_z(st, work64, Si, hb, nullptr, nullptr, EPI_REDUCE, 2, partials, tb64, &nb)));
-        k_sum_partials<<<1, 1024, 0, st>>>(partials, nb, sums + ns + s, 1, nullptr);
-    }
+    // all shells in one sweep over the spectrum (Parseval): sums of |dk|^2 in
+    // FP64 and exact counts; per-shell inverse transforms (six passes and two
+    // reductions each) took 1.45 ms for 32 shells at 64^3
+    k_pair2_lut<<<dim3(4, nch), 256, 0, st>>>(d->chunks, d->iv, lut);
+    k_pair2_sweep<float><<<blocks, kP2Threads, 0, st>>>(N, spec32, S32, d->chunks, nch, lut, partials);
     const double n3 = (double)N * (double)N * (double)N;
+    k_pair2_finish<<<nch, 256, 0, st>>>(d->chunks, partials, d->idx, n3, sums, sums + ns);
     k_noalloc_finalize<<<(ns + 127) / 128, 128, 0, st>>>(ns, host_norm_coef(L, N, 2), n3, sums, out);
     PS_LCK(cudaGetLastError());
     static thread_local double hout[2 * PS_NOALLOC_MAX_SHELLS];
@@ -188,9 +188,13 @@ extern "C" int ps_gpu_power_spectrum_noalloc(int nbins, double boxsize, const fl
     unsigned char* base = nullptr;
     PS_LTRY(noalloc_scratch_ptr(dev, &base));
     cudaStream_t st = (cudaStream_t)stream;
-    switch (nbins) {
-    case 16: return run_noalloc<16>(st, base, boxsize, field_dev, use_only_phase, nshell, k, kbinwidth, P, Npoly);
-    case 32: return run_noalloc<32>(st, base, boxsize, field_dev, use_only_phase, nshell, k, kbinwidth, P, Npoly);
-    default: return run_noalloc<64>(st, base, boxsize, field_dev, use_only_phase, nshell, k, kbinwidth, P, Npoly);
+    try {
+        switch (nbins) {
+        case 16: return run_noalloc<16>(st, base, boxsize, field_dev, use_only_phase, nshell, k, kbinwidth, P, Npoly);
+        case 32: return run_noalloc<32>(st, base, boxsize, field_dev, use_only_phase, nshell, k, kbinwidth, P, Npoly);
+        default: return run_noalloc<64>(st, base, boxsize, field_dev, use_only_phase, nshell, k, kbinwidth, P, Npoly);
+        }
+    } catch (const std::exception&) {  // the host's small tables
+        return report_error(PS_ERR_OOM, "host memory");
     }
 }
