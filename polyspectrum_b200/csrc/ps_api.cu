@@ -1908,8 +1908,8 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
         for (int x = 0; x < ch.cnt; x++) idx_all.push_back(pairs2[q0 + x]);
         p2.push_back(ch);
     }
-    int p2_lut = 0, p2_blocks = 0;
-    const std::vector<P2Chunk> chunks = pair2_chunks(iv, N, 148 * 9 * 2, &p2_lut);
+    int p2_blocks = 0;
+    const std::vector<P2Chunk> chunks = pair2_chunks(iv, N, 148 * 12 * 2);
     if (!chunks.empty()) p2_blocks = chunks.back().block0 + chunks.back().nblocks;
     const int iv_ofs = (int)idx_all.size();
     for (int q : iv_cfg) idx_all.push_back(q);
@@ -1940,14 +1940,10 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
     double* dcoef = nullptr;
     PS_TRY(plan_upload(P, &dcoef, coef));
     P2Chunk* dchunks = nullptr;
-    unsigned short* dp2lut = nullptr;
+    P2Range* div = nullptr;
     if (!chunks.empty()) {
-        P2Range* div = nullptr;
         PS_TRY(plan_upload(P, &dchunks, chunks));
         PS_TRY(plan_upload(P, &div, iv));
-        PS_TRY(plan_alloc(P, &dp2lut, (size_t)std::max(p2_lut, 1)));
-        k_pair2_lut<<<dim3(16, (unsigned)chunks.size()), 256, 0, c->stream>>>(dchunks, div, dp2lut);
-        PS_CK(launch_status());
     }
     const size_t gs = std::max<size_t>(nconf, 2 * MAX_DOT_SHELLS);
     double *sumD = nullptr, *sumI = nullptr, *sumA = nullptr, *gD = nullptr;  // gD: n = 2 chunk sums
@@ -1975,7 +1971,7 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
     {
         const size_t pen32 = (size_t)N * (c->f.S / pw<float>(N)), pen64 = (size_t)N * (c->d.S / pw<double>(N));
         const size_t np = std::max({(size_t)N * N, pen32 * MAX_DOT_SHELLS, pen64 * MAX_DOT_SHELLS,
-                                    (size_t)148 * 8 * 2 * MAX_DOT_SHELLS, (size_t)p2_blocks * 2 * kP2Shells});
+                                    (size_t)148 * 8 * 2 * MAX_DOT_SHELLS, (size_t)p2_blocks * kP2Shells + iv.size() * kP2CountParts});
         PS_TRY(ensure_partials(c, np));
         PS_TRY(ensure_lut(c, (size_t)3 * (N / 2) * (N / 2) + 2));
         if (!groups.empty()) {
@@ -2227,20 +2223,26 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
     auto& tail = P->ops_tail;
     // ---- n = 2 (Parseval)
     if (!chunks.empty()) {
-        const int nch = (int)chunks.size();
+        const int nch = (int)chunks.size(), niv = (int)iv.size();
         double modes = 0.0;
         for (const P2Chunk& ch : chunks)  // half-spectrum modes of the chunk's radius range
             modes += 2.0 / 3.0 * 3.14159 * (pow((double)std::max(ch.hi, 0), 1.5) - pow((double)ch.lo, 1.5));
         tail.push_back([=]() {
             {
                 Prof pf(c);
-                k_pair2_sweep<float><<<p2_blocks, kP2Threads, 0, c->stream>>>(N, c->f.spec, c->f.S, dchunks, nch, dp2lut,
+                k_pair2_sweep<float><<<p2_blocks, kP2Threads, 0, c->stream>>>(N, c->f.spec, c->f.S, dchunks, nch, div,
                                                                               c->partials);
                 pf.end(KF_PAIR2, modes * sizeof(V2<float>));
             }
+            double* cparts = c->partials + (size_t)p2_blocks * kP2Shells;
+            {
+                Prof pf(c);
+                k_pair2_counts<<<dim3(niv, kP2CountParts), 256, 0, c->stream>>>(N, div, cparts);
+                pf.end(KF_PAIR_COUNTS, 0.0);
+            }
             Prof pf(c);
-            k_pair2_finish<<<nch, 256, 0, c->stream>>>(dchunks, c->partials, didx + iv_ofs, n3, sumD, sumI);
-            pf.end(KF_SUM, 16.0 * p2_blocks * kP2Shells);
+            k_pair2_finish<<<nch, 256, 0, c->stream>>>(dchunks, c->partials, didx + iv_ofs, n3, sumD, cparts, sumI);
+            pf.end(KF_SUM, 8.0 * p2_blocks * kP2Shells);
             return PS_OK;
         });
     }

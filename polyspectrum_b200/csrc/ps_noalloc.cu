@@ -121,8 +121,7 @@ int run_noalloc(cudaStream_t st, unsigned char* base, double L, const float* fie
         h.iv[s] = iv[s] = by_cfg[order[s]];
         h.idx[s] = order[s];
     }
-    int lut_size = 0;
-    const std::vector<P2Chunk> chunks = pair2_chunks(iv, N, 148 * 4, &lut_size);
+    const std::vector<P2Chunk> chunks = pair2_chunks(iv, N, 148 * 4);
     std::copy(chunks.begin(), chunks.end(), h.chunks);
     const int nch = (int)chunks.size(), blocks = chunks.back().block0 + chunks.back().nblocks;
 
@@ -134,8 +133,8 @@ int run_noalloc(cudaStream_t st, unsigned char* base, double L, const float* fie
     };
     V32* spec32 = (V32*)carve(sizeof(V32) * (size_t)N * N * S32);
     Head* d = (Head*)carve(sizeof(Head));
-    unsigned short* lut = (unsigned short*)carve(sizeof(unsigned short) * (size_t)(lut_size + 1));
-    double* partials = (double*)carve(sizeof(double) * (size_t)blocks * 2 * kP2Shells);
+    double* cparts = (double*)carve(sizeof(double) * (size_t)ns * kP2CountParts);
+    double* partials = (double*)carve(sizeof(double) * (size_t)blocks * kP2Shells);
     double* sums = (double*)carve(sizeof(double) * 2 * PS_NOALLOC_MAX_SHELLS);
     double* out = (double*)carve(sizeof(double) * 2 * PS_NOALLOC_MAX_SHELLS);
     if (off > PS_NOALLOC_SCRATCH_BYTES) return report_error(PS_ERR_ARG, "no-alloc scratch too small");
@@ -150,10 +149,10 @@ int run_noalloc(cudaStream_t st, unsigned char* base, double L, const float* fie
     // all shells in one sweep over the spectrum (Parseval): sums of |dk|^2 in
     // FP64 and exact counts; per-shell inverse transforms (six passes and two
     // reductions each) took 1.45 ms for 32 shells at 64^3
-    k_pair2_lut<<<dim3(4, nch), 256, 0, st>>>(d->chunks, d->iv, lut);
-    k_pair2_sweep<float><<<blocks, kP2Threads, 0, st>>>(N, spec32, S32, d->chunks, nch, lut, partials);
     const double n3 = (double)N * (double)N * (double)N;
-    k_pair2_finish<<<nch, 256, 0, st>>>(d->chunks, partials, d->idx, n3, sums, sums + ns);
+    k_pair2_sweep<float><<<blocks, kP2Threads, 0, st>>>(N, spec32, S32, d->chunks, nch, d->iv, partials);
+    k_pair2_counts<<<dim3(ns, kP2CountParts), 256, 0, st>>>(N, d->iv, cparts);
+    k_pair2_finish<<<nch, 256, 0, st>>>(d->chunks, partials, d->idx, n3, sums, cparts, sums + ns);
     k_noalloc_finalize<<<(ns + 127) / 128, 128, 0, st>>>(ns, host_norm_coef(L, N, 2), n3, sums, out);
     PS_LCK(cudaGetLastError());
     static thread_local double hout[2 * PS_NOALLOC_MAX_SHELLS];
