@@ -253,6 +253,20 @@ struct PendingSubmit {
     ps_cfg* cfgs_out;
 };
 
+// Device memory of a plan's tables with a page-locked host mirror: the host
+// writes the mirror while planning, one copy per piece brings it over.  A
+// context keeps the arenas of destroyed plans, so evaluating a list once
+// (ps_gpu_polyspectrum_batch) allocates nothing after its first call: about 25
+// device and page-locked allocations, copies and frees per call took 2.5 to 9 ms.
+struct PlanArena {
+    unsigned char* dev = nullptr;
+    unsigned char* host = nullptr;
+    size_t cap = 0, used = 0, flushed = 0;
+};
+constexpr size_t kArenaBytes = (size_t)1 << 20;  // smallest arena
+constexpr size_t kSpareArenas = 4;
+constexpr size_t kSpareBytes = (size_t)64 << 20;  // larger arenas are given back at once
+
 struct ps_gpu_ctx {
     int N = 0;
     double L = 0.0;  // (double)(float) box size, grid.h:9
@@ -269,17 +283,15 @@ struct ps_gpu_ctx {
     unsigned short* side_lut = nullptr;
     size_t side_lut_cap = 0;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-    // second field lane: the pair groups of a plan split over two streams (the
-    // main one and this), each with its own FP32 work spectra, partial sums and
-    // shell table, so the kernels of different groups overlap
+    // field lanes: the batches of pair groups of a plan split over two streams
+    // (0 the main one, 1 lane2_stream), each with its own workspace (leg and
+    // product spectra, block sums), so the kernels of different batches overlap
     cudaStream_t lane2_stream = nullptr;
-    double* lane2_partials = nullptr;
-    size_t lane2_partials_cap = 0;
-    unsigned short* lane2_lut = nullptr;
-    size_t lane2_lut_cap = 0;
-    V2<float>* lane2_work[3] = {nullptr, nullptr, nullptr};
-    size_t lane2_work_cap = 0;  // elements of each
+    unsigned char* lane_work[2] = {nullptr, nullptr};
+    size_t lane_work_cap[2] = {0, 0};  // bytes
     cudaEvent_t ev_join2 = nullptr;
+    // memory of destroyed plans kept for the next ones (at most kSpareArenas)
+    std::vector<PlanArena> spare_arenas;
     PrecBufs<float> f;
     PrecBufs<double> d;
     double* partials = nullptr;
@@ -597,40 +609,29 @@ struct SideLane {
     }
 };
 
-// While alive, the context's stream, partial sums, shell table and FP32 work
-// spectra are those of the second field lane (not while profiling: then
-// everything runs on the main lane, one launch at a time).
+// While alive, the context's stream is that of the second field lane (not while
+// profiling: then everything runs on the main lane, one launch at a time).
 struct Lane2 {
     ps_gpu_ctx* c;
     bool on;
-    explicit Lane2(ps_gpu_ctx* cc, bool always = false) : c(cc), on(always || !cc->prof_on) { swap(); }
+    explicit Lane2(ps_gpu_ctx* cc, bool second = true) : c(cc), on(second && !cc->prof_on) { swap(); }
     ~Lane2() { swap(); }
     void swap()
     {
-        if (!on) return;
-        std::swap(c->stream, c->lane2_stream);
-        std::swap(c->partials, c->lane2_partials);
-        std::swap(c->partials_cap, c->lane2_partials_cap);
-        std::swap(c->dlut, c->lane2_lut);
-        std::swap(c->dlut_cap, c->lane2_lut_cap);
-        std::swap(c->f.work, c->lane2_work[0]);
-        std::swap(c->f.work2, c->lane2_work[1]);
-        std::swap(c->f.work3, c->lane2_work[2]);
+        if (on) std::swap(c->stream, c->lane2_stream);
     }
 };
 
-// FP32 work spectra of the second lane, n elements each (replaced ones are
-// retired: a captured graph may still point at them).
-int ensure_lane2_work(ps_gpu_ctx* c, size_t n)
+// Workspace of a field lane, at least `bytes` (a replaced one is retired: a
+// captured graph or a plan's tables may still point at it).
+int ensure_lane_work(ps_gpu_ctx* c, int lane, size_t bytes)
 {
-    if (n <= c->lane2_work_cap) return PS_OK;
-    for (auto& p : c->lane2_work) {
-        if (p) c->retired.push_back(p);
-        p = nullptr;
-    }
-    c->lane2_work_cap = 0;
-    for (auto& p : c->lane2_work) PS_TRY(alloc_dev(&p, n));
-    c->lane2_work_cap = n;
+    if (bytes <= c->lane_work_cap[lane]) return PS_OK;
+    if (c->lane_work[lane]) c->retired.push_back(c->lane_work[lane]);
+    c->lane_work[lane] = nullptr;
+    c->lane_work_cap[lane] = 0;
+    PS_TRY(alloc_dev(&c->lane_work[lane], bytes));
+    c->lane_work_cap[lane] = bytes;
     return PS_OK;
 }
 
@@ -923,9 +924,13 @@ template <typename T> int forward_field(ps_gpu_ctx* c, int kind, const void* a, 
     {
         Prof pf(c);
         const double rows = band < N / 2 ? (double)N * (2 * band + 1) : NN2;
-        PS_SWITCH_N(N, PS_TRY((L3<T, NN>::fwd_x(c->stream, B.spec, B.S, hcols, epi, B.spec, B.S, nullptr, 0,
-                                                nullptr, 0, nullptr, 0, nullptr, B.tables(), nullptr, 1.0, 0, 0,
-                                                0x7fffffff, mod, ncols, band < N / 2 ? band : NN))));
+        FwdXItem<T> it{};
+        it.data = B.spec;
+        it.stride = B.S;
+        it.hvalid = hcols;
+        it.ncols = ncols;
+        PS_SWITCH_N(N, PS_TRY((L3<T, NN>::fwd_x(c->stream, &it, 1, ncols, epi, B.spec, B.S, nullptr, 0,
+                                                B.tables(), nullptr, 0, 0, mod, band < N / 2 ? band : NN))));
         pf.end(fam<T>(KF_FWD_X_STORE), rows * H * V + (band < N / 2 ? (double)(2 * band + 1) : (double)N) *
                                                          (2 * band + 1 < N ? 2 * band + 1 : N) * H * V, N);
     }
@@ -968,17 +973,31 @@ int dot_pass(ps_gpu_ctx* c, V2<T>* data, int epi, int S, int hvalid, const Shell
             PS_TRY(ensure_lut(c, (size_t)std::max(lut_size, 1)));
             Prof pf(c);
             if (lut_size > 0)
-                k_shell_lut<<<(lut_size + 255) / 256, 256, 0, c->stream>>>(dshells + s0, cnt, lut_size, c->dlut);
+                {
+                    Items<LutItem> one{};
+                    one.at[0] = LutItem{dshells + s0, c->dlut, cnt, lut_size};
+                    k_shell_lut<<<(lut_size + 255) / 256, 256, 0, c->stream>>>(one);
+                }
             pf.end(KF_LUT, 2.0 * lut_size);
             lut = c->dlut;
         }
         int nb = 0;
         {
             Prof pf(c);
-            PS_SWITCH_N(N, PS_TRY((L3<T, NN>::fwd_x(c->stream, data, S, hvalid, epi, nullptr, 0, B.spec, B.S,
-                                                    dshells + s0, cnt, lut, lut_size, c->partials, tb, &nb,
-                                                    weight, quad, c->N, (int)std::min<long long>(r2max, 0x7fffffff),
-                                                    nullptr, 0, NN, dot_alt_of<T>(c, N)))));
+            FwdXItem<T> it{};
+            it.data = data;
+            it.stride = S;
+            it.hvalid = hvalid;
+            it.ncols = S;
+            it.nshell = cnt;
+            it.shells = dshells + s0;
+            it.lut = lut;
+            it.lut_size = lut_size;
+            it.r2max = (int)std::min<long long>(r2max, 0x7fffffff);
+            it.weight = weight;
+            it.partials = c->partials;
+            PS_SWITCH_N(N, PS_TRY((L3<T, NN>::fwd_x(c->stream, &it, 1, S, epi, nullptr, 0, B.spec, B.S, tb, &nb,
+                                                    quad, c->N, nullptr, NN, dot_alt_of<T>(c, N)))));
             const double q = quad ? (double)(N / 2 + 1) * (N / 2 + 1) / ((double)N * N) : 1.0;
             pf.end(fam<T>(KF_FWD_X_DOT), q * N * N * hvalid * sizeof(V2<T>) * (epi == SPEC_DOT ? 2.0 : 1.0), N);
         }
@@ -1420,14 +1439,14 @@ struct ps_gpu_plan {
     std::vector<std::function<int()>> ops_counts;  // exact polygon counts per pair group (no field)
     std::vector<std::function<int()>> ops_groups;  // the pair groups' field parts (main or second lane)
     std::vector<std::function<int()>> ops_tail;    // n = 2 and leg-by-leg configurations, finalisation
-    bool has_groups = false;
-    std::vector<void*> owned;               // device buffers of this plan
+    bool has_groups = false, two_lanes = false;
+    std::vector<PlanArena> arenas;          // this plan's device tables and their host mirrors
     double* dres = nullptr;                 // B, Npoly per configuration
     double* dsumA = nullptr;                // sum |terms| (condition numbers)
     double* dsumD = nullptr;
     double* dwb = nullptr;                  // derived k ranges, 6 per configuration
     int* derr = nullptr;
-    double* hres = nullptr;  // pinned host copy of dres | dwb | dsumA | dsumD | err
+    double* hres = nullptr;  // page-locked host copy of dres | dwb | dsumA | dsumD | err
     std::vector<int> derived_cfgs;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -1447,18 +1466,69 @@ struct ps_gpu_plan {
 
 namespace {
 
-template <typename T> int plan_alloc(ps_gpu_plan* P, T** p, size_t count)
+// `bytes` of the plan's arenas: device address in *dev, host mirror in *host.
+int arena_take(ps_gpu_plan* P, size_t bytes, void** dev, void** host)
 {
-    *p = nullptr;
-    PS_TRY(alloc_dev(p, count));
-    P->owned.push_back(*p);
+    ps_gpu_ctx* c = P->ctx;
+    bytes = (bytes + 255) / 256 * 256;
+    if (P->arenas.empty() || P->arenas.back().cap - P->arenas.back().used < bytes) {
+        PlanArena a;
+        size_t best = c->spare_arenas.size();
+        for (size_t q = 0; q < c->spare_arenas.size(); q++)
+            if (c->spare_arenas[q].cap >= bytes && (best == c->spare_arenas.size() || c->spare_arenas[q].cap > c->spare_arenas[best].cap))
+                best = q;
+        if (best < c->spare_arenas.size()) {
+            a = c->spare_arenas[best];
+            c->spare_arenas.erase(c->spare_arenas.begin() + (long)best);
+        } else {
+            // the next piece of a growing plan doubles, so a few pieces hold any plan
+            const size_t prev = P->arenas.empty() ? 0 : P->arenas.back().cap;
+            const size_t cap = std::max({bytes, kArenaBytes, std::min(2 * prev, kSpareBytes)});
+            PS_TRY(alloc_dev(&a.dev, cap));
+            if (fault_hit(FAULT_ALLOC) || cudaHostAlloc((void**)&a.host, cap, cudaHostAllocDefault) != cudaSuccess) {
+                cudaFree(a.dev);
+                return fail(PS_ERR_OOM, "page-locked plan tables of %zu bytes", cap);
+            }
+            a.cap = cap;
+        }
+        a.used = a.flushed = 0;
+        P->arenas.push_back(a);
+    }
+    PlanArena& a = P->arenas.back();
+    *dev = a.dev + a.used;
+    *host = a.host + a.used;
+    a.used += bytes;
     return PS_OK;
 }
 
-template <typename T> int plan_upload(ps_gpu_plan* P, T** p, const std::vector<T>& h)
+// Queues the copies of what was written to the mirrors since the last flush;
+// before the first launch that reads the plan's tables.
+int plan_flush(ps_gpu_plan* P)
 {
-    PS_TRY(plan_alloc(P, p, std::max<size_t>(h.size(), 1)));
-    if (!h.empty()) PS_CK(cudaMemcpy(*p, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice));
+    for (PlanArena& a : P->arenas) {
+        if (a.used == a.flushed) continue;
+        PS_CK(cudaMemcpyAsync(a.dev + a.flushed, a.host + a.flushed, a.used - a.flushed, cudaMemcpyHostToDevice,
+                              P->ctx->stream));
+        a.flushed = a.used;
+    }
+    return PS_OK;
+}
+
+template <typename T> int plan_alloc(ps_gpu_plan* P, T** p, size_t count)  // zero-filled
+{
+    void *d = nullptr, *h = nullptr;
+    PS_TRY(arena_take(P, sizeof(T) * std::max<size_t>(count, 1), &d, &h));
+    memset(h, 0, sizeof(T) * std::max<size_t>(count, 1));
+    *p = (T*)d;
+    return PS_OK;
+}
+
+template <typename T> int plan_upload(ps_gpu_plan* P, T** p, const std::vector<T>& v)
+{
+    void *d = nullptr, *h = nullptr;
+    PS_TRY(arena_take(P, sizeof(T) * std::max<size_t>(v.size(), 1), &d, &h));
+    if (!v.empty()) memcpy(h, v.data(), sizeof(T) * v.size());
+    *p = (T*)d;
     return PS_OK;
 }
 
@@ -1503,7 +1573,9 @@ bool grid_supported(int M)
 // timed over three runs with CUDA events on the context's stream; the fastest
 // wins.  Every candidate gives the same counts and the same sums up to FP32
 // rounding of the transforms.
-int tune_grid(ps_gpu_ctx* c, const std::function<std::function<int()>(int)>& group_op, int M0, int* best)
+// flush: queues the copies of the tables that group_op made.
+int tune_grid(ps_gpu_ctx* c, const std::function<std::function<int()>(int)>& group_op, int M0, int* best,
+              const std::function<int()>& flush)
 {
     std::vector<int> cands;
     for (int q : kGridSizes)
@@ -1524,6 +1596,7 @@ int tune_grid(ps_gpu_ctx* c, const std::function<std::function<int()>(int)>& gro
             if ((rc = tables_for<float>(c, M, &t32)) != PS_OK || (rc = tables_for<double>(c, M, &t64)) != PS_OK) break;
         }
         const auto op = group_op(M);
+        if ((rc = flush()) != PS_OK) break;
         if ((rc = op()) != PS_OK) break;
         cudaEventRecord(e0, c->stream);
         for (int r = 0; r < 3 && rc == PS_OK; r++) rc = op();
@@ -1812,32 +1885,45 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
     const int nu = (int)uniq.size();
     auto host_shell_of = [&](int u) -> const Shell& { return uniq[u].sh; };
 
-    // ---- plan: pair groups (n = 3 sharing a leg pair), n = 2 (Parseval), the rest leg by leg
+    // ---- plan: pair groups (n = 3: configurations sharing a leg pair, alone if
+    // none does), n = 2 (Parseval), n > 3 leg by leg
     std::vector<Group> groups;
     std::vector<int> direct, pairs2;
     {
+        // freq: configurations holding a pair (each pair of one counted once)
         std::map<std::pair<int, int>, int> freq;
+        const auto pair_of = [&](int q, int z) {  // the two legs other than z
+            const auto& v = lid[q];
+            const int x = v[(z + 1) % 3], y = v[(z + 2) % 3];
+            return std::pair<int, int>{std::min(x, y), std::max(x, y)};
+        };
         for (int q = 0; q < nconf; q++)
             if (cfgs[q].n == 3) {
-                const auto& v = lid[q];
-                for (int x = 0; x < 3; x++)
-                    for (int y = x + 1; y < 3; y++) freq[{std::min(v[x], v[y]), std::max(v[x], v[y])}]++;
+                const std::set<std::pair<int, int>> own = {pair_of(q, 0), pair_of(q, 1), pair_of(q, 2)};
+                for (const auto& pr : own) freq[pr]++;
             }
         std::map<std::pair<int, int>, int> gidx;
         for (int q = 0; q < nconf; q++) {
             const int n = cfgs[q].n;
             if (n == 2) { pairs2.push_back(q); continue; }
             if (n != 3) { direct.push_back(q); continue; }
-            const auto& v = lid[q];
-            int best = -1, bx = 0, by = 1;
-            for (int x = 0; x < 3; x++)
-                for (int y = x + 1; y < 3; y++) {
-                    const int f = freq[{std::min(v[x], v[y]), std::max(v[x], v[y])}];
-                    if (f > best) { best = f; bx = x; by = y; }
+            // the pair most configurations share; among equals one of equal legs
+            // (one inverse transform less), then host-known legs (their counts can be
+            // enumerated), then the widest closing shell (it is transformed once, a
+            // leg three times)
+            int bz = 2;
+            std::array<int, 4> best = {-1, 0, 0, 0};
+            for (int z = 2; z >= 0; z--) {
+                const auto pr = pair_of(q, z);
+                const std::array<int, 4> score = {freq[pr], pr.first == pr.second ? 1 : 0,
+                                                  uniq[pr.first].tag == 0 && uniq[pr.second].tag == 0 ? 1 : 0,
+                                                  host_shell_of(lid[q][z]).band};
+                if (score > best) {
+                    best = score;
+                    bz = z;
                 }
-            if (best < 2) { direct.push_back(q); continue; }
-            const int z = 3 - bx - by;
-            std::pair<int, int> key{std::min(v[bx], v[by]), std::max(v[bx], v[by])};
+            }
+            const auto key = pair_of(q, bz);
             auto it = gidx.find(key);
             if (it == gidx.end()) {
                 gidx[key] = (int)groups.size();
@@ -1845,7 +1931,7 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
                 it = gidx.find(key);
             }
             groups[it->second].cfg.push_back(q);
-            groups[it->second].third.push_back(v[z]);
+            groups[it->second].third.push_back(lid[q][bz]);
         }
     }
 
@@ -1953,32 +2039,21 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
     PS_TRY(plan_alloc(P, &gD, gs));
     PS_TRY(plan_alloc(P, &P->dres, 2 * (size_t)nconf));
     PS_TRY(plan_alloc(P, &P->dwb, 6 * (size_t)nconf));
-    PS_CK(cudaMemset(P->dwb, 0, 48 * (size_t)nconf));  // entries of non-DERIVED configurations stay 0
     PS_TRY(plan_alloc(P, &P->derr, 1));
-    PS_CK(cudaMemset(P->derr, 0, sizeof(int)));
-    if (fault_hit(FAULT_ALLOC) ||
-        cudaHostAlloc((void**)&P->hres, (10 * (size_t)nconf + 1) * sizeof(double), cudaHostAllocDefault) !=
-        cudaSuccess) {
-        P->hres = nullptr;
-        return fail(PS_ERR_OOM, "pinned result buffer of %d configurations", nconf);
+    {
+        void *dev = nullptr, *host = nullptr;  // the results' host copy: a piece of the mirror
+        PS_TRY(arena_take(P, (10 * (size_t)nconf + 1) * sizeof(double), &dev, &host));
+        P->hres = (double*)host;
     }
     P->dsumA = sumA;
     P->dsumD = sumD;
-    if (!groups.empty()) {
-        PS_TRY(ensure_pair_bufs(c, c->f));
-        PS_TRY(ensure_pair_bufs(c, c->d));
-    }
     {
         const size_t pen32 = (size_t)N * (c->f.S / pw<float>(N)), pen64 = (size_t)N * (c->d.S / pw<double>(N));
         const size_t np = std::max({(size_t)N * N, pen32 * MAX_DOT_SHELLS, pen64 * MAX_DOT_SHELLS,
-                                    (size_t)148 * 8 * 2 * MAX_DOT_SHELLS, (size_t)p2_blocks * kP2Shells + iv.size() * kP2CountParts});
+                                    (size_t)148 * 8 * 2 * MAX_DOT_SHELLS,
+                                    (size_t)p2_blocks * kP2Shells + iv.size() * kP2CountParts});
         PS_TRY(ensure_partials(c, np));
         PS_TRY(ensure_lut(c, (size_t)3 * (N / 2) * (N / 2) + 2));
-        if (!groups.empty()) {
-            SideLane lane(c, true);  // the side lane's own scratch, profiling or not
-            PS_TRY(ensure_partials(c, np));
-            PS_TRY(ensure_lut(c, (size_t)3 * (N / 2) * (N / 2) + 2));
-        }
     }
     const double n3 = (double)N * (double)N * (double)N;
     const double pi = ref_pi();
@@ -2019,206 +2094,495 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
             return PS_OK;
         });
     }
-    // ---- pair groups, split over the main and the second field lane
-    bool prefix_done = false;
-    std::vector<std::function<int()>> group_dop(groups.size()), group_iop(groups.size());
-    std::vector<int> group_M(groups.size(), 0);
-    std::vector<size_t> group_need(groups.size(), 0);
+    // ---- pair groups: legs, sub-grid, closing shells' r^2 tables
+    P->has_groups = !groups.empty();
+    struct GroupInfo {
+        Shell sa, sb;
+        int hmax = 0, M = 0;
+        bool two = false;                // distinct legs
+        std::vector<Shell> gtable;       // host copies of the closing shells
+        std::vector<unsigned short*> lut;  // per 16 closing shells: r^2 -> bitmask (NULL: compared directly)
+        bool enum_counts = false;
+        PairCountLists lists;
+    };
+    std::vector<GroupInfo> info(groups.size());
+    std::vector<LutItem> luts;
+    int lut_max = 0;
     for (size_t g = 0; g < groups.size(); g++) {
-        const Group G = groups[g];
-        const Shell sa = host_shell_of(G.a), sb = host_shell_of(G.b);
-        int hmax = 0;
-        for (int s : G.third) hmax = std::max(hmax, std::min(host_shell_of(s).band, N / 2));
-        const int hout = hmax + 1;
+        const Group& G = groups[g];
+        GroupInfo& I = info[g];
+        I.sa = host_shell_of(G.a);
+        I.sb = host_shell_of(G.b);
+        I.two = G.a != G.b;
+        for (int s : G.third) I.hmax = std::max(I.hmax, std::min(host_shell_of(s).band, N / 2));
         const int ng = (int)G.cfg.size();
-        const int go = gofs[g], io = gidx_ofs[g];
-        const Shell* hsh = table.data();  // host copy kept alive by the closure below
-        std::vector<Shell> gtable(table.begin() + go, table.begin() + go + ng);
-        // the group's transforms run on an M-grid on which no triple of its
-        // modes aliases (scale of the product spectrum: (N/M)^3): the smallest
-        // one, or the fastest candidate when autotuned
-        const int ba = std::min(sa.band, N / 2), bb = std::min(sb.band, N / 2);
-        // D part (FP32 field products) and I part (FP64 counts on the xy-quadrant:
-        // unit filters are even in every axis) of the group on an M-grid
-        auto d_part = [=](int M) -> std::function<int()> {
-            const double wD = ((double)N / M) * ((double)N / M) * ((double)N / M);
-            return [=]() {
-                int Sa = 0, ha = 0, Sb = 0, hbb = 0, S = 0;
-                PS_TRY(c2r_xy<float>(c, LOAD_MASKED, dtable + G.a, sa.band, c->f.work, &Sa, &ha, 0, M));
-                if (G.a != G.b)
-                    PS_TRY(c2r_xy<float>(c, LOAD_MASKED, dtable + G.b, sb.band, c->f.work2, &Sb, &hbb, 0, M));
-                PS_TRY(pair_spectrum<float>(c, c->f.work, Sa, ha, G.a != G.b ? c->f.work2 : nullptr, Sb, hbb, hout,
-                                            &S, 0, M));
-                PS_TRY(dot_pass<float>(c, c->f.work3, SPEC_DOT, S, hout, dtable + go, gtable.data(), ng, sumD, 0, M,
-                                       wD, didx + io));
-                if (kappa)
-                    PS_TRY(dot_pass<float>(c, c->f.work3, SPEC_DOT_ABS, S, hout, dtable + go, gtable.data(), ng, sumA,
-                                           0, M, wD, didx + io));
+        I.gtable.assign(table.begin() + gofs[g], table.begin() + gofs[g] + ng);
+        for (int s0 = 0; s0 < ng; s0 += MAX_DOT_SHELLS) {
+            const int cnt = std::min(MAX_DOT_SHELLS, ng - s0);
+            bool interval = true;
+            int size = 0;
+            for (int q = s0; q < s0 + cnt; q++) {
+                if (I.gtable[q].kind > SHELL_RANGE) interval = false;
+                size = std::max(size, I.gtable[q].r2hi + 1);
+            }
+            unsigned short* lut = nullptr;
+            // one or two intervals are compared in the dot pass itself; a table
+            // pays from three shells on (sixteen compares per mode against one load)
+            if (interval && cnt > 2 && size > 0) {
+                PS_TRY(plan_alloc(P, &lut, (size_t)size));
+                luts.push_back(LutItem{dtable + gofs[g] + s0, lut, cnt, size});
+                lut_max = std::max(lut_max, size);
+            }
+            I.lut.push_back(lut);
+        }
+    }
+    for (size_t q0 = 0; q0 < luts.size(); q0 += kItems) {  // after the DERIVED chain, which fills closing shells
+        const int nl = (int)std::min<size_t>(kItems, luts.size() - q0);
+        Items<LutItem> items{};
+        double bytes = 0.0;
+        for (int q = 0; q < nl; q++) {
+            items.at[q] = luts[q0 + q];
+            bytes += 2.0 * luts[q0 + q].size;
+        }
+        ops.push_back([=]() {
+            Prof pf(c);
+            k_shell_lut<<<dim3((lut_max + 255) / 256, nl), 256, 0, c->stream>>>(items);
+            pf.end(KF_LUT, bytes);
+            return PS_OK;
+        });
+    }
+
+    // ---- field part of a batch of groups on the M-grid, on lane `lane`: masked
+    // inverse X and Y of every leg, the products' row passes, forward Y, and the
+    // dot passes, one launch each
+    const auto sum_bytes = [&](size_t g, int M) {  // block sums of a group (twice with the condition numbers')
+        const int Sp = round_up(info[g].hmax + 1, pw<float>(M));
+        return sizeof(double) * (size_t)M * (size_t)(Sp / pw<float>(M)) * info[g].gtable.size() * (kappa ? 2 : 1);
+    };
+    const auto group_bytes = [&](size_t g, int M) {  // spectra of a group
+        const GroupInfo& I = info[g];
+        const int w = pw<float>(M);
+        const size_t rows = (size_t)M * M;
+        const int Sa = round_up(std::min(I.sa.band, M / 2) + 1, w), Sb = round_up(std::min(I.sb.band, M / 2) + 1, w);
+        const int Sp = round_up(I.hmax + 1, w);
+        return rows * (size_t)(Sa + (I.two ? Sb : 0) + Sp) * sizeof(V2<float>) + 1024;
+    };
+    // The lane's workspace holds the block sums of all its batches first (from
+    // sums_at on those of this one), then the spectra of the batch at work.
+    std::vector<FwdXItem<float>> sums, sums_abs;  // every dot pass of the plan, for the final sums
+    auto batch_op = [&](const std::vector<size_t>& gs, int M, int lane, size_t sums_at, size_t spectra_at,
+                        std::function<int()>* op) -> int {
+        const int w = pw<float>(M);
+        const size_t rows = (size_t)M * M;
+        unsigned char* at = c->lane_work[lane] + spectra_at;
+        double* part = (double*)(c->lane_work[lane] + sums_at);
+        auto carve = [&](size_t n) {
+            unsigned char* p = at;
+            at += (n + 255) / 256 * 256;
+            return p;
+        };
+        std::vector<XItem<float>> xi;
+        std::vector<YItem<float>> yi, yf;
+        std::vector<PairItem<float>> pi_;
+        std::vector<FwdXItem<float>> fx, fa;
+        int Smax = 0, Pmax = 0, ha_max = 0, hb_max = 0, ninputs = 1;
+        double bx = 0.0, by = 0.0, bp = 0.0, byf = 0.0, bd = 0.0;  // algorithmic bytes
+        const double V = sizeof(V2<float>), NN2 = (double)rows;
+        const double wD = ((double)N / M) * ((double)N / M) * ((double)N / M);
+        for (size_t g : gs) {
+            const Group& G = groups[g];
+            const GroupInfo& I = info[g];
+            auto leg = [&](int shell, const Shell& sh, int* S, int* h) {
+                const int band = std::min(sh.band, M / 2);
+                *h = band + 1;
+                *S = round_up(*h, w);
+                V2<float>* dst = (V2<float>*)carve(rows * (size_t)*S * sizeof(V2<float>));
+                xi.push_back(XItem<float>{dst, *S, M / 2 + 1, dtable + shell});
+                yi.push_back(YItem<float>{dst, *S, *S, band, M});
+                Smax = std::max(Smax, *S);
+                bx += NN2 * (*S + *h) * V;
+                by += 2.0 * NN2 * *S * V;
+                return dst;
+            };
+            int Sa = 0, ha = 0, Sb = 0, hb = 0;
+            const V2<float>* A = leg(G.a, I.sa, &Sa, &ha);
+            const V2<float>* B = I.two ? leg(G.b, I.sb, &Sb, &hb) : nullptr;
+            const int hout = I.hmax + 1, Sp = round_up(hout, w);
+            V2<float>* D = (V2<float>*)carve(rows * (size_t)Sp * sizeof(V2<float>));
+            pi_.push_back(PairItem<float>{A, B, D, Sa, ha, Sb, hb, Sp, hout});
+            yf.push_back(YItem<float>{D, Sp, Sp, M, hout - 1});
+            ha_max = std::max(ha_max, ha);
+            hb_max = std::max(hb_max, hb);
+            if (B) ninputs = 2;
+            Pmax = std::max(Pmax, Sp);
+            bp += NN2 * (ha + hb + hout) * V;
+            byf += 2.0 * NN2 * Sp * V;
+            const int ng = (int)I.gtable.size();
+            for (int s0 = 0, ch = 0; s0 < ng; s0 += MAX_DOT_SHELLS, ch++) {
+                FwdXItem<float> it{};
+                it.data = D;
+                it.stride = it.ncols = Sp;
+                it.hvalid = hout;
+                it.nshell = std::min(MAX_DOT_SHELLS, ng - s0);
+                it.shells = dtable + gofs[g] + s0;
+                it.lut = I.lut[ch];
+                bool interval = true;
+                long long r2max = 0;  // no mode of these shells lies outside |m|^2 <= r2max
+                for (int q = s0; q < s0 + it.nshell; q++) {
+                    const Shell& h = I.gtable[q];
+                    const bool iv_shell = h.kind <= SHELL_RANGE;
+                    interval = interval && iv_shell;
+                    it.lut_size = std::max(it.lut_size, h.r2hi + 1);
+                    const long long b = std::min(h.band, N / 2);
+                    r2max = std::max(r2max, iv_shell ? (long long)h.r2hi : 3 * b * b);
+                }
+                it.interval = interval && it.nshell <= 2;
+                it.r2max = (int)std::min<long long>(r2max, 0x7fffffff);
+                it.weight = wD;
+                it.nblk = M * (Sp / w);
+                it.idx = didx + gidx_ofs[g] + s0;
+                it.partials = part;
+                it.out = sumD;
+                part += (size_t)it.nblk * it.nshell;
+                fx.push_back(it);
+                if (kappa) {
+                    it.partials = part;
+                    it.out = sumA;
+                    part += (size_t)it.nblk * it.nshell;
+                    fa.push_back(it);
+                }
+                bd += NN2 * hout * V * 2.0;
+            }
+        }
+        Tables<float> tb;
+        PS_TRY(tables_for<float>(c, M, &tb));
+        sums.insert(sums.end(), fx.begin(), fx.end());
+        sums_abs.insert(sums_abs.end(), fa.begin(), fa.end());
+        const int nx = (int)xi.size(), ngr = (int)gs.size(), nf = (int)fx.size();
+        *op = [=]() -> int {
+            const int N = M;  // PS_SWITCH_N's subject
+            // f(first, n): one launch per kItems items, its bytes in proportion
+            const auto launches = [&](int family, double bytes, int total, const std::function<int(int, int)>& f) -> int {
+                for (int q = 0; q < total; q += kItems) {
+                    const int n = std::min(kItems, total - q);
+                    Prof pf(c);
+                    PS_TRY(f(q, n));
+                    pf.end(family, bytes * n / total, M);
+                }
                 return PS_OK;
             };
-        };
-        // exact counts by enumeration when every shell of the group is an r^2
-        // interval known on the host (closing shells may come from the DERIVED
-        // chain: their intervals are read on the device); else FP64 transforms
-        bool enum_counts = !(P->flags & PS_PLAN_FFT_COUNTS) && uniq[G.a].tag == 0 && uniq[G.b].tag == 0 &&
-                           (sa.kind == SHELL_DEFAULT || sa.kind == SHELL_RANGE) &&
-                           (sb.kind == SHELL_DEFAULT || sb.kind == SHELL_RANGE);
-        for (int s3 : G.third) {
-            const Shell& h3 = host_shell_of(s3);
-            enum_counts = enum_counts && (h3.kind == SHELL_DEFAULT || h3.kind == SHELL_RANGE);
-        }
-        PairCountLists lists;
-        if (enum_counts) enum_counts = pair_count_lists(sa, sb, N, &lists);
-        int4* dreps = nullptr;
-        short4* dmodes = nullptr;
-        unsigned long long* dcounts = nullptr;
-        if (enum_counts) {
-            PS_TRY(plan_upload(P, &dreps, lists.reps));
-            PS_TRY(plan_upload(P, &dmodes, lists.modes));
-            PS_TRY(plan_alloc(P, &dcounts, (size_t)ng));
-        }
-        const int nrep = (int)lists.reps.size(), nmodes = (int)lists.modes.size();
-        const int s_lo = lists.s_lo, nbins = lists.nbins;
-        const bool wrap = lists.wrap;
-        int sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-        // one CTA of kCountThreads per SM over about eight work items each: the
-        // count lane runs beside the field load and the field lanes, and one
-        // histogram per SM leaves the rest of each SM's shared memory to their
-        // passes
-        const size_t csmem = kCountStageBytes + (size_t)nbins * sizeof(unsigned int);
-        int cgrid = 1, rep_slice = kCountRepChunk;
-        if (enum_counts) {
-            // the shared-memory limit is a property of the kernel, not of a
-            // launch (every group's launch, replayed from a graph too, must fit
-            // under it): the largest histogram any group may have
-            constexpr int kLimit = (int)(kCountStageBytes + kCountMaxBins * sizeof(unsigned int));
-            PS_CK(cudaFuncSetAttribute(k_pair_counts<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLimit));
-            PS_CK(cudaFuncSetAttribute(k_pair_counts<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLimit));
-            const int nmc = (nmodes + kCountThreads * kCountBPT - 1) / (kCountThreads * kCountBPT);
-            const int nrs = std::min(nrep, std::max(1, (8 * sms + nmc - 1) / nmc));
-            rep_slice = std::min(kCountRepChunk, std::max(8, (nrep + nrs - 1) / nrs));
-            const int nitems = nmc * ((nrep + rep_slice - 1) / rep_slice);
-            cgrid = std::max(1, std::min(nitems, sms));
-        }
-        auto enum_part = [=]() -> int {
-            PS_CK(cudaMemsetAsync(dcounts, 0, sizeof(unsigned long long) * ng, c->stream));
-            Prof pf(c);
-            if (wrap)
-                k_pair_counts<true><<<cgrid, kCountThreads, csmem, c->stream>>>(
-                    dreps, nrep, dmodes, nmodes, N, s_lo, nbins, rep_slice, dtable + go, ng, dcounts);
-            else
-                k_pair_counts<false><<<cgrid, kCountThreads, csmem, c->stream>>>(
-                    dreps, nrep, dmodes, nmodes, N, s_lo, nbins, rep_slice, dtable + go, ng, dcounts);
-            pf.end(KF_PAIR_COUNTS, 8.0 * nmodes + 16.0 * nrep);
-            k_counts_out<<<(ng + 127) / 128, 128, 0, c->stream>>>(ng, dcounts, didx + io, sumI);
+            const int ya = pencil_alt_of<float>(c, M);
+            PS_TRY(launches(KF_INV_X, bx, nx, [&](int q, int n) -> int {
+                PS_SWITCH_N(N, PS_TRY((L3<float, NN>::inv_x_b(c->stream, c->f.spec, c->f.S, xi.data() + q, n, Smax,
+                                                              LOAD_MASKED, tb, 0, c->N, 1))));
+                return PS_OK;
+            }));
+            PS_TRY(launches(KF_PASS_Y, by, nx, [&](int q, int n) -> int {
+                PS_SWITCH_N(N, PS_TRY((L3<float, NN>::pass_y_b(c->stream, yi.data() + q, n, Smax, true, tb, 0, ya))));
+                return PS_OK;
+            }));
+            PS_TRY(launches(KF_PAIR_Z, bp, ngr, [&](int q, int n) -> int {
+                PS_SWITCH_N(N, PS_TRY((L3<float, NN>::pair_z_b(c->stream, pi_.data() + q, n, ninputs, ha_max, hb_max, tb, 0,
+                                                               pair_var_of<float>(c, M)))));
+                return PS_OK;
+            }));
+            // rows |my| >= hout lie outside every shell a product is dotted with
+            PS_TRY(launches(KF_PASS_Y, byf, ngr, [&](int q, int n) -> int {
+                PS_SWITCH_N(N, PS_TRY((L3<float, NN>::pass_y_b(c->stream, yf.data() + q, n, Pmax, false, tb, 0, ya))));
+                return PS_OK;
+            }));
+            for (int abs_pass = 0; abs_pass < (kappa ? 2 : 1); abs_pass++)
+                PS_TRY(launches(KF_FWD_X_DOT, bd, nf, [&](int q, int n) -> int {
+                    PS_SWITCH_N(N, PS_TRY((L3<float, NN>::fwd_x(c->stream, (abs_pass ? fa : fx).data() + q, n, Pmax,
+                                                                abs_pass ? SPEC_DOT_ABS : SPEC_DOT, nullptr, 0, c->f.spec,
+                                                                c->f.S, tb, nullptr, 0, c->N, nullptr, NN,
+                                                                dot_alt_of<float>(c, M)))));
+                    return PS_OK;
+                }));
             PS_CK(launch_status());
             return PS_OK;
         };
-        auto i_part = [=](int M) -> std::function<int()> {
-            if (enum_counts) return enum_part;
-            return [=]() {
-                int Sa = 0, ha = 0, Sb = 0, hbb = 0, S = 0;
-                PS_TRY(c2r_xy<double>(c, LOAD_UNIT, dtable + G.a, sa.band, c->d.work, &Sa, &ha, 1, M));
-                if (G.a != G.b)
-                    PS_TRY(c2r_xy<double>(c, LOAD_UNIT, dtable + G.b, sb.band, c->d.work2, &Sb, &hbb, 1, M));
-                PS_TRY(pair_spectrum<double>(c, c->d.work, Sa, ha, G.a != G.b ? c->d.work2 : nullptr, Sb, hbb, hout,
-                                             &S, 1, M));
-                PS_TRY(dot_pass<double>(c, c->d.work3, SPEC_COUNT, S, hout, dtable + go, gtable.data(), ng, sumI, 1,
-                                        M, 1.0, didx + io));
-                return PS_OK;
-            };
+        return PS_OK;
+    };
+
+    // ---- counts: exact, by enumeration, when every shell of the group is an
+    // r^2 interval and the legs are known on the host (closing shells may come
+    // from the DERIVED chain: their intervals are read on the device); else
+    // FP64 transforms of the unit shells on the xy-quadrant (unit filters are
+    // even in every axis)
+    bool any_fft = false;
+    for (size_t g = 0; g < groups.size(); g++) {
+        const Group& G = groups[g];
+        GroupInfo& I = info[g];
+        I.enum_counts = !(P->flags & PS_PLAN_FFT_COUNTS) && uniq[G.a].tag == 0 && uniq[G.b].tag == 0 &&
+                        I.sa.kind <= SHELL_RANGE && I.sb.kind <= SHELL_RANGE;
+        for (const Shell& h : I.gtable) I.enum_counts = I.enum_counts && h.kind <= SHELL_RANGE;
+        if (I.enum_counts) I.enum_counts = pair_count_lists(I.sa, I.sb, N, &I.lists);
+        any_fft = any_fft || !I.enum_counts;
+    }
+    if (any_fft) {
+        PS_TRY(ensure_pair_bufs(c, c->d));
+        SideLane lane(c, true);  // the side lane's own scratch, profiling or not
+        PS_TRY(ensure_partials(c, std::max((size_t)N * N, (size_t)N * (c->d.S / pw<double>(N)) * MAX_DOT_SHELLS)));
+        PS_TRY(ensure_lut(c, (size_t)3 * (N / 2) * (N / 2) + 2));
+    }
+    auto fft_counts = [&](size_t g, int M) -> std::function<int()> {
+        const Group G = groups[g];
+        const Shell sa = info[g].sa, sb = info[g].sb;
+        const std::vector<Shell> gtable = info[g].gtable;
+        const int hout = info[g].hmax + 1, go = gofs[g], io = gidx_ofs[g];
+        return [=]() {
+            int Sa = 0, ha = 0, Sb = 0, hbb = 0, S = 0;
+            PS_TRY(c2r_xy<double>(c, LOAD_UNIT, dtable + G.a, sa.band, c->d.work, &Sa, &ha, 1, M));
+            if (G.a != G.b)
+                PS_TRY(c2r_xy<double>(c, LOAD_UNIT, dtable + G.b, sb.band, c->d.work2, &Sb, &hbb, 1, M));
+            PS_TRY(pair_spectrum<double>(c, c->d.work, Sa, ha, G.a != G.b ? c->d.work2 : nullptr, Sb, hbb, hout, &S, 1, M));
+            PS_TRY(dot_pass<double>(c, c->d.work3, SPEC_COUNT, S, hout, dtable + go, gtable.data(), (int)gtable.size(), sumI,
+                                    1, M, 1.0, didx + io));
+            return PS_OK;
         };
-        auto group_op = [=](int M) -> std::function<int()> {
-            const auto dp = d_part(M), ip = i_part(M);
-            return [=]() {
-                PS_TRY(dp());
-                return ip();
-            };
-        };
-        int M = alias_free_grid(N, ba, bb, hmax);
-        const std::array<int, 4> key = {N, ba, bb, hmax};
+    };
+
+    // ---- sub-grids: the smallest alias-free one, or the fastest candidate.  Groups
+    // below 96 points are launch-bound and run in batches: timing one alone would
+    // say nothing, they keep the smallest
+    bool prefix_done = false;
+    auto prefix = [&]() -> int {  // the DERIVED chain fills the closing shells the candidates read
+        PS_TRY(plan_flush(P));
+        if (!prefix_done)
+            for (auto& op : ops) PS_TRY(op());
+        prefix_done = true;
+        return PS_OK;
+    };
+    for (size_t g = 0; g < groups.size(); g++) {
+        GroupInfo& I = info[g];
+        const int ba = std::min(I.sa.band, N / 2), bb = std::min(I.sb.band, N / 2);
+        int M = alias_free_grid(N, ba, bb, I.hmax);
+        const std::array<int, 4> key = {N, ba, bb, I.hmax};
         auto known = c->tune_grid.find(key);
+        const auto field_op = [&](int m) -> std::function<int()> {
+            std::function<int()> op;
+            const size_t at = (sum_bytes(g, m) + 255) / 256 * 256;
+            int rc = ensure_lane_work(c, 0, at + group_bytes(g, m));
+            if (rc == PS_OK) rc = batch_op({g}, m, 0, 0, at, &op);
+            if (rc == PS_OK) return op;
+            return [rc]() { return rc; };
+        };
         if (known != c->tune_grid.end() && known->second >= M && known->second <= N && grid_supported(known->second)) {
             M = known->second;
-        } else if (P->flags & PS_PLAN_AUTOTUNE) {
-            if (!prefix_done) {  // the DERIVED chain fills the closing shells the candidates read
-                for (auto& op : ops) PS_TRY(op());
-                prefix_done = true;
-            }
-            PS_TRY(tune_grid(c, group_op, M, &M));
+        } else if ((P->flags & PS_PLAN_AUTOTUNE) && M >= 96) {
+            const auto group_op = [&](int m) -> std::function<int()> {
+                const auto dp = field_op(m);
+                if (I.enum_counts) return dp;  // the counts do not depend on m
+                const auto ip = fft_counts(g, m);
+                return [=]() {
+                    PS_TRY(dp());
+                    return ip();
+                };
+            };
+            PS_TRY(prefix());
+            size_t most = 0;  // workspace of the largest candidate, so that it grows once
+            for (int q : kGridSizes)
+                if (q >= M && q <= N) {
+                    most = std::max(most, sum_bytes(g, q) + 256 + group_bytes(g, q));
+                    if (q != M && (q >= 2 * M || most > ((size_t)1 << 30))) break;
+                }
+            PS_TRY(ensure_lane_work(c, 0, most));
+            PS_TRY(tune_grid(c, group_op, M, &M, [&]() { return plan_flush(P); }));
             c->tune_grid[key] = M;
         }
         if (M < N) {
             Tables<float> t32;
-            Tables<double> t64;
             PS_TRY(tables_for<float>(c, M, &t32));
-            PS_TRY(tables_for<double>(c, M, &t64));
+            Tables<double> t64;
+            if (!I.enum_counts) PS_TRY(tables_for<double>(c, M, &t64));
         }
         if (P->flags & PS_PLAN_AUTOTUNE) {  // the FP32 pair kernel variant and dot pass geometry of this size
-            PS_TRY(tune_pair(c, M, std::min(sa.band, M / 2) + 1, G.a != G.b ? std::min(sb.band, M / 2) + 1 : 0,
-                             hout));
+            PS_TRY(tune_pair(c, M, std::min(I.sa.band, M / 2) + 1, I.two ? std::min(I.sb.band, M / 2) + 1 : 0,
+                             I.hmax + 1));
             if (!c->dot_alt.count(M)) {
-                if (!prefix_done) {  // the DERIVED chain fills the closing shells the group reads
-                    for (auto& op : ops) PS_TRY(op());
-                    prefix_done = true;
-                }
-                PS_TRY(tune_dot(c, d_part(M), M));
+                const auto op = field_op(M);
+                PS_TRY(prefix());
+                PS_TRY(tune_dot(c, op, M));
             }
         }
-        group_dop[g] = d_part(M);
-        group_iop[g] = i_part(M);
-        group_M[g] = M;
-        {   // FP32 work spectra the group's field part writes on its M-grid
-            const int w32 = pw<float>(M);
-            const int s_ab = round_up(std::max(std::min(sa.band, M / 2), std::min(sb.band, M / 2)) + 1, w32);
-            group_need[g] = (size_t)M * M * (size_t)std::max(s_ab, round_up(hout, w32));
-        }
-        (void)hsh;
+        I.M = M;
     }
     if (P->flags & PS_PLAN_AUTOTUNE) {  // the FP32 Y pass geometry of the pair groups' transform sizes
-        for (size_t g = 0; g < groups.size(); g++) PS_TRY(tune_pencil(c, group_M[g]));
+        for (const GroupInfo& I : info) PS_TRY(tune_pencil(c, I.M));
     }
-    // lanes: the groups by decreasing transform volume, each onto the less
-    // loaded of the main and the second field lane (one lane when profiling
-    // or with a single group)
-    std::vector<int> group_lane(groups.size(), 0);
-    if (groups.size() > 1) {
+
+    // ---- batches: groups of one size together while their spectra stay in L2
+    // (64 MB of 126), larger groups alone; then the batches by decreasing volume,
+    // each onto the less loaded of the two field lanes
+    {
+        constexpr size_t kBatchBytes = (size_t)64 << 20;
+        struct Batch {
+            int M;
+            std::vector<size_t> g;
+            double cost;
+        };
         std::vector<size_t> order(groups.size());
         for (size_t g = 0; g < groups.size(); g++) order[g] = g;
-        std::stable_sort(order.begin(), order.end(),
-                         [&](size_t x, size_t y) { return group_M[x] > group_M[y]; });
-        double load[2] = {0.0, 0.0};
-        size_t need2 = 0;
+        std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) { return info[x].M > info[y].M; });
+        std::vector<Batch> batches;
+        size_t bytes = 0;
         for (size_t g : order) {
-            const int l = load[1] < load[0] ? 1 : 0;
-            group_lane[g] = l;
-            load[l] += (double)group_M[g] * group_M[g] * group_M[g];
-            if (l == 1) need2 = std::max(need2, group_need[g]);
+            const int M = info[g].M;
+            const size_t b = group_bytes(g, M);
+            if (batches.empty() || batches.back().M != M || bytes + b > kBatchBytes) {
+                batches.push_back(Batch{M, {}, 3e6});  // a launch sequence's latency, in cells
+                bytes = 0;
+            }
+            batches.back().g.push_back(g);
+            batches.back().cost += (double)M * M * M;
+            bytes += b;
         }
-        if (need2 > 0) {
-            PS_TRY(ensure_lane2_work(c, need2));
-            const size_t pen32 = (size_t)N * (c->f.S / pw<float>(N));
-            const size_t np = std::max({(size_t)N * N, pen32 * MAX_DOT_SHELLS, (size_t)148 * 8 * 2 * MAX_DOT_SHELLS});
-            Lane2 lane(c, true);  // the second lane's own scratch, profiling or not
-            PS_TRY(ensure_partials(c, np));
-            PS_TRY(ensure_lut(c, (size_t)3 * (N / 2) * (N / 2) + 2));
+        std::stable_sort(batches.begin(), batches.end(), [](const Batch& x, const Batch& y) { return x.cost > y.cost; });
+        double load[2] = {0.0, 0.0};
+        std::vector<int> lane(batches.size());
+        size_t need[2] = {0, 0}, nsums[2] = {0, 0};
+        std::vector<size_t> sums_at(batches.size());
+        for (size_t q = 0; q < batches.size(); q++) {
+            const int l = lane[q] = load[1] < load[0] ? 1 : 0;
+            load[l] += batches[q].cost;
+            size_t spectra = 0;
+            sums_at[q] = nsums[l];
+            for (size_t g : batches[q].g) {
+                spectra += group_bytes(g, batches[q].M);
+                nsums[l] += sum_bytes(g, batches[q].M);
+            }
+            need[l] = std::max(need[l], spectra);
+        }
+        for (int l = 0; l < 2; l++) {  // final size before any batch takes addresses
+            nsums[l] = (nsums[l] + 255) / 256 * 256;
+            if (need[l]) PS_TRY(ensure_lane_work(c, l, nsums[l] + need[l]));
+        }
+        sums.clear();  // of the tuning's candidates
+        sums_abs.clear();
+        for (size_t q = 0; q < batches.size(); q++) {
+            std::function<int()> op;
+            const bool second = lane[q] == 1;
+            PS_TRY(batch_op(batches[q].g, batches[q].M, lane[q], sums_at[q], nsums[lane[q]], &op));
+            P->two_lanes = P->two_lanes || second;
+            P->ops_groups.push_back([=]() {
+                Lane2 l(c, second);
+                return op();
+            });
+        }
+        sums.insert(sums.end(), sums_abs.begin(), sums_abs.end());
+        for (size_t q0 = 0; q0 < sums.size(); q0 += kItems) {
+            const int n = (int)std::min<size_t>(kItems, sums.size() - q0);
+            const auto items = pack(sums.data() + q0, n);
+            double bytes = 0.0;
+            for (int q = 0; q < n; q++) bytes += 8.0 * items.at[q].nblk * items.at[q].nshell;
+            P->ops_tail.push_back([=]() {
+                Prof pf(c);
+                k_sum_items<float><<<dim3(MAX_DOT_SHELLS, n), 256, 0, c->stream>>>(items);
+                pf.end(KF_SUM, bytes);
+                PS_CK(launch_status());
+                return PS_OK;
+            });
         }
     }
-    // the groups' counts (run on the side lane) and field parts (main or
-    // second lane); the lanes are forked and joined where the parts are enqueued
-    P->has_groups = !groups.empty();
-    for (size_t g = 0; g < groups.size(); g++) {
-        const auto dop = group_dop[g];
-        const bool second = group_lane[g] == 1;
-        P->ops_counts.push_back(group_iop[g]);
-        P->ops_groups.push_back([=]() {
-            if (second) {
-                Lane2 lane(c);
-                return dop();
+
+    // ---- the counts' launches: enumerated groups together (by histogram size, so
+    // small ones do not hold a large one's shared memory), then the FFT ones
+    {
+        struct Launch {
+            CountItem* items;
+            int n, grid;
+            size_t smem;
+            bool wrap;
+        };
+        std::vector<Launch> launches;
+        std::vector<int> order;  // configurations of the enumerated groups
+        double bytes = 0.0;
+        size_t total = 0;
+        for (size_t g = 0; g < groups.size(); g++)
+            if (info[g].enum_counts) total += info[g].gtable.size();
+        unsigned long long* dcounts = nullptr;
+        if (total) PS_TRY(plan_alloc(P, &dcounts, total));
+        int sms = 148;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+        constexpr int kClass[3] = {2048, 12 * 1024, kCountMaxBins};  // bins
+        for (int wrap = 0; wrap < 2; wrap++)
+            for (int cl = 0; cl < 3; cl++) {
+                std::vector<CountItem> items;
+                std::vector<double> pairs;
+                double sum = 0.0;
+                int nb_max = 0;
+                for (size_t g = 0; g < groups.size(); g++) {
+                    const GroupInfo& I = info[g];
+                    if (!I.enum_counts || (int)I.lists.wrap != wrap) continue;
+                    if (I.lists.nbins > kClass[cl] || (cl > 0 && I.lists.nbins <= kClass[cl - 1])) continue;
+                    CountItem it{};
+                    int4* dreps = nullptr;
+                    short4* dmodes = nullptr;
+                    PS_TRY(plan_upload(P, &dreps, I.lists.reps));
+                    PS_TRY(plan_upload(P, &dmodes, I.lists.modes));
+                    it.reps = dreps;
+                    it.modes = dmodes;
+                    it.closing = dtable + gofs[g];
+                    it.counts = dcounts + order.size();
+                    it.nrep = (int)I.lists.reps.size();
+                    it.nb = (int)I.lists.modes.size();
+                    it.s_lo = I.lists.s_lo;
+                    it.nbins = I.lists.nbins;
+                    it.ncl = (int)I.gtable.size();
+                    items.push_back(it);
+                    pairs.push_back((double)it.nrep * it.nb);
+                    sum += pairs.back();
+                    nb_max = std::max(nb_max, it.nbins);
+                    bytes += 8.0 * it.nb + 16.0 * it.nrep;
+                    for (int q : groups[g].cfg) order.push_back(q);
+                }
+                if (items.empty()) continue;
+                // about one CTA of kCountThreads per SM in all, shared out by pairs, over
+                // about eight work items each: the count lane runs beside the field load
+                // and the field lanes, and one histogram per SM leaves the rest of each SM's
+                // shared memory to their passes
+                int cta = 0;
+                for (size_t q = 0; q < items.size(); q++) {
+                    CountItem& it = items[q];
+                    const int share = std::max(1, (int)(sms * pairs[q] / std::max(sum, 1.0)));
+                    const int nmc = std::max(1, (it.nb + kCountThreads * kCountBPT - 1) / (kCountThreads * kCountBPT));
+                    const int nrs = std::max(1, std::min(it.nrep, (8 * share + nmc - 1) / nmc));
+                    it.rep_slice = std::min(kCountRepChunk, std::max(8, (it.nrep + nrs - 1) / nrs));
+                    const int nitems = nmc * ((it.nrep + it.rep_slice - 1) / it.rep_slice);
+                    it.cta0 = cta;
+                    it.nctas = std::max(1, std::min(nitems, share));
+                    cta += it.nctas;
+                }
+                Launch L{nullptr, (int)items.size(), cta, kCountStageBytes + (size_t)nb_max * sizeof(unsigned int), wrap != 0};
+                PS_TRY(plan_upload(P, &L.items, items));
+                launches.push_back(L);
             }
-            return dop();
-        });
+        if (!launches.empty()) {
+            // the shared-memory limit is a property of the kernel, not of a launch
+            // (every launch, replayed from a graph too, must fit under it): the
+            // largest histogram any group may have
+            constexpr int kLimit = (int)(kCountStageBytes + kCountMaxBins * sizeof(unsigned int));
+            PS_CK(cudaFuncSetAttribute(k_pair_counts<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLimit));
+            PS_CK(cudaFuncSetAttribute(k_pair_counts<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLimit));
+            int* dorder = nullptr;
+            PS_TRY(plan_upload(P, &dorder, order));
+            const int nc = (int)order.size();
+            P->ops_counts.push_back([=]() -> int {
+                PS_CK(cudaMemsetAsync(dcounts, 0, sizeof(unsigned long long) * (size_t)nc, c->stream));
+                for (const Launch& L : launches) {
+                    Prof pf(c);
+                    if (L.wrap) k_pair_counts<true><<<L.grid, kCountThreads, L.smem, c->stream>>>(L.items, L.n, N);
+                    else k_pair_counts<false><<<L.grid, kCountThreads, L.smem, c->stream>>>(L.items, L.n, N);
+                    pf.end(KF_PAIR_COUNTS, bytes / (double)launches.size());
+                }
+                k_counts_out<<<(nc + 127) / 128, 128, 0, c->stream>>>(nc, dcounts, dorder, sumI);
+                PS_CK(launch_status());
+                return PS_OK;
+            });
+        }
+        for (size_t g = 0; g < groups.size(); g++)
+            if (!info[g].enum_counts) P->ops_counts.push_back(fft_counts(g, info[g].M));
     }
     auto& tail = P->ops_tail;
     // ---- n = 2 (Parseval)
@@ -2332,12 +2696,12 @@ int enqueue_part(ps_gpu_ctx* c, ps_gpu_plan* P, int part)
     case PART_COUNTS:
         return enqueue_ops(P->ops_counts);
     case PART_GROUPS:
-        if (P->has_groups && !c->prof_on) {
+        if (P->two_lanes && !c->prof_on) {
             PS_CK(cudaEventRecord(c->ev_fork, c->stream));
             PS_CK(cudaStreamWaitEvent(c->lane2_stream, c->ev_fork, 0));
         }
         PS_TRY(enqueue_ops(P->ops_groups));
-        if (P->has_groups && !c->prof_on) {
+        if (P->two_lanes && !c->prof_on) {
             PS_CK(cudaEventRecord(c->ev_join2, c->lane2_stream));
             PS_CK(cudaStreamWaitEvent(c->stream, c->ev_join2, 0));
         }
@@ -2470,8 +2834,9 @@ int submit_slot(ps_gpu_ctx* c, size_t len, double** host, cudaEvent_t* ev)
     return PS_OK;
 }
 
-// Device and pinned memory of a plan (the plan object itself stays).
-void plan_release(ps_gpu_plan* P)
+// Graphs and tables of a plan (the plan object itself stays); keep: its memory
+// goes back to the context for the next plan, else it is freed.
+void plan_release(ps_gpu_plan* P, bool keep)
 {
     if (P->exec) cudaGraphExecDestroy(P->exec);
     if (P->graph) cudaGraphDestroy(P->graph);
@@ -2490,17 +2855,29 @@ void plan_release(ps_gpu_plan* P)
     P->ops_counts.clear();
     P->ops_groups.clear();
     P->ops_tail.clear();
-    for (void* p : P->owned) cudaFree(p);
-    P->owned.clear();
-    if (P->hres) cudaFreeHost(P->hres);
-    P->hres = nullptr;
     P->ops.clear();
+    if (!P->arenas.empty()) {
+        // nothing may still read the tables or their mirrors when the next plan writes them
+        ps_gpu_ctx* c = P->ctx;
+        for (cudaStream_t st : {c->stream, c->side_stream, c->lane2_stream})
+            if (st) cudaStreamSynchronize(st);
+        for (PlanArena& a : P->arenas) {
+            if (keep && a.cap <= kSpareBytes && c->spare_arenas.size() < kSpareArenas) {
+                c->spare_arenas.push_back(a);
+            } else {
+                cudaFree(a.dev);
+                cudaFreeHost(a.host);
+            }
+        }
+        P->arenas.clear();
+    }
+    P->hres = nullptr;
 }
 
 void plan_free(ps_gpu_plan* P)
 {
     if (!P) return;
-    plan_release(P);
+    plan_release(P, P->ctx != nullptr);
     delete P;
 }
 
@@ -2591,6 +2968,7 @@ int batched(ps_gpu_ctx* c, int nconf, ps_cfg* cfgs, double* B, double* Np, doubl
     P->flags = kappa ? PS_PLAN_KAPPA : 0;
     P->cfgs.assign(cfgs, cfgs + nconf);
     int rc = plan_batched(c, P);
+    if (rc == PS_OK) rc = plan_flush(P);
     if (rc == PS_OK) rc = check_band(c, P->band);
     if (rc == PS_OK) rc = plan_enqueue(c, P);
     if (rc == PS_OK) rc = plan_finish(c, P, B, Np, kappa, cfgs);
@@ -2649,9 +3027,15 @@ int grad_impl(ps_gpu_ctx* c, int n, const std::vector<Shell>& legs, double scale
             const int hout = std::min(legs[li].band, N / 2) + 1;
             PS_TRY(pair_spectrum<T>(c, B.work, Sa, ha, same ? nullptr : B.work2, Sb, hbb, hout, &S));
             Prof pf(c);
-            PS_SWITCH_N(N, PS_TRY((L3<T, NN>::fwd_x(c->stream, B.work3, S, hout, SPEC_MASK_ADD, B.hacc, B.S, nullptr,
-                                                    0, c->dshells + li, 1, nullptr, 0, nullptr, B.tables(),
-                                                    nullptr, (double)tm.second))));
+            FwdXItem<T> it{};
+            it.data = B.work3;
+            it.stride = it.ncols = S;
+            it.hvalid = hout;
+            it.shells = c->dshells + li;
+            it.nshell = 1;
+            it.weight = (double)tm.second;
+            PS_SWITCH_N(N, PS_TRY((L3<T, NN>::fwd_x(c->stream, &it, 1, S, SPEC_MASK_ADD, B.hacc, B.S, nullptr, 0,
+                                                    B.tables(), nullptr))));
             pf.end(fam<T>(KF_GRAD), 3.0 * N * N * S * sizeof(V2<T>), N);
         }
     }
@@ -3395,7 +3779,10 @@ int ps_gpu_plan_create(ps_gpu_ctx* c, int method, int nconf, const ps_cfg* cfgs,
     P->flags = method == PS_FP32_BATCHED ? flags : (flags & PS_PLAN_KAPPA);
     P->cfgs.assign(cfgs, cfgs + nconf);
     if (method == PS_FP32_BATCHED && nconf > 0) {
-        const int rc = plan_batched(c, P);
+        int rc = plan_batched(c, P);
+        if (rc == PS_OK) rc = plan_flush(P);
+        // executions may run on another stream (ps_gpu_set_stream)
+        if (rc == PS_OK && cudaStreamSynchronize(c->stream) != cudaSuccess) rc = fail(PS_ERR_CUDA, "plan upload failed");
         if (rc != PS_OK) {
             plan_free(P);
             return rc;
@@ -3698,10 +4085,14 @@ void ps_gpu_finalize(ps_gpu_ctx* c)
     for (auto& hb : c->spare_host) cudaFreeHost(hb.first);
     for (cudaEvent_t e : c->spare_events) cudaEventDestroy(e);
     for (ps_gpu_plan* P : c->plans) {  // plans outliving their context keep only their host part
-        plan_release(P);
+        plan_release(P, false);
         P->ctx = nullptr;
     }
     c->plans.clear();
+    for (PlanArena& a : c->spare_arenas) {
+        cudaFree(a.dev);
+        cudaFreeHost(a.host);
+    }
     free_prec(c->f);
     free_prec(c->d);
     cudaFree(c->partials);
@@ -3736,9 +4127,7 @@ void ps_gpu_finalize(ps_gpu_ctx* c)
         cudaStreamSynchronize(c->lane2_stream);
         cudaStreamDestroy(c->lane2_stream);
     }
-    cudaFree(c->lane2_partials);
-    cudaFree(c->lane2_lut);
-    for (auto& p : c->lane2_work) cudaFree(p);
+    for (auto& p : c->lane_work) cudaFree(p);
     if (c->ev_join2) cudaEventDestroy(c->ev_join2);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);

@@ -4,9 +4,7 @@
 #pragma once
 
 #include <algorithm>
-#include <array>
 #include <cmath>
-#include <map>
 #include <vector>
 
 #include "ps_common.cuh"
@@ -25,7 +23,7 @@ namespace ps {
 // flips with their orbit sizes as weights: S_b, the closing shells and |w(.)|^2
 // are invariant under them.  The pairs are cut into work items (a chunk of
 // THREADS BPT modes of S_b times a slice of rep_slice representatives); each CTA
-// of a grid of resident CTAs takes items blockIdx.x, + gridDim.x, ... into
+// of a group takes every nctas-th item into
 // its own histogram of |w(m_a + m_b)|^2 - s_lo over nbins bins in shared
 // memory (integer atomics: the result does not depend on their order), so
 // the clearing and the interval sums are paid once per CTA.  Each CTA then sums each closing shell's
@@ -40,12 +38,33 @@ constexpr int kCountRepChunk = 512;  // largest rep_slice
 constexpr size_t kCountStageBytes = kCountRepChunk * (sizeof(int4) + sizeof(int));
 constexpr int kCountMaxBins = 44 * 1024;  // 176 KB of uint32 bins beside the staged representatives
 
+// One launch counts for a list of groups: group g has the CTAs cta0 .. cta0 +
+// nctas - 1 (about in proportion to its pairs), each with a histogram of its own.
+struct CountItem {
+    const int4* reps;
+    const short4* modes;
+    const Shell* closing;
+    unsigned long long* counts;
+    int nrep, nb, s_lo, nbins, rep_slice, ncl;
+    int cta0, nctas;
+};
 template <bool WRAP, int BPT = kCountBPT, int THREADS = kCountThreads>
 __global__ void __launch_bounds__(THREADS)
-    k_pair_counts(const int4* __restrict__ reps, int nrep, const short4* __restrict__ modes, int nb, int n, int s_lo,
-                  int nbins, int rep_slice, const Shell* __restrict__ closing, int ncl,
-                  unsigned long long* __restrict__ counts)
+    k_pair_counts(const CountItem* __restrict__ items, int ngroups, int n)
 {
+    int gi = 0;  // the group of this CTA
+    for (int e = ngroups; gi + 1 < e;) {
+        const int mid = (gi + e) >> 1;
+        if (items[mid].cta0 <= (int)blockIdx.x) gi = mid;
+        else e = mid;
+    }
+    const CountItem it = items[gi];
+    const int4* __restrict__ reps = it.reps;
+    const short4* __restrict__ modes = it.modes;
+    const Shell* __restrict__ closing = it.closing;
+    unsigned long long* __restrict__ counts = it.counts;
+    const int nrep = it.nrep, nb = it.nb, s_lo = it.s_lo, nbins = it.nbins, ncl = it.ncl;
+    int rep_slice = it.rep_slice;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     int4* srep = reinterpret_cast<int4*>(smem_raw);
     int* snorm = reinterpret_cast<int*>(smem_raw + kCountRepChunk * sizeof(int4));
@@ -56,7 +75,7 @@ __global__ void __launch_bounds__(THREADS)
     rep_slice = max(1, min(rep_slice, kCountRepChunk));  // the staging buffer's size
     const int nmc = (nb + kChunk - 1) / kChunk, nrs = (nrep + rep_slice - 1) / rep_slice;
     const int nitems = nmc * nrs;
-    for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+    for (int item = (int)blockIdx.x - it.cta0; item < nitems; item += it.nctas) {
         const int mc = item % nmc, r0 = (item / nmc) * rep_slice;
         const int cnt = min(rep_slice, nrep - r0);
         int bx[BPT], by[BPT], bz[BPT], bn[BPT];
@@ -159,13 +178,32 @@ inline std::vector<short4> interval_modes(const Shell& sh, int N)
     return out;
 }
 
-// Canonical member of a mode's orbit under axis permutations and sign flips
-// on the N-grid: components |x| (as indices, -N/2 stays N/2 = -N/2), sorted.
-inline std::array<int, 3> orbit_key(int x, int y, int z)
+// Representatives 0 <= x <= y <= z (as indices, N/2 stands for -N/2) of the
+// orbits of an interval shell's modes under the 48 axis permutations and sign
+// flips, with the orbit sizes: 6, 3 or 1 permutations, two signs per component
+// but for 0 and the single index of |N/2|.
+inline std::vector<int4> interval_orbits(const Shell& sh, int N)
 {
-    std::array<int, 3> k = {std::abs(x), std::abs(y), std::abs(z)};
-    std::sort(k.begin(), k.end());
-    return k;
+    std::vector<int4> out;
+    if (sh.r2hi < 0 || sh.r2lo > sh.r2hi) return out;
+    const int b = std::min(sh.band, N / 2);
+    const auto signs = [&](int v) { return v == 0 || v == N / 2 ? 1 : 2; };
+    const auto lattice = [&](int v) { return v == N / 2 ? -(N / 2) : v; };
+    for (int x = 0; x <= b && 3 * x * x <= sh.r2hi; x++)
+        for (int y = x; y <= b && x * x + 2 * y * y <= sh.r2hi; y++) {
+            const int s = x * x + y * y;
+            int z = y;
+            if (sh.r2lo - s > z * z) {
+                z = (int)sqrt((double)(sh.r2lo - s));
+                while (z * z < sh.r2lo - s) z++;
+                while (z > y && (z - 1) * (z - 1) >= sh.r2lo - s) z--;
+            }
+            for (; z <= b && s + z * z <= sh.r2hi; z++) {
+                const int perms = x == y && y == z ? 1 : x == y || y == z ? 3 : 6;
+                out.push_back(int4{lattice(x), lattice(y), lattice(z), perms * signs(x) * signs(y) * signs(z)});
+            }
+        }
+    return out;
 }
 
 // The lists of a group with interval legs a, b on an N-grid; false when the
@@ -175,19 +213,14 @@ inline bool pair_count_lists(const Shell& sa, const Shell& sb, int N, PairCountL
     // host work O(b^2 + |S|); the enumeration itself |S_a| |S_b| / 48 pairs
     const double est = 4.0 * 3.14159 * (double)std::max(sa.r2hi, 1) * 4.0 * 3.14159 * (double)std::max(sb.r2hi, 1);
     if (std::max(sa.band, sb.band) > 300 || est / 48.0 > 4e10) return false;
-    std::vector<short4> ma = interval_modes(sa, N), mb = interval_modes(sb, N);
-    if ((double)ma.size() * (double)mb.size() / 48.0 > 4e9) return false;
-    if (ma.size() > mb.size()) std::swap(ma, mb);  // representatives from the smaller shell
-    std::map<std::array<int, 3>, int> orbits;
-    for (const short4& m : ma) orbits[orbit_key(m.x, m.y, m.z)]++;
-    L->reps.clear();
-    for (const auto& kv : orbits) {
-        // a representative as lattice frequencies (N/2 is the index of -N/2)
-        int v[3];
-        for (int q = 0; q < 3; q++) v[q] = kv.first[q] == N / 2 ? -(N / 2) : kv.first[q];
-        L->reps.push_back(int4{v[0], v[1], v[2], kv.second});
-    }
-    L->modes = mb;
+    // representatives from the smaller shell
+    const Shell *pa = &sa, *pb = &sb;
+    const auto volume = [](const Shell& h) { return pow((double)std::max(h.r2hi, 0), 1.5) - pow((double)std::max(h.r2lo, 0), 1.5); };
+    if (volume(sa) > volume(sb)) std::swap(pa, pb);
+    L->reps = interval_orbits(*pa, N);
+    if (48.0 * (double)L->reps.size() * 4.19 * std::max(volume(*pb), 1.0) / 48.0 > 1.2e10) return false;
+    L->modes = interval_modes(*pb, N);
+    if ((double)L->reps.size() * (double)L->modes.size() > 4e9) return false;
     const int bmax_a = std::min(sa.band, N / 2), bmax_b = std::min(sb.band, N / 2);
     L->wrap = bmax_a + bmax_b >= N / 2;
     const double ra_hi = sqrt((double)std::max(sa.r2hi, 0)), rb_hi = sqrt((double)std::max(sb.r2hi, 0));
@@ -197,7 +230,7 @@ inline bool pair_count_lists(const Shell& sa, const Shell& sb, int N, PairCountL
     const double dmin = L->wrap ? 0.0 : std::max({0.0, ra_lo - rb_hi, rb_lo - ra_hi});
     L->s_lo = std::max(0, (int)floor(dmin * dmin) - 1);
     const long long s_hi = (long long)ceil(smax) + 1;
-    if (s_hi - L->s_lo + 1 > kCountMaxBins || ma.empty() || mb.empty()) return false;
+    if (s_hi - L->s_lo + 1 > kCountMaxBins) return false;
     L->nbins = (int)(s_hi - L->s_lo + 1);
     return true;
 }

@@ -89,12 +89,14 @@ double time_pass_y(int reps, float2* data, int S, int ncols, int jband, int jout
     int per_sm = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, G::THREADS, G::SMEM));
     const unsigned blocks = (unsigned)(M * (ncols / G::W));
+    const YItem<float> item{data, S, ncols, jband, jout};
+    const auto items = pack(&item, 1);
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
-    for (int it = 0; it < 3; it++) kern<<<blocks, G::THREADS, G::SMEM>>>(data, S, ncols, 0, jband, jout, tw);
+    for (int it = 0; it < 3; it++) kern<<<blocks, G::THREADS, G::SMEM>>>(items, 0, tw);
     CK(cudaEventRecord(e0));
-    for (int it = 0; it < reps; it++) kern<<<blocks, G::THREADS, G::SMEM>>>(data, S, ncols, 0, jband, jout, tw);
+    for (int it = 0; it < reps; it++) kern<<<blocks, G::THREADS, G::SMEM>>>(items, 0, tw);
     CK(cudaEventRecord(e1));
     CK(cudaEventSynchronize(e1));
     CK(cudaGetLastError());
@@ -133,16 +135,18 @@ double time_pair(int reps, const float2* wa, int Sa, int ba, const float2* wb, i
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, G::THREADS, smem));
+    const PairItem<float> item{wa, wb, w3, Sa, ba + 1, Sb, bb + 1, S, bc + 1};
+    const auto items = pack(&item, 1);
     const int nrows = M * M, tiles = (nrows + G::WZ - 1) / G::WZ;
     const int grid = std::min(tiles, std::max(per_sm, 1) * sms);
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
     for (int it = 0; it < 3; it++)
-        kern<<<grid, G::THREADS, smem>>>(wa, Sa, ba + 1, wb, Sb, bb + 1, w3, S, bc + 1, nrows, twr, twpp);
+        kern<<<grid, G::THREADS, smem>>>(items, nrows, twr, twpp);
     CK(cudaEventRecord(e0));
     for (int it = 0; it < reps; it++)
-        kern<<<grid, G::THREADS, smem>>>(wa, Sa, ba + 1, wb, Sb, bb + 1, w3, S, bc + 1, nrows, twr, twpp);
+        kern<<<grid, G::THREADS, smem>>>(items, nrows, twr, twpp);
     CK(cudaEventRecord(e1));
     CK(cudaEventSynchronize(e1));
     CK(cudaGetLastError());
@@ -177,10 +181,14 @@ double time_counts(int reps, const PairCountLists& L, const int4* dreps, const s
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
     float total = 0.f;
+    const CountItem item{dreps, dmodes, dcl, dcounts, nrep, nb, L.s_lo, L.nbins, rep_slice, ncl, 0, grid};
+    CountItem* ditem;
+    CK(cudaMalloc(&ditem, sizeof(CountItem)));
+    CK(cudaMemcpy(ditem, &item, sizeof(CountItem), cudaMemcpyHostToDevice));
     for (int it = 0; it < reps + 2; it++) {
         CK(cudaMemset(dcounts, 0, sizeof(unsigned long long) * ncl));
         CK(cudaEventRecord(e0));
-        kern<<<grid, THREADS, smem>>>(dreps, nrep, dmodes, nb, N, L.s_lo, L.nbins, rep_slice, dcl, ncl, dcounts);
+        kern<<<grid, THREADS, smem>>>(ditem, 1, N);
         CK(cudaEventRecord(e1));
         CK(cudaEventSynchronize(e1));
         float ms = 0.f;
@@ -247,17 +255,30 @@ int main(int argc, char** argv)
         LT(L5::fwd_z(0, SRC_XHI_F32, da, db, spec, SN, hcols, T5, 1)); tm.lap();
         LT(L5::fwd_z(0, SRC_XHI_F32, da, db, spec, SN, hcols, T5, 1, 0, status)); tm.lap();
         LT(L5::pass_y(0, spec, SN, false, T5, 0, N, 176)); tm.lap();
-        LT(L5::fwd_x(0, spec, SN, hcols, SPEC_STORE_PHASE, spec, SN, nullptr, 0, nullptr, 0, nullptr, 0, nullptr, T5,
-                     nullptr, 1.0, 0, 0, 0x7fffffff, nullptr, 176, 164)); tm.lap();
+        FwdXItem<float> store{};
+        store.data = spec;
+        store.stride = SN;
+        store.hvalid = hcols;
+        store.ncols = 176;
+        LT(L5::fwd_x(0, &store, 1, 176, SPEC_STORE_PHASE, spec, SN, nullptr, 0, T5, nullptr, 0, 0, nullptr, 164));
+        tm.lap();
         LT(L4::inv_x(0, spec, SN, wa, Sa, LOAD_MASKED, dsh, M / 2 + 1, T3, 0, N, 1)); tm.lap();
         LT(L4::pass_y(0, wa, Sa, true, T3, 0, ba)); tm.lap();
         LT(L4::inv_x(0, spec, SN, wb, Sb, LOAD_MASKED, dsh + 1, M / 2 + 1, T3, 0, N, 1)); tm.lap();
         LT(L4::pass_y(0, wb, Sb, true, T3, 0, bb)); tm.lap();
         LT(L4::pair_z(0, wa, Sa, ba + 1, wb, Sb, bb + 1, w3, S, bc + 1, T3)); tm.lap();
         LT(L4::pass_y(0, w3, S, false, T3, 0, M, 0, bc)); tm.lap();
-        int nb = 0;
-        LT(L4::fwd_x(0, w3, S, bc + 1, SPEC_DOT, nullptr, 0, spec, SN, nullptr, 16, dlut, lut_size, partials, T3, &nb,
-                     1.0, 0, N, lut_size - 1)); tm.lap();
+        FwdXItem<float> dot{};
+        dot.data = w3;
+        dot.stride = dot.ncols = S;
+        dot.hvalid = bc + 1;
+        dot.nshell = 16;
+        dot.lut = dlut;
+        dot.lut_size = lut_size;
+        dot.r2max = lut_size - 1;
+        dot.weight = 1.0;
+        dot.partials = partials;
+        LT(L4::fwd_x(0, &dot, 1, S, SPEC_DOT, nullptr, 0, spec, SN, T3, nullptr, 0, N)); tm.lap();
         CK(cudaGetLastError());
         if (it == 2) { CK(cudaDeviceSynchronize()); tm.acc.assign(NK, 0.0); } else tm.collect();
     }

@@ -51,6 +51,13 @@ template <typename K> int persistent_grid(K kernel, int threads, size_t smem, in
     return PS_OK;
 }
 
+template <class I> inline Items<I> pack(const I* items, int n)
+{
+    Items<I> b;
+    for (int q = 0; q < kItems; q++) b.at[q] = items[q < n ? q : 0];
+    return b;
+}
+
 // Twiddle tables of one precision: twp = Stockham table of the pencil
 // transforms (length N), twr = of the row transforms (length N/2), twpp =
 // W_N^k for the r2c / c2r pre- and post-processing (k < N).
@@ -83,13 +90,28 @@ template <typename T, int N> struct L3 {
     // skip_dead: tiles of all-zero pencils (|my| above the shell's band) are
     // left unwritten; the following pass_y must then be given that band
     static int inv_x(cudaStream_t st, const V* src, int ss, V* dst, int ds, int mode, const Shell* sh,
-                     int hvalid, const Tables<T>& tb, int quad = 0, int nsrc = 0, int skip_dead = 0);
+                     int hvalid, const Tables<T>& tb, int quad = 0, int nsrc = 0, int skip_dead = 0)
+    {
+        const XItem<T> it{dst, ds, hvalid, sh};
+        return inv_x_b(st, src, ss, &it, 1, ds, mode, tb, quad, nsrc, skip_dead);
+    }
+    // The batched forms take nitems <= kItems descriptions (copied into the launch);
+    // ds, ncols, hva, hvb: the widest of the batch.
+    static int inv_x_b(cudaStream_t st, const V* src, int ss, const XItem<T>* items, int nitems,
+                       int ds, int mode, const Tables<T>& tb, int quad, int nsrc, int skip_dead);
     // jband < N/2: input rows with |my| > jband are zero and are not read
     // ncols (0: stride): only columns h < ncols, a multiple of the pencil width
     // jout < N/2: output rows with |my| > jout are not stored
     // alt: the alternative geometry (PencilAlt) when this length has one
     static int pass_y(cudaStream_t st, V* data, int stride, bool inv, const Tables<T>& tb, int quad = 0,
-                      int jband = N, int ncols = 0, int jout = N, int alt = 0);
+                      int jband = N, int ncols = 0, int jout = N, int alt = 0)
+    {
+        const int nc = ncols > 0 ? ncols : stride;
+        const YItem<T> it{data, stride, nc, jband, jout};
+        return pass_y_b(st, &it, 1, nc, inv, tb, quad, alt);
+    }
+    static int pass_y_b(cudaStream_t st, const YItem<T>* items, int nitems, int ncols, bool inv,
+                        const Tables<T>& tb, int quad, int alt);
     static int inv_z(cudaStream_t st, const V* src, int ss, int hvalid, T* out, const T* aux, int epi,
                      int power, double* partials, const Tables<T>& tb, int* nblocks);
     // stage: 1 copies the input rows to shared memory first (k_fwd_z STAGED),
@@ -101,20 +123,27 @@ template <typename T, int N> struct L3 {
     // array and tile) whose bounded wait sets *status to 1 if it expires
     static int fwd_z(cudaStream_t st, int kind, const void* a, const void* b, V* dst, int ds, int hout,
                      const Tables<T>& tb, int stage = -1, size_t nrows = 0, int* status = nullptr, int tx_extra = 0);
-    template <int RX, bool KEEP>
-    static int pair_z_v(cudaStream_t st, const V* a, int sa, int hva, const V* b, int sb, int hvb, V* dst, int ds,
-                        int hout, const V* twr, const V* twpp, int quad);
     // variant: the autotuned pair kernel variant (PairVariants; 0 the default,
     // and the default wherever the length lacks the one asked for)
     static int pair_z(cudaStream_t st, const V* a, int sa, int hva, const V* b, int sb, int hvb, V* dst,
-                      int ds, int hout, const Tables<T>& tb, int quad = 0, int variant = 0);
-    // ndk: grid size of the field spectrum dk (0: N); r2max: bound of the
-    // launch's shells' |m|^2 for the sum epilogues (tiles outside are skipped)
-    static int fwd_x(cudaStream_t st, V* data, int stride, int hvalid, int epi, V* out, int ostride,
-                     const V* dk, int dks, const Shell* shells, int nshell, const unsigned short* lut,
-                     int lut_size, double* partials, const Tables<T>& tb, int* nblocks, double weight = 1.0,
-                     int quad = 0, int ndk = 0, int r2max = 0x7fffffff, T* mod_out = nullptr, int ncols = 0,
-                     int jband = N, int alt = 0);
+                      int ds, int hout, const Tables<T>& tb, int quad = 0, int variant = 0)
+    {
+        const PairItem<T> it{a, b, dst, sa, hva, sb, hvb, ds, hout};
+        return pair_z_b(st, &it, 1, b ? 2 : 1, hva, hvb, tb, quad,
+                        variant);
+    }
+    // hva, hvb: the widest legs of the batch; ninputs: 2 when any item has two
+    static int pair_z_b(cudaStream_t st, const PairItem<T>* items, int nitems, int ninputs,
+                        int hva, int hvb, const Tables<T>& tb, int quad, int variant);
+    template <int RX, bool KEEP>
+    static int pair_z_v(cudaStream_t st, const PairItem<T>* items, int nitems, int ninputs,
+                        int hva, int hvb, const V* twr, const V* twpp, int quad);
+    // The forward X pass, storing (epi SPEC_STORE, SPEC_STORE_PHASE, SPEC_MASK_ADD)
+    // or summing per shell; ndk: grid size of the field spectrum dk (0: N).
+    // Returns the blocks per item of the widest spectrum in *nblocks.
+    static int fwd_x(cudaStream_t st, const FwdXItem<T>* items, int nitems, int ncols, int epi,
+                     V* out, int ostride, const V* dk, int dks, const Tables<T>& tb, int* nblocks, int quad = 0,
+                     int ndk = 0, T* mod_out = nullptr, int jband = N, int alt = 0);
 };
 
 // Grid sizes.  Powers of two 16..1024, the 3 2^k / 5 2^k sizes of the

@@ -51,46 +51,34 @@ void L3<T, N>::host_tables(V* twp, V* twr)
 }
 
 template <typename T, int N>
-int L3<T, N>::inv_x(cudaStream_t st, const V* src, int ss, V* dst, int ds, int mode, const Shell* sh,
-                 int hvalid, const Tables<T>& tb, int quad, int nsrc, int skip_dead)
+int L3<T, N>::inv_x_b(cudaStream_t st, const V* src, int ss, const XItem<T>* items, int nitems,
+                      int ds, int mode, const Tables<T>& tb, int quad, int nsrc, int skip_dead)
 {
     PS_LTRY(set_smem(k_inv_x<T, N>, PG::SMEM));
     const int nj = quad ? N / 2 + 1 : N;
-    k_inv_x<T, N><<<(unsigned)(nj * (ds / PG::W)), PG::THREADS, PG::SMEM, st>>>(
-        src, ss, nsrc > 0 ? nsrc : N, dst, ds, mode, sh, hvalid, quad, skip_dead, tb.twp);
+    k_inv_x<T, N><<<dim3((unsigned)(nj * (ds / PG::W)), (unsigned)nitems), PG::THREADS, PG::SMEM, st>>>(
+        src, ss, nsrc > 0 ? nsrc : N, pack(items, nitems), mode, quad, skip_dead, tb.twp);
     return PS_OK;
 }
 
 template <typename T, int N>
-int L3<T, N>::pass_y(cudaStream_t st, V* data, int stride, bool inv, const Tables<T>& tb, int quad,
-                  int jband, int ncols, int jout, int alt)
+int L3<T, N>::pass_y_b(cudaStream_t st, const YItem<T>* items, int nitems, int ncols, bool inv,
+                       const Tables<T>& tb, int quad, int alt)
 {
-    const int ni = quad ? N / 2 + 1 : N;
-    const int nc = ncols > 0 ? ncols : stride;
-    const unsigned blocks = (unsigned)(ni * (nc / PG::W));
+    const dim3 grid((unsigned)((quad ? N / 2 + 1 : N) * (ncols / PG::W)), (unsigned)nitems);
+    auto go = [&](auto kernel, int threads, size_t smem, const V* tw) -> int {
+        PS_LTRY(set_smem(kernel, smem));
+        kernel<<<grid, threads, smem, st>>>(pack(items, nitems), quad, tw);
+        return PS_OK;
+    };
     if constexpr (ALT > 0) {
-        if (alt && tb.twp_alt) {
-            using PA = PencilGeom<T, N, ALT>;
-            if (inv) {
-                PS_LTRY(set_smem(k_pass_y<T, N, true, ALT>, PA::SMEM));
-                k_pass_y<T, N, true, ALT><<<blocks, PA::THREADS, PA::SMEM, st>>>(data, stride, nc, quad, jband, jout,
-                                                                                 tb.twp_alt);
-            } else {
-                PS_LTRY(set_smem(k_pass_y<T, N, false, ALT>, PA::SMEM));
-                k_pass_y<T, N, false, ALT><<<blocks, PA::THREADS, PA::SMEM, st>>>(data, stride, nc, quad, jband,
-                                                                                  jout, tb.twp_alt);
-            }
-            return PS_OK;
-        }
+        using PA = PencilGeom<T, N, ALT>;
+        if (alt && tb.twp_alt)
+            return inv ? go(k_pass_y<T, N, true, ALT>, PA::THREADS, PA::SMEM, tb.twp_alt)
+                       : go(k_pass_y<T, N, false, ALT>, PA::THREADS, PA::SMEM, tb.twp_alt);
     }
-    if (inv) {
-        PS_LTRY(set_smem(k_pass_y<T, N, true>, PG::SMEM));
-        k_pass_y<T, N, true><<<blocks, PG::THREADS, PG::SMEM, st>>>(data, stride, nc, quad, jband, jout, tb.twp);
-    } else {
-        PS_LTRY(set_smem(k_pass_y<T, N, false>, PG::SMEM));
-        k_pass_y<T, N, false><<<blocks, PG::THREADS, PG::SMEM, st>>>(data, stride, nc, quad, jband, jout, tb.twp);
-    }
-    return PS_OK;
+    return inv ? go(k_pass_y<T, N, true>, PG::THREADS, PG::SMEM, tb.twp)
+               : go(k_pass_y<T, N, false>, PG::THREADS, PG::SMEM, tb.twp);
 }
 
 template <typename T, int N>
@@ -140,74 +128,65 @@ int L3<T, N>::fwd_z(cudaStream_t st, int kind, const void* a, const void* b, V* 
 
 template <typename T, int N>
 template <int RX, bool KEEP>
-int L3<T, N>::pair_z_v(cudaStream_t st, const V* a, int sa, int hva, const V* b, int sb, int hvb, V* dst, int ds,
-                    int hout, const V* twr, const V* twpp, int quad)
+int L3<T, N>::pair_z_v(cudaStream_t st, const PairItem<T>* items, int nitems, int ninputs,
+                       int hva, int hvb, const V* twr, const V* twpp, int quad)
 {
     using G = RowGeom<T, N, RX>;
     using PGm = PairGeom<T, N, RX, KEEP>;
-    const size_t smem = PGm::smem(b ? 2 : 1, hva, hvb);
+    const size_t smem = PGm::smem(ninputs, hva, hvb);
     PS_LTRY(set_smem(k_pair_z<T, N, RX, KEEP>, PGm::smem(2, N / 2 + 1, N / 2 + 1)));
     const int nrows = quad ? (N / 2 + 1) * (N / 2 + 1) : N * N;
-    int grid = 0;
-    PS_LTRY(persistent_grid(k_pair_z<T, N, RX, KEEP>, G::THREADS, smem, (nrows + G::WZ - 1) / G::WZ, &grid));
-    k_pair_z<T, N, RX, KEEP><<<grid, G::THREADS, smem, st>>>(a, sa, hva, b, sb, hvb, dst, ds, hout, nrows, twr,
-                                                             twpp);
+    const int tiles = (nrows + G::WZ - 1) / G::WZ;
+    int grid = 0;  // resident CTAs, shared out among the items
+    PS_LTRY(persistent_grid(k_pair_z<T, N, RX, KEEP>, G::THREADS, smem, tiles * nitems, &grid));
+    grid = std::max(1, std::min(tiles, grid / nitems));
+    k_pair_z<T, N, RX, KEEP><<<dim3((unsigned)grid, (unsigned)nitems), G::THREADS, smem, st>>>(pack(items, nitems), nrows, twr, twpp);
     return PS_OK;
 }
 
 template <typename T, int N>
-int L3<T, N>::pair_z(cudaStream_t st, const V* a, int sa, int hva, const V* b, int sb, int hvb, V* dst,
-                  int ds, int hout, const Tables<T>& tb, int quad, int variant)
+int L3<T, N>::pair_z_b(cudaStream_t st, const PairItem<T>* items, int nitems, int ninputs,
+                       int hva, int hvb, const Tables<T>& tb, int quad, int variant)
 {
     if constexpr (PAIR_RX2 > 0) {
         if constexpr (PairGeom<T, N, PAIR_RX2, true>::FITS) {
             if (variant == 2 && tb.twr_alt && !quad)
-                return pair_z_v<PAIR_RX2, true>(st, a, sa, hva, b, sb, hvb, dst, ds, hout, tb.twr_alt, tb.twpp,
-                                                quad);
+                return pair_z_v<PAIR_RX2, true>(st, items, nitems, ninputs, hva, hvb, tb.twr_alt, tb.twpp, quad);
         }
     }
     if constexpr (PairVariants<T, N>::KEEP_OK) {
         if (variant == 1 && !quad)
-            return pair_z_v<0, true>(st, a, sa, hva, b, sb, hvb, dst, ds, hout, tb.twr, tb.twpp, quad);
+            return pair_z_v<0, true>(st, items, nitems, ninputs, hva, hvb, tb.twr, tb.twpp, quad);
     }
-    return pair_z_v<0, false>(st, a, sa, hva, b, sb, hvb, dst, ds, hout, tb.twr, tb.twpp, quad);
+    return pair_z_v<0, false>(st, items, nitems, ninputs, hva, hvb, tb.twr, tb.twpp, quad);
 }
 
 template <typename T, int N>
-int L3<T, N>::fwd_x(cudaStream_t st, V* data, int stride, int hvalid, int epi, V* out, int ostride,
-                 const V* dk, int dks, const Shell* shells, int nshell, const unsigned short* lut,
-                 int lut_size, double* partials, const Tables<T>& tb, int* nblocks, double weight,
-                 int quad, int ndk, int r2max, T* mod_out, int ncols,
-                 int jband, int alt)
+int L3<T, N>::fwd_x(cudaStream_t st, const FwdXItem<T>* items, int nitems, int ncols, int epi,
+                    V* out, int ostride, const V* dk, int dks, const Tables<T>& tb, int* nblocks, int quad, int ndk,
+                    T* mod_out, int jband, int alt)
 {
-    const int nj = quad ? N / 2 + 1 : N;
-    const int nc = ncols > 0 ? ncols : stride;
-    const unsigned blocks = (unsigned)(nj * (nc / PG::W));
+    const dim3 grid((unsigned)((quad ? N / 2 + 1 : N) * (ncols / PG::W)), (unsigned)nitems);
     const bool dot = epi == SPEC_DOT || epi == SPEC_COUNT || epi == SPEC_DOT_ABS;
+    if (nblocks) *nblocks = (int)grid.x;
+    auto go = [&](auto batch, auto kernel, int threads, size_t smem, const V* tw) -> int {
+        PS_LTRY(set_smem(kernel, smem));
+        if constexpr (std::is_same_v<decltype(batch), std::true_type>)
+            kernel<<<grid, threads, smem, st>>>(pack(items, nitems), epi, out, ostride, dk, dks, ndk > 0 ? ndk : N, quad,
+                                                tw, mod_out, jband);
+        else
+            kernel<<<grid, threads, smem, st>>>(items[0], epi, out, ostride, dk, dks, ndk > 0 ? ndk : N, quad, tw, mod_out,
+                                                jband);
+        return PS_OK;
+    };
     if constexpr (ALT > 0) {  // alt: the dot pass in the alternative geometry (PencilAlt)
-        if (dot && alt && tb.twp_alt) {
-            using PA = PencilGeom<T, N, ALT>;
-            PS_LTRY(set_smem(k_fwd_x<T, N, true, ALT>, PA::SMEM_DOT));
-            k_fwd_x<T, N, true, ALT><<<blocks, PA::THREADS, PA::SMEM_DOT, st>>>(
-                data, stride, hvalid, epi, out, ostride, dk, dks, ndk > 0 ? ndk : N, shells, nshell, lut, lut_size,
-                weight, quad, r2max, partials, tb.twp_alt, mod_out, nc, jband);
-            if (nblocks) *nblocks = (int)blocks;
-            return PS_OK;
-        }
+        using PA = PencilGeom<T, N, ALT>;
+        if (dot && alt && tb.twp_alt)
+            return go(std::true_type{}, k_fwd_x<T, N, FWD_SUMS, ALT>, PA::THREADS, PA::SMEM_DOT, tb.twp_alt);
     }
-    if (dot) {
-        PS_LTRY(set_smem(k_fwd_x<T, N, true>, PG::SMEM_DOT));
-        k_fwd_x<T, N, true><<<blocks, PG::THREADS, PG::SMEM_DOT, st>>>(
-            data, stride, hvalid, epi, out, ostride, dk, dks, ndk > 0 ? ndk : N, shells, nshell, lut, lut_size,
-            weight, quad, r2max, partials, tb.twp, mod_out, nc, jband);
-    } else {
-        PS_LTRY(set_smem(k_fwd_x<T, N, false>, PG::SMEM));
-        k_fwd_x<T, N, false><<<blocks, PG::THREADS, PG::SMEM, st>>>(
-            data, stride, hvalid, epi, out, ostride, dk, dks, ndk > 0 ? ndk : N, shells, nshell, lut, lut_size,
-            weight, quad, r2max, partials, tb.twp, mod_out, nc, jband);
-    }
-    if (nblocks) *nblocks = (int)blocks;
-    return PS_OK;
+    if (dot) return go(std::true_type{}, k_fwd_x<T, N, FWD_SUMS>, PG::THREADS, PG::SMEM_DOT, tb.twp);
+    return epi == SPEC_MASK_ADD ? go(std::false_type{}, k_fwd_x<T, N, FWD_MASK>, PG::THREADS, PG::SMEM, tb.twp)
+                                : go(std::false_type{}, k_fwd_x<T, N, FWD_STORE>, PG::THREADS, PG::SMEM, tb.twp);
 }
 
 }  // namespace ps

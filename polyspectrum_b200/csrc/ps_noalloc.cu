@@ -144,8 +144,12 @@ int run_noalloc(cudaStream_t st, unsigned char* base, double L, const float* fie
     // forward transform of the field (get_FT_field + optional phase normalisation)
     PS_LTRY((L3<float, N>::fwd_z(st, SRC_F32, field, nullptr, spec32, S32, N / 2 + 1, tb32)));
     PS_LTRY((L3<float, N>::pass_y(st, spec32, S32, false, tb32)));
-    PS_LTRY((L3<float, N>::fwd_x(st, spec32, S32, N / 2 + 1, phase == 1 ? SPEC_STORE_PHASE : SPEC_STORE,
-                                 spec32, S32, nullptr, 0, nullptr, 0, nullptr, 0, nullptr, tb32, nullptr)));
+    FwdXItem<float> it{};
+    it.data = spec32;
+    it.stride = it.ncols = S32;
+    it.hvalid = N / 2 + 1;
+    PS_LTRY((L3<float, N>::fwd_x(st, &it, 1, S32, phase == 1 ? SPEC_STORE_PHASE : SPEC_STORE, spec32, S32,
+                                 nullptr, 0, tb32, nullptr)));
     // all shells in one sweep over the spectrum (Parseval): sums of |dk|^2 in
     // FP64 and exact counts; per-shell inverse transforms (six passes and two
     // reductions each) took 1.45 ms for 32 shells at 64^3
