@@ -285,10 +285,11 @@ struct ps_gpu_ctx {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     // field lanes: the batches of pair groups of a plan split over two streams
     // (0 the main one, 1 lane2_stream), each with its own workspace (leg and
-    // product spectra, block sums), so the kernels of different batches overlap
+    // product spectra, block sums), so the kernels of different batches overlap;
+    // workspace 2 is the products' (prod_ops)
     cudaStream_t lane2_stream = nullptr;
-    unsigned char* lane_work[2] = {nullptr, nullptr};
-    size_t lane_work_cap[2] = {0, 0};  // bytes
+    unsigned char* lane_work[3] = {nullptr, nullptr, nullptr};
+    size_t lane_work_cap[3] = {0, 0, 0};  // bytes
     cudaEvent_t ev_join2 = nullptr;
     // memory of destroyed plans kept for the next ones (at most kSpareArenas)
     std::vector<PlanArena> spare_arenas;
@@ -296,8 +297,6 @@ struct ps_gpu_ctx {
     PrecBufs<double> d;
     double* partials = nullptr;
     size_t partials_cap = 0;
-    double* dsums = nullptr;  // device scalars
-    size_t dsums_cap = 0;
     Shell* dshells = nullptr;
     size_t dshells_cap = 0;
     unsigned long long* dminmax = nullptr;
@@ -559,16 +558,6 @@ int ensure_partials(ps_gpu_ctx* c, size_t n)
     c->partials_cap = n;
     return PS_OK;
 }
-int ensure_sums(ps_gpu_ctx* c, size_t n)
-{
-    if (n <= c->dsums_cap) return PS_OK;
-    if (c->dsums) c->retired.push_back(c->dsums);
-    c->dsums = nullptr;
-    c->dsums_cap = 0;
-    PS_TRY(alloc_dev(&c->dsums, n));
-    c->dsums_cap = n;
-    return PS_OK;
-}
 int ensure_shells(ps_gpu_ctx* c, size_t n)
 {
     if (n <= c->dshells_cap) return PS_OK;
@@ -773,7 +762,7 @@ int c2r_xy(ps_gpu_ctx* c, int mode, const Shell* dshell, int band, V2<T>* dst, i
     Tables<T> tb;
     PS_TRY(tables_for<T>(c, N, &tb));
     const int hb = std::min(band, N / 2) + 1;
-    const int S = round_up(hb, pw<T>(N));
+    const int S = round_up(quad ? (hb + 1) / 2 : hb, pw<T>(N));  // quad: two columns per element
     const double V = sizeof(V2<T>), NN2 = (double)N * N;
     {
         Prof pf(c);
@@ -832,14 +821,14 @@ int pair_spectrum(ps_gpu_ctx* c, const V2<T>* A, int Sa, int hba, const V2<T>* B
     const int N = M > 0 ? M : c->N;
     Tables<T> tb;
     PS_TRY(tables_for<T>(c, N, &tb));
-    const int S = round_up(hout, pw<T>(N));
+    const int S = round_up(quad ? (hout + 1) / 2 : hout, pw<T>(N));
     const double V = sizeof(V2<T>), NN2 = (double)N * N;
     const double q = quad ? (double)(N / 2 + 1) * (N / 2 + 1) / NN2 : 1.0;
     {
         Prof pf(c);
         PS_SWITCH_N(N, PS_TRY((L3<T, NN>::pair_z(c->stream, A, Sa, hba, Bq, Sb, hbb, B.work3, S, hout, tb, quad,
                                                  pair_var_of<T>(c, N)))));
-        pf.end(fam<T>(KF_PAIR_Z), q * NN2 * (hba + (Bq ? hbb : 0) + hout) * V, N);
+        pf.end(fam<T>(KF_PAIR_Z), q * NN2 * (hba + (Bq ? hbb : 0) + hout) * (quad ? V / 2 : V), N);
     }
     {
         Prof pf(c);
@@ -999,7 +988,7 @@ int dot_pass(ps_gpu_ctx* c, V2<T>* data, int epi, int S, int hvalid, const Shell
             PS_SWITCH_N(N, PS_TRY((L3<T, NN>::fwd_x(c->stream, &it, 1, S, epi, nullptr, 0, B.spec, B.S, tb, &nb,
                                                     quad, c->N, nullptr, NN, dot_alt_of<T>(c, N)))));
             const double q = quad ? (double)(N / 2 + 1) * (N / 2 + 1) / ((double)N * N) : 1.0;
-            pf.end(fam<T>(KF_FWD_X_DOT), q * N * N * hvalid * sizeof(V2<T>) * (epi == SPEC_DOT ? 2.0 : 1.0), N);
+            pf.end(fam<T>(KF_FWD_X_DOT), q * N * N * hvalid * sizeof(V2<T>) * (epi == SPEC_DOT ? 2.0 : quad ? 0.5 : 1.0), N);
         }
         PS_TRY(didx ? sum_partials(c, nb, cnt, dout, 1, didx + s0) : sum_partials(c, nb, cnt, dout + s0, 1));
     }
@@ -1262,69 +1251,7 @@ void remember_npoly(ps_gpu_ctx* c, int method, int nconf, const ps_cfg* in, cons
     for (int q = 0; q < nconf; q++) c->npoly_cache[npoly_key(method, in[q])] = Np[q];
 }
 
-int plain_batch(ps_gpu_ctx* c, int nconf, ps_cfg* cfgs, double* B, double* Np, double* kappa)
-{
-    if (!c->d.have_spec) return fail(PS_ERR_ARG, "FP64 spectrum not available (methods mask)");
-    std::vector<std::vector<Shell>> legs;
-    const int N = c->N;
-    PS_TRY(ensure_sums(c, 4 * (size_t)nconf + 8));
-    PS_TRY(ensure_shells(c, PS_MAX_LEGS));
-    std::vector<double> coef(nconf), habs(nconf, 0.0);
-    for (int q = 0; q < nconf; q++) {
-        PS_TRY(resolve_legs(c, 1, cfgs + q, legs));
-        PS_TRY(check_band(c, legs_band(legs[0], N)));
-        const int n = cfgs[q].n;
-        PS_CK(cudaMemcpyAsync(c->dshells, legs[0].data(), sizeof(Shell) * n, cudaMemcpyHostToDevice,
-                              c->stream));
-        double* sD = c->dsums + q;
-        double* sI = c->dsums + nconf + q;
-        for (int pass = 0; pass < 2; pass++) {  // 0: D = IFFT[F dk], 1: I = IFFT[F]
-            const int mode = pass == 0 ? LOAD_MASKED : LOAD_UNIT;
-            double* prod = pass == 0 ? c->d.ra : c->d.rb;
-            for (int l = 0; l < n; l++) {
-                const int epi = l == 0 ? EPI_STORE : (l < n - 1 ? EPI_MUL_STORE : EPI_MUL_REDUCE);
-                PS_TRY(c2r_shell<double>(c, mode, c->dshells + l, legs[0][l].band, prod, prod, epi, 1,
-                                         pass == 0 ? sD : sI));
-                if (kappa && pass == 0 && l == n - 1) {  // sum |prod D| for the condition number
-                    double* sA = c->dsums + 3 * nconf + q;
-                    PS_TRY(c2r_shell<double>(c, mode, c->dshells + l, legs[0][l].band, prod, prod,
-                                             EPI_MUL_REDUCE_ABS, 1, sA));
-                    PS_CK(cudaMemcpyAsync(&habs[q], sA, 8, cudaMemcpyDeviceToHost, c->stream));
-                }
-            }
-        }
-        coef[q] = norm_coef(c->L, N, n);
-        // the host shell table is rewritten by the next config: keep order
-        PS_CK(cudaStreamSynchronize(c->stream));
-    }
-    double* dcoef = c->dsums + 2 * nconf;
-    PS_CK(cudaMemcpyAsync(dcoef, coef.data(), sizeof(double) * nconf, cudaMemcpyHostToDevice, c->stream));
-    double* dout = nullptr;
-    PS_TRY(alloc_dev(&dout, 2 * (size_t)nconf));
-    const double inv_n3 = 1.0 / ((double)N * (double)N * (double)N);
-    {
-        Prof pf(c);
-        k_finalize<<<(nconf + 127) / 128, 128, 0, c->stream>>>(nconf, dcoef, c->dsums, c->dsums + nconf,
-                                                               inv_n3, 0, dout);
-        pf.end(KF_FINAL, 0.0);
-    }
-    std::vector<double> h(2 * nconf);
-    std::vector<double> hD(nconf);
-    cudaError_t e1 = cudaMemcpyAsync(h.data(), dout, sizeof(double) * 2 * nconf, cudaMemcpyDeviceToHost,
-                                     c->stream);
-    if (e1 == cudaSuccess && kappa)
-        e1 = cudaMemcpyAsync(hD.data(), c->dsums, sizeof(double) * nconf, cudaMemcpyDeviceToHost, c->stream);
-    cudaError_t e2 = cudaStreamSynchronize(c->stream);
-    cudaFree(dout);
-    PS_CK(e1);
-    PS_CK(e2);
-    for (int q = 0; q < nconf; q++) {
-        B[q] = h[2 * q];
-        Np[q] = h[2 * q + 1];
-        if (kappa) kappa[q] = habs[q] / fabs(hD[q]);
-    }
-    return PS_OK;
-}
+int plain_batch(ps_gpu_ctx* c, int nconf, ps_cfg* cfgs, double* B, double* Np, double* kappa);
 
 // =========================================================================
 // method 2: batched FP32 (FP64 counts)
@@ -1553,13 +1480,13 @@ struct LegKey {
 // keeps every mode of a shell on its own M-grid index.  N when none fits.
 const int kGridSizes[] = {16, 32, 64, 96, 128, 192, 256, 320, 384, 512, 1024};
 
-int alias_free_grid(int N, int ba, int bb, int bc)
+int alias_free_grid_n(int N, int bsum, int bmax)
 {
-    const int bmax = std::max({ba, bb, bc});
     for (int M : kGridSizes)
-        if (M < N && M > ba + bb + bc && M > 2 * bmax) return M;
+        if (M < N && M > bsum && M > 2 * bmax) return M;
     return N;
 }
+int alias_free_grid(int N, int ba, int bb, int bc) { return alias_free_grid_n(N, ba + bb + bc, std::max({ba, bb, bc})); }
 
 bool grid_supported(int M)
 {
@@ -1780,6 +1707,194 @@ int scatter_dev(ps_gpu_ctx* c, const double* src, const int* didx, int count, do
     Prof pf(c);
     k_scatter<<<(count + 127) / 128, 128, 0, c->stream>>>(src, didx, count, dst);
     pf.end(KF_SUM, 16.0 * count);
+    return PS_OK;
+}
+
+// =========================================================================
+// grid sums of products of n filtered fields
+// =========================================================================
+struct ProdCfg {
+    std::vector<std::pair<int, int>> f;  // (shell table index, power)
+    int out;                             // column of the results
+};
+
+// Bytes of one shell's inverse transform (X and Y passes) on the M-grid; unit:
+// the shell itself on the xy-quadrant.
+template <typename T> size_t prod_spectrum_bytes(const Shell& sh, int M, bool unit)
+{
+    const int hb = std::min(sh.band, M / 2) + 1;
+    const int S = round_up(unit ? (hb + 1) / 2 : hb, pw<T>(M));
+    const size_t rows = unit ? (size_t)(M / 2 + 1) * (M / 2 + 1) : (size_t)M * M;
+    return (rows * (size_t)S * sizeof(V2<T>) + 255) / 256 * 256;
+}
+
+// A configuration's legs must all be in memory at once; above this (two or more
+// full-band legs at 1024 points in FP64) they are taken one by one with the running
+// product on a real grid, which needs one spectrum however many legs there are.
+constexpr size_t kProdMost = (size_t)16 << 30;
+constexpr size_t kProdBatch = (size_t)64 << 20;  // spectra of a batch: they stay in L2
+
+// Launch sequence of the grid sums of `cfgs` on the M-grid, `scale` times each into
+// out[cfg.out] (and of the terms' absolute values into out_abs, if not NULL).  unit:
+// sums of products of the shells themselves (T double).  The distinct shells of a
+// batch of configurations are transformed along X and Y once, in one launch each;
+// k_prod_z does the rows, the product and the sum.
+template <typename T>
+int prod_ops(ps_gpu_ctx* c, const std::vector<Shell>& host, const Shell* dtable, const std::vector<ProdCfg>& cfgs, int M,
+             bool unit, double scale, double* out, double* out_abs, std::vector<std::function<int()>>* ops)
+{
+    struct Batch {
+        std::vector<int> shells;
+        std::vector<size_t> at;  // offsets of their spectra
+        std::vector<const ProdCfg*> cfgs;
+        size_t bytes = 0;
+    };
+    std::vector<Batch> batches;
+    for (const ProdCfg& g : cfgs) {
+        size_t more = 0;
+        std::vector<int> add;
+        const auto missing = [&](const Batch* b) {
+            more = 0;
+            add.clear();
+            for (const auto& f : g.f)
+                if ((!b || std::find(b->shells.begin(), b->shells.end(), f.first) == b->shells.end()) &&
+                    std::find(add.begin(), add.end(), f.first) == add.end()) {
+                    add.push_back(f.first);
+                    more += prod_spectrum_bytes<T>(host[f.first], M, unit);
+                }
+        };
+        missing(batches.empty() ? nullptr : &batches.back());
+        if (batches.empty() || batches.back().bytes + more > kProdBatch) {
+            batches.emplace_back();
+            missing(nullptr);
+        }
+        Batch& b = batches.back();
+        for (int sidx : add) {
+            b.shells.push_back(sidx);
+            b.at.push_back(b.bytes);
+            b.bytes += prod_spectrum_bytes<T>(host[sidx], M, unit);
+        }
+        b.cfgs.push_back(&g);
+    }
+    int most = 0;  // partial sums of a product
+    {
+        const int N = M;
+        PS_SWITCH_N(N, (most = L3<T, NN>::prod_blocks(unit)));
+    }
+    size_t spectra = 0;
+    for (const Batch& b : batches) spectra = std::max(spectra, b.bytes);
+    PS_TRY(ensure_lane_work(c, 2, spectra + sizeof(double) * (size_t)most * kItems));
+    Tables<T> tb;
+    PS_TRY(tables_for<T>(c, M, &tb));
+    unsigned char* base = c->lane_work[2];
+    double* partials = (double*)(base + spectra);
+    for (const Batch& b : batches) {
+        std::vector<XItem<T>> xi;
+        std::vector<YItem<T>> yi;
+        std::map<int, std::pair<V2<T>*, std::pair<int, int>>> where;  // shell -> spectrum, stride, columns
+        int Smax = 0;
+        const double V = sizeof(V2<T>), rows = unit ? (double)(M / 2 + 1) * (M / 2 + 1) : (double)M * M;
+        double bx = 0.0, by = 0.0, bz = 0.0;
+        for (size_t q = 0; q < b.shells.size(); q++) {
+            const Shell& sh = host[b.shells[q]];
+            const int band = std::min(sh.band, M / 2), hb = band + 1, S = round_up(unit ? (hb + 1) / 2 : hb, pw<T>(M));
+            V2<T>* dst = (V2<T>*)(base + b.at[q]);
+            xi.push_back(XItem<T>{dst, S, M / 2 + 1, dtable + b.shells[q]});
+            yi.push_back(YItem<T>{dst, S, S, band, M});
+            where[b.shells[q]] = {dst, {S, hb}};
+            Smax = std::max(Smax, S);
+            bx += rows * S * V + (unit ? 0.0 : rows * hb * V);
+            by += 2.0 * rows * S * V;
+        }
+        std::vector<ProdItem<T>> pi;
+        std::vector<int> cols;
+        int hv = 1;
+        for (const ProdCfg* g : b.cfgs) {
+            ProdItem<T> it{};
+            it.nf = (int)g->f.size();
+            for (int f = 0; f < it.nf; f++) {
+                const auto& w = where[g->f[f].first];
+                it.src[f] = w.first;
+                it.stride[f] = w.second.first;
+                it.hv[f] = (short)w.second.second;
+                it.power[f] = (short)g->f[f].second;
+                hv = std::max(hv, w.second.second);
+                bz += rows * w.second.second * (unit ? V / 2 : V);
+            }
+            pi.push_back(it);
+            cols.push_back(g->out);
+        }
+        const int nx = (int)xi.size(), np = (int)pi.size();
+        ops->push_back([=]() -> int {
+            const int N = M;  // PS_SWITCH_N's subject
+            const int quad = unit ? 1 : 0, mode = unit ? LOAD_UNIT : LOAD_MASKED;
+            const PrecBufs<T>& F = bufs<T>(c);
+            for (int q = 0; q < nx; q += kItems) {
+                const int n = std::min(kItems, nx - q);
+                Prof pf(c);
+                PS_SWITCH_N(N, PS_TRY((L3<T, NN>::inv_x_b(c->stream, F.spec, F.S, xi.data() + q, n, Smax, mode, tb, quad,
+                                                          c->N, 1))));
+                pf.end(fam<T>(KF_INV_X), bx * n / nx, M);
+            }
+            for (int q = 0; q < nx; q += kItems) {
+                const int n = std::min(kItems, nx - q);
+                Prof pf(c);
+                PS_SWITCH_N(N, PS_TRY((L3<T, NN>::pass_y_b(c->stream, yi.data() + q, n, Smax, true, tb, quad,
+                                                           pencil_alt_of<T>(c, M)))));
+                pf.end(fam<T>(KF_PASS_Y), by * n / nx, M);
+            }
+            for (int q = 0; q < np; q += kItems) {
+                const int n = std::min(kItems, np - q);
+                for (int ab = 0; ab < (out_abs ? 2 : 1); ab++) {
+                    Items<SumItem> si{};
+                    std::vector<ProdItem<T>> part(pi.begin() + q, pi.begin() + q + n);
+                    for (int x = 0; x < n; x++) part[x].partials = partials + (size_t)x * most;
+                    int nblk = 0;
+                    {
+                        Prof pf(c);
+                        PS_SWITCH_N(N, PS_TRY((L3<T, NN>::prod_z(c->stream, part.data(), n, hv, unit, ab, tb, &nblk))));
+                        pf.end(fam<T>(KF_INV_Z), bz * n / np, M);
+                    }
+                    for (int x = 0; x < n; x++)
+                        si.at[x] = SumItem{partials + (size_t)x * most, nblk, 1, scale, (ab ? out_abs : out) + cols[q + x],
+                                           nullptr};
+                    Prof pf(c);
+                    k_sum_items<<<dim3(1, n), 256, 0, c->stream>>>(si);
+                    pf.end(KF_SUM, 8.0 * nblk * n);
+                }
+            }
+            PS_CK(launch_status());
+            return PS_OK;
+        });
+    }
+    return PS_OK;
+}
+
+// Whether a product's legs fit (kProdMost).
+template <typename T> bool prod_fits(const std::vector<Shell>& host, const ProdCfg& g, int M, bool unit)
+{
+    size_t sum = 0;
+    for (const auto& f : g.f) sum += prod_spectrum_bytes<T>(host[f.first], M, unit);
+    return sum <= kProdMost;
+}
+
+// Sum of a product whose legs are transformed one by one, the running product on a
+// real grid (configurations above kProdMost).
+template <typename T>
+int legwise_sum(ps_gpu_ctx* c, const std::vector<Shell>& host, const Shell* dtable, const ProdCfg& g, double* out,
+                double* out_abs)
+{
+    PrecBufs<T>& F = bufs<T>(c);
+    const int r = (int)g.f.size();
+    for (int x = 0; x < r; x++) {
+        const int epi = r == 1 ? EPI_REDUCE : (x == 0 ? EPI_STORE : (x < r - 1 ? EPI_MUL_STORE : EPI_MUL_REDUCE));
+        const Shell* sh = dtable + g.f[x].first;
+        const int band = host[g.f[x].first].band, power = g.f[x].second;
+        PS_TRY(c2r_shell<T>(c, LOAD_MASKED, sh, band, F.ra, F.ra, epi, power, out));
+        if (out_abs && x == r - 1)
+            PS_TRY(c2r_shell<T>(c, LOAD_MASKED, sh, band, F.ra, F.ra, r == 1 ? EPI_REDUCE_ABS : EPI_MUL_REDUCE_ABS, power,
+                                out_abs));
+    }
     return PS_OK;
 }
 
@@ -2169,7 +2284,7 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
     };
     // The lane's workspace holds the block sums of all its batches first (from
     // sums_at on those of this one), then the spectra of the batch at work.
-    std::vector<FwdXItem<float>> sums, sums_abs;  // every dot pass of the plan, for the final sums
+    std::vector<SumItem> sums;  // every dot pass of the plan, for the final sums
     auto batch_op = [&](const std::vector<size_t>& gs, int M, int lane, size_t sums_at, size_t spectra_at,
                         std::function<int()>* op) -> int {
         const int w = pw<float>(M);
@@ -2239,25 +2354,18 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
                 it.interval = interval && it.nshell <= 2;
                 it.r2max = (int)std::min<long long>(r2max, 0x7fffffff);
                 it.weight = wD;
-                it.nblk = M * (Sp / w);
-                it.idx = didx + gidx_ofs[g] + s0;
-                it.partials = part;
-                it.out = sumD;
-                part += (size_t)it.nblk * it.nshell;
-                fx.push_back(it);
-                if (kappa) {
+                const int nblk = M * (Sp / w);
+                for (int ab = 0; ab < (kappa ? 2 : 1); ab++) {
                     it.partials = part;
-                    it.out = sumA;
-                    part += (size_t)it.nblk * it.nshell;
-                    fa.push_back(it);
+                    part += (size_t)nblk * it.nshell;
+                    (ab ? fa : fx).push_back(it);
+                    sums.push_back(SumItem{it.partials, nblk, it.nshell, 1.0, ab ? sumA : sumD, didx + gidx_ofs[g] + s0});
                 }
                 bd += NN2 * hout * V * 2.0;
             }
         }
         Tables<float> tb;
         PS_TRY(tables_for<float>(c, M, &tb));
-        sums.insert(sums.end(), fx.begin(), fx.end());
-        sums_abs.insert(sums_abs.end(), fa.begin(), fa.end());
         const int nx = (int)xi.size(), ngr = (int)gs.size(), nf = (int)fx.size();
         *op = [=]() -> int {
             const int N = M;  // PS_SWITCH_N's subject
@@ -2459,7 +2567,6 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
             if (need[l]) PS_TRY(ensure_lane_work(c, l, nsums[l] + need[l]));
         }
         sums.clear();  // of the tuning's candidates
-        sums_abs.clear();
         for (size_t q = 0; q < batches.size(); q++) {
             std::function<int()> op;
             const bool second = lane[q] == 1;
@@ -2470,15 +2577,14 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
                 return op();
             });
         }
-        sums.insert(sums.end(), sums_abs.begin(), sums_abs.end());
         for (size_t q0 = 0; q0 < sums.size(); q0 += kItems) {
             const int n = (int)std::min<size_t>(kItems, sums.size() - q0);
             const auto items = pack(sums.data() + q0, n);
             double bytes = 0.0;
-            for (int q = 0; q < n; q++) bytes += 8.0 * items.at[q].nblk * items.at[q].nshell;
+            for (int q = 0; q < n; q++) bytes += 8.0 * items.at[q].nblk * items.at[q].ncol;
             P->ops_tail.push_back([=]() {
                 Prof pf(c);
-                k_sum_items<float><<<dim3(MAX_DOT_SHELLS, n), 256, 0, c->stream>>>(items);
+                k_sum_items<<<dim3(MAX_DOT_SHELLS, n), 256, 0, c->stream>>>(items);
                 pf.end(KF_SUM, bytes);
                 PS_CK(launch_status());
                 return PS_OK;
@@ -2627,38 +2733,44 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
             return PS_OK;
         });
     }
-    // ---- leg by leg (singletons, n > 3): running products with powers
-    for (int q : direct) {
-        std::vector<std::pair<int, int>> up;  // (shell, multiplicity)
-        for (int sidx : lid[q]) {
-            bool found = false;
-            for (auto& pr : up)
-                if (pr.first == sidx) { pr.second++; found = true; }
-            if (!found) up.push_back({sidx, 1});
-        }
-        std::vector<int> bands;
-        for (auto& pr : up) bands.push_back(host_shell_of(pr.first).band);
-        tail.push_back([=]() {
-            const int r = (int)up.size();
-            for (int pass = 0; pass < 2; pass++)
-                for (int x = 0; x < r; x++) {
-                    const int epi = r == 1 ? EPI_REDUCE : (x == 0 ? EPI_STORE : (x < r - 1 ? EPI_MUL_STORE : EPI_MUL_REDUCE));
-                    if (pass == 0) {
-                        PS_TRY(c2r_shell<float>(c, LOAD_MASKED, dtable + up[x].first, bands[x], c->f.ra, c->f.ra, epi,
-                                                up[x].second, sumD + q));
-                        if (kappa && x == r - 1)
-                            PS_TRY(c2r_shell<float>(c, LOAD_MASKED, dtable + up[x].first, bands[x], c->f.ra, c->f.ra,
-                                                    r == 1 ? EPI_REDUCE_ABS : EPI_MUL_REDUCE_ABS, up[x].second,
-                                                    sumA + q));
-                    } else {
-                        PS_TRY(c2r_shell<double>(c, LOAD_UNIT, dtable + up[x].first, bands[x], c->d.ra, c->d.ra, epi,
-                                                 up[x].second, sumI + q));
-                    }
-                }
-            return PS_OK;
-        });
-    }
+    // ---- n > 3: grid sums of products on the smallest grid that holds the polygons
+    // without wrap-around (b_1 + ... + b_n < M and 2 max b < M, as for pairs)
     if (!direct.empty()) {
+        std::map<int, std::vector<ProdCfg>> by_size;
+        std::vector<ProdCfg> large;
+        for (int q : direct) {
+            ProdCfg g;
+            g.out = q;
+            int total = 0, bmax = 0;
+            for (int sidx : lid[q]) {
+                const int b = std::min(host_shell_of(sidx).band, N / 2);
+                total += b;
+                bmax = std::max(bmax, b);
+                bool found = false;
+                for (auto& f : g.f)
+                    if (f.first == sidx) {
+                        f.second++;
+                        found = true;
+                    }
+                if (!found) g.f.push_back({sidx, 1});
+            }
+            const int M = alias_free_grid_n(N, total, bmax);
+            (prod_fits<float>(table, g, M, false) ? by_size[M] : large).push_back(g);
+        }
+        for (const auto& kv : by_size) {
+            const double up = ((double)N / kv.first) * ((double)N / kv.first) * ((double)N / kv.first);
+            PS_TRY(prod_ops<float>(c, table, dtable, kv.second, kv.first, false, up, sumD, kappa ? sumA : nullptr, &tail));
+            PS_TRY(prod_ops<double>(c, table, dtable, kv.second, kv.first, true, up, sumI, nullptr, &tail));
+        }
+        if (!large.empty()) {
+            PS_TRY(prod_ops<double>(c, table, dtable, large, N, true, 1.0, sumI, nullptr, &tail));
+            const std::vector<Shell> host = table;
+            tail.push_back([=]() {
+                for (const ProdCfg& g : large)
+                    PS_TRY(legwise_sum<float>(c, host, dtable, g, sumD + g.out, kappa ? sumA + g.out : nullptr));
+                return PS_OK;
+            });
+        }
         const int nr = (int)direct.size();
         tail.push_back([=]() {
             Prof pf(c);
@@ -2956,6 +3068,86 @@ int plan_prepare(ps_gpu_ctx* c, ps_gpu_plan* P)
     PS_CK(cudaEventRecord(P->ev_counts, c->stream));
     P->prepared = true;
     return PS_OK;
+}
+
+// PS_FP64_PLAIN: every configuration's grid sums on the full grid in FP64, products
+// of its n filtered fields and of its n shells, reference normalisation.
+int plain_batch(ps_gpu_ctx* c, int nconf, ps_cfg* cfgs, double* B, double* Np, double* kappa)
+{
+    if (!c->d.have_spec) return fail(PS_ERR_ARG, "FP64 spectrum not available (methods mask)");
+    const int N = c->N;
+    std::vector<std::vector<Shell>> legs;
+    PS_TRY(resolve_legs(c, nconf, cfgs, legs));
+    std::vector<Shell> table;
+    std::vector<ProdCfg> prods(nconf);
+    std::vector<double> coef(nconf);
+    for (int q = 0; q < nconf; q++) {
+        PS_TRY(check_band(c, legs_band(legs[q], N)));
+        prods[q].out = q;
+        for (const Shell& sh : legs[q]) {
+            int id = -1;
+            for (size_t u = 0; u < table.size() && id < 0; u++)
+                if (same_shell(table[u], sh)) id = (int)u;
+            if (id < 0) {
+                id = (int)table.size();
+                table.push_back(sh);
+            }
+            bool found = false;
+            for (auto& f : prods[q].f)
+                if (f.first == id) {
+                    f.second++;
+                    found = true;
+                }
+            if (!found) prods[q].f.push_back({id, 1});
+        }
+        coef[q] = norm_coef(c->L, N, cfgs[q].n);
+    }
+    ps_gpu_plan tmp;  // its arenas hold the call's tables
+    tmp.ctx = c;
+    const double inv_n3 = 1.0 / ((double)N * (double)N * (double)N);
+    const auto run = [&]() -> int {
+        Shell* dtable = nullptr;
+        double *dcoef = nullptr, *sums = nullptr, *dout = nullptr;
+        PS_TRY(plan_upload(&tmp, &dtable, table));
+        PS_TRY(plan_upload(&tmp, &dcoef, coef));
+        PS_TRY(plan_alloc(&tmp, &sums, 3 * (size_t)nconf));
+        PS_TRY(plan_alloc(&tmp, &dout, 2 * (size_t)nconf));
+        void *dh = nullptr, *hh = nullptr;
+        PS_TRY(arena_take(&tmp, sizeof(double) * 4 * (size_t)nconf, &dh, &hh));
+        double* h = (double*)hh;  // B, Npoly | sum D | sum |D|
+        PS_TRY(plan_flush(&tmp));
+        double *sD = sums, *sI = sums + nconf, *sA = sums + 2 * (size_t)nconf;
+        std::vector<ProdCfg> fit, large;
+        for (const ProdCfg& g : prods) (prod_fits<double>(table, g, N, false) ? fit : large).push_back(g);
+        std::vector<std::function<int()>> ops;
+        if (!fit.empty()) PS_TRY(prod_ops<double>(c, table, dtable, fit, N, false, 1.0, sD, kappa ? sA : nullptr, &ops));
+        PS_TRY(enqueue_ops(ops));
+        ops.clear();
+        PS_TRY(prod_ops<double>(c, table, dtable, prods, N, true, 1.0, sI, nullptr, &ops));
+        PS_TRY(enqueue_ops(ops));
+        for (const ProdCfg& g : large) PS_TRY(legwise_sum<double>(c, table, dtable, g, sD + g.out, kappa ? sA + g.out : nullptr));
+        {
+            Prof pf(c);
+            k_finalize<<<(nconf + 127) / 128, 128, 0, c->stream>>>(nconf, dcoef, sD, sI, inv_n3, 0, dout);
+            pf.end(KF_FINAL, 0.0);
+        }
+        PS_CK(launch_status());
+        PS_CK(cudaMemcpyAsync(h, dout, sizeof(double) * 2 * nconf, cudaMemcpyDeviceToHost, c->stream));
+        if (kappa) {
+            PS_CK(cudaMemcpyAsync(h + 2 * (size_t)nconf, sD, sizeof(double) * nconf, cudaMemcpyDeviceToHost, c->stream));
+            PS_CK(cudaMemcpyAsync(h + 3 * (size_t)nconf, sA, sizeof(double) * nconf, cudaMemcpyDeviceToHost, c->stream));
+        }
+        PS_CK(cudaStreamSynchronize(c->stream));
+        for (int q = 0; q < nconf; q++) {
+            B[q] = h[2 * q];
+            Np[q] = h[2 * q + 1];
+            if (kappa) kappa[q] = h[3 * (size_t)nconf + q] / fabs(h[2 * (size_t)nconf + q]);
+        }
+        return PS_OK;
+    };
+    const int rc = run();
+    plan_release(&tmp, true);
+    return rc;
 }
 
 int batched(ps_gpu_ctx* c, int nconf, ps_cfg* cfgs, double* B, double* Np, double* kappa)
@@ -4097,7 +4289,6 @@ void ps_gpu_finalize(ps_gpu_ctx* c)
     free_prec(c->d);
     cudaFree(c->partials);
     cudaFree(c->dstatus);
-    cudaFree(c->dsums);
     cudaFree(c->dshells);
     cudaFree(c->dminmax);
     cudaFree(c->dlut);

@@ -18,6 +18,12 @@
 //   fwd_x  : along i; epilogue stores the spectrum (optionally phase only) or
 //            folds it into per-shell dot products
 //
+// Unit shells (polygon counts) are even in every axis, so their transforms are
+// real and even too and are kept on the xy-quadrant i, j <= N/2 as real numbers
+// ("quad" below, FP64): a row of the quadrant spectrum holds columns 2p and
+// 2p + 1 as the two lanes of complex element p, and one complex transform along x
+// or y of the pair is the transform of both columns, each staying in its lane.
+//
 // Every kernel stages the twiddle table W_N^m (m < N) in shared memory first;
 // row kernels synchronise per row (warp or named barrier), pencil kernels per
 // CTA (a pencil's threads span several warps).
@@ -239,13 +245,10 @@ template <typename T> struct FwdXItem {  // forward X
     int r2max;                  // no shell holds a mode with |m|^2 > r2max
     double weight;
     double* partials;           // [nshell][blocks]
-    double* out;                // k_sum_items: the sum of column c lands at out[idx[c]]
-    const int* idx;
-    int nblk;                   // k_sum_items: blocks of this item
 };
 
 // ------------------------------------------------------------------ inverse X
-enum InvLoad : int { LOAD_PLAIN = 0, LOAD_MASKED = 1, LOAD_UNIT = 2 };
+enum InvLoad : int { LOAD_PLAIN = 0, LOAD_MASKED = 1, LOAD_UNIT = 2 };  // LOAD_UNIT: quad only
 
 template <typename T, int N>
 __global__ void __launch_bounds__(PencilGeom<T, N>::THREADS)
@@ -272,7 +275,8 @@ __global__ void __launch_bounds__(PencilGeom<T, N>::THREADS)
     SmemInterleaved<V, G::W> sm{reinterpret_cast<V*>(smem_raw + G::TW_BYTES), (int)(threadIdx.x % G::W)};
     const int w = threadIdx.x % G::W, t = threadIdx.x / G::W;
     // quad: pencils j <= N/2 only, outputs i <= N/2 only, stored [i][j][h] with
-    // N/2+1 rows per plane (the unit filter is even in every axis).
+    // N/2+1 rows per plane; column element h holds the unit filter's columns 2h
+    // and 2h + 1.
     // nsrc: grid size of the source spectrum ([nsrc][nsrc][src_stride]); a mode
     // m of this N-grid is read at index m mod nsrc there (nsrc >= N, and the
     // shell's band is below N/2, so every selected mode has one home in both).
@@ -286,7 +290,7 @@ __global__ void __launch_bounds__(PencilGeom<T, N>::THREADS)
     Shell sh;
     if (mode != LOAD_PLAIN) sh = *shell_p;
     const bool pencil_live =
-        col_ok && (mode == LOAD_PLAIN || (abs(my) <= sh.band && abs(mz) <= sh.band));
+        !quad && col_ok && (mode == LOAD_PLAIN || (abs(my) <= sh.band && abs(mz) <= sh.band));
     // filter bits of this thread's R modes, one predicate instance (loop not unrolled)
     unsigned bits = 0u;
     if (pencil_live) {
@@ -304,13 +308,33 @@ __global__ void __launch_bounds__(PencilGeom<T, N>::THREADS)
         }
     }
     V a[G::R];
+    if constexpr (sizeof(T) == 8) {
+        if (quad) {
+#pragma unroll
+            for (int e = 0; e < G::R; e++) a[e] = czero<V>();
+            for (int lane = 0; lane < 2; lane++) {
+                const int hz = 2 * h + lane, mzq = hz == N / 2 ? -(N / 2) : hz;
+                if (hz > N / 2 || hz >= hvalid || abs(my) > sh.band || abs(mzq) > sh.band) continue;
+                unsigned in = 0u;
+#pragma unroll 1
+                for (int e = 0; e < G::R; e++) {
+                    if (!G::live(t + G::TPF * e)) continue;
+                    const int mx = lattice_freq(t + G::TPF * e, N);
+                    if (abs(mx) <= sh.band && shell_bit(sh, mx, my, mzq)) in |= 1u << e;
+                }
+#pragma unroll
+                for (int e = 0; e < G::R; e++)
+                    if ((in >> e) & 1u) (lane ? a[e].y : a[e].x) = (T)1;
+            }
+        }
+    }
 #pragma unroll
     for (int e = 0; e < G::R; e++) {
+        if (sizeof(T) == 8 && quad) break;
         const int mx = lattice_freq(t + G::TPF * e, N);
         V v = czero<V>();
         if ((bits >> e) & 1u) {
-            if (mode == LOAD_UNIT) v = V{(T)1, (T)0};
-            else v = src[((size_t)(mx < 0 ? mx + nsrc : mx) * nsrc + js) * src_stride + h];
+            v = src[((size_t)(mx < 0 ? mx + nsrc : mx) * nsrc + js) * src_stride + h];
         }
         a[e] = v;
     }
@@ -423,10 +447,36 @@ __device__ __forceinline__ void c2r_row(const V2<T>* zr, int hv, RowCtx<T, N, RX
     rc.sync();
 }
 
-// r2c of a real row held in registers (canonical pairs), writing h < hout.
+// The same of a real spectrum row (quad layout: the transform of an even row).
 template <typename T, int N, int RX = 0>
-__device__ __forceinline__ void r2c_row(V2<T> (&a)[RowGeom<T, N, RX>::R], RowCtx<T, N, RX>& rc, V2<T>* __restrict__ xo,
-                                        int hout)
+__device__ __forceinline__ void c2r_row_real(const T* zr, int hv, RowCtx<T, N, RX>& rc,
+                                             V2<T> (&a)[RowGeom<T, N, RX>::R])
+{
+    using G = RowGeom<T, N, RX>;
+    using V = V2<T>;
+    constexpr int NH = G::NH;
+#pragma unroll
+    for (int e = 0; e < G::R; e++) {
+        const int k = rc.t + G::TPF * e;
+        if (!G::live(k)) {
+            a[e] = czero<V>();
+            continue;
+        }
+        const T zk = k < hv ? zr[k] : (T)0, zm = (NH - k) < hv ? zr[NH - k] : (T)0;
+        const T A = zk + zm, D = zk - zm;
+        const V w = rc.twpp[k];  // B = D conj(w)
+        a[e] = V{A + D * w.y, D * w.x};
+    }
+    SmemRow<V> sm{rc.rowbuf};
+    fft_any<V, NH, G::R, G::TPF, true>(a, rc.t, sm, rc.twr, rc.sync);
+    rc.sync();
+}
+
+// r2c of a real row held in registers (canonical pairs), writing h < hout (REAL:
+// the real parts only, for even rows).
+template <typename T, int N, int RX = 0, bool REAL = false>
+__device__ __forceinline__ void r2c_row(V2<T> (&a)[RowGeom<T, N, RX>::R], RowCtx<T, N, RX>& rc,
+                                        std::conditional_t<REAL, T, V2<T>>* __restrict__ xo, int hout)
 {
     using G = RowGeom<T, N, RX>;
     using V = V2<T>;
@@ -445,8 +495,12 @@ __device__ __forceinline__ void r2c_row(V2<T> (&a)[RowGeom<T, N, RX>::R], RowCtx
         const V E = V{(yk.x + ym.x) * half, (yk.y + ym.y) * half};
         const V D = csub(yk, ym);
         const V O = V{D.y * half, -D.x * half};  // D / (2i)
-        xo[k] = cadd(E, cmul(rc.twpp[k], O));
+        const V X = cadd(E, cmul(rc.twpp[k], O));
+        if constexpr (REAL) xo[k] = X.x;
+        else xo[k] = X;
     }
+    // the partner lane of an odd last column: the complex passes mix lanes that are not real and even
+    if (REAL && (hout & 1) && rc.t == 0) reinterpret_cast<T*>(xo)[hout] = (T)0;
     rc.sync();
 }
 
@@ -751,7 +805,9 @@ template <typename T, int N> struct PairVariants {
     static constexpr int ALT_RX = REG && (N / 2) % RX2 == 0 && (N / 2) / RX2 >= 4 ? RX2 : 0;
 };
 
-template <typename T, int N, int RX = 0, bool KEEP = false>
+//   REAL : rows of the quad layout (real spectra, two columns per element;
+//          hva, hvb, hout count columns)
+template <typename T, int N, int RX = 0, bool KEEP = false, bool REAL = false>
 __global__ void __launch_bounds__(RowGeom<T, N, RX>::THREADS)
     k_pair_z(const __grid_constant__ Items<PairItem<T>> items, int nrows,
              const V2<T>* __restrict__ twr_g, const V2<T>* __restrict__ twpp_g)
@@ -763,8 +819,14 @@ __global__ void __launch_bounds__(RowGeom<T, N, RX>::THREADS)
     const V* __restrict__ srcA = it.A;
     const V* __restrict__ srcB = it.B;
     V* __restrict__ dst = it.dst;
-    const int sa = it.sa, hva = it.hva, sb = it.sb, hvb = it.hvb, ds = it.ds, hout = it.hout;
+    const int sa = it.sa, sb = it.sb, ds = it.ds, hout = it.hout;
     RowCtx<T, N, RX> rc(smem_raw, twr_g, twpp_g);
+    // elements of a staged row
+    const int hva = REAL ? (it.hva + 1) / 2 : it.hva, hvb = REAL ? (it.hvb + 1) / 2 : it.hvb;
+    auto c2r = [&](const V* z, int hv, V(&x)[G::R]) {
+        if constexpr (REAL) c2r_row_real<T, N, RX>(reinterpret_cast<const T*>(z), hv, rc, x);
+        else c2r_row<T, N, RX>(z, hv, rc, x);
+    };
     const bool two = srcB != nullptr;
     const int PA = G::pitch(hva), PB = two ? G::pitch(hvb) : 0;
     V* stA = reinterpret_cast<V*>(smem_raw + G::STAGE_OFF);
@@ -795,13 +857,13 @@ __global__ void __launch_bounds__(RowGeom<T, N, RX>::THREADS)
             continue;
         }
         V a[G::R];
-        c2r_row<T, N, RX>(stA + st * G::WZ * PA + rc.w * PA, hva, rc, a);
+        c2r(stA + st * G::WZ * PA + rc.w * PA, it.hva, a);
         if (two) {
             if constexpr (KEEP) {
 #pragma unroll
                 for (int e = 0; e < G::R; e++)
                     if (G::live(rc.t + G::TPF * e)) keep[rc.t + G::TPF * e] = a[e];
-                c2r_row<T, N, RX>(stB + st * G::WZ * PB + rc.w * PB, hvb, rc, a);
+                c2r(stB + st * G::WZ * PB + rc.w * PB, it.hvb, a);
 #pragma unroll
                 for (int e = 0; e < G::R; e++) {
                     const V q = G::live(rc.t + G::TPF * e) ? keep[rc.t + G::TPF * e] : czero<V>();
@@ -809,7 +871,7 @@ __global__ void __launch_bounds__(RowGeom<T, N, RX>::THREADS)
                 }
             } else {
                 V b[G::R];
-                c2r_row<T, N, RX>(stB + st * G::WZ * PB + rc.w * PB, hvb, rc, b);
+                c2r(stB + st * G::WZ * PB + rc.w * PB, it.hvb, b);
 #pragma unroll
                 for (int e = 0; e < G::R; e++) a[e] = V{a[e].x * b[e].x, a[e].y * b[e].y};
             }
@@ -818,9 +880,92 @@ __global__ void __launch_bounds__(RowGeom<T, N, RX>::THREADS)
             for (int e = 0; e < G::R; e++) a[e] = V{a[e].x * a[e].x, a[e].y * a[e].y};
         }
         // the products sit in canonical layout as (x[2n], x[2n+1]): r2c input as is
-        r2c_row<T, N, RX>(a, rc, dst + row * ds, hout);
+        if constexpr (REAL) r2c_row<T, N, RX, true>(a, rc, reinterpret_cast<T*>(dst + row * ds), hout);
+        else r2c_row<T, N, RX>(a, rc, dst + row * ds, hout);
         __syncthreads();
     }
+}
+
+// ------------------------------------------------------------------ products of n fields
+// Grid sums of prod_f x_f^p_f over the rows of up to kMaxFactors inverse
+// transforms: every row's factors are brought back to real space one after the
+// other and multiplied in registers, so no real field is stored or read (three
+// legs as separate passes moved 6 N^3 values beside the spectra).  Persistent and
+// double-buffered over the (row tile, factor) sequence.  REAL: quad rows, weighted
+// by the points each stands for.
+constexpr int kMaxFactors = 8;
+template <typename T> struct ProdItem {
+    const V2<T>* src[kMaxFactors];
+    int stride[kMaxFactors];
+    short hv[kMaxFactors];     // columns
+    short power[kMaxFactors];
+    int nf;
+    double* partials;          // one per block
+};
+template <typename T, int N, bool REAL>
+__global__ void __launch_bounds__(RowGeom<T, N>::THREADS)
+    k_prod_z(const __grid_constant__ Items<ProdItem<T>> items, int P, int abs_terms, const V2<T>* __restrict__ twr_g,
+             const V2<T>* __restrict__ twpp_g)
+{
+    using G = RowGeom<T, N>;
+    using V = V2<T>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ double red[(G::THREADS + 31) / 32];
+    const ProdItem<T>& it = item_at(items);
+    RowCtx<T, N> rc(smem_raw, twr_g, twpp_g);
+    V* stage = reinterpret_cast<V*>(smem_raw + G::STAGE_OFF);  // two tiles of pitch P
+    constexpr int NQ = N / 2 + 1;
+    constexpr int nrows = REAL ? NQ * NQ : N * N, ntiles = (nrows + G::WZ - 1) / G::WZ;
+    const int nf = it.nf;
+    auto fetch = [&](int tile, int f, int buf) {
+        if (tile < ntiles)
+            stage_rows<V, G::WZ, G::THREADS>(stage + buf * G::WZ * P, P, it.src[f], (size_t)tile * G::WZ, it.stride[f],
+                                             REAL ? (it.hv[f] + 1) / 2 : it.hv[f], nrows);
+        cp_async_commit();
+    };
+    int buf = 0;
+    fetch(blockIdx.x, 0, 0);
+    double acc = 0.0;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int row = tile * G::WZ + rc.w;
+        const bool live = row < nrows;
+        V prod[G::R];
+        for (int f = 0; f < nf; f++, buf ^= 1) {
+            const bool last = f + 1 == nf;
+            fetch(last ? tile + gridDim.x : tile, last ? 0 : f + 1, buf ^ 1);
+            cp_async_wait_prev();
+            __syncthreads();
+            if (live) {  // whole row groups
+                V a[G::R];
+                const V* z = stage + buf * G::WZ * P + rc.w * P;
+                if constexpr (REAL) c2r_row_real<T, N>(reinterpret_cast<const T*>(z), it.hv[f], rc, a);
+                else c2r_row<T, N>(z, it.hv[f], rc, a);
+                const int p = it.power[f];
+                double s = 0.0;
+#pragma unroll
+                for (int e = 0; e < G::R; e++) {
+                    const T x0 = ipow(a[e].x, p), x1 = ipow(a[e].y, p);
+                    if (!last) {
+                        prod[e] = f == 0 ? V{x0, x1} : V{prod[e].x * x0, prod[e].y * x1};
+                    } else if (G::live(rc.t + G::TPF * e)) {
+                        const double y0 = f == 0 ? (double)x0 : (double)prod[e].x * (double)x0;
+                        const double y1 = f == 0 ? (double)x1 : (double)prod[e].y * (double)x1;
+                        s += abs_terms ? fabs(y0) + fabs(y1) : y0 + y1;
+                    }
+                }
+                if (last) {
+                    if constexpr (REAL) {
+                        const int i = row / NQ, j = row - i * NQ;
+                        s *= (double)((i == 0 || i == N / 2 ? 1 : 2) * (j == 0 || j == N / 2 ? 1 : 2));
+                    }
+                    acc += s;
+                }
+            }
+            __syncthreads();  // this buffer is refilled by the next fetch but one
+        }
+    }
+    const double total = block_sum<G::THREADS>(acc, red);
+    if (threadIdx.x == 0) it.partials[blockIdx.x] = total;
 }
 
 // ------------------------------------------------------------------ forward X
@@ -870,13 +1015,16 @@ __global__ void __launch_bounds__(PencilGeom<T, N, RX>::THREADS,
     // |my| exceeds it and write only modes with |mx| <= jband
     const int tiles_per_row = ncols / G::W;
     // quad (counts only): pencils j <= N/2 of data even in x and y stored
-    // [i <= N/2][j <= N/2][h]; plane N-i read as plane i; interior j weigh 2
+    // [i <= N/2][j <= N/2][h]; plane N-i read as plane i; interior j weigh 2;
+    // column element h holds columns 2h (real part) and 2h + 1 (imaginary part)
     const int nj = quad ? N / 2 + 1 : N;
     const int j = blockIdx.x / tiles_per_row;
     const int h = (blockIdx.x % tiles_per_row) * G::W + w;
-    const bool col_ok = h < hvalid && h <= N / 2;
+    const bool packed = DOT && sizeof(T) == 8 && quad;
+    const int hz = packed ? 2 * h : h;
+    const bool col_ok = hz < hvalid && hz <= N / 2;
     const int my = lattice_freq(j, N);
-    const int mz = h == N / 2 ? -(N / 2) : h;
+    const int mz = hz == N / 2 ? -(N / 2) : hz;
     if constexpr (!DOT) {
         if (jband < N / 2 && abs(my) > jband) return;  // rows outside the field's band
     }
@@ -917,9 +1065,10 @@ __global__ void __launch_bounds__(PencilGeom<T, N, RX>::THREADS,
     // sums: the shell bits depend on indices only and are found before the
     // transform (16 bits per mode, two modes per register)
     unsigned bits2[(G::R + 1) / 2];
+    [[maybe_unused]] unsigned bits2b[(G::R + 1) / 2];  // packed: of the odd column
     if constexpr (DOT) {
 #pragma unroll
-        for (int e = 0; e < (G::R + 1) / 2; e++) bits2[e] = 0u;
+        for (int e = 0; e < (G::R + 1) / 2; e++) bits2[e] = bits2b[e] = 0u;
         const auto each = [&](auto&& bits_of) {  // bits_of(mx) of every mode of this thread
 #pragma unroll
             for (int e = 0; e < G::R; e++) {
@@ -941,6 +1090,21 @@ __global__ void __launch_bounds__(PencilGeom<T, N, RX>::THREADS,
             each([&](int mx) { return mx * mx + s2 < lut_size ? (unsigned)__ldg(lut + mx * mx + s2) : 0u; });
         } else {
             each([&](int mx) { return shell_bits(it.shells, it.nshell, mx, my, mz); });
+        }
+        if constexpr (sizeof(T) == 8) {
+            if (packed && hz + 1 < hvalid && hz + 1 <= N / 2) {
+                const int mzb = hz + 1 == N / 2 ? -(N / 2) : hz + 1;
+                const unsigned short* __restrict__ lut = it.lut;
+                const int s2b = my * my + mzb * mzb;
+#pragma unroll
+                for (int e = 0; e < G::R; e++) {
+                    if (!G::live(t + G::TPF * e)) continue;
+                    const int mx = lattice_freq(t + G::TPF * e, N), r2 = mx * mx + s2b;
+                    const unsigned bb = lut ? (r2 < it.lut_size ? (unsigned)__ldg(lut + r2) : 0u)
+                                            : shell_bits(it.shells, it.nshell, mx, my, mzb);
+                    bits2b[e / 2] |= (bb & 0xffffu) << (16 * (e & 1));
+                }
+            }
         }
     }
     const V* tw = stage_table<V>(smem_raw, tw_g, N);
@@ -1010,7 +1174,7 @@ __global__ void __launch_bounds__(PencilGeom<T, N, RX>::THREADS,
         }
         // DOT sums carry `weight` (the (N_field / N)^3 of a sub-grid product spectrum)
         const double wgt =
-            (double)(herm_weight(h, N) * (quad && j != 0 && j != N / 2 ? 2 : 1)) * (use_dk ? it.weight : 1.0);
+            (double)(herm_weight(hz, N) * (quad && j != 0 && j != N / 2 ? 2 : 1)) * (use_dk ? it.weight : 1.0);
         const double inv_n3 = 1.0 / ((double)N * (double)N * (double)N);
         // the 16 shells in two halves of 8 (8 FP64 accumulators live at a
         // time; a mode's term is formed once per half it has shells in).
@@ -1049,6 +1213,21 @@ __global__ void __launch_bounds__(PencilGeom<T, N, RX>::THREADS,
 #pragma unroll
                     for (int c = 0; c < 8; c++)
                         if ((b >> c) & 1u) acc[c] += val;
+                }
+            }
+            if constexpr (sizeof(T) == 8) {
+                if (packed) {
+                    const double wgtb = (double)(herm_weight(hz + 1, N) * (j != 0 && j != N / 2 ? 2 : 1));
+#pragma unroll
+                    for (int e = 0; e < G::R; e++) {
+                        const unsigned b = (bits2b[e / 2] >> (16 * (e & 1) + 8 * half)) & 0xffu;
+                        if (b) {
+                            const double val = wgtb * rint((double)a[e].y * inv_n3);
+#pragma unroll
+                            for (int c = 0; c < 8; c++)
+                                if ((b >> c) & 1u) acc[c] += val;
+                        }
+                    }
                 }
             }
             halve_sums<8, 16>(acc, lane);
@@ -1231,22 +1410,28 @@ static __global__ void k_sum_partials(const double* __restrict__ partials, int n
     if (threadIdx.x == 0) out[idx ? (size_t)idx[blockIdx.x] : (size_t)blockIdx.x * out_stride] = s;
 }
 
-// Column blockIdx.x of item blockIdx.y of a list of dot passes, in a fixed order:
-// one launch for all pair groups of a plan.  (Summed by the last block of each dot
-// pass instead, the 384-point pass took 0.203 against 0.145 + 0.008 ms: every
-// block then waits for a fence and an atomic before it leaves its SM.)
-template <typename T>
-__global__ void __launch_bounds__(256) k_sum_items(const __grid_constant__ Items<FwdXItem<T>> items)
+// Column blockIdx.x of item blockIdx.y of a list of partial sums, in a fixed
+// order: one launch for all pair groups of a plan.  (Summed by the last block of
+// each dot pass instead, the 384-point pass took 0.203 against 0.145 + 0.008 ms:
+// every block then waits for a fence and an atomic before it leaves its SM.)
+struct SumItem {
+    const double* partials;  // [ncol][nblk]
+    int nblk, ncol;
+    double scale;
+    double* out;             // column c lands at out[idx[c]], or out[c] (idx NULL)
+    const int* idx;
+};
+static __global__ void __launch_bounds__(256) k_sum_items(const __grid_constant__ Items<SumItem> items)
 {
-    const FwdXItem<T>& it = item_at(items);
+    const SumItem& it = item_at(items);
     const int c = blockIdx.x;
-    if (c >= it.nshell) return;
+    if (c >= it.ncol) return;
     __shared__ double red[8];
     const double* p = it.partials + (size_t)c * it.nblk;
     double s = 0.0;
     for (int b = threadIdx.x; b < it.nblk; b += 256) s += p[b];
     s = block_sum<256>(s, red);
-    if (threadIdx.x == 0) it.out[it.idx[c]] = s;
+    if (threadIdx.x == 0) it.out[it.idx ? it.idx[c] : c] = it.scale * s;
 }
 
 // ------------------------------------------------------------------ DERIVED k-range

@@ -135,9 +135,17 @@ template <typename T, int N> struct L3 {
     // hva, hvb: the widest legs of the batch; ninputs: 2 when any item has two
     static int pair_z_b(cudaStream_t st, const PairItem<T>* items, int nitems, int ninputs,
                         int hva, int hvb, const Tables<T>& tb, int quad, int variant);
-    template <int RX, bool KEEP>
+    template <int RX, bool KEEP, bool REAL = false>
     static int pair_z_v(cudaStream_t st, const PairItem<T>* items, int nitems, int ninputs,
                         int hva, int hvb, const V* twr, const V* twpp, int quad);
+    // Grid sums of products (k_prod_z) of nitems lists of factors, the widest row of
+    // hv columns; real: quad rows.  Partials per item: *nblocks (at most prod_blocks()).
+    static int prod_z(cudaStream_t st, const ProdItem<T>* items, int nitems, int hv, bool real, int abs_terms,
+                      const Tables<T>& tb, int* nblocks);
+    static constexpr int prod_blocks(bool real)
+    {
+        return ((real ? (N / 2 + 1) * (N / 2 + 1) : N * N) + RG::WZ - 1) / RG::WZ;
+    }
     // The forward X pass, storing (epi SPEC_STORE, SPEC_STORE_PHASE, SPEC_MASK_ADD)
     // or summing per shell; ndk: grid size of the field spectrum dk (0: N).
     // Returns the blocks per item of the widest spectrum in *nblocks.

@@ -127,20 +127,20 @@ int L3<T, N>::fwd_z(cudaStream_t st, int kind, const void* a, const void* b, V* 
 }
 
 template <typename T, int N>
-template <int RX, bool KEEP>
+template <int RX, bool KEEP, bool REAL>
 int L3<T, N>::pair_z_v(cudaStream_t st, const PairItem<T>* items, int nitems, int ninputs,
                        int hva, int hvb, const V* twr, const V* twpp, int quad)
 {
     using G = RowGeom<T, N, RX>;
     using PGm = PairGeom<T, N, RX, KEEP>;
-    const size_t smem = PGm::smem(ninputs, hva, hvb);
-    PS_LTRY(set_smem(k_pair_z<T, N, RX, KEEP>, PGm::smem(2, N / 2 + 1, N / 2 + 1)));
+    const size_t smem = PGm::smem(ninputs, REAL ? (hva + 1) / 2 : hva, REAL ? (hvb + 1) / 2 : hvb);
+    PS_LTRY(set_smem(k_pair_z<T, N, RX, KEEP, REAL>, PGm::smem(2, N / 2 + 1, N / 2 + 1)));
     const int nrows = quad ? (N / 2 + 1) * (N / 2 + 1) : N * N;
     const int tiles = (nrows + G::WZ - 1) / G::WZ;
     int grid = 0;  // resident CTAs, shared out among the items
-    PS_LTRY(persistent_grid(k_pair_z<T, N, RX, KEEP>, G::THREADS, smem, tiles * nitems, &grid));
+    PS_LTRY(persistent_grid(k_pair_z<T, N, RX, KEEP, REAL>, G::THREADS, smem, tiles * nitems, &grid));
     grid = std::max(1, std::min(tiles, grid / nitems));
-    k_pair_z<T, N, RX, KEEP><<<dim3((unsigned)grid, (unsigned)nitems), G::THREADS, smem, st>>>(pack(items, nitems), nrows, twr, twpp);
+    k_pair_z<T, N, RX, KEEP, REAL><<<dim3((unsigned)grid, (unsigned)nitems), G::THREADS, smem, st>>>(pack(items, nitems), nrows, twr, twpp);
     return PS_OK;
 }
 
@@ -158,7 +158,32 @@ int L3<T, N>::pair_z_b(cudaStream_t st, const PairItem<T>* items, int nitems, in
         if (variant == 1 && !quad)
             return pair_z_v<0, true>(st, items, nitems, ninputs, hva, hvb, tb.twr, tb.twpp, quad);
     }
+    if constexpr (sizeof(T) == 8) {
+        if (quad) return pair_z_v<0, false, true>(st, items, nitems, ninputs, hva, hvb, tb.twr, tb.twpp, quad);
+    }
     return pair_z_v<0, false>(st, items, nitems, ninputs, hva, hvb, tb.twr, tb.twpp, quad);
+}
+
+template <typename T, int N>
+int L3<T, N>::prod_z(cudaStream_t st, const ProdItem<T>* items, int nitems, int hv, bool real, int abs_terms,
+                     const Tables<T>& tb, int* nblocks)
+{
+    const int P = RG::pitch(real ? (hv + 1) / 2 : hv);
+    const size_t smem = RG::STAGE_OFF + (size_t)2 * RG::WZ * P * sizeof(V);
+    auto go = [&](auto kernel) -> int {
+        PS_LTRY(set_smem(kernel, RG::smem(1, N / 2 + 1, 0)));
+        int grid = 0;  // resident CTAs, shared out among the items
+        PS_LTRY(persistent_grid(kernel, RG::THREADS, smem, prod_blocks(real) * nitems, &grid));
+        grid = std::max(1, std::min(prod_blocks(real), grid / nitems));
+        kernel<<<dim3((unsigned)grid, (unsigned)nitems), RG::THREADS, smem, st>>>(pack(items, nitems), P, abs_terms, tb.twr,
+                                                                                  tb.twpp);
+        *nblocks = grid;
+        return PS_OK;
+    };
+    if constexpr (sizeof(T) == 8) {
+        if (real) return go(k_prod_z<T, N, true>);
+    }
+    return go(k_prod_z<T, N, false>);
 }
 
 template <typename T, int N>
