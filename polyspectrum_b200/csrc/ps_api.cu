@@ -292,7 +292,7 @@ struct ps_gpu_ctx {
     size_t lane_work_cap[3] = {0, 0, 0};  // bytes
     cudaEvent_t ev_join2 = nullptr;
     // memory of destroyed plans kept for the next ones (at most kSpareArenas)
-    std::vector<PlanArena> spare_arenas;
+    std::vector<PlanArena> spare_arenas, spare_device;
     PrecBufs<float> f;
     PrecBufs<double> d;
     double* partials = nullptr;
@@ -937,7 +937,7 @@ template <typename T> int forward_field(ps_gpu_ctx* c, int kind, const void* a, 
 template <typename T>
 int dot_pass(ps_gpu_ctx* c, V2<T>* data, int epi, int S, int hvalid, const Shell* dshells,
              const Shell* hsh, int ns, double* dout, int quad = 0, int M = 0, double weight = 1.0,
-             const int* didx = nullptr)
+             const int* didx = nullptr, const std::vector<unsigned short*>* vol = nullptr, int vol_band = 0)
 {
     PrecBufs<T>& B = bufs<T>(c);
     const int N = M > 0 ? M : c->N;
@@ -982,6 +982,8 @@ int dot_pass(ps_gpu_ctx* c, V2<T>* data, int epi, int S, int hvalid, const Shell
             it.shells = dshells + s0;
             it.lut = lut;
             it.lut_size = lut_size;
+            if (vol) it.vol = (*vol)[(size_t)(s0 / MAX_DOT_SHELLS)];
+            it.vol_band = vol_band;
             it.r2max = (int)std::min<long long>(r2max, 0x7fffffff);
             it.weight = weight;
             it.partials = c->partials;
@@ -1368,6 +1370,8 @@ struct ps_gpu_plan {
     std::vector<std::function<int()>> ops_tail;    // n = 2 and leg-by-leg configurations, finalisation
     bool has_groups = false, two_lanes = false;
     std::vector<PlanArena> arenas;          // this plan's device tables and their host mirrors
+    std::vector<PlanArena> device_only;     // tables made on the device (no mirror)
+    std::vector<std::function<int()>> ops_once;  // their launches, after the next flush
     double* dres = nullptr;                 // B, Npoly per configuration
     double* dsumA = nullptr;                // sum |terms| (condition numbers)
     double* dsumD = nullptr;
@@ -1428,8 +1432,28 @@ int arena_take(ps_gpu_plan* P, size_t bytes, void** dev, void** host)
     return PS_OK;
 }
 
-// Queues the copies of what was written to the mirrors since the last flush;
-// before the first launch that reads the plan's tables.
+// Device memory of the plan without a mirror.
+int device_take(ps_gpu_plan* P, size_t bytes, void** dev)
+{
+    ps_gpu_ctx* c = P->ctx;
+    PlanArena a;
+    for (size_t q = 0; q < c->spare_device.size() && !a.dev; q++)
+        if (c->spare_device[q].cap >= bytes) {
+            a = c->spare_device[q];
+            c->spare_device.erase(c->spare_device.begin() + (long)q);
+        }
+    if (!a.dev) {
+        PS_TRY(alloc_dev(&a.dev, bytes));
+        a.cap = bytes;
+    }
+    P->device_only.push_back(a);
+    *dev = a.dev;
+    return PS_OK;
+}
+
+// Queues the copies of what was written to the mirrors since the last flush, and
+// the launches that make tables from them; before the first launch that reads the
+// plan's tables.
 int plan_flush(ps_gpu_plan* P)
 {
     for (PlanArena& a : P->arenas) {
@@ -1438,6 +1462,8 @@ int plan_flush(ps_gpu_plan* P)
                               P->ctx->stream));
         a.flushed = a.used;
     }
+    for (auto& op : P->ops_once) PS_TRY(op());
+    P->ops_once.clear();
     return PS_OK;
 }
 
@@ -2217,6 +2243,7 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
         bool two = false;                // distinct legs
         std::vector<Shell> gtable;       // host copies of the closing shells
         std::vector<unsigned short*> lut;  // per 16 closing shells: r^2 -> bitmask (NULL: compared directly)
+        std::vector<unsigned short*> vol;  // or octant -> bitmask, components <= hmax (shells that are no intervals)
         bool enum_counts = false;
         PairCountLists lists;
     };
@@ -2248,7 +2275,21 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
                 luts.push_back(LutItem{dtable + gofs[g] + s0, lut, cnt, size});
                 lut_max = std::max(lut_max, size);
             }
+            unsigned short* vol = nullptr;
+            const size_t side = (size_t)I.hmax + 1, vbytes = side * side * side * sizeof(unsigned short);
+            if (!interval && vbytes <= kSpareBytes) {
+                PS_TRY(device_take(P, vbytes, (void**)&vol));
+                const Shell* sh = dtable + gofs[g] + s0;
+                const int band = I.hmax;
+                P->ops_once.push_back([=]() {
+                    k_shell_volume<<<(unsigned)std::min<size_t>((side * side * side + 255) / 256, 148 * 16), 256, 0, c->stream>>>(
+                        sh, cnt, band, vol);
+                    PS_CK(launch_status());
+                    return PS_OK;
+                });
+            }
             I.lut.push_back(lut);
+            I.vol.push_back(vol);
         }
     }
     for (size_t q0 = 0; q0 < luts.size(); q0 += kItems) {  // after the DERIVED chain, which fills closing shells
@@ -2341,6 +2382,8 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
                 it.nshell = std::min(MAX_DOT_SHELLS, ng - s0);
                 it.shells = dtable + gofs[g] + s0;
                 it.lut = I.lut[ch];
+                it.vol = I.vol[ch];
+                it.vol_band = I.hmax;
                 bool interval = true;
                 long long r2max = 0;  // no mode of these shells lies outside |m|^2 <= r2max
                 for (int q = s0; q < s0 + it.nshell; q++) {
@@ -2425,7 +2468,13 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
         I.enum_counts = !(P->flags & PS_PLAN_FFT_COUNTS) && uniq[G.a].tag == 0 && uniq[G.b].tag == 0 &&
                         I.sa.kind <= SHELL_RANGE && I.sb.kind <= SHELL_RANGE;
         for (const Shell& h : I.gtable) I.enum_counts = I.enum_counts && h.kind <= SHELL_RANGE;
-        if (I.enum_counts) I.enum_counts = pair_count_lists(I.sa, I.sb, N, &I.lists);
+        // squared radii the closing shells hold: known on the host but for DERIVED ones
+        int c_lo = 0x7fffffff, c_hi = 0;
+        for (size_t q = 0; q < I.gtable.size(); q++) {
+            c_lo = std::min(c_lo, uniq[G.third[q]].tag == 0 ? std::max(I.gtable[q].r2lo, 0) : 0);
+            c_hi = std::max(c_hi, uniq[G.third[q]].tag == 0 ? I.gtable[q].r2hi : 0x7fffffff);
+        }
+        if (I.enum_counts) I.enum_counts = pair_count_lists(I.sa, I.sb, N, c_lo, c_hi, I.gtable.size() == 1, &I.lists);
         any_fft = any_fft || !I.enum_counts;
     }
     if (any_fft) {
@@ -2438,6 +2487,8 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
         const Group G = groups[g];
         const Shell sa = info[g].sa, sb = info[g].sb;
         const std::vector<Shell> gtable = info[g].gtable;
+        const std::vector<unsigned short*> vol = info[g].vol;
+        const int hmax = info[g].hmax;
         const int hout = info[g].hmax + 1, go = gofs[g], io = gidx_ofs[g];
         return [=]() {
             int Sa = 0, ha = 0, Sb = 0, hbb = 0, S = 0;
@@ -2446,7 +2497,7 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
                 PS_TRY(c2r_xy<double>(c, LOAD_UNIT, dtable + G.b, sb.band, c->d.work2, &Sb, &hbb, 1, M));
             PS_TRY(pair_spectrum<double>(c, c->d.work, Sa, ha, G.a != G.b ? c->d.work2 : nullptr, Sb, hbb, hout, &S, 1, M));
             PS_TRY(dot_pass<double>(c, c->d.work3, SPEC_COUNT, S, hout, dtable + go, gtable.data(), (int)gtable.size(), sumI,
-                                    1, M, 1.0, didx + io));
+                                    1, M, 1.0, didx + io, &vol, hmax));
             return PS_OK;
         };
     };
@@ -2600,6 +2651,7 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
             int n, grid;
             size_t smem;
             bool wrap;
+            int cl;
         };
         std::vector<Launch> launches;
         std::vector<int> order;  // configurations of the enumerated groups
@@ -2611,9 +2663,9 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
         if (total) PS_TRY(plan_alloc(P, &dcounts, total));
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-        constexpr int kClass[3] = {2048, 12 * 1024, kCountMaxBins};  // bins
+        constexpr int kClass[4] = {0, kCountSmallBins, 12 * 1024, kCountMaxBins};  // bins (0: one closing shell)
         for (int wrap = 0; wrap < 2; wrap++)
-            for (int cl = 0; cl < 3; cl++) {
+            for (int cl = 0; cl < 4; cl++) {
                 std::vector<CountItem> items;
                 std::vector<double> pairs;
                 double sum = 0.0;
@@ -2644,23 +2696,27 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
                     for (int q : groups[g].cfg) order.push_back(q);
                 }
                 if (items.empty()) continue;
-                // about one CTA of kCountThreads per SM in all, shared out by pairs, over
-                // about eight work items each: the count lane runs beside the field load
-                // and the field lanes, and one histogram per SM leaves the rest of each SM's
-                // shared memory to their passes
+                // about one CTA of kCountThreads per SM in all (short histograms: six of
+                // kCountSmallThreads), shared out by pairs, over about eight work items
+                // each: the count lane runs beside the field load and the field lanes, and
+                // one histogram per SM leaves the rest of each SM's shared memory to their
+                // passes
+                const bool small = cl <= 1;
+                const int threads = small ? kCountSmallThreads : kCountThreads, total_ctas = small ? 6 * sms : sms;
                 int cta = 0;
                 for (size_t q = 0; q < items.size(); q++) {
                     CountItem& it = items[q];
-                    const int share = std::max(1, (int)(sms * pairs[q] / std::max(sum, 1.0)));
-                    const int nmc = std::max(1, (it.nb + kCountThreads * kCountBPT - 1) / (kCountThreads * kCountBPT));
-                    const int nrs = std::max(1, std::min(it.nrep, (8 * share + nmc - 1) / nmc));
+                    const double part = total_ctas * pairs[q] / std::max(sum, 1.0);
+                    const int share = std::max(1, (int)(small ? ceil(part) : part));
+                    const int nmc = std::max(1, (it.nb + threads * kCountBPT - 1) / (threads * kCountBPT));
+                    const int nrs = std::max(1, std::min(it.nrep, ((small ? 2 : 8) * share + nmc - 1) / nmc));
                     it.rep_slice = std::min(kCountRepChunk, std::max(8, (it.nrep + nrs - 1) / nrs));
                     const int nitems = nmc * ((it.nrep + it.rep_slice - 1) / it.rep_slice);
                     it.cta0 = cta;
                     it.nctas = std::max(1, std::min(nitems, share));
                     cta += it.nctas;
                 }
-                Launch L{nullptr, (int)items.size(), cta, kCountStageBytes + (size_t)nb_max * sizeof(unsigned int), wrap != 0};
+                Launch L{nullptr, (int)items.size(), cta, kCountStageBytes + (size_t)nb_max * sizeof(unsigned int), wrap != 0, cl};
                 PS_TRY(plan_upload(P, &L.items, items));
                 launches.push_back(L);
             }
@@ -2678,8 +2734,15 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
                 PS_CK(cudaMemsetAsync(dcounts, 0, sizeof(unsigned long long) * (size_t)nc, c->stream));
                 for (const Launch& L : launches) {
                     Prof pf(c);
-                    if (L.wrap) k_pair_counts<true><<<L.grid, kCountThreads, L.smem, c->stream>>>(L.items, L.n, N);
-                    else k_pair_counts<false><<<L.grid, kCountThreads, L.smem, c->stream>>>(L.items, L.n, N);
+                    const auto go = [&](auto kernel, int threads) {
+                        kernel<<<L.grid, threads, L.smem, c->stream>>>(L.items, L.n, N);
+                    };
+                    if (L.cl == 0 && L.wrap) go(k_pair_counts<true, kCountBPT, kCountSmallThreads, true>, kCountSmallThreads);
+                    else if (L.cl == 0) go(k_pair_counts<false, kCountBPT, kCountSmallThreads, true>, kCountSmallThreads);
+                    else if (L.cl == 1 && L.wrap) go(k_pair_counts<true, kCountBPT, kCountSmallThreads>, kCountSmallThreads);
+                    else if (L.cl == 1) go(k_pair_counts<false, kCountBPT, kCountSmallThreads>, kCountSmallThreads);
+                    else if (L.wrap) go(k_pair_counts<true>, kCountThreads);
+                    else go(k_pair_counts<false>, kCountThreads);
                     pf.end(KF_PAIR_COUNTS, bytes / (double)launches.size());
                 }
                 k_counts_out<<<(nc + 127) / 128, 128, 0, c->stream>>>(nc, dcounts, dorder, sumI);
@@ -2982,7 +3045,13 @@ void plan_release(ps_gpu_plan* P, bool keep)
             }
         }
         P->arenas.clear();
+        for (PlanArena& a : P->device_only) {
+            if (keep && a.cap <= kSpareBytes && c->spare_device.size() < kSpareArenas) c->spare_device.push_back(a);
+            else cudaFree(a.dev);
+        }
+        P->device_only.clear();
     }
+    P->ops_once.clear();
     P->hres = nullptr;
 }
 
@@ -4285,6 +4354,7 @@ void ps_gpu_finalize(ps_gpu_ctx* c)
         cudaFree(a.dev);
         cudaFreeHost(a.host);
     }
+    for (PlanArena& a : c->spare_device) cudaFree(a.dev);
     free_prec(c->f);
     free_prec(c->d);
     cudaFree(c->partials);

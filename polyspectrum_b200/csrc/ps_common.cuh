@@ -76,26 +76,26 @@ struct Shell {
 __device__ __forceinline__ int lattice_freq(int idx, int n) { return idx < (n >> 1) ? idx : idx - n; }
 
 // get_corners (filter.c:257-289) on squared radii: min/max over the 8 corners
-// of the cube of half-width e around m, folded into (min2, max2).
+// of the cube of half-width e around m, folded into (min2, max2).  Rounded
+// addition is monotone, so the smallest of the eight sums (x + y) + z is the sum
+// of the smaller squares of each axis, and the largest that of the larger ones:
+// the same bits as folding all eight.
+__device__ __forceinline__ void axis_extremes(int v, double e, double& lo, double& hi)
+{
+    const double m = __dsub_rn((double)v, e), p = __dadd_rn((double)v, e);
+    const double m2 = __dmul_rn(m, m), p2 = __dmul_rn(p, p);
+    lo = fmin(m2, p2);
+    hi = fmax(m2, p2);
+}
 __device__ __forceinline__ void corners_fold(int mx, int my, int mz, double e, double& min2,
                                              double& max2)
 {
-    const double x = (double)mx, y = (double)my, z = (double)mz;
-    const double xm = __dmul_rn(__dsub_rn(x, e), __dsub_rn(x, e));
-    const double xp = __dmul_rn(__dadd_rn(x, e), __dadd_rn(x, e));
-    const double ym = __dmul_rn(__dsub_rn(y, e), __dsub_rn(y, e));
-    const double yp = __dmul_rn(__dadd_rn(y, e), __dadd_rn(y, e));
-    const double zm = __dmul_rn(__dsub_rn(z, e), __dsub_rn(z, e));
-    const double zp = __dmul_rn(__dadd_rn(z, e), __dadd_rn(z, e));
-    const double c[8] = {__dadd_rn(__dadd_rn(xm, ym), zm), __dadd_rn(__dadd_rn(xp, ym), zm),
-                         __dadd_rn(__dadd_rn(xm, yp), zm), __dadd_rn(__dadd_rn(xm, ym), zp),
-                         __dadd_rn(__dadd_rn(xp, yp), zm), __dadd_rn(__dadd_rn(xp, ym), zp),
-                         __dadd_rn(__dadd_rn(xm, yp), zp), __dadd_rn(__dadd_rn(xp, yp), zp)};
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-        if (c[q] > max2) max2 = c[q];
-        if (c[q] < min2) min2 = c[q];
-    }
+    double xl, xh, yl, yh, zl, zh;
+    axis_extremes(mx, e, xl, xh);
+    axis_extremes(my, e, yl, yh);
+    axis_extremes(mz, e, zl, zh);
+    min2 = fmin(min2, __dadd_rn(__dadd_rn(xl, yl), zl));
+    max2 = fmax(max2, __dadd_rn(__dadd_rn(xh, yh), zh));
 }
 
 // The DEFAULT and RANGE predicates (filter.c:57-59, :155-158) depend on the
@@ -148,30 +148,30 @@ __host__ __device__ inline void shell_r2_interval(Shell& s, int n)
     s.r2hi = a;
 }
 
+// The WATKINSON predicates on the smallest and largest corner radius of a cell.
+__device__ __forceinline__ bool corner_bit(const Shell& s, double pmin, double pmax)
+{
+    if (s.kind == SHELL_WATKINSON) return pmin <= s.kk && s.kk <= pmax;
+    return (pmax >= s.mmax && pmin <= s.mmax) || (pmax <= s.mmax && pmin >= s.mmin) ||
+           (pmax >= s.mmin && pmin <= s.mmin);
+}
+__device__ __forceinline__ void corner_radii(const Shell& s, int mx, int my, int mz, double& pmin, double& pmax)
+{
+    double min2 = s.min2_init, max2 = 0.0;
+    corners_fold(mx, my, mz, s.half, min2, max2);
+    pmin = __dsqrt_rn(min2);
+    pmax = __dsqrt_rn(max2);
+}
+
 __device__ __forceinline__ bool shell_bit(const Shell& s, int mx, int my, int mz)
 {
-    switch (s.kind) {
-    case SHELL_DEFAULT:
-    case SHELL_RANGE: {
+    if (s.kind == SHELL_DEFAULT || s.kind == SHELL_RANGE) {
         const int r2 = mx * mx + my * my + mz * mz;
         return r2 >= s.r2lo && r2 <= s.r2hi;
     }
-    case SHELL_WATKINSON: {
-        double min2 = s.min2_init, max2 = 0.0;
-        corners_fold(mx, my, mz, s.half, min2, max2);
-        const double pmin = __dsqrt_rn(min2), pmax = __dsqrt_rn(max2);
-        return pmin <= s.kk && s.kk <= pmax;
-    }
-    case SHELL_WATKINSON_RANGE: {
-        double min2 = s.min2_init, max2 = 0.0;
-        corners_fold(mx, my, mz, s.half, min2, max2);
-        const double pmin = __dsqrt_rn(min2), pmax = __dsqrt_rn(max2);
-        return (pmax >= s.mmax && pmin <= s.mmax) || (pmax <= s.mmax && pmin >= s.mmin) ||
-               (pmax >= s.mmin && pmin <= s.mmin);
-    }
-    default:
-        return false;
-    }
+    double pmin, pmax;
+    corner_radii(s, mx, my, mz, pmin, pmax);
+    return corner_bit(s, pmin, pmax);
 }
 
 // Cheap necessary condition: outside the band cube nothing is selected.
@@ -181,13 +181,26 @@ __device__ __forceinline__ bool in_band(const Shell& s, int mx, int my, int mz)
 }
 
 // Bitmask of the shells (of ns <= 32) that select mode m; one out-of-line
-// instance so the callers' unrolled loops stay small.
+// instance so the callers' unrolled loops stay small.  The corner radii depend on
+// the bin width only and are found once for all shells of one width.
 static __device__ __noinline__ unsigned shell_bits(const Shell* __restrict__ sh, int ns, int mx, int my, int mz)
 {
     unsigned bits = 0u;
+    const int r2 = mx * mx + my * my + mz * mz, r = max(abs(mx), max(abs(my), abs(mz)));
+    double half = 0.0, init = -1.0, pmin = 0.0, pmax = 0.0;
     for (int c = 0; c < ns; c++) {
-        const Shell s = sh[c];
-        if (in_band(s, mx, my, mz) && shell_bit(s, mx, my, mz)) bits |= 1u << c;
+        const Shell& s = sh[c];
+        if (r > s.band) continue;
+        if (s.kind <= SHELL_RANGE) {
+            bits |= (unsigned)(r2 >= s.r2lo && r2 <= s.r2hi) << c;
+        } else {
+            if (s.half != half || s.min2_init != init) {
+                half = s.half;
+                init = s.min2_init;
+                corner_radii(s, mx, my, mz, pmin, pmax);
+            }
+            bits |= (unsigned)corner_bit(s, pmin, pmax) << c;
+        }
     }
     return bits;
 }

@@ -32,10 +32,23 @@ namespace ps {
 // (2x, 2y, 2z, weight) beside |m_a|^2 - s_lo, the modes keep |m_b|^2 (a large
 // negative value for the idle slots past nb), so a pair costs three
 // multiply-adds, an add and the range test before its atomic.
+// WRAP: with a >= 0 and b >= -n/2 a component q = a + b can pass the upper edge
+// only, and (q - n)^2 - q^2 = n (n - 2 q) is at most 0 exactly where q >= n/2, so the
+// wrapped norm is the plain one plus min(0, n^2 - 2 n q) per component: one fused
+// add-minimum each (compares and selects per component took 27 instructions a pair,
+// 0.24 ms for the 2.2e8 wrapping pairs of 64 equilateral triangles at 128^3).
 constexpr int kCountBPT = 4;
 constexpr int kCountThreads = 1024;  // one CTA per SM: 32 warps to hide the atomics' latency
+// Lists of groups with one closing shell each (equilateral and single triangles)
+// need no histogram: a pair inside the shell's interval adds its weight in a
+// register (ONE), about seven instructions a pair without a branch or an atomic.
+// They and short histograms hold no SM's shared memory, and such a list is cut
+// finer: CTAs of 256 threads, six per SM in all, so that no group's last CTA is
+// left over.  64 equilateral triangles at 128^3: 0.42 ms with histograms and CTAs of
+// 1024 threads.
+constexpr int kCountSmallBins = 2048, kCountSmallThreads = 256;
 constexpr int kCountRepChunk = 512;  // largest rep_slice
-constexpr size_t kCountStageBytes = kCountRepChunk * (sizeof(int4) + sizeof(int));
+constexpr size_t kCountStageBytes = kCountRepChunk * 2 * sizeof(int4);
 constexpr int kCountMaxBins = 44 * 1024;  // 176 KB of uint32 bins beside the staged representatives
 
 // One launch counts for a list of groups: group g has the CTAs cta0 .. cta0 +
@@ -48,8 +61,8 @@ struct CountItem {
     int nrep, nb, s_lo, nbins, rep_slice, ncl;
     int cta0, nctas;
 };
-template <bool WRAP, int BPT = kCountBPT, int THREADS = kCountThreads>
-__global__ void __launch_bounds__(THREADS)
+template <bool WRAP, int BPT = kCountBPT, int THREADS = kCountThreads, bool ONE = false>
+__global__ void __launch_bounds__(THREADS, THREADS == kCountSmallThreads ? 6 : 1)
     k_pair_counts(const CountItem* __restrict__ items, int ngroups, int n)
 {
     int gi = 0;  // the group of this CTA
@@ -67,10 +80,19 @@ __global__ void __launch_bounds__(THREADS)
     int rep_slice = it.rep_slice;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     int4* srep = reinterpret_cast<int4*>(smem_raw);
-    int* snorm = reinterpret_cast<int*>(smem_raw + kCountRepChunk * sizeof(int4));
+    int4* sedge = srep + kCountRepChunk;  // -2 n a (WRAP), |a|^2 - base
     unsigned int* hist = reinterpret_cast<unsigned int*>(smem_raw + kCountStageBytes);
-    for (int i = threadIdx.x; i < nbins; i += blockDim.x) hist[i] = 0u;
-    const int half = n >> 1;
+    int one_lo = 0;
+    unsigned one_span = 0u;
+    unsigned long long inside = 0ull;
+    if constexpr (ONE) {  // the interval, empty as one no value falls into
+        const int lo = closing[0].r2lo, hi = closing[0].r2hi;
+        one_lo = hi >= lo ? lo : 0x7fffffff;
+        one_span = hi >= lo ? (unsigned)(hi - lo) : 0u;
+    } else {
+        for (int i = threadIdx.x; i < nbins; i += blockDim.x) hist[i] = 0u;
+    }
+    const int base = ONE ? one_lo : s_lo;  // bins count from here
     constexpr int kChunk = THREADS * BPT;
     rep_slice = max(1, min(rep_slice, kCountRepChunk));  // the staging buffer's size
     const int nmc = (nb + kChunk - 1) / kChunk, nrs = (nrep + rep_slice - 1) / rep_slice;
@@ -79,6 +101,7 @@ __global__ void __launch_bounds__(THREADS)
         const int mc = item % nmc, r0 = (item / nmc) * rep_slice;
         const int cnt = min(rep_slice, nrep - r0);
         int bx[BPT], by[BPT], bz[BPT], bn[BPT];
+        int ex[BPT], ey[BPT], ez[BPT];  // n^2 - 2 n b
 #pragma unroll
         for (int u = 0; u < BPT; u++) {
             const int idx = mc * kChunk + u * THREADS + (int)threadIdx.x;
@@ -89,33 +112,38 @@ __global__ void __launch_bounds__(THREADS)
             bz[u] = m.z;
             // idle slots: every bin index of theirs is negative (|.|^2 sums stay below 2^29)
             bn[u] = valid ? m.x * m.x + m.y * m.y + m.z * m.z : -(1 << 30);
+            ex[u] = n * (n - 2 * m.x);
+            ey[u] = n * (n - 2 * m.y);
+            ez[u] = n * (n - 2 * m.z);
         }
         __syncthreads();  // the previous item's representatives are no longer read
         for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
             const int4 a = reps[r0 + i];
-            srep[i] = WRAP ? a : int4{2 * a.x, 2 * a.y, 2 * a.z, a.w};
-            snorm[i] = a.x * a.x + a.y * a.y + a.z * a.z - s_lo;
+            srep[i] = int4{2 * a.x, 2 * a.y, 2 * a.z, a.w};
+            sedge[i] = int4{-2 * n * a.x, -2 * n * a.y, -2 * n * a.z, a.x * a.x + a.y * a.y + a.z * a.z - base};
         }
         __syncthreads();
+        unsigned here = 0u;  // ONE: at most rep_slice BPT 48
 #pragma unroll 2
         for (int r = 0; r < cnt; r++) {
             const int4 a = srep[r];
-            const int an = snorm[r];
+            const int4 d = sedge[r];
 #pragma unroll
             for (int u = 0; u < BPT; u++) {
-                int sb;
-                if constexpr (WRAP) {
-                    int qx = a.x + bx[u], qy = a.y + by[u], qz = a.z + bz[u];
-                    qx += (qx < -half) * n - (qx >= half) * n;
-                    qy += (qy < -half) * n - (qy >= half) * n;
-                    qz += (qz < -half) * n - (qz >= half) * n;
-                    sb = bn[u] < 0 ? -1 : qx * qx + qy * qy + qz * qz - s_lo;
-                } else {
-                    sb = an + bn[u] + a.x * bx[u] + a.y * by[u] + a.z * bz[u];
-                }
-                if ((unsigned)sb < (unsigned)nbins) atomicAdd(&hist[sb], (unsigned)a.w);
+                int sb = d.w + bn[u] + a.x * bx[u] + a.y * by[u] + a.z * bz[u];
+                if constexpr (WRAP)
+                    sb += __viaddmin_s32(d.x, ex[u], 0) + __viaddmin_s32(d.y, ey[u], 0) + __viaddmin_s32(d.z, ez[u], 0);
+                if constexpr (ONE) here += (unsigned)sb <= one_span ? (unsigned)a.w : 0u;
+                else if ((unsigned)sb < (unsigned)nbins) atomicAdd(&hist[sb], (unsigned)a.w);
             }
         }
+        inside += here;
+    }
+    if constexpr (ONE) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) inside += __shfl_xor_sync(0xffffffffu, inside, o);
+        if ((threadIdx.x & 31) == 0 && inside) atomicAdd(&counts[0], inside);
+        return;
     }
     __syncthreads();
     // closing shell c: the bins of its interval (clamped to the histogram)
@@ -178,7 +206,7 @@ inline std::vector<short4> interval_modes(const Shell& sh, int N)
     return out;
 }
 
-// Representatives 0 <= x <= y <= z (as indices, N/2 stands for -N/2) of the
+// Representatives 0 <= x <= y <= z (N/2 stands for -N/2, which is the same index) of the
 // orbits of an interval shell's modes under the 48 axis permutations and sign
 // flips, with the orbit sizes: 6, 3 or 1 permutations, two signs per component
 // but for 0 and the single index of |N/2|.
@@ -188,7 +216,6 @@ inline std::vector<int4> interval_orbits(const Shell& sh, int N)
     if (sh.r2hi < 0 || sh.r2lo > sh.r2hi) return out;
     const int b = std::min(sh.band, N / 2);
     const auto signs = [&](int v) { return v == 0 || v == N / 2 ? 1 : 2; };
-    const auto lattice = [&](int v) { return v == N / 2 ? -(N / 2) : v; };
     for (int x = 0; x <= b && 3 * x * x <= sh.r2hi; x++)
         for (int y = x; y <= b && x * x + 2 * y * y <= sh.r2hi; y++) {
             const int s = x * x + y * y;
@@ -200,15 +227,18 @@ inline std::vector<int4> interval_orbits(const Shell& sh, int N)
             }
             for (; z <= b && s + z * z <= sh.r2hi; z++) {
                 const int perms = x == y && y == z ? 1 : x == y || y == z ? 3 : 6;
-                out.push_back(int4{lattice(x), lattice(y), lattice(z), perms * signs(x) * signs(y) * signs(z)});
+                out.push_back(int4{x, y, z, perms * signs(x) * signs(y) * signs(z)});
             }
         }
     return out;
 }
 
-// The lists of a group with interval legs a, b on an N-grid; false when the
-// enumeration does not apply (histogram too large for shared memory).
-inline bool pair_count_lists(const Shell& sa, const Shell& sb, int N, PairCountLists* L)
+// The lists of a group with interval legs a, b on an N-grid, the histogram over
+// the squared radii [c_lo, c_hi] its closing shells may hold (one: a single closing
+// shell, no histogram); false when the
+// enumeration does not apply (histogram too large for shared memory, or more
+// pairs than the FP64 transforms of the shells would cost).
+inline bool pair_count_lists(const Shell& sa, const Shell& sb, int N, int c_lo, int c_hi, bool one, PairCountLists* L)
 {
     // host work O(b^2 + |S|); the enumeration itself |S_a| |S_b| / 48 pairs
     const double est = 4.0 * 3.14159 * (double)std::max(sa.r2hi, 1) * 4.0 * 3.14159 * (double)std::max(sb.r2hi, 1);
@@ -229,7 +259,12 @@ inline bool pair_count_lists(const Shell& sa, const Shell& sb, int N, PairCountL
     if (L->wrap) smax = std::min(smax, 3.0 * (N / 2) * (N / 2));
     const double dmin = L->wrap ? 0.0 : std::max({0.0, ra_lo - rb_hi, rb_lo - ra_hi});
     L->s_lo = std::max(0, (int)floor(dmin * dmin) - 1);
-    const long long s_hi = (long long)ceil(smax) + 1;
+    L->s_lo = std::max(L->s_lo, c_lo);
+    const long long s_hi = std::max<long long>(L->s_lo, std::min<long long>((long long)ceil(smax) + 1, c_hi));
+    if (one) {
+        L->nbins = 0;
+        return true;
+    }
     if (s_hi - L->s_lo + 1 > kCountMaxBins) return false;
     L->nbins = (int)(s_hi - L->s_lo + 1);
     return true;
