@@ -158,8 +158,7 @@ template <typename T> struct PrecBufs {
     V2<T>* work2 = nullptr; // second and third work spectra (pair groups; allocated on use)
     V2<T>* work3 = nullptr;
     V2<T>* hacc = nullptr;  // adjoint spectrum accumulator (allocated on use)
-    T* ra = nullptr;        // real grids
-    T* rb = nullptr;
+    T* ra = nullptr;        // real grid
     T* mod = nullptr;       // |X| of a phase-only field (ps_gpu_keep_modulus)
     int S = 0;
     bool have_spec = false;
@@ -290,6 +289,7 @@ struct ps_gpu_ctx {
     cudaStream_t lane2_stream = nullptr;
     unsigned char* lane_work[3] = {nullptr, nullptr, nullptr};
     size_t lane_work_cap[3] = {0, 0, 0};  // bytes
+    bool lane_work_own[3] = {false, false, false};  // allocated for it (else one of the buffers below)
     cudaEvent_t ev_join2 = nullptr;
     // memory of destroyed plans kept for the next ones (at most kSpareArenas)
     std::vector<PlanArena> spare_arenas, spare_device;
@@ -459,7 +459,6 @@ template <typename T> int init_prec(ps_gpu_ctx* c, PrecBufs<T>& b)
     PS_TRY(alloc_dev(&b.spec, nspec));
     PS_TRY(alloc_dev(&b.work, nspec));
     PS_TRY(alloc_dev(&b.ra, nreal));
-    PS_TRY(alloc_dev(&b.rb, nreal));
     std::vector<V2<T>> h(N);
     const long double two_pi = 6.283185307179586476925286766559005768L;
     for (int m = 0; m < N; m++) {
@@ -536,7 +535,6 @@ template <typename T> void free_prec(PrecBufs<T>& b)
     cudaFree(b.hacc);
     cudaFree(b.mod);
     cudaFree(b.ra);
-    cudaFree(b.rb);
     b = PrecBufs<T>();
 }
 
@@ -611,16 +609,30 @@ struct Lane2 {
     }
 };
 
-// Workspace of a field lane, at least `bytes` (a replaced one is retired: a
-// captured graph or a plan's tables may still point at it).
+// Workspace of a field lane, at least `bytes`.  A buffer of the context that nothing
+// else uses while the lane works serves as long as it is large enough: lane 0 the FP32
+// work spectrum, lane 1 an FP32 real grid, the products (2) the FP64 work spectrum
+// (FP64 counts use it on the side lane, which is joined first).  A replaced own one is
+// retired: a captured graph or a plan's launches may still point at it.
 int ensure_lane_work(ps_gpu_ctx* c, int lane, size_t bytes)
 {
     if (bytes <= c->lane_work_cap[lane]) return PS_OK;
-    if (c->lane_work[lane]) c->retired.push_back(c->lane_work[lane]);
+    const size_t rows = (size_t)c->N * c->N;
+    unsigned char* const base[3] = {(unsigned char*)c->f.work, (unsigned char*)c->f.ra, (unsigned char*)c->d.work};
+    const size_t size[3] = {rows * (size_t)c->f.S * sizeof(V2<float>), rows * (size_t)c->N * sizeof(float),
+                            rows * (size_t)c->d.S * sizeof(V2<double>)};
+    if (base[lane] && bytes <= size[lane]) {
+        c->lane_work[lane] = base[lane];
+        c->lane_work_cap[lane] = size[lane];
+        return PS_OK;
+    }
+    if (c->lane_work_own[lane]) c->retired.push_back(c->lane_work[lane]);
     c->lane_work[lane] = nullptr;
     c->lane_work_cap[lane] = 0;
+    c->lane_work_own[lane] = false;
     PS_TRY(alloc_dev(&c->lane_work[lane], bytes));
     c->lane_work_cap[lane] = bytes;
+    c->lane_work_own[lane] = true;
     return PS_OK;
 }
 
@@ -1825,7 +1837,7 @@ int prod_ops(ps_gpu_ctx* c, const std::vector<Shell>& host, const Shell* dtable,
             const Shell& sh = host[b.shells[q]];
             const int band = std::min(sh.band, M / 2), hb = band + 1, S = round_up(unit ? (hb + 1) / 2 : hb, pw<T>(M));
             V2<T>* dst = (V2<T>*)(base + b.at[q]);
-            xi.push_back(XItem<T>{dst, S, M / 2 + 1, dtable + b.shells[q]});
+            xi.push_back(XItem<T>{dst, S, M / 2 + 1, dtable + b.shells[q], 0});
             yi.push_back(YItem<T>{dst, S, S, band, M});
             where[b.shells[q]] = {dst, {S, hb}};
             Smax = std::max(Smax, S);
@@ -2353,7 +2365,7 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
                 *h = band + 1;
                 *S = round_up(*h, w);
                 V2<float>* dst = (V2<float>*)carve(rows * (size_t)*S * sizeof(V2<float>));
-                xi.push_back(XItem<float>{dst, *S, M / 2 + 1, dtable + shell});
+                xi.push_back(XItem<float>{dst, *S, M / 2 + 1, dtable + shell, 0});
                 yi.push_back(YItem<float>{dst, *S, *S, band, M});
                 Smax = std::max(Smax, *S);
                 bx += NN2 * (*S + *h) * V;
@@ -3185,6 +3197,9 @@ int plain_batch(ps_gpu_ctx* c, int nconf, ps_cfg* cfgs, double* B, double* Np, d
         PS_TRY(arena_take(&tmp, sizeof(double) * 4 * (size_t)nconf, &dh, &hh));
         double* h = (double*)hh;  // B, Npoly | sum D | sum |D|
         PS_TRY(plan_flush(&tmp));
+        // the counts of a prepared plan may still use the FP64 work spectrum
+        PS_CK(cudaEventRecord(c->ev_join, c->side_stream));
+        PS_CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
         double *sD = sums, *sI = sums + nconf, *sA = sums + 2 * (size_t)nconf;
         std::vector<ProdCfg> fit, large;
         for (const ProdCfg& g : prods) (prod_fits<double>(table, g, N, false) ? fit : large).push_back(g);
@@ -3252,16 +3267,29 @@ int grad_impl(ps_gpu_ctx* c, int n, const std::vector<Shell>& legs, double scale
     PS_TRY(alloc_dev(&B.hacc, nspec));
     PS_TRY(ensure_shells(c, PS_MAX_LEGS));
     PS_CK(cudaMemcpyAsync(c->dshells, legs.data(), sizeof(Shell) * n, cudaMemcpyHostToDevice, c->stream));
-    PS_CK(cudaMemsetAsync(B.hacc, 0, sizeof(V2<T>) * nspec, c->stream));
-    int hb = 1;
-    for (int l = 0; l < n; l++) hb = std::max(hb, std::min(legs[l].band, N / 2) + 1);
+    int band = 0;  // the gradient spectrum lives on the cube |components| <= band
+    for (int l = 0; l < n; l++) band = std::max(band, std::min(legs[l].band, N / 2));
+    const double cube = (double)(2 * band + 1) * (2 * band + 1) * (band + 1);
     if (n == 2) {
         Prof pf(c);
-        k_grad_pair2<T><<<148 * 8, 256, 0, c->stream>>>(N, B.spec, B.S, c->dshells, B.hacc, B.S, hb);
-        pf.end(fam<T>(KF_GRAD), 2.0 * N * N * hb * sizeof(V2<T>), N);
+        k_grad_pair2<T><<<148 * 8, 256, 0, c->stream>>>(N, B.spec, B.S, c->dshells, B.hacc, B.S, band);
+        pf.end(fam<T>(KF_GRAD), 2.0 * cube * sizeof(V2<T>), N);
     } else {
         // leg i: FFT of the product of the other two legs, masked by F_i;
-        // identical (mask, pair) terms are folded into one with a weight
+        // identical (mask, pair) terms are folded into one with a weight.  The products
+        // are formed on the smallest grid on which no triple of modes wraps around
+        // (alias_free_grid: the modes a mask keeps are then the full grid's, up to the
+        // factor (N/M)^3): 96 instead of 256 points for k = 0.8 at 256^3, L = 200.
+        const int M = alias_free_grid(N, std::min(legs[0].band, N / 2), std::min(legs[1].band, N / 2),
+                                      std::min(legs[2].band, N / 2));
+        const double up = ((double)N / M) * ((double)N / M) * ((double)N / M);
+        Tables<T> tm;
+        PS_TRY(tables_for<T>(c, M, &tm));
+        {
+            Prof pf(c);
+            k_zero_cube<T><<<148 * 8, 256, 0, c->stream>>>(N, band, B.hacc, B.S);
+            pf.end(fam<T>(KF_GRAD), cube * sizeof(V2<T>), N);
+        }
         std::vector<std::pair<std::vector<int>, int>> terms;
         for (int i = 0; i < 3; i++) {
             std::vector<int> key = {i, (i + 1) % 3, (i + 2) % 3};
@@ -3279,14 +3307,15 @@ int grad_impl(ps_gpu_ctx* c, int n, const std::vector<Shell>& legs, double scale
             }
             if (!found) terms.push_back({key, 1});
         }
-        for (const auto& tm : terms) {
-            const int li = tm.first[0], la = tm.first[1], lb = tm.first[2];
+        for (const auto& term : terms) {
+            const int li = term.first[0], la = term.first[1], lb = term.first[2];
             const bool same = same_shell(legs[la], legs[lb]);
             int Sa = 0, ha = 0, Sb = 0, hbb = 0, S = 0;
-            PS_TRY(c2r_xy<T>(c, LOAD_MASKED, c->dshells + la, legs[la].band, B.work, &Sa, &ha));
-            if (!same) PS_TRY(c2r_xy<T>(c, LOAD_MASKED, c->dshells + lb, legs[lb].band, B.work2, &Sb, &hbb));
+            PS_TRY(c2r_xy<T>(c, LOAD_MASKED, c->dshells + la, legs[la].band, B.work, &Sa, &ha, 0, M));
+            if (!same) PS_TRY(c2r_xy<T>(c, LOAD_MASKED, c->dshells + lb, legs[lb].band, B.work2, &Sb, &hbb, 0, M));
             const int hout = std::min(legs[li].band, N / 2) + 1;
-            PS_TRY(pair_spectrum<T>(c, B.work, Sa, ha, same ? nullptr : B.work2, Sb, hbb, hout, &S));
+            PS_TRY(pair_spectrum<T>(c, B.work, Sa, ha, same ? nullptr : B.work2, Sb, hbb, hout, &S, 0, M));
+            const int N = M;  // PS_SWITCH_N's subject
             Prof pf(c);
             FwdXItem<T> it{};
             it.data = B.work3;
@@ -3294,44 +3323,48 @@ int grad_impl(ps_gpu_ctx* c, int n, const std::vector<Shell>& legs, double scale
             it.hvalid = hout;
             it.shells = c->dshells + li;
             it.nshell = 1;
-            it.weight = (double)tm.second;
-            PS_SWITCH_N(N, PS_TRY((L3<T, NN>::fwd_x(c->stream, &it, 1, S, SPEC_MASK_ADD, B.hacc, B.S, nullptr, 0,
-                                                    B.tables(), nullptr))));
+            it.weight = up * (double)term.second;
+            PS_SWITCH_N(N, PS_TRY((L3<T, NN>::fwd_x(c->stream, &it, 1, S, SPEC_MASK_ADD, B.hacc, B.S, nullptr, 0, tm,
+                                                    nullptr, 0, c->N))));
             pf.end(fam<T>(KF_GRAD), 3.0 * N * N * S * sizeof(V2<T>), N);
         }
     }
     if (c->use_only_phase == 1) {  // the field entered through z/|z|
         Prof pf(c);
-        k_phase_adjoint<T><<<148 * 8, 256, 0, c->stream>>>((size_t)N * N, hb, B.hacc, B.S, B.spec, B.mod);
-        pf.end(fam<T>(KF_GRAD), 4.0 * N * N * hb * sizeof(V2<T>), N);
+        k_phase_adjoint<T><<<148 * 8, 256, 0, c->stream>>>(N, band, B.hacc, B.S, B.spec, B.mod);
+        pf.end(fam<T>(KF_GRAD), 4.0 * cube * sizeof(V2<T>), N);
     }
-    // inverse transform of the accumulated spectrum into B.ra, then scale
-    const int S = round_up(hb, pw<T>(N));
-    int nb = 0;
-    {
-        Prof pf(c);
-        PS_SWITCH_N(N, PS_TRY((L3<T, NN>::inv_x(c->stream, B.hacc, B.S, B.work, S, LOAD_PLAIN, nullptr, hb, B.tables()))));
-        pf.end(fam<T>(KF_INV_X), 2.0 * N * N * S * sizeof(V2<T>), N);
-    }
-    {
-        Prof pf(c);
-        PS_SWITCH_N(N, PS_TRY((L3<T, NN>::pass_y(c->stream, B.work, S, true, B.tables()))));
-        pf.end(fam<T>(KF_PASS_Y), 2.0 * N * N * S * sizeof(V2<T>), N);
-    }
-    {
-        Prof pf(c);
-        PS_SWITCH_N(N, PS_TRY((L3<T, NN>::inv_z(c->stream, B.work, S, hb, B.ra, nullptr, EPI_STORE, 1, nullptr,
-                                                B.tables(), &nb))));
-        pf.end(fam<T>(KF_INV_Z), (double)N * N * hb * sizeof(V2<T>) + (double)n3 * sizeof(T), N);
-    }
+    // inverse transform of the accumulated spectrum, scaled as it is stored: into
+    // out itself when that is device memory of the transform's type, else through
+    // B.ra and a conversion
     void* dst = out;
     void* stage = nullptr;
     const size_t out_bytes = n3 * (out_is_double ? 8 : 4);
+    const bool direct = out_mem == PS_MEM_DEVICE && (out_is_double != 0) == (sizeof(T) == 8) && (uintptr_t)out % sizeof(V2<T>) == 0;
     if (out_mem == PS_MEM_HOST) {
         PS_TRY(alloc_dev((unsigned char**)&stage, out_bytes));
         dst = stage;
     }
+    const int hb = band + 1, S = round_up(hb, pw<T>(N));
+    int nb = 0;
     {
+        Prof pf(c);
+        PS_SWITCH_N(N, PS_TRY((L3<T, NN>::inv_x(c->stream, B.hacc, B.S, B.work, S, LOAD_PLAIN, nullptr, hb, B.tables(), 0, 0,
+                                                1, band))));
+        pf.end(fam<T>(KF_INV_X), (double)N * N * S * sizeof(V2<T>) + cube * sizeof(V2<T>), N);
+    }
+    {
+        Prof pf(c);
+        PS_SWITCH_N(N, PS_TRY((L3<T, NN>::pass_y(c->stream, B.work, S, true, B.tables(), 0, band))));
+        pf.end(fam<T>(KF_PASS_Y), 2.0 * N * N * S * sizeof(V2<T>), N);
+    }
+    {
+        Prof pf(c);
+        PS_SWITCH_N(N, PS_TRY((L3<T, NN>::inv_z(c->stream, B.work, S, hb, direct ? (T*)out : B.ra, nullptr,
+                                                direct ? EPI_SCALE : EPI_STORE, 1, nullptr, B.tables(), &nb, scale))));
+        pf.end(fam<T>(KF_INV_Z), (double)N * N * hb * sizeof(V2<T>) + (double)n3 * sizeof(T), N);
+    }
+    if (!direct) {
         Prof pf(c);
         if (out_is_double)
             k_scale_out<T, double><<<148 * 8, 256, 0, c->stream>>>(B.ra, (double*)dst, n3, scale);
@@ -4388,7 +4421,8 @@ void ps_gpu_finalize(ps_gpu_ctx* c)
         cudaStreamSynchronize(c->lane2_stream);
         cudaStreamDestroy(c->lane2_stream);
     }
-    for (auto& p : c->lane_work) cudaFree(p);
+    for (int l = 0; l < 3; l++)
+        if (c->lane_work_own[l]) cudaFree(c->lane_work[l]);
     if (c->ev_join2) cudaEventDestroy(c->ev_join2);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);

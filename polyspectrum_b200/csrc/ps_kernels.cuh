@@ -221,6 +221,7 @@ template <typename T> struct XItem {  // inverse X
     int ds;              // row stride, a multiple of the pencil width
     int hvalid;
     const Shell* shell;  // NULL for plain loads
+    int band;            // plain loads: components above it are zero and not read
 };
 template <typename T> struct YItem {  // Y pass
     V2<T>* data;
@@ -270,7 +271,7 @@ __global__ void __launch_bounds__(PencilGeom<T, N>::THREADS)
     // skip_dead: a filtered tile whose |my| exceeds the shell's band holds only
     // zeros and is not written (the inverse Y pass then treats those rows as
     // zero, its jband)
-    if (skip_dead && mode != LOAD_PLAIN && abs(lattice_freq((int)(blockIdx.x / tiles_per_row), N)) > shell_p->band)
+    if (skip_dead && abs(lattice_freq((int)(blockIdx.x / tiles_per_row), N)) > (mode == LOAD_PLAIN ? it.band : shell_p->band))
         return;
     const V* tw = stage_table<V>(smem_raw, tw_g, N);
     __syncthreads();
@@ -291,15 +292,16 @@ __global__ void __launch_bounds__(PencilGeom<T, N>::THREADS)
     const size_t js = (size_t)(my < 0 ? my + nsrc : my);
     Shell sh;
     if (mode != LOAD_PLAIN) sh = *shell_p;
+    else sh.band = it.band;
     const bool pencil_live =
-        !quad && col_ok && (mode == LOAD_PLAIN || (abs(my) <= sh.band && abs(mz) <= sh.band));
+        !quad && col_ok && abs(my) <= sh.band && abs(mz) <= sh.band;
     // filter bits of this thread's R modes, one predicate instance (loop not unrolled)
     unsigned bits = 0u;
     if (pencil_live) {
         if (mode == LOAD_PLAIN) {
 #pragma unroll
             for (int e = 0; e < G::R; e++)
-                if (G::live(t + G::TPF * e)) bits |= 1u << e;
+                if (G::live(t + G::TPF * e) && abs(lattice_freq(t + G::TPF * e, N)) <= sh.band) bits |= 1u << e;
         } else {
 #pragma unroll 1
             for (int e = 0; e < G::R; e++) {
@@ -513,7 +515,8 @@ enum RealEpi : int {
     EPI_MUL_REDUCE = 2, // sum x^p * aux
     EPI_REDUCE = 3,     // sum x^p
     EPI_MUL_REDUCE_ABS = 4,  // sum |x^p * aux|  (condition numbers)
-    EPI_REDUCE_ABS = 5       // sum |x^p|
+    EPI_REDUCE_ABS = 5,      // sum |x^p|
+    EPI_SCALE = 6            // out = scale * x, the product in FP64
 };
 
 template <typename T> __device__ __forceinline__ T ipow(T x, int p)
@@ -528,7 +531,7 @@ template <typename T> __device__ __forceinline__ T ipow(T x, int p)
 template <typename T, int N>
 __global__ void __launch_bounds__(RowGeom<T, N>::THREADS)
     k_inv_z(const V2<T>* __restrict__ src, int src_stride, int hvalid, T* out, const T* aux,
-            int epi, int power, double* __restrict__ partials, const V2<T>* __restrict__ twr_g,
+            int epi, int power, double scale, double* __restrict__ partials, const V2<T>* __restrict__ twr_g,
             const V2<T>* __restrict__ twpp_g)
 {
     using G = RowGeom<T, N>;
@@ -563,6 +566,8 @@ __global__ void __launch_bounds__(RowGeom<T, N>::THREADS)
             T x0 = ipow(a[e].x, power), x1 = ipow(a[e].y, power);
             if (epi == EPI_STORE) {
                 *reinterpret_cast<V*>(orow + n2) = V{x0, x1};
+            } else if (epi == EPI_SCALE) {
+                *reinterpret_cast<V*>(orow + n2) = V{(T)(scale * (double)x0), (T)(scale * (double)x1)};
             } else if (epi == EPI_MUL_STORE) {
                 const V q = *reinterpret_cast<const V*>(arow + n2);
                 *reinterpret_cast<V*>(orow + n2) = V{x0 * q.x, x1 * q.y};
@@ -580,7 +585,7 @@ __global__ void __launch_bounds__(RowGeom<T, N>::THREADS)
         }
         __syncthreads();  // stage st is refilled two tiles later
     }
-    if (epi >= EPI_MUL_REDUCE) {
+    if (epi >= EPI_MUL_REDUCE && epi != EPI_SCALE) {
         const double s = block_sum<G::THREADS>(acc, red);
         if (threadIdx.x == 0) partials[blockIdx.x] = s;
     }
@@ -976,7 +981,7 @@ enum SpecEpi : int {
     SPEC_STORE_PHASE = 1,  // out = X / |X|  (utils_fftw.c:78-93)
     SPEC_DOT = 2,          // per shell c: sum_m w(h) F_c(m) Re(dk(m) conj(X(m)))
     SPEC_COUNT = 3,        // per shell c: sum_m w(h) F_c(m) rint(Re X(m) / N^3)
-    SPEC_MASK_ADD = 4,     // out += weight * F(m) X(m) where F selects (adjoint)
+    SPEC_MASK_ADD = 4,     // out += weight * F(m) X(m) where F selects (adjoint); out is of an ndk-grid
     SPEC_DOT_ABS = 5       // as SPEC_DOT with |term| (condition numbers)
 };
 
@@ -1145,7 +1150,9 @@ __global__ void __launch_bounds__(PencilGeom<T, N, RX>::THREADS,
             V v = a[e];
             if constexpr (KIND == FWD_MASK) {
                 if (!((keep >> e) & 1u)) continue;
-                V* o = out + ((size_t)i * N + j) * out_stride + h;
+                // mode m of this grid sits at m mod ndk of the accumulated spectrum
+                const int mx = lattice_freq(i, N);
+                V* o = out + ((size_t)(mx < 0 ? mx + ndk : mx) * ndk + jdk) * out_stride + h;
                 const V prev = *o;
                 *o = V{prev.x + (T)it.weight * v.x, prev.y + (T)it.weight * v.y};
                 continue;
@@ -1292,47 +1299,68 @@ static __global__ void __launch_bounds__(256)
 }
 
 // ------------------------------------------------------------------ adjoint helpers
+// Mode q of the cube |components| <= band of an n-grid's half spectrum (stride S):
+// its index, or false for +n/2 (the index of -n/2, visited as such).
+__device__ __forceinline__ bool cube_index(size_t q, int n, int band, int S, size_t& idx)
+{
+    const int side = 2 * band + 1, hb = band + 1;
+    const int h = (int)(q % hb);
+    const int my = (int)(q / hb % side) - band, mx = (int)(q / hb / side) - band;
+    if (mx >= n / 2 || my >= n / 2) return false;
+    idx = ((size_t)(mx < 0 ? mx + n : mx) * n + (my < 0 ? my + n : my)) * S + h;
+    return true;
+}
 // n = 2: dB/d(delta) needs L_a D_b + L_b D_a = IFFT[F_a FFT[D_b] + F_b FFT[D_a]]
 // with FFT[D] = N^3 F dk (the inverse transform is unnormalised), i.e.
-// IFFT[2 N^3 F_a F_b dk]; this writes that spectrum on the band h < hb (stride S).
+// IFFT[2 N^3 F_a F_b dk]; this writes that spectrum on the cube |components| <= band.
 template <typename T>
 __global__ void k_grad_pair2(int n, const V2<T>* __restrict__ dk, int dks, const Shell* __restrict__ shells,
-                             V2<T>* __restrict__ hacc, int S, int hb)
+                             V2<T>* __restrict__ hacc, int S, int band)
 {
-    const size_t total = (size_t)n * n * hb;
+    const size_t total = (size_t)(2 * band + 1) * (2 * band + 1) * (band + 1);
     for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (size_t)gridDim.x * blockDim.x) {
-        const int h = (int)(q % hb);
-        const size_t r = q / hb;
-        const int j = (int)(r % n), i = (int)(r / n);
-        const int mx = lattice_freq(i, n), my = lattice_freq(j, n), mz = h == n / 2 ? -(n / 2) : h;
+        size_t idx;
+        if (!cube_index(q, n, band, S, idx)) continue;
+        const int h = (int)(q % (band + 1));
+        const int my = (int)(q / (band + 1) % (2 * band + 1)) - band, mx = (int)(q / (band + 1) / (2 * band + 1)) - band;
+        const int mz = h == n / 2 ? -(n / 2) : h;
         V2<T> v = czero<V2<T>>();
-        if (h <= n / 2 && in_band(shells[0], mx, my, mz) && shell_bit(shells[0], mx, my, mz) &&
-            in_band(shells[1], mx, my, mz) && shell_bit(shells[1], mx, my, mz)) {
-            const V2<T> d = dk[r * dks + h];
+        if (in_band(shells[0], mx, my, mz) && shell_bit(shells[0], mx, my, mz) && in_band(shells[1], mx, my, mz) &&
+            shell_bit(shells[1], mx, my, mz)) {
+            const V2<T> d = dk[idx / S * dks + h];
             const T f = (T)(2.0 * (double)n * (double)n * (double)n);
             v = V2<T>{f * d.x, f * d.y};
         }
-        hacc[r * S + h] = v;
+        hacc[idx] = v;
     }
 }
 
 // Phase-only adjoint: the field enters through phi = z/|z| per mode, whose
 // differential is (dz - phi Re(conj(phi) dz)) / |z|; its transpose maps the
 // accumulated gradient spectrum H to (H - phi Re(conj(phi) H)) / |z| (in
-// place, rows of the half spectrum, h < hb).  Modes with H = 0 stay 0.
+// place, on the cube |components| <= band).  Modes with H = 0 stay 0.
 template <typename T>
-__global__ void k_phase_adjoint(size_t rows, int hb, V2<T>* __restrict__ hacc, int S,
-                                const V2<T>* __restrict__ phi, const T* __restrict__ mod)
+__global__ void k_phase_adjoint(int n, int band, V2<T>* __restrict__ hacc, int S, const V2<T>* __restrict__ phi,
+                                const T* __restrict__ mod)
 {
-    const size_t total = rows * (size_t)hb;
+    const size_t total = (size_t)(2 * band + 1) * (2 * band + 1) * (band + 1);
     for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (size_t)gridDim.x * blockDim.x) {
-        const size_t r = q / hb, idx = r * S + q % hb;
+        size_t idx;
+        if (!cube_index(q, n, band, S, idx)) continue;
         const V2<T> H = hacc[idx];
         if (H.x == (T)0 && H.y == (T)0) continue;
         const V2<T> u = phi[idx];
         const T m = mod[idx];
         const T p = u.x * H.x + u.y * H.y;  // Re(conj(phi) H)
         hacc[idx] = V2<T>{(H.x - u.x * p) / m, (H.y - u.y * p) / m};
+    }
+}
+template <typename T> __global__ void k_zero_cube(int n, int band, V2<T>* __restrict__ hacc, int S)
+{
+    const size_t total = (size_t)(2 * band + 1) * (2 * band + 1) * (band + 1);
+    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (size_t)gridDim.x * blockDim.x) {
+        size_t idx;
+        if (cube_index(q, n, band, S, idx)) hacc[idx] = czero<V2<T>>();
     }
 }
 

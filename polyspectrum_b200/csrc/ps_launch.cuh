@@ -90,9 +90,9 @@ template <typename T, int N> struct L3 {
     // skip_dead: tiles of all-zero pencils (|my| above the shell's band) are
     // left unwritten; the following pass_y must then be given that band
     static int inv_x(cudaStream_t st, const V* src, int ss, V* dst, int ds, int mode, const Shell* sh,
-                     int hvalid, const Tables<T>& tb, int quad = 0, int nsrc = 0, int skip_dead = 0)
+                     int hvalid, const Tables<T>& tb, int quad = 0, int nsrc = 0, int skip_dead = 0, int band = N)
     {
-        const XItem<T> it{dst, ds, hvalid, sh};
+        const XItem<T> it{dst, ds, hvalid, sh, band};
         return inv_x_b(st, src, ss, &it, 1, ds, mode, tb, quad, nsrc, skip_dead);
     }
     // The batched forms take nitems <= kItems descriptions (copied into the launch);
@@ -113,7 +113,7 @@ template <typename T, int N> struct L3 {
     static int pass_y_b(cudaStream_t st, const YItem<T>* items, int nitems, int ncols, bool inv,
                         const Tables<T>& tb, int quad, int alt);
     static int inv_z(cudaStream_t st, const V* src, int ss, int hvalid, T* out, const T* aux, int epi,
-                     int power, double* partials, const Tables<T>& tb, int* nblocks);
+                     int power, double* partials, const Tables<T>& tb, int* nblocks, double scale = 1.0);
     // stage: 1 copies the input rows to shared memory first (k_fwd_z STAGED),
     // 0 loads them straight into registers, -1 picks staging when it applies
     // (16-byte aligned inputs of 4- or 8-byte values, tile fits shared memory)

@@ -83,13 +83,13 @@ int L3<T, N>::pass_y_b(cudaStream_t st, const YItem<T>* items, int nitems, int n
 
 template <typename T, int N>
 int L3<T, N>::inv_z(cudaStream_t st, const V* src, int ss, int hvalid, T* out, const T* aux, int epi,
-                 int power, double* partials, const Tables<T>& tb, int* nblocks)
+                 int power, double* partials, const Tables<T>& tb, int* nblocks, double scale)
 {
     const size_t smem = RG::smem(1, hvalid, 0);
     PS_LTRY(set_smem(k_inv_z<T, N>, RG::smem(1, N / 2 + 1, 0)));
     int grid = 0;
     PS_LTRY(persistent_grid(k_inv_z<T, N>, RG::THREADS, smem, N * N / RG::WZ, &grid));
-    k_inv_z<T, N><<<grid, RG::THREADS, smem, st>>>(src, ss, hvalid, out, aux, epi, power, partials,
+    k_inv_z<T, N><<<grid, RG::THREADS, smem, st>>>(src, ss, hvalid, out, aux, epi, power, scale, partials,
                                                    tb.twr, tb.twpp);
     if (nblocks) *nblocks = grid;
     return PS_OK;
