@@ -2353,7 +2353,8 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
         std::vector<YItem<float>> yi, yf;
         std::vector<PairItem<float>> pi_;
         std::vector<FwdXItem<float>> fx, fa;
-        int Smax = 0, Pmax = 0, ha_max = 0, hb_max = 0, ninputs = 1;
+        int Smax = 0, Pmax = 0, ha_max = 0, hb_max = 0;
+        std::vector<PairItem<float>> sq;  // groups of one leg, after the two-leg ones in pi_
         double bx = 0.0, by = 0.0, bp = 0.0, byf = 0.0, bd = 0.0;  // algorithmic bytes
         const double V = sizeof(V2<float>), NN2 = (double)rows;
         const double wD = ((double)N / M) * ((double)N / M) * ((double)N / M);
@@ -2377,11 +2378,10 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
             const V2<float>* B = I.two ? leg(G.b, I.sb, &Sb, &hb) : nullptr;
             const int hout = I.hmax + 1, Sp = round_up(hout, w);
             V2<float>* D = (V2<float>*)carve(rows * (size_t)Sp * sizeof(V2<float>));
-            pi_.push_back(PairItem<float>{A, B, D, Sa, ha, Sb, hb, Sp, hout});
+            (B ? pi_ : sq).push_back(PairItem<float>{A, B, D, Sa, ha, Sb, hb, Sp, hout});
             yf.push_back(YItem<float>{D, Sp, Sp, M, hout - 1});
             ha_max = std::max(ha_max, ha);
             hb_max = std::max(hb_max, hb);
-            if (B) ninputs = 2;
             Pmax = std::max(Pmax, Sp);
             bp += NN2 * (ha + hb + hout) * V;
             byf += 2.0 * NN2 * Sp * V;
@@ -2421,7 +2421,8 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
         }
         Tables<float> tb;
         PS_TRY(tables_for<float>(c, M, &tb));
-        const int nx = (int)xi.size(), ngr = (int)gs.size(), nf = (int)fx.size();
+        const int nx = (int)xi.size(), ngr = (int)gs.size(), nf = (int)fx.size(), ntwo = (int)pi_.size();
+        pi_.insert(pi_.end(), sq.begin(), sq.end());
         *op = [=]() -> int {
             const int N = M;  // PS_SWITCH_N's subject
             // f(first, n): one launch per kItems items, its bytes in proportion
@@ -2444,11 +2445,14 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
                 PS_SWITCH_N(N, PS_TRY((L3<float, NN>::pass_y_b(c->stream, yi.data() + q, n, Smax, true, tb, 0, ya))));
                 return PS_OK;
             }));
-            PS_TRY(launches(KF_PAIR_Z, bp, ngr, [&](int q, int n) -> int {
-                PS_SWITCH_N(N, PS_TRY((L3<float, NN>::pair_z_b(c->stream, pi_.data() + q, n, ninputs, ha_max, hb_max, tb, 0,
-                                                               pair_var_of<float>(c, M)))));
-                return PS_OK;
-            }));
+            for (int two = 1; two >= 0; two--)
+                PS_TRY(launches(KF_PAIR_Z, bp * (two ? ntwo : ngr - ntwo) / ngr, two ? ntwo : ngr - ntwo,
+                                [&](int q, int n) -> int {
+                                    PS_SWITCH_N(N, PS_TRY((L3<float, NN>::pair_z_b(
+                                                       c->stream, pi_.data() + (two ? 0 : ntwo) + q, n, two ? 2 : 1, ha_max,
+                                                       hb_max, tb, 0, pair_var_of<float>(c, M)))));
+                                    return PS_OK;
+                                }));
             // rows |my| >= hout lie outside every shell a product is dotted with
             PS_TRY(launches(KF_PASS_Y, byf, ngr, [&](int q, int n) -> int {
                 PS_SWITCH_N(N, PS_TRY((L3<float, NN>::pass_y_b(c->stream, yf.data() + q, n, Pmax, false, tb, 0, ya))));

@@ -250,7 +250,9 @@ inline bool pair_count_lists(const Shell& sa, const Shell& sb, int N, int c_lo, 
     L->reps = interval_orbits(*pa, N);
     if (48.0 * (double)L->reps.size() * 4.19 * std::max(volume(*pb), 1.0) / 48.0 > 1.2e10) return false;
     L->modes = interval_modes(*pb, N);
-    if ((double)L->reps.size() * (double)L->modes.size() > 4e9) return false;
+    // about 5 (wrapping 1.2) pairs in a nanosecond; the transforms take 1.5 ms at 600 points
+    const bool wraps = std::min(sa.band, N / 2) + std::min(sb.band, N / 2) >= N / 2;
+    if ((double)L->reps.size() * (double)L->modes.size() > (wraps ? 1.5e9 : 4e9)) return false;
     const int bmax_a = std::min(sa.band, N / 2), bmax_b = std::min(sb.band, N / 2);
     L->wrap = bmax_a + bmax_b >= N / 2;
     const double ra_hi = sqrt((double)std::max(sa.r2hi, 0)), rb_hi = sqrt((double)std::max(sb.r2hi, 0));

@@ -2,8 +2,8 @@
 //
 // A transform of length N is done by TPF = N/R threads.  Thread t holds
 // a[e] = x[t + TPF*e] ("canonical layout") on entry and X[t + TPF*e] on exit.
-// N is a power of two, or 3 or 5 times one, for the register passes below;
-// other lengths 2^a 3^b 5^c take the shared-memory passes (GenericPlan).  Passes are
+// N is a power of two, or 3 or 5 times one, for the register passes below; the
+// other lengths 2^a 3^b 5^c are two passes of unequal radices (SplitPlan).  Passes are
 // radix-R (for N = f 2^k, R = f 2^r: radix-2^r passes, one of a smaller power
 // of two if needed, then one radix-R pass last); each thread does R/Rp
 // butterflies per pass.  Pass p with radix Rp and span Ns (product of the
@@ -95,10 +95,51 @@ template <int R, int K, bool INV, typename V> __device__ __forceinline__ V twidd
 }
 
 // Decimation-in-frequency DFT of length R in registers, natural order in and
-// out: even R splits into two halves, R = 3 and 5 are direct butterflies.
+// out: even R splits into two halves, R = 3 and 5 are direct butterflies, 15 and 25
+// go through columns of five.
 template <int R, bool INV> struct Dft {
-    static_assert(R % 2 == 0, "odd DFT lengths other than 3 and 5 are not provided");
+    static_assert(R % 2 == 0 || R == 15 || R == 25, "odd DFT lengths other than 3, 5, 15 and 25 are not provided");
+    // R = P Q odd: x[Q i + j] -> P-point DFTs over i, twiddles W_R^{j k}, Q-point
+    // DFTs over j, output P l + k
+    template <int J, int K, typename V> static __device__ __forceinline__ void twist(V* y)
+    {
+        constexpr int P = R / 5;
+        if constexpr (K < P) {
+            y[K] = twiddle_const<R, (J * K) % R, INV>(y[K]);
+            twist<J, K + 1>(y);
+        }
+    }
+    template <int J, typename V> static __device__ __forceinline__ void columns(const V* a, V (&y)[5][R / 5])
+    {
+        constexpr int P = R / 5;
+        if constexpr (J < 5) {
+#pragma unroll
+            for (int i = 0; i < P; i++) y[J][i] = a[5 * i + J];
+            Dft<P, INV>::run(y[J]);
+            twist<J, 0>(y[J]);
+            columns<J + 1>(a, y);
+        }
+    }
     template <typename V> static __device__ __forceinline__ void run(V* a)
+    {
+        if constexpr (R % 2 != 0) {
+            constexpr int P = R / 5;
+            V y[5][P];
+            columns<0>(a, y);
+#pragma unroll
+            for (int k = 0; k < P; k++) {
+                V z[5];
+#pragma unroll
+                for (int j = 0; j < 5; j++) z[j] = y[j][k];
+                Dft<5, INV>::run(z);
+#pragma unroll
+                for (int l = 0; l < 5; l++) a[P * l + k] = z[l];
+            }
+        } else {
+            halves(a);
+        }
+    }
+    template <typename V> static __device__ __forceinline__ void halves(V* a)
     {
         constexpr int H = R / 2;
         V b[H], c[H];
@@ -213,15 +254,33 @@ template <int N> struct DefaultRadix {
                                : N <= 16 ? N : (N == 32 || N == 64 || N == 128 || N == 512) ? 8 : 16;
 };
 
-// Thread layout of a transform of length L: R elements per thread, TPF
-// threads per transform (a power of two, so rows pack whole warps).  Lengths
-// whose odd part is 1, 3 or 5 use the register plan (TPF = L / R); the others
-// ("ragged": 30, 60, 150, 300, 600, ...) take TPF threads with R = ceil(L/TPF)
-// slots each, the last ones past L idle, and the shared-memory passes.
+// Lengths whose odd part is not 1, 3 or 5: N = RA RB in two passes, the factors as
+// equal as they come (the second at least the first), so that either pass is one
+// butterfly per thread and one exchange through shared memory lies between them.
+// Thread t does the butterflies v = t, t + TPF, ... of a pass: slot u R + q of its
+// array holds element v + q N / R, v = t + TPF u; slots of v >= N / R are idle.  The
+// layouts of input (pass A) and output (pass B) therefore differ, see SplitGeom.  A
+// sequence of radix-8/4/2, 3 and 5 passes through shared memory (five exchanges at 600
+// points) took 0.54 ms for a Y pass of 600^2 x 304 columns.
+template <int N> struct SplitPlan {
+    static constexpr int RA = N == 30 ? 5 : N == 60 ? 6 : N == 150 ? 10 : N == 300 ? 15 : N == 600 ? 24 : 0;
+    static constexpr int RB = RA ? N / RA : 0;
+    static constexpr bool value = RA > 0;
+};
+template <int N, int TPF> struct SplitGeom {
+    static constexpr int RA = SplitPlan<N>::RA, RB = SplitPlan<N>::RB;
+    static constexpr int BA = (RB + TPF - 1) / TPF, BB = (RA + TPF - 1) / TPF;  // butterflies per thread (N / RA = RB)
+    static constexpr int RI = BA * RA, RO = BB * RB;                            // slots in, out
+    __device__ static constexpr int ip(int t, int e) { return t + TPF * (e / RA) + (e % RA) * RB; }
+    __device__ static constexpr bool il(int t, int e) { return t + TPF * (e / RA) < RB; }
+    __device__ static constexpr int op(int t, int e) { return t + TPF * (e / RB) + (e % RB) * RA; }
+    __device__ static constexpr bool ol(int t, int e) { return t + TPF * (e / RB) < RA; }
+};
+
 template <int L> struct LenKind {
     __host__ __device__ static constexpr int odd_of(int n) { return n % 2 ? n : odd_of(n / 2); }
-    static constexpr bool RAGGED = !(odd_of(L) == 1 || odd_of(L) == 3 || odd_of(L) == 5);
-    static constexpr int RAGGED_TPF = L <= 32 ? 4 : L <= 64 ? 8 : L <= 160 ? 16 : 32;
+    static constexpr bool SPLIT = SplitPlan<L>::value;
+    static_assert(SPLIT || odd_of(L) == 1 || odd_of(L) == 3 || odd_of(L) == 5, "no plan for this length");
 };
 
 // Synchronisation between passes: the whole CTA (pencil kernels, whose
@@ -291,121 +350,64 @@ __device__ __forceinline__ void fft_passes(V (&a)[R], int t, Acc& sm, const V* _
     }
 }
 
-// Pass sequence of lengths N = 2^a 3^b 5^c whose odd part does not fit one
-// register pass ("ragged" transforms, e.g. 60, 150, 300, 600): radix-8 passes,
-// one radix-4 or -2 pass for the rest of the power of two, then one radix-3
-// pass per factor 3 and one radix-5 pass per factor 5.  Such transforms keep
-// their data in shared memory between passes; each thread does the
-// butterflies v = t, t + TPF, ... of a pass.
-template <int N> struct GenericPlan {
-    __host__ __device__ static constexpr int pow2_of(int n) { return n % 2 ? 1 : 2 * pow2_of(n / 2); }
-    __host__ __device__ static constexpr int count_of(int n, int f) { return n % f ? 0 : 1 + count_of(n / f, f); }
-    __host__ __device__ static constexpr int ilog2(int v) { return v > 1 ? 1 + ilog2(v / 2) : 0; }
-    static constexpr int A = ilog2(pow2_of(N));
-    static constexpr int B3 = count_of(N, 3), C5 = count_of(N, 5);
-    static constexpr int P8 = A / 3, PR = A % 3 ? 1 : 0;
-    static constexpr int P = P8 + PR + B3 + C5;
-    __host__ __device__ static constexpr int radix(int p)
-    {
-        return p < P8 ? 8 : (p < P8 + PR ? (A % 3 == 2 ? 4 : 2) : (p < P8 + PR + B3 ? 3 : 5));
-    }
-    __host__ __device__ static constexpr int span(int p)
-    {
-        int s = 1;
-        for (int q = 0; q < p; q++) s *= radix(q);
-        return s;
-    }
-    __host__ __device__ static constexpr int tw_off(int p)
-    {
-        int o = 0;
-        for (int q = 0; q < p; q++) o += span(q) * (radix(q) - 1);
-        return o;
-    }
-    __host__ __device__ static constexpr int product()
-    {
-        int s = 1;
-        for (int q = 0; q < P; q++) s *= radix(q);
-        return s;
-    }
-    static_assert(product() == N, "length must be 2^a 3^b 5^c");
-};
-
-// Whether a transform of N elements over TPF threads with R elements each
-// runs the register passes (RadixPlan; N = R * TPF with the odd part of N in
-// R) or the shared-memory passes of GenericPlan.
-template <int N, int R, int TPF> struct UseRegisterPlan {
-    __host__ __device__ static constexpr int odd_of(int n) { return n % 2 ? n : odd_of(n / 2); }
-    static constexpr bool value = R * TPF == N && odd_of(R) == odd_of(N) &&
-                                  (odd_of(R) == 1 || odd_of(R) == 3 || odd_of(R) == 5) &&
-                                  (odd_of(R) == 1 || R / odd_of(R) >= 2 || N == R);
-};
-
-// The passes of GenericPlan<N> on the transform held in shared memory behind
-// `sm` (positions 0..N-1); each thread does butterflies t, t + TPF, ...
-template <typename V, int N, int R, int TPF, bool INV, int P_ = 0, class Acc, class Sync>
-__device__ __forceinline__ void generic_passes(Acc& sm, int t, const V* __restrict__ twt, const Sync& sync)
+// The two passes of N = RA RB (see SplitPlan).  twt holds W_N^{k q}, k < A, q in
+// [1, B), at k (B - 1) + q - 1 for the factors A <= B of SplitPlan; with SWAP the
+// passes run as RB RA (RA, RB here being the swapped pair) on the same table.
+template <typename V, int N, int RA, int RB, int TPF, bool INV, bool SWAP, int SLOTS, class Acc, class Sync>
+__device__ __forceinline__ void split_passes(V (&a)[SLOTS], int t, Acc& sm, const V* __restrict__ twt, const Sync& sync)
 {
-    using Plan = GenericPlan<N>;
-    if constexpr (P_ < Plan::P) {
-        constexpr int Rp = Plan::radix(P_);
-        constexpr int Ns = Plan::span(P_);
-        constexpr int NB = N / Rp;                   // butterflies of the pass
-        constexpr int BPT = (NB + TPF - 1) / TPF;    // per thread (the last ones partly idle)
-        V b[BPT][Rp];
+    constexpr int BA = (RB + TPF - 1) / TPF, BB = (RA + TPF - 1) / TPF;
+    static_assert(BA * RA <= SLOTS && BB * RB <= SLOTS && RA * RB == N, "slots");
 #pragma unroll
-        for (int u = 0; u < BPT; u++) {
-            const int v = t + TPF * u;
-            if (v < NB) {
+    for (int u = 0; u < BA; u++) {
+        const int v = t + TPF * u;
+        if (v < RB) {
+            Dft<RA, INV>::run(&a[u * RA]);
 #pragma unroll
-                for (int q = 0; q < Rp; q++) b[u][q] = sm.ld(v + q * NB);
-            }
+            for (int q = 0; q < RA; q++) sm.st(v * RA + q, a[u * RA + q]);
         }
-        sync();
+    }
+    sync();
 #pragma unroll
-        for (int u = 0; u < BPT; u++) {
-            const int v = t + TPF * u;
-            if (v < NB) {
-                const int k = v % Ns;
-                if constexpr (Ns > 1) {
-                    const V* tp = twt + Plan::tw_off(P_) + k * (Rp - 1);
+    for (int u = 0; u < BB; u++) {
+        const int v = t + TPF * u;
+        if (v < RA) {
 #pragma unroll
-                    for (int q = 1; q < Rp; q++) {
-                        V w = tp[q - 1];
-                        if constexpr (INV) w.y = -w.y;
-                        b[u][q] = cmul(b[u][q], w);
-                    }
+            for (int q = 0; q < RB; q++) a[u * RB + q] = sm.ld(v + q * RA);
+        }
+    }
+    sync();
+#pragma unroll
+    for (int u = 0; u < BB; u++) {
+        const int v = t + TPF * u;
+        if (v < RA) {
+#pragma unroll
+            for (int q = 1; q < RB; q++) {
+                V w;
+                if constexpr (!SWAP) {
+                    w = twt[v * (RB - 1) + q - 1];
+                } else {  // entry (k = q, q = v), 1 for v = 0
+                    w = v > 0 ? twt[q * (RA - 1) + v - 1] : V{1, 0};
                 }
-                Dft<Rp, INV>::run(b[u]);
-                const int j = (v / Ns) * Ns * Rp + k;
-#pragma unroll
-                for (int q = 0; q < Rp; q++) sm.st(j + q * Ns, b[u][q]);
+                if constexpr (INV) w.y = -w.y;
+                a[u * RB + q] = cmul(a[u * RB + q], w);
             }
+            Dft<RB, INV>::run(&a[u * RB]);
         }
-        sync();
-        generic_passes<V, N, R, TPF, INV, P_ + 1>(sm, t, twt, sync);
     }
 }
 
-// A transform of length N held by TPF threads, R elements each (canonical
-// layout a[e] = x[t + TPF e]; with R * TPF > N the entries past N are not
-// part of the transform and are left as they are).  Register passes when the
-// length allows them, else shared-memory passes; either way the buffer behind
-// `sm` holds N elements.
-template <typename V, int N, int R, int TPF, bool INV, class Acc, class Sync>
-__device__ __forceinline__ void fft_any(V (&a)[R], int t, Acc& sm, const V* __restrict__ twt, const Sync& sync)
+// A transform in the geometry G of a kernel (input layout G::ip, output G::op; SWAP:
+// the other way round), register passes or split.
+template <class G, typename V, int N, bool INV, bool SWAP = false, class Acc, class Sync>
+__device__ __forceinline__ void fft_geom(V (&a)[G::R], int t, Acc& sm, const V* __restrict__ twt, const Sync& sync)
 {
-    if constexpr (UseRegisterPlan<N, R, TPF>::value) {
-        fft_passes<V, N, R, INV>(a, t, sm, twt, sync);
+    if constexpr (!LenKind<N>::SPLIT) {
+        fft_passes<V, N, G::R, INV>(a, t, sm, twt, sync);
+    } else if constexpr (SWAP) {
+        split_passes<V, N, SplitPlan<N>::RB, SplitPlan<N>::RA, G::TPF, INV, true>(a, t, sm, twt, sync);
     } else {
-#pragma unroll
-        for (int e = 0; e < R; e++)
-            if (t + TPF * e < N) sm.st(t + TPF * e, a[e]);
-        sync();
-        generic_passes<V, N, R, TPF, INV>(sm, t, twt, sync);
-#pragma unroll
-        for (int e = 0; e < R; e++)
-            if (t + TPF * e < N) a[e] = sm.ld(t + TPF * e);
-        sync();
+        split_passes<V, N, SplitPlan<N>::RA, SplitPlan<N>::RB, G::TPF, INV, false>(a, t, sm, twt, sync);
     }
 }
 
@@ -425,12 +427,21 @@ template <typename V, class Plan> inline void plan_table(V* out)
             }
     }
 }
-template <typename V, int N, int R> inline void stockham_table(V* out) { plan_table<V, RadixPlan<N, R>>(out); }
-// the table of the transform fft_any<V, N, R, TPF> runs
-template <typename V, int N, int R, int TPF> inline void transform_table(V* out)
+// the table of the transform fft_geom runs with R elements per thread
+template <typename V, int N, int R> inline void transform_table(V* out)
 {
-    if constexpr (UseRegisterPlan<N, R, TPF>::value) plan_table<V, RadixPlan<N, R>>(out);
-    else plan_table<V, GenericPlan<N>>(out);
+    if constexpr (!LenKind<N>::SPLIT) {
+        plan_table<V, RadixPlan<N, R>>(out);
+    } else {
+        const long double two_pi = 6.283185307179586476925286766559005768L;
+        constexpr int RA = SplitPlan<N>::RA, RB = SplitPlan<N>::RB;
+        for (int k = 0; k < RA; k++)
+            for (int q = 1; q < RB; q++) {
+                const long double a = two_pi * (long double)(q * k) / (long double)N;
+                out[k * (RB - 1) + q - 1].x = (decltype(out->x))cosl(a);
+                out[k * (RB - 1) + q - 1].y = (decltype(out->x))(-sinl(a));
+            }
+    }
 }
 
 // Shared-memory accessor for pencil passes: W transforms interleaved, element

@@ -80,7 +80,7 @@ double time_pass_y(int reps, float2* data, int S, int ncols, int jband, int jout
 {
     using G = PencilGeom<float, M, RX>;
     std::vector<float2> hp(M);
-    transform_table<float2, M, G::R, G::TPF>(hp.data());
+    transform_table<float2, M, G::R>(hp.data());
     float2* tw;
     CK(cudaMalloc(&tw, M * 8));
     CK(cudaMemcpy(tw, hp.data(), M * 8, cudaMemcpyHostToDevice));
@@ -112,7 +112,7 @@ template <int M, int RX> float2* pair_row_table()
 {
     using G = RowGeom<float, M, RX>;
     std::vector<float2> hr(M / 2);
-    transform_table<float2, M / 2, G::R, G::TPF>(hr.data());
+    transform_table<float2, M / 2, G::R>(hr.data());
     float2* d;
     CK(cudaMalloc(&d, M / 2 * 8));
     CK(cudaMemcpy(d, hr.data(), M / 2 * 8, cudaMemcpyHostToDevice));
@@ -143,10 +143,10 @@ double time_pair(int reps, const float2* wa, int Sa, int ba, const float2* wb, i
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
     for (int it = 0; it < 3; it++)
-        kern<<<grid, G::THREADS, smem>>>(items, nrows, twr, twpp);
+        kern<<<grid, G::THREADS, smem>>>(items, nrows, 0, twr, twpp);
     CK(cudaEventRecord(e0));
     for (int it = 0; it < reps; it++)
-        kern<<<grid, G::THREADS, smem>>>(items, nrows, twr, twpp);
+        kern<<<grid, G::THREADS, smem>>>(items, nrows, 0, twr, twpp);
     CK(cudaEventRecord(e1));
     CK(cudaEventSynchronize(e1));
     CK(cudaGetLastError());

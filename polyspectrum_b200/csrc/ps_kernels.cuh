@@ -43,20 +43,26 @@ template <typename T> struct PencilWidth { static constexpr int value = 128 / (i
 
 // Threads per pencil (strided-axis) transform: N / (register-plan radix),
 // with radix 16 for FP32 at N = 512 so a CTA of 16 pencils is 512 threads;
-// ragged lengths take LenKind's thread count (64 for FP64 pencils above 512).
+// split lengths take the larger factor, rounded up so that a CTA is whole warps.
 template <typename T, int N> struct PencilThreads {
-    static constexpr int value = LenKind<N>::RAGGED ? ((sizeof(T) == 8 && N > 512) ? 64 : LenKind<N>::RAGGED_TPF)
+    static constexpr int split(int v) { return v * PencilWidth<T>::value % 32 ? split(v + 1) : v; }
+    static constexpr int value = LenKind<N>::SPLIT ? split(SplitPlan<N>::RB)
                                : N / ((sizeof(T) == 4 && N == 512) ? 16 : DefaultRadix<N>::value);
 };
 // RX > 0 overrides the elements per thread of a register-plan pencil length
 // (pass variants with fewer, larger radix passes).
 template <typename T, int N, int RX = 0> struct PencilGeom {
-    static constexpr int TPF = RX > 0 && !LenKind<N>::RAGGED ? N / RX : PencilThreads<T, N>::value;
-    static constexpr int R = (N + TPF - 1) / TPF;
-    // element e of thread t is position t + TPF e of the transform; with
-    // R * TPF > N (ragged lengths) the positions past N are idle slots
-    static constexpr bool FULL = R * TPF == N;
-    __device__ static constexpr bool live(int pos) { return FULL || pos < N; }
+    static constexpr bool SPLIT = LenKind<N>::SPLIT;
+    static constexpr int TPF = RX > 0 && !SPLIT ? N / RX : PencilThreads<T, N>::value;
+    using SG = SplitGeom<SPLIT ? N : 600, TPF>;
+    // slots of a thread going in and coming out, and what they hold: position
+    // ip(t, e) where il(t, e), op and ol likewise (register plans: t + TPF e, all live)
+    static constexpr int RI = SPLIT ? SG::RI : N / TPF, RO = SPLIT ? SG::RO : N / TPF;
+    static constexpr int R = RI > RO ? RI : RO;
+    __device__ static constexpr int ip(int t, int e) { return SPLIT ? SG::ip(t, e) : t + TPF * e; }
+    __device__ static constexpr bool il(int t, int e) { return !SPLIT || SG::il(t, e); }
+    __device__ static constexpr int op(int t, int e) { return SPLIT ? SG::op(t, e) : t + TPF * e; }
+    __device__ static constexpr bool ol(int t, int e) { return !SPLIT || SG::ol(t, e); }
     // one 128-byte segment per row, whole warps per CTA, at most 512 threads
     // (so an epilogue keeps 16 FP64 accumulators in registers)
     static constexpr int W0 = PencilWidth<T>::value * TPF >= 32 ? PencilWidth<T>::value : 32 / TPF;
@@ -76,7 +82,7 @@ template <typename T, int N, int RX = 0> struct PencilGeom {
 // pencil, one radix pass fewer (0: none).  Chosen per length by the plan
 // autotuner against the default.
 template <typename T, int N> struct PencilAlt {
-    static constexpr int value = (sizeof(T) == 4 && !LenKind<N>::RAGGED && N >= 128 && N <= 512) ? 2 * PencilGeom<T, N>::R : 0;
+    static constexpr int value = (sizeof(T) == 4 && !LenKind<N>::SPLIT && N >= 128 && N <= 512) ? 2 * PencilGeom<T, N>::R : 0;
 };
 
 // Elements per thread of the row (contiguous-axis) transforms of length NH:
@@ -93,18 +99,38 @@ template <typename T, int NH> struct RowRadix {
 // (the pair kernel's variants).
 template <typename T, int N, int RX = 0> struct RowGeom {
     static constexpr int NH = N / 2;
-    static constexpr int TPF = LenKind<NH>::RAGGED ? LenKind<NH>::RAGGED_TPF : NH / (RX > 0 ? RX : RowRadix<T, NH>::value);
-    static constexpr int R = (NH + TPF - 1) / TPF;
-    // element e of thread t is pair t + TPF e of the row; with R * TPF > NH
-    // (ragged lengths) the pairs past NH are idle slots
-    static constexpr bool FULL = R * TPF == NH;
-    __device__ static constexpr bool live(int n) { return FULL || n < NH; }
+    static constexpr bool SPLIT = LenKind<NH>::SPLIT;
+    // split rows (30, 150, 300): a power of two of threads, so that rows pack warps
+    static constexpr int TPF = SPLIT ? (NH == 30 ? 8 : NH == 150 ? 16 : sizeof(T) == 4 ? 16 : 32)
+                                     : NH / (RX > 0 ? RX : RowRadix<T, NH>::value);
+    using SG = SplitGeom<SPLIT ? NH : 300, TPF>;
+    // slots of a thread on the spectrum side (kp, kl: column k) and on the real side
+    // (tp, tl: pair n of the row); register plans: t + TPF e on both, all live
+    static constexpr int RK = SPLIT ? SG::RI : NH / TPF, RT = SPLIT ? SG::RO : NH / TPF;
+    static constexpr int R = RK > RT ? RK : RT;
+    __device__ static constexpr int kp(int t, int e) { return SPLIT ? SG::ip(t, e) : t + TPF * e; }
+    __device__ static constexpr bool kl(int t, int e) { return !SPLIT || SG::il(t, e); }
+    __device__ static constexpr int tp(int t, int e) { return SPLIT ? SG::op(t, e) : t + TPF * e; }
+    __device__ static constexpr bool tl(int t, int e) { return !SPLIT || SG::ol(t, e); }
     static constexpr int EPC = 16 / (int)sizeof(V2<T>);  // complex elements per 16-byte copy
+    // Rows shorter than a 128-byte block of threads share a warp: their buffers are
+    // set apart by SKEW elements modulo a block, so that the rows of a warp fall on
+    // different banks (rows of 4 threads at 96 points: two of three shared-memory
+    // accesses were conflicts, pair kernel of 13 equilateral groups at 128 points
+    // 0.134 -> @@ ms).
+    static constexpr int BLOCK = 128 / (int)sizeof(V2<T>);
+    static constexpr int SKEW = TPF < BLOCK ? (TPF < EPC ? EPC : TPF) : 0;
     // rows per CTA (tile): up to 256 threads and 32 rows, and as many as fit
     // in 227 KB of shared memory with two double-buffered full-length inputs
     static constexpr int WZ0 = (256 / TPF) < 32 ? (256 / TPF) : 32;
-    static constexpr size_t ROW_BYTES =
-        (size_t)((NH < 16 ? NH : (NH + 15) / 16 * 16) + 4 * ((NH + 1 + EPC - 1) / EPC * EPC)) * sizeof(V2<T>);
+    static constexpr int ROWBUF = (NH < 16 ? NH : (NH + 15) / 16 * 16) + SKEW;
+    // input stage pitch (elements) for rows of hv valid entries
+    __host__ __device__ static constexpr int pitch(int hv)
+    {
+        const int p = (hv + EPC - 1) / EPC * EPC;
+        return SKEW ? p + (SKEW + BLOCK - p % BLOCK) % BLOCK : p;
+    }
+    static constexpr size_t ROW_BYTES = (size_t)(ROWBUF + 4 * pitch(NH + 1)) * sizeof(V2<T>);
     static constexpr int WZ_FIT = (int)((227 * 1024 - (size_t)(2 * NH + 2) * sizeof(V2<T>)) / ROW_BYTES);
     __host__ __device__ static constexpr int pow2_floor(int v) { return v >= 2 ? 2 * pow2_floor(v / 2) : 1; }
     // and a divisor of the N^2 rows, so whole tiles cover the grid
@@ -117,11 +143,8 @@ template <typename T, int N, int RX = 0> struct RowGeom {
     static constexpr size_t TWPP_OFF = TWR_OFF + (size_t)NH * sizeof(V2<T>);
     static constexpr size_t ROWBUF_OFF = TWPP_OFF + (size_t)(NH + 2) * sizeof(V2<T>);
     // row exchange buffers hold whole swizzle blocks of SmemRow (16 elements:
-    // its XOR stays inside a block, which a ragged NH may end in the middle of)
-    static constexpr int ROWBUF = NH < 16 ? NH : (NH + 15) / 16 * 16;
+    // its XOR stays inside a block, which a split NH may end in the middle of)
     static constexpr size_t STAGE_OFF = ROWBUF_OFF + (size_t)WZ * ROWBUF * sizeof(V2<T>);
-    // input stage pitch (elements) for rows of hv valid entries
-    __host__ __device__ static constexpr int pitch(int hv) { return (hv + EPC - 1) / EPC * EPC; }
     // dynamic shared memory of a kernel with `ninputs` double-buffered inputs
     __host__ __device__ static constexpr size_t smem(int ninputs, int hva, int hvb)
     {
@@ -300,13 +323,13 @@ __global__ void __launch_bounds__(PencilGeom<T, N>::THREADS)
     if (pencil_live) {
         if (mode == LOAD_PLAIN) {
 #pragma unroll
-            for (int e = 0; e < G::R; e++)
-                if (G::live(t + G::TPF * e) && abs(lattice_freq(t + G::TPF * e, N)) <= sh.band) bits |= 1u << e;
+            for (int e = 0; e < G::RI; e++)
+                if (G::il(t, e) && abs(lattice_freq(G::ip(t, e), N)) <= sh.band) bits |= 1u << e;
         } else {
 #pragma unroll 1
-            for (int e = 0; e < G::R; e++) {
-                if (!G::live(t + G::TPF * e)) continue;
-                const int mx = lattice_freq(t + G::TPF * e, N);
+            for (int e = 0; e < G::RI; e++) {
+                if (!G::il(t, e)) continue;
+                const int mx = lattice_freq(G::ip(t, e), N);
                 if (abs(mx) <= sh.band && shell_bit(sh, mx, my, mz)) bits |= 1u << e;
             }
         }
@@ -315,38 +338,38 @@ __global__ void __launch_bounds__(PencilGeom<T, N>::THREADS)
     if constexpr (sizeof(T) == 8) {
         if (quad) {
 #pragma unroll
-            for (int e = 0; e < G::R; e++) a[e] = czero<V>();
+            for (int e = 0; e < G::RI; e++) a[e] = czero<V>();
             for (int lane = 0; lane < 2; lane++) {
                 const int hz = 2 * h + lane, mzq = hz == N / 2 ? -(N / 2) : hz;
                 if (hz > N / 2 || hz >= hvalid || abs(my) > sh.band || abs(mzq) > sh.band) continue;
                 unsigned in = 0u;
 #pragma unroll 1
-                for (int e = 0; e < G::R; e++) {
-                    if (!G::live(t + G::TPF * e)) continue;
-                    const int mx = lattice_freq(t + G::TPF * e, N);
+                for (int e = 0; e < G::RI; e++) {
+                    if (!G::il(t, e)) continue;
+                    const int mx = lattice_freq(G::ip(t, e), N);
                     if (abs(mx) <= sh.band && shell_bit(sh, mx, my, mzq)) in |= 1u << e;
                 }
 #pragma unroll
-                for (int e = 0; e < G::R; e++)
+                for (int e = 0; e < G::RI; e++)
                     if ((in >> e) & 1u) (lane ? a[e].y : a[e].x) = (T)1;
             }
         }
     }
 #pragma unroll
-    for (int e = 0; e < G::R; e++) {
+    for (int e = 0; e < G::RI; e++) {
         if (sizeof(T) == 8 && quad) break;
-        const int mx = lattice_freq(t + G::TPF * e, N);
+        const int mx = lattice_freq(G::ip(t, e), N);
         V v = czero<V>();
         if ((bits >> e) & 1u) {
             v = src[((size_t)(mx < 0 ? mx + nsrc : mx) * nsrc + js) * src_stride + h];
         }
         a[e] = v;
     }
-    fft_any<V, N, G::R, G::TPF, true>(a, t, sm, tw, BlockSync{});
+    fft_geom<G, V, N, true>(a, t, sm, tw, BlockSync{});
 #pragma unroll
-    for (int e = 0; e < G::R; e++) {
-        const int i = t + G::TPF * e;
-        if (G::live(i) && (!quad || i <= N / 2)) dst[((size_t)i * nj + j) * dst_stride + h] = a[e];
+    for (int e = 0; e < G::RO; e++) {
+        const int i = G::op(t, e);
+        if (G::ol(t, e) && (!quad || i <= N / 2)) dst[((size_t)i * nj + j) * dst_stride + h] = a[e];
     }
 }
 
@@ -375,21 +398,21 @@ __global__ void __launch_bounds__(PencilGeom<T, N, RX>::THREADS)
     // pass of a band-limited shell leaves them unwritten)
     V a[G::R];
 #pragma unroll
-    for (int e = 0; e < G::R; e++) {
-        const int j = t + G::TPF * e;
+    for (int e = 0; e < G::RI; e++) {
+        const int j = G::ip(t, e);
         const int jr = quad && j > N / 2 ? N - j : j;
-        a[e] = G::live(j) && (jband >= N / 2 || abs(lattice_freq(j, N)) <= jband) ? base[(size_t)jr * stride]
+        a[e] = G::il(t, e) && (jband >= N / 2 || abs(lattice_freq(j, N)) <= jband) ? base[(size_t)jr * stride]
                                                                                   : czero<V>();
     }
     const V* tw = stage_table<V>(smem_raw, tw_g, N);
     __syncthreads();
     SmemInterleaved<V, G::W> sm{reinterpret_cast<V*>(smem_raw + G::TW_BYTES), w};
-    fft_any<V, N, G::R, G::TPF, INV>(a, t, sm, tw, BlockSync{});
+    fft_geom<G, V, N, INV>(a, t, sm, tw, BlockSync{});
 #pragma unroll
-    for (int e = 0; e < G::R; e++) {
-        const int j = t + G::TPF * e;
+    for (int e = 0; e < G::RO; e++) {
+        const int j = G::op(t, e);
         // jout < N/2: rows with |my| > jout are read by no later pass and not stored
-        if (G::live(j) && (!quad || j <= N / 2) && (jout >= N / 2 || abs(lattice_freq(j, N)) <= jout))
+        if (G::ol(t, e) && (!quad || j <= N / 2) && (jout >= N / 2 || abs(lattice_freq(j, N)) <= jout))
             base[(size_t)j * stride] = a[e];
     }
 }
@@ -434,9 +457,9 @@ __device__ __forceinline__ void c2r_row(const V2<T>* zr, int hv, RowCtx<T, N, RX
     using V = V2<T>;
     constexpr int NH = G::NH;
 #pragma unroll
-    for (int e = 0; e < G::R; e++) {
-        const int k = rc.t + G::TPF * e;
-        if (!G::live(k)) {
+    for (int e = 0; e < G::RK; e++) {
+        const int k = G::kp(rc.t, e);
+        if (!G::kl(rc.t, e)) {
             a[e] = czero<V>();
             continue;
         }
@@ -446,8 +469,9 @@ __device__ __forceinline__ void c2r_row(const V2<T>* zr, int hv, RowCtx<T, N, RX
         const V B = cmul(csub(zk, zm), cconj(rc.twpp[k]));  // exp(+2 pi i k / N)
         a[e] = V{A.x - B.y, A.y + B.x};
     }
+    rc.sync();  // the exchange buffer may be the row just read
     SmemRow<V> sm{rc.rowbuf};
-    fft_any<V, NH, G::R, G::TPF, true>(a, rc.t, sm, rc.twr, rc.sync);
+    fft_geom<G, V, NH, true>(a, rc.t, sm, rc.twr, rc.sync);
     rc.sync();
 }
 
@@ -460,9 +484,9 @@ __device__ __forceinline__ void c2r_row_real(const T* zr, int hv, RowCtx<T, N, R
     using V = V2<T>;
     constexpr int NH = G::NH;
 #pragma unroll
-    for (int e = 0; e < G::R; e++) {
-        const int k = rc.t + G::TPF * e;
-        if (!G::live(k)) {
+    for (int e = 0; e < G::RK; e++) {
+        const int k = G::kp(rc.t, e);
+        if (!G::kl(rc.t, e)) {
             a[e] = czero<V>();
             continue;
         }
@@ -471,8 +495,9 @@ __device__ __forceinline__ void c2r_row_real(const T* zr, int hv, RowCtx<T, N, R
         const V w = rc.twpp[k];  // B = D conj(w)
         a[e] = V{A + D * w.y, D * w.x};
     }
+    rc.sync();  // the exchange buffer may be the row just read
     SmemRow<V> sm{rc.rowbuf};
-    fft_any<V, NH, G::R, G::TPF, true>(a, rc.t, sm, rc.twr, rc.sync);
+    fft_geom<G, V, NH, true>(a, rc.t, sm, rc.twr, rc.sync);
     rc.sync();
 }
 
@@ -486,11 +511,11 @@ __device__ __forceinline__ void r2c_row(V2<T> (&a)[RowGeom<T, N, RX>::R], RowCtx
     using V = V2<T>;
     constexpr int NH = G::NH;
     SmemRow<V> sm{rc.rowbuf};
-    fft_any<V, NH, G::R, G::TPF, false>(a, rc.t, sm, rc.twr, rc.sync);
+    fft_geom<G, V, NH, false, true>(a, rc.t, sm, rc.twr, rc.sync);
     rc.sync();
 #pragma unroll
-    for (int e = 0; e < G::R; e++)
-        if (G::live(rc.t + G::TPF * e)) sm.st(rc.t + G::TPF * e, a[e]);
+    for (int e = 0; e < G::RK; e++)
+        if (G::kl(rc.t, e)) sm.st(G::kp(rc.t, e), a[e]);
     rc.sync();
     const T half = (T)0.5;
     for (int k = rc.t; k <= NH && k < hout; k += G::TPF) {
@@ -560,9 +585,9 @@ __global__ void __launch_bounds__(RowGeom<T, N>::THREADS)
         T* orow = out ? out + row * N : nullptr;
         const T* arow = aux ? aux + row * N : nullptr;
 #pragma unroll
-        for (int e = 0; e < G::R; e++) {
-            if (!G::live(rc.t + G::TPF * e)) continue;
-            const int n2 = 2 * (rc.t + G::TPF * e);
+        for (int e = 0; e < G::RT; e++) {
+            if (!G::tl(rc.t, e)) continue;
+            const int n2 = 2 * (G::tp(rc.t, e));
             T x0 = ipow(a[e].x, power), x1 = ipow(a[e].y, power);
             if (epi == EPI_STORE) {
                 *reinterpret_cast<V*>(orow + n2) = V{x0, x1};
@@ -750,27 +775,27 @@ __global__ void __launch_bounds__(RowGeom<T, N>::THREADS,
         const unsigned char* ra = sa + (size_t)w0 * N * eb;
         const unsigned char* rb = gb ? sb + (size_t)w0 * N * eb : nullptr;
 #pragma unroll
-        for (int e = 0; e < G::R; e++)
-            a[e] = G::live(t0 + G::TPF * e) ? load_pair<T>(kind, ra, rb, t0 + G::TPF * e) : czero<V>();
+        for (int e = 0; e < G::RT; e++)
+            a[e] = G::tl(t0, e) ? load_pair<T>(kind, ra, rb, G::tp(t0, e)) : czero<V>();
         r2c_row<T, N>(a, rc, dst + row * dst_stride, hout);
     } else {
         if (kind == SRC_T) {
             const V* xr = reinterpret_cast<const V*>((const T*)a_src + row * N);
 #pragma unroll
-            for (int e = 0; e < G::R; e++) a[e] = G::live(t0 + G::TPF * e) ? xr[t0 + G::TPF * e] : czero<V>();
+            for (int e = 0; e < G::RT; e++) a[e] = G::tl(t0, e) ? xr[G::tp(t0, e)] : czero<V>();
         } else if (vec) {
             // both values of a pair in one 8- or 16-byte load per array
             const int eb = (kind == SRC_F32 || kind == SRC_XHI_F32) ? 4 : 8;
             const unsigned char* ra = reinterpret_cast<const unsigned char*>(a_src) + row * N * eb;
             const unsigned char* rb = b_src ? reinterpret_cast<const unsigned char*>(b_src) + row * N * eb : nullptr;
 #pragma unroll
-            for (int e = 0; e < G::R; e++)
-                a[e] = G::live(t0 + G::TPF * e) ? load_pair<T>(kind, ra, rb, t0 + G::TPF * e) : czero<V>();
+            for (int e = 0; e < G::RT; e++)
+                a[e] = G::tl(t0, e) ? load_pair<T>(kind, ra, rb, G::tp(t0, e)) : czero<V>();
         } else {
 #pragma unroll
-            for (int e = 0; e < G::R; e++) {
-                const size_t n2 = row * N + 2 * (t0 + G::TPF * e);
-                a[e] = G::live(t0 + G::TPF * e)
+            for (int e = 0; e < G::RT; e++) {
+                const size_t n2 = row * N + 2 * (G::tp(t0, e));
+                a[e] = G::tl(t0, e)
                            ? V{load_real<T>(kind, a_src, b_src, n2), load_real<T>(kind, a_src, b_src, n2 + 1)}
                            : czero<V>();
             }
@@ -793,9 +818,12 @@ __global__ void __launch_bounds__(RowGeom<T, N>::THREADS,
 template <typename T, int N, int RX, bool KEEP> struct PairGeom {
     using G = RowGeom<T, N, RX>;
     // dynamic shared memory: the row kernels' layout, then the keep buffers
-    __host__ __device__ static constexpr size_t smem(int ninputs, int hva, int hvb)
+    __host__ __device__ static constexpr size_t smem(int ninputs, int hva, int hvb, bool alias = false)
     {
-        return G::smem(ninputs, hva, hvb) + (KEEP ? (size_t)G::WZ * G::ROWBUF * sizeof(V2<T>) : 0);
+        const int pa = G::pitch(hva);
+        return (alias ? G::ROWBUF_OFF + (size_t)2 * G::WZ * ((pa > G::ROWBUF ? pa : G::ROWBUF) + (ninputs > 1 ? G::pitch(hvb) : 0)) * sizeof(V2<T>)
+                      : G::smem(ninputs, hva, hvb)) +
+               (KEEP ? (size_t)G::WZ * G::ROWBUF * sizeof(V2<T>) : 0);
     }
     static constexpr bool FITS = smem(2, N / 2 + 1, N / 2 + 1) <= 227 * 1024;
 };
@@ -806,7 +834,7 @@ template <typename T, int N, int RX, bool KEEP> struct PairGeom {
 // thread (one radix pass fewer, half the threads per row).  KEEP_OK /
 // ALT_RX (0: none) say which exist for a length.
 template <typename T, int N> struct PairVariants {
-    static constexpr bool REG = sizeof(T) == 4 && !LenKind<N / 2>::RAGGED && N >= 128 && N <= 512;
+    static constexpr bool REG = sizeof(T) == 4 && !LenKind<N / 2>::SPLIT && N >= 128 && N <= 512;
     static constexpr int RX2 = 2 * RowGeom<T, N>::R;
     static constexpr bool KEEP_OK = REG && PairGeom<T, N, 0, true>::FITS;
     static constexpr int ALT_RX = REG && (N / 2) % RX2 == 0 && (N / 2) / RX2 >= 4 ? RX2 : 0;
@@ -814,9 +842,12 @@ template <typename T, int N> struct PairVariants {
 
 //   REAL : rows of the quad layout (real spectra, two columns per element;
 //          hva, hvb, hout count columns)
-template <typename T, int N, int RX = 0, bool KEEP = false, bool REAL = false>
-__global__ void __launch_bounds__(RowGeom<T, N, RX>::THREADS)
-    k_pair_z(const __grid_constant__ Items<PairItem<T>> items, int nrows,
+//   TWO  : two legs (else A squared: no second row in registers)
+// alias: the exchange buffer of a row is its current stage buffer of A, whose pitch
+// is then at least ROWBUF (full-band legs: a third less shared memory per row).
+template <typename T, int N, int RX = 0, bool KEEP = false, bool REAL = false, bool TWO = true>
+__global__ void __launch_bounds__(RowGeom<T, N, RX>::THREADS, (sizeof(T) == 4 && LenKind<N / 2>::SPLIT) ? 2 : 0)
+    k_pair_z(const __grid_constant__ Items<PairItem<T>> items, int nrows, int alias,
              const V2<T>* __restrict__ twr_g, const V2<T>* __restrict__ twpp_g)
 {
     using G = RowGeom<T, N, RX>;
@@ -834,9 +865,9 @@ __global__ void __launch_bounds__(RowGeom<T, N, RX>::THREADS)
         if constexpr (REAL) c2r_row_real<T, N, RX>(reinterpret_cast<const T*>(z), hv, rc, x);
         else c2r_row<T, N, RX>(z, hv, rc, x);
     };
-    const bool two = srcB != nullptr;
-    const int PA = G::pitch(hva), PB = two ? G::pitch(hvb) : 0;
-    V* stA = reinterpret_cast<V*>(smem_raw + G::STAGE_OFF);
+    constexpr bool two = TWO;
+    const int PA = alias ? max(G::pitch(hva), G::ROWBUF) : G::pitch(hva), PB = two ? G::pitch(hvb) : 0;
+    V* stA = reinterpret_cast<V*>(smem_raw + (alias ? G::ROWBUF_OFF : G::STAGE_OFF));
     V* stB = stA + 2 * G::WZ * PA;
     V* keep = stB + 2 * G::WZ * PB + rc.w * G::ROWBUF;  // KEEP: this row's slots
     const int ntiles = (nrows + G::WZ - 1) / G::WZ;
@@ -863,28 +894,29 @@ __global__ void __launch_bounds__(RowGeom<T, N, RX>::THREADS)
             __syncthreads();
             continue;
         }
+        if (alias) rc.rowbuf = stA + st * G::WZ * PA + rc.w * PA;
         V a[G::R];
         c2r(stA + st * G::WZ * PA + rc.w * PA, it.hva, a);
-        if (two) {
+        if constexpr (two) {
             if constexpr (KEEP) {
 #pragma unroll
-                for (int e = 0; e < G::R; e++)
-                    if (G::live(rc.t + G::TPF * e)) keep[rc.t + G::TPF * e] = a[e];
+                for (int e = 0; e < G::RT; e++)
+                    if (G::tl(rc.t, e)) keep[G::tp(rc.t, e)] = a[e];
                 c2r(stB + st * G::WZ * PB + rc.w * PB, it.hvb, a);
 #pragma unroll
-                for (int e = 0; e < G::R; e++) {
-                    const V q = G::live(rc.t + G::TPF * e) ? keep[rc.t + G::TPF * e] : czero<V>();
+                for (int e = 0; e < G::RT; e++) {
+                    const V q = G::tl(rc.t, e) ? keep[G::tp(rc.t, e)] : czero<V>();
                     a[e] = V{a[e].x * q.x, a[e].y * q.y};
                 }
             } else {
                 V b[G::R];
                 c2r(stB + st * G::WZ * PB + rc.w * PB, it.hvb, b);
 #pragma unroll
-                for (int e = 0; e < G::R; e++) a[e] = V{a[e].x * b[e].x, a[e].y * b[e].y};
+                for (int e = 0; e < G::RT; e++) a[e] = V{a[e].x * b[e].x, a[e].y * b[e].y};
             }
         } else {
 #pragma unroll
-            for (int e = 0; e < G::R; e++) a[e] = V{a[e].x * a[e].x, a[e].y * a[e].y};
+            for (int e = 0; e < G::RT; e++) a[e] = V{a[e].x * a[e].x, a[e].y * a[e].y};
         }
         // the products sit in canonical layout as (x[2n], x[2n+1]): r2c input as is
         if constexpr (REAL) r2c_row<T, N, RX, true>(a, rc, reinterpret_cast<T*>(dst + row * ds), hout);
@@ -911,7 +943,7 @@ template <typename T> struct ProdItem {
 };
 template <typename T, int N, bool REAL>
 __global__ void __launch_bounds__(RowGeom<T, N>::THREADS)
-    k_prod_z(const __grid_constant__ Items<ProdItem<T>> items, int P, int abs_terms, const V2<T>* __restrict__ twr_g,
+    k_prod_z(const __grid_constant__ Items<ProdItem<T>> items, int P, int alias, int abs_terms, const V2<T>* __restrict__ twr_g,
              const V2<T>* __restrict__ twpp_g)
 {
     using G = RowGeom<T, N>;
@@ -920,7 +952,7 @@ __global__ void __launch_bounds__(RowGeom<T, N>::THREADS)
     __shared__ double red[(G::THREADS + 31) / 32];
     const ProdItem<T>& it = item_at(items);
     RowCtx<T, N> rc(smem_raw, twr_g, twpp_g);
-    V* stage = reinterpret_cast<V*>(smem_raw + G::STAGE_OFF);  // two tiles of pitch P
+    V* stage = reinterpret_cast<V*>(smem_raw + (alias ? G::ROWBUF_OFF : G::STAGE_OFF));  // two tiles of pitch P
     constexpr int NQ = N / 2 + 1;
     constexpr int nrows = REAL ? NQ * NQ : N * N, ntiles = (nrows + G::WZ - 1) / G::WZ;
     const int nf = it.nf;
@@ -944,17 +976,18 @@ __global__ void __launch_bounds__(RowGeom<T, N>::THREADS)
             __syncthreads();
             if (live) {  // whole row groups
                 V a[G::R];
-                const V* z = stage + buf * G::WZ * P + rc.w * P;
+                V* z = stage + buf * G::WZ * P + rc.w * P;
+                if (alias) rc.rowbuf = z;  // the row's own stage buffer is its exchange buffer
                 if constexpr (REAL) c2r_row_real<T, N>(reinterpret_cast<const T*>(z), it.hv[f], rc, a);
                 else c2r_row<T, N>(z, it.hv[f], rc, a);
                 const int p = it.power[f];
                 double s = 0.0;
 #pragma unroll
-                for (int e = 0; e < G::R; e++) {
+                for (int e = 0; e < G::RT; e++) {
                     const T x0 = ipow(a[e].x, p), x1 = ipow(a[e].y, p);
                     if (!last) {
                         prod[e] = f == 0 ? V{x0, x1} : V{prod[e].x * x0, prod[e].y * x1};
-                    } else if (G::live(rc.t + G::TPF * e)) {
+                    } else if (G::tl(rc.t, e)) {
                         const double y0 = f == 0 ? (double)x0 : (double)prod[e].x * (double)x0;
                         const double y1 = f == 0 ? (double)x1 : (double)prod[e].y * (double)x1;
                         s += abs_terms ? fabs(y0) + fabs(y1) : y0 + y1;
@@ -1065,22 +1098,22 @@ __global__ void __launch_bounds__(PencilGeom<T, N, RX>::THREADS,
     }
     V a[G::R];
 #pragma unroll
-    for (int e = 0; e < G::R; e++) {
-        const int i = t + G::TPF * e;
-        a[e] = G::live(i) ? data[((size_t)(quad && i > N / 2 ? N - i : i) * nj + j) * stride + h] : czero<V>();
+    for (int e = 0; e < G::RI; e++) {
+        const int i = G::ip(t, e);
+        a[e] = G::il(t, e) ? data[((size_t)(quad && i > N / 2 ? N - i : i) * nj + j) * stride + h] : czero<V>();
     }
     // sums: the shell bits depend on indices only and are found before the
     // transform (16 bits per mode, two modes per register)
-    unsigned bits2[(G::R + 1) / 2];
-    [[maybe_unused]] unsigned bits2b[(G::R + 1) / 2];  // packed: of the odd column
+    unsigned bits2[(G::RO + 1) / 2];
+    [[maybe_unused]] unsigned bits2b[(G::RO + 1) / 2];  // packed: of the odd column
     if constexpr (DOT) {
 #pragma unroll
-        for (int e = 0; e < (G::R + 1) / 2; e++) bits2[e] = bits2b[e] = 0u;
+        for (int e = 0; e < (G::RO + 1) / 2; e++) bits2[e] = bits2b[e] = 0u;
         const auto each = [&](auto&& bits_of) {  // bits_of(mx) of every mode of this thread
 #pragma unroll
-            for (int e = 0; e < G::R; e++) {
-                if (col_ok && G::live(t + G::TPF * e))
-                    bits2[e / 2] |= (bits_of(lattice_freq(t + G::TPF * e, N)) & 0xffffu) << (16 * (e & 1));
+            for (int e = 0; e < G::RO; e++) {
+                if (col_ok && G::ol(t, e))
+                    bits2[e / 2] |= (bits_of(lattice_freq(G::op(t, e), N)) & 0xffffu) << (16 * (e & 1));
             }
         };
         const int s2 = my * my + mz * mz;
@@ -1110,9 +1143,9 @@ __global__ void __launch_bounds__(PencilGeom<T, N, RX>::THREADS,
                 const unsigned short* __restrict__ lut = it.lut;
                 const int s2b = my * my + mzb * mzb;
 #pragma unroll
-                for (int e = 0; e < G::R; e++) {
-                    if (!G::live(t + G::TPF * e)) continue;
-                    const int mx = lattice_freq(t + G::TPF * e, N), r2 = mx * mx + s2b;
+                for (int e = 0; e < G::RO; e++) {
+                    if (!G::ol(t, e)) continue;
+                    const int mx = lattice_freq(G::op(t, e), N), r2 = mx * mx + s2b;
                     const int vb = it.vol_band;
                     unsigned bb = 0u;
                     if (lut) bb = r2 < it.lut_size ? (unsigned)__ldg(lut + r2) : 0u;
@@ -1127,25 +1160,25 @@ __global__ void __launch_bounds__(PencilGeom<T, N, RX>::THREADS,
     const V* tw = stage_table<V>(smem_raw, tw_g, N);
     __syncthreads();
     SmemInterleaved<V, G::W> sm{reinterpret_cast<V*>(smem_raw + G::TW_BYTES), w};
-    fft_any<V, N, G::R, G::TPF, false>(a, t, sm, tw, BlockSync{});
+    fft_geom<G, V, N, false>(a, t, sm, tw, BlockSync{});
     if constexpr (!DOT) {
         unsigned keep = 0u;
         if constexpr (KIND == FWD_MASK) {
             const Shell sh = it.shells[0];
             if (col_ok) {
 #pragma unroll 1
-                for (int e = 0; e < G::R; e++) {
-                    if (!G::live(t + G::TPF * e)) continue;
-                    const int mx = lattice_freq(t + G::TPF * e, N);
+                for (int e = 0; e < G::RO; e++) {
+                    if (!G::ol(t, e)) continue;
+                    const int mx = lattice_freq(G::op(t, e), N);
                     if (in_band(sh, mx, my, mz) && shell_bit(sh, mx, my, mz)) keep |= 1u << e;
                 }
             }
         }
         if (h >= out_stride) return;
 #pragma unroll
-        for (int e = 0; e < G::R; e++) {
-            const int i = t + G::TPF * e;
-            if (!G::live(i)) continue;
+        for (int e = 0; e < G::RO; e++) {
+            const int i = G::op(t, e);
+            if (!G::ol(t, e)) continue;
             if (jband < N / 2 && abs(lattice_freq(i, N)) > jband) continue;
             V v = a[e];
             if constexpr (KIND == FWD_MASK) {
@@ -1212,16 +1245,16 @@ __global__ void __launch_bounds__(PencilGeom<T, N, RX>::THREADS,
 #pragma unroll
             for (int c = 0; c < 8; c++) acc[c] = 0.0;
 #pragma unroll
-            for (int e = 0; e < G::R; e++) {
+            for (int e = 0; e < G::RO; e++) {
                 const unsigned b = (bits2[e / 2] >> (16 * (e & 1) + 8 * half)) & 0xffu;
                 if (b) {
                     double val;
                     if (use_dk) {
                         V d;
                         if constexpr (G::DK_SMEM) {
-                            d = sdk[(t + G::TPF * e) * G::W + w];
+                            d = sdk[G::op(t, e) * G::W + w];
                         } else {
-                            const int mx = lattice_freq(t + G::TPF * e, N);
+                            const int mx = lattice_freq(G::op(t, e), N);
                             d = dk[((size_t)(mx < 0 ? mx + ndk : mx) * ndk + jdk) * dk_stride + h];
                         }
                         val = wgt * ((double)d.x * (double)a[e].x + (double)d.y * (double)a[e].y);
@@ -1238,7 +1271,7 @@ __global__ void __launch_bounds__(PencilGeom<T, N, RX>::THREADS,
                 if (packed) {
                     const double wgtb = (double)(herm_weight(hz + 1, N) * (j != 0 && j != N / 2 ? 2 : 1));
 #pragma unroll
-                    for (int e = 0; e < G::R; e++) {
+                    for (int e = 0; e < G::RO; e++) {
                         const unsigned b = (bits2b[e / 2] >> (16 * (e & 1) + 8 * half)) & 0xffu;
                         if (b) {
                             const double val = wgtb * rint((double)a[e].y * inv_n3);

@@ -135,7 +135,7 @@ template <typename T, int N> struct L3 {
     // hva, hvb: the widest legs of the batch; ninputs: 2 when any item has two
     static int pair_z_b(cudaStream_t st, const PairItem<T>* items, int nitems, int ninputs,
                         int hva, int hvb, const Tables<T>& tb, int quad, int variant);
-    template <int RX, bool KEEP, bool REAL = false>
+    template <int RX, bool KEEP, bool REAL, bool TWO>
     static int pair_z_v(cudaStream_t st, const PairItem<T>* items, int nitems, int ninputs,
                         int hva, int hvb, const V* twr, const V* twpp, int quad);
     // Grid sums of products (k_prod_z) of nitems lists of factors, the widest row of

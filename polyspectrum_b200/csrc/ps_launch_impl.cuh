@@ -11,7 +11,7 @@ bool L3<T, N>::host_alt_table(V* twp_alt)
 {
     if constexpr (ALT > 0) {
         static_assert(PencilGeom<T, N, ALT>::W == PG::W, "same pencil tile width");
-        transform_table<V, N, ALT, PencilGeom<T, N, ALT>::TPF>(twp_alt);
+        transform_table<V, N, ALT>(twp_alt);
         return true;
     } else {
         (void)twp_alt;
@@ -24,7 +24,7 @@ bool L3<T, N>::host_pair_alt_table(V* twr_alt)
 {
     if constexpr (PAIR_RX2 > 0) {
         using G2 = RowGeom<T, N, PAIR_RX2>;
-        transform_table<V, N / 2, G2::R, G2::TPF>(twr_alt);
+        transform_table<V, N / 2, G2::R>(twr_alt);
         return true;
     } else {
         (void)twr_alt;
@@ -46,8 +46,8 @@ int L3<T, N>::pair_variants()
 template <typename T, int N>
 void L3<T, N>::host_tables(V* twp, V* twr)
 {
-    transform_table<V, N, PG::R, PG::TPF>(twp);
-    transform_table<V, N / 2, RG::R, RG::TPF>(twr);
+    transform_table<V, N, PG::R>(twp);
+    transform_table<V, N / 2, RG::R>(twr);
 }
 
 template <typename T, int N>
@@ -127,20 +127,22 @@ int L3<T, N>::fwd_z(cudaStream_t st, int kind, const void* a, const void* b, V* 
 }
 
 template <typename T, int N>
-template <int RX, bool KEEP, bool REAL>
+template <int RX, bool KEEP, bool REAL, bool TWO>
 int L3<T, N>::pair_z_v(cudaStream_t st, const PairItem<T>* items, int nitems, int ninputs,
                        int hva, int hvb, const V* twr, const V* twpp, int quad)
 {
     using G = RowGeom<T, N, RX>;
     using PGm = PairGeom<T, N, RX, KEEP>;
-    const size_t smem = PGm::smem(ninputs, REAL ? (hva + 1) / 2 : hva, REAL ? (hvb + 1) / 2 : hvb);
-    PS_LTRY(set_smem(k_pair_z<T, N, RX, KEEP, REAL>, PGm::smem(2, N / 2 + 1, N / 2 + 1)));
+    const int ea = REAL ? (hva + 1) / 2 : hva, eb = REAL ? (hvb + 1) / 2 : hvb;
+    const bool alias = PGm::smem(ninputs, ea, eb, true) < PGm::smem(ninputs, ea, eb, false);
+    const size_t smem = PGm::smem(ninputs, ea, eb, alias);
+    PS_LTRY(set_smem(k_pair_z<T, N, RX, KEEP, REAL, TWO>, PGm::smem(2, N / 2 + 1, N / 2 + 1)));
     const int nrows = quad ? (N / 2 + 1) * (N / 2 + 1) : N * N;
     const int tiles = (nrows + G::WZ - 1) / G::WZ;
     int grid = 0;  // resident CTAs, shared out among the items
-    PS_LTRY(persistent_grid(k_pair_z<T, N, RX, KEEP, REAL>, G::THREADS, smem, tiles * nitems, &grid));
+    PS_LTRY(persistent_grid(k_pair_z<T, N, RX, KEEP, REAL, TWO>, G::THREADS, smem, tiles * nitems, &grid));
     grid = std::max(1, std::min(tiles, grid / nitems));
-    k_pair_z<T, N, RX, KEEP, REAL><<<dim3((unsigned)grid, (unsigned)nitems), G::THREADS, smem, st>>>(pack(items, nitems), nrows, twr, twpp);
+    k_pair_z<T, N, RX, KEEP, REAL, TWO><<<dim3((unsigned)grid, (unsigned)nitems), G::THREADS, smem, st>>>(pack(items, nitems), nrows, alias ? 1 : 0, twr, twpp);
     return PS_OK;
 }
 
@@ -148,34 +150,39 @@ template <typename T, int N>
 int L3<T, N>::pair_z_b(cudaStream_t st, const PairItem<T>* items, int nitems, int ninputs,
                        int hva, int hvb, const Tables<T>& tb, int quad, int variant)
 {
+    if constexpr (sizeof(T) == 8) {
+        if (quad)
+            return ninputs > 1 ? pair_z_v<0, false, true, true>(st, items, nitems, ninputs, hva, hvb, tb.twr, tb.twpp, quad)
+                               : pair_z_v<0, false, true, false>(st, items, nitems, ninputs, hva, hvb, tb.twr, tb.twpp, quad);
+    }
+    if (ninputs == 1)  // one leg squared: one row transform in registers anyway
+        return pair_z_v<0, false, false, false>(st, items, nitems, 1, hva, 0, tb.twr, tb.twpp, quad);
     if constexpr (PAIR_RX2 > 0) {
         if constexpr (PairGeom<T, N, PAIR_RX2, true>::FITS) {
-            if (variant == 2 && tb.twr_alt && !quad)
-                return pair_z_v<PAIR_RX2, true>(st, items, nitems, ninputs, hva, hvb, tb.twr_alt, tb.twpp, quad);
+            if (variant == 2 && tb.twr_alt)
+                return pair_z_v<PAIR_RX2, true, false, true>(st, items, nitems, 2, hva, hvb, tb.twr_alt, tb.twpp, quad);
         }
     }
     if constexpr (PairVariants<T, N>::KEEP_OK) {
-        if (variant == 1 && !quad)
-            return pair_z_v<0, true>(st, items, nitems, ninputs, hva, hvb, tb.twr, tb.twpp, quad);
+        if (variant == 1) return pair_z_v<0, true, false, true>(st, items, nitems, 2, hva, hvb, tb.twr, tb.twpp, quad);
     }
-    if constexpr (sizeof(T) == 8) {
-        if (quad) return pair_z_v<0, false, true>(st, items, nitems, ninputs, hva, hvb, tb.twr, tb.twpp, quad);
-    }
-    return pair_z_v<0, false>(st, items, nitems, ninputs, hva, hvb, tb.twr, tb.twpp, quad);
+    return pair_z_v<0, false, false, true>(st, items, nitems, 2, hva, hvb, tb.twr, tb.twpp, quad);
 }
 
 template <typename T, int N>
 int L3<T, N>::prod_z(cudaStream_t st, const ProdItem<T>* items, int nitems, int hv, bool real, int abs_terms,
                      const Tables<T>& tb, int* nblocks)
 {
-    const int P = RG::pitch(real ? (hv + 1) / 2 : hv);
-    const size_t smem = RG::STAGE_OFF + (size_t)2 * RG::WZ * P * sizeof(V);
+    const int P0 = RG::pitch(real ? (hv + 1) / 2 : hv);
+    const bool alias = 2 * std::max(P0, RG::ROWBUF) < 2 * P0 + RG::ROWBUF;  // rows' exchange buffers in their stages
+    const int P = alias ? std::max(P0, RG::ROWBUF) : P0;
+    const size_t smem = (alias ? RG::ROWBUF_OFF : RG::STAGE_OFF) + (size_t)2 * RG::WZ * P * sizeof(V);
     auto go = [&](auto kernel) -> int {
         PS_LTRY(set_smem(kernel, RG::smem(1, N / 2 + 1, 0)));
         int grid = 0;  // resident CTAs, shared out among the items
         PS_LTRY(persistent_grid(kernel, RG::THREADS, smem, prod_blocks(real) * nitems, &grid));
         grid = std::max(1, std::min(prod_blocks(real), grid / nitems));
-        kernel<<<dim3((unsigned)grid, (unsigned)nitems), RG::THREADS, smem, st>>>(pack(items, nitems), P, abs_terms, tb.twr,
+        kernel<<<dim3((unsigned)grid, (unsigned)nitems), RG::THREADS, smem, st>>>(pack(items, nitems), P, alias ? 1 : 0, abs_terms, tb.twr,
                                                                                   tb.twpp);
         *nblocks = grid;
         return PS_OK;
