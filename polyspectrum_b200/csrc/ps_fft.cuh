@@ -337,13 +337,13 @@ __device__ __forceinline__ void fft_passes(V (&a)[R], int t, Acc& sm, const V* _
             } else {
                 const int j = (v / Ns) * Ns * Rp + k;
 #pragma unroll
-                for (int q = 0; q < Rp; q++) sm.template st<Rp, Ns>(j + q * Ns, b[q]);
+                for (int q = 0; q < Rp; q++) sm.template st<Rp, Ns>(j, q * Ns, b[q]);
             }
         }
         if constexpr (!LAST) {
             sync();
 #pragma unroll
-            for (int e = 0; e < R; e++) a[e] = sm.template ld<Rp, Ns>(t + TPF * e);
+            for (int e = 0; e < R; e++) a[e] = sm.template ld<Rp, Ns>(t, TPF * e);
             sync();
             fft_passes<V, N, R, INV, P_ + 1>(a, t, sm, twt, sync);
         }
@@ -364,7 +364,7 @@ __device__ __forceinline__ void split_passes(V (&a)[SLOTS], int t, Acc& sm, cons
         if (v < RB) {
             Dft<RA, INV>::run(&a[u * RA]);
 #pragma unroll
-            for (int q = 0; q < RA; q++) sm.st(v * RA + q, a[u * RA + q]);
+            for (int q = 0; q < RA; q++) sm.template st_split<RA, RB>(v, q, a[u * RA + q]);
         }
     }
     sync();
@@ -373,7 +373,7 @@ __device__ __forceinline__ void split_passes(V (&a)[SLOTS], int t, Acc& sm, cons
         const int v = t + TPF * u;
         if (v < RA) {
 #pragma unroll
-            for (int q = 0; q < RB; q++) a[u * RB + q] = sm.ld(v + q * RA);
+            for (int q = 0; q < RB; q++) a[u * RB + q] = sm.template ld_split<RA, RB>(v, q);
         }
     }
     sync();
@@ -446,48 +446,74 @@ template <typename V, int N, int R> inline void transform_table(V* out)
 
 // Shared-memory accessor for pencil passes: W transforms interleaved, element
 // `pos` of transform `lane` at s[pos*W + lane] (conflict-free when W*sizeof(V)
-// = 128 bytes, the tile width of one global row segment).
+// = 128 bytes, the tile width of one global row segment).  In the exchange of the
+// split passes butterfly v of the first stores its output q, and butterfly v of the
+// second loads its input q.
 template <typename V, int W> struct SmemInterleaved {
     V* s;
     int lane;
-    template <int Rp, int Ns> __device__ __forceinline__ void st(int pos, V v) { s[pos * W + lane] = v; }
-    template <int Rp, int Ns> __device__ __forceinline__ V ld(int pos) const { return s[pos * W + lane]; }
-    __device__ __forceinline__ void st(int pos, V v) { s[pos * W + lane] = v; }
-    __device__ __forceinline__ V ld(int pos) const { return s[pos * W + lane]; }
+    template <int Rp, int Ns> __device__ __forceinline__ void st(int base, int off, V v) { s[(base + off) * W + lane] = v; }
+    template <int Rp, int Ns> __device__ __forceinline__ V ld(int base, int off) const { return s[(base + off) * W + lane]; }
+    template <int RA, int RB> __device__ __forceinline__ void st_split(int v, int q, V x) { s[(v * RA + q) * W + lane] = x; }
+    template <int RA, int RB> __device__ __forceinline__ V ld_split(int v, int q) const { return s[(v + q * RA) * W + lane]; }
 };
 
-// Shared-memory accessor for row passes: one row per transform, XOR-swizzled
-// within blocks of G = 2^LB elements (128 bytes): element pos of block
-// a = pos >> LB lives at pos ^ g(a).
-//  * Exchange after a pass of radix Rp and span Ns (both powers of two): the
-//    stores of one instruction put lane t at (t/Ns)*Ns*Rp + t%Ns + q*Ns.
-//    When Ns*Rp < G the lanes that share an offset within their block differ
-//    in a mod Rp, and g(a) = a*Ns moves them apart on the log2(Rp) bits that
-//    q occupies; when Ns*Rp >= G they differ in a / K (K = Ns*Rp/G) and
-//    g(a) = (a/K)*Ns does the same.  The loads that follow (consecutive
-//    positions, one block per G lanes) stay conflict-free under any g.
-//  * Elsewhere (r2c post-processing): g(a) = a.
+// Shared-memory accessor for row passes: one row per transform, padded per exchange
+// so that no store of an instruction meets another on a bank and every address is a
+// thread's base plus a constant (no arithmetic per element; an XOR swizzle took two
+// instructions for each, a fifth of the row kernels').  Blocks are G elements (128
+// bytes).
+//  * Exchange after a pass of radix Rp and span Ns (powers of two): lane t stores at
+//    (t/Ns)*Ns*Rp + t%Ns + q*Ns; block a is moved up by a*PAD elements.  When Ns*Rp <=
+//    G the lanes that share an offset lie in Rp consecutive blocks and PAD = Ns moves
+//    them apart; else they lie K = Ns*Rp/G blocks apart and PAD = Ns/K = G/Rp does.  From
+//    Ns = G on the lanes are consecutive anyway.  The loads that follow (consecutive
+//    positions, one block per G lanes) stay conflict-free.
+//  * Split passes: output q of butterfly v at q * pitch + v, so both the stores
+//    (consecutive v) and the loads (v of the second pass pitch apart, the pitch odd)
+//    are conflict-free.
+//  * r2c post-processing: consecutive positions both ways, no padding.
 template <typename V> struct SmemRow {
-    static constexpr int LB = sizeof(V) == 16 ? 3 : 4;
-    static constexpr int G = 1 << LB;
+    static constexpr int G = 128 / (int)sizeof(V);
     V* s;
-    __host__ __device__ static constexpr int ilog2(int v) { return v > 1 ? 1 + ilog2(v / 2) : 0; }
-    template <int Rp, int Ns> __device__ __forceinline__ static int phys_x(int pos)
+    template <int Rp, int Ns> __host__ __device__ static constexpr int pad()
     {
-        const int a = pos >> LB;
-        if constexpr (Ns >= G || (Rp & (Rp - 1)) != 0 || (Ns & (Ns - 1)) != 0) {
-            return pos ^ (a & (G - 1));
-        } else if constexpr (Ns * Rp < G) {
-            return pos ^ ((a * Ns) & (G - 1));
+        static_assert((Rp & (Rp - 1)) == 0 && (Ns & (Ns - 1)) == 0, "power-of-two passes go through shared memory");
+        return Ns >= G ? 0 : Ns * Rp <= G ? Ns : Rp >= G ? 1 : G / Rp;
+    }
+    // base: the thread's part of the position, off: the constant part; their offsets
+    // within a block never add up to a whole one (a store's base is r < Ns past a
+    // multiple of min(Ns Rp, G), its off a multiple of Ns below Ns Rp; a load's base is
+    // t and its off a multiple of TPF), so the padded position is the sum of both
+    template <int Rp, int Ns> __device__ __forceinline__ static int at(int pos) { return pos + pos / G * pad<Rp, Ns>(); }
+    template <int Rp, int Ns> __device__ __forceinline__ void st(int base, int off, V v) { s[at<Rp, Ns>(base) + at<Rp, Ns>(off)] = v; }
+    template <int Rp, int Ns> __device__ __forceinline__ V ld(int base, int off) const { return s[at<Rp, Ns>(base) + at<Rp, Ns>(off)]; }
+    __host__ __device__ static constexpr int pitch(int rb) { return rb | 1; }
+    template <int RA, int RB> __device__ __forceinline__ void st_split(int v, int q, V x) { s[q * pitch(RB) + v] = x; }
+    template <int RA, int RB> __device__ __forceinline__ V ld_split(int v, int q) const { return s[v * pitch(RB) + q]; }
+    __device__ __forceinline__ void st(int pos, V v) { s[pos] = v; }
+    __device__ __forceinline__ V ld(int pos) const { return s[pos]; }
+    // elements a row of N takes through the passes of radix R (register plan) or split
+    template <int N, int R, int P = 0> __host__ __device__ static constexpr int size_reg()
+    {
+        using Plan = RadixPlan<N, R>;
+        if constexpr (P + 1 >= Plan::P) {
+            return N;
         } else {
-            return pos ^ (((a >> ilog2(Ns * Rp / G)) * Ns) & (G - 1));
+            constexpr int here = N + (N + G - 1) / G * pad<Plan::radix(P), Plan::span(P)>(), rest = size_reg<N, R, P + 1>();
+            return here > rest ? here : rest;
         }
     }
-    __device__ __forceinline__ static int phys(int pos) { return pos ^ ((pos >> LB) & (G - 1)); }
-    template <int Rp, int Ns> __device__ __forceinline__ void st(int pos, V v) { s[phys_x<Rp, Ns>(pos)] = v; }
-    template <int Rp, int Ns> __device__ __forceinline__ V ld(int pos) const { return s[phys_x<Rp, Ns>(pos)]; }
-    __device__ __forceinline__ void st(int pos, V v) { s[phys(pos)] = v; }
-    __device__ __forceinline__ V ld(int pos) const { return s[phys(pos)]; }
+    template <int N, int R> __host__ __device__ static constexpr int size()
+    {
+        if constexpr (LenKind<N>::SPLIT) {
+            constexpr int A = SplitPlan<N>::RA, B = SplitPlan<N>::RB;
+            constexpr int x = A * pitch(B), y = B * pitch(A);
+            return x > y ? x : y;
+        } else {
+            return size_reg<N, R>();
+        }
+    }
 };
 
 }  // namespace ps

@@ -123,7 +123,9 @@ template <typename T, int N, int RX = 0> struct RowGeom {
     // rows per CTA (tile): up to 256 threads and 32 rows, and as many as fit
     // in 227 KB of shared memory with two double-buffered full-length inputs
     static constexpr int WZ0 = (256 / TPF) < 32 ? (256 / TPF) : 32;
-    static constexpr int ROWBUF = (NH < 16 ? NH : (NH + 15) / 16 * 16) + SKEW;
+    // exchange buffer of a row: its padded passes, rounded up to the skew
+    static constexpr int ROWBUF0 = (SmemRow<V2<T>>::template size<NH, R>() + EPC - 1) / EPC * EPC;
+    static constexpr int ROWBUF = SKEW ? ROWBUF0 + (SKEW + BLOCK - ROWBUF0 % BLOCK) % BLOCK : ROWBUF0;
     // input stage pitch (elements) for rows of hv valid entries
     __host__ __device__ static constexpr int pitch(int hv)
     {
@@ -142,8 +144,6 @@ template <typename T, int N, int RX = 0> struct RowGeom {
     static constexpr size_t TWR_OFF = 0;
     static constexpr size_t TWPP_OFF = TWR_OFF + (size_t)NH * sizeof(V2<T>);
     static constexpr size_t ROWBUF_OFF = TWPP_OFF + (size_t)(NH + 2) * sizeof(V2<T>);
-    // row exchange buffers hold whole swizzle blocks of SmemRow (16 elements:
-    // its XOR stays inside a block, which a split NH may end in the middle of)
     static constexpr size_t STAGE_OFF = ROWBUF_OFF + (size_t)WZ * ROWBUF * sizeof(V2<T>);
     // dynamic shared memory of a kernel with `ninputs` double-buffered inputs
     __host__ __device__ static constexpr size_t smem(int ninputs, int hva, int hvb)
@@ -518,7 +518,11 @@ __device__ __forceinline__ void r2c_row(V2<T> (&a)[RowGeom<T, N, RX>::R], RowCtx
         if (G::kl(rc.t, e)) sm.st(G::kp(rc.t, e), a[e]);
     rc.sync();
     const T half = (T)0.5;
-    for (int k = rc.t; k <= NH && k < hout; k += G::TPF) {
+    // column k from elements k and NH - k; column NH (element 0 twice) by thread 0
+#pragma unroll
+    for (int e = 0; e <= (NH + G::TPF - 1) / G::TPF; e++) {
+        const int k = e * G::TPF >= NH ? NH : rc.t + e * G::TPF;
+        if ((e * G::TPF >= NH && rc.t != 0) || (e * G::TPF < NH && k >= NH) || k >= hout) continue;
         const V yk = sm.ld(k == NH ? 0 : k);
         const V ym = cconj(sm.ld(k == 0 ? 0 : NH - k));
         const V E = V{(yk.x + ym.x) * half, (yk.y + ym.y) * half};
