@@ -667,7 +667,7 @@ template <typename T> int dot_alt_of(const ps_gpu_ctx* c, int M)
 {
     if (sizeof(T) != 4) return 0;
     const auto it = c->dot_alt.find(M);
-    return it == c->dot_alt.end() ? 0 : it->second;
+    return it == c->dot_alt.end() ? (M == 384 ? L3<T, 384>::DOT_ALT : 0) : it->second;
 }
 
 // Pair kernel variant of an M-point transform of precision T (autotuned choice).

@@ -254,16 +254,21 @@ template <int N> struct DefaultRadix {
                                : N <= 16 ? N : (N == 32 || N == 64 || N == 128 || N == 512) ? 8 : 16;
 };
 
-// Lengths whose odd part is not 1, 3 or 5: N = RA RB in two passes, the factors as
+// Lengths whose odd part is not 1, 3 or 5, and those with a factor 3 or 5 whose
+// register plan needs three or more passes: N = RA RB in two passes, the factors as
 // equal as they come (the second at least the first), so that either pass is one
 // butterfly per thread and one exchange through shared memory lies between them.
 // Thread t does the butterflies v = t, t + TPF, ... of a pass: slot u R + q of its
 // array holds element v + q N / R, v = t + TPF u; slots of v >= N / R are idle.  The
 // layouts of input (pass A) and output (pass B) therefore differ, see SplitGeom.  A
 // sequence of radix-8/4/2, 3 and 5 passes through shared memory (five exchanges at 600
-// points) took 0.54 ms for a Y pass of 600^2 x 304 columns.
+// points) took 0.54 ms for a Y pass of 600^2 x 304 columns.  Against the register plans
+// (160: 2 2 2 2 10, 192: 4 4 12, 320: 4 4 20, 384: 4 4 2 12): pair kernel at 320 points
+// 0.170 -> 0.135 ms, at 384 points 0.224 -> 0.215 ms, inverse X pass at 384 points 0.048
+// -> 0.041 ms, Y passes at 320 points 9% and at 384 points 10 to 14% faster.
 template <int N> struct SplitPlan {
-    static constexpr int RA = N == 30 ? 5 : N == 60 ? 6 : N == 150 ? 10 : N == 300 ? 15 : N == 600 ? 24 : 0;
+    static constexpr int RA = N == 30 ? 5 : N == 60 ? 6 : N == 96 ? 8 : N == 150 || N == 160 ? 10 : N == 192 ? 12
+                            : N == 300 ? 15 : N == 320 || N == 384 ? 16 : N == 600 ? 24 : 0;
     static constexpr int RB = RA ? N / RA : 0;
     static constexpr bool value = RA > 0;
 };
@@ -402,7 +407,7 @@ __device__ __forceinline__ void split_passes(V (&a)[SLOTS], int t, Acc& sm, cons
 template <class G, typename V, int N, bool INV, bool SWAP = false, class Acc, class Sync>
 __device__ __forceinline__ void fft_geom(V (&a)[G::R], int t, Acc& sm, const V* __restrict__ twt, const Sync& sync)
 {
-    if constexpr (!LenKind<N>::SPLIT) {
+    if constexpr (!G::SPLIT) {
         fft_passes<V, N, G::R, INV>(a, t, sm, twt, sync);
     } else if constexpr (SWAP) {
         split_passes<V, N, SplitPlan<N>::RB, SplitPlan<N>::RA, G::TPF, INV, true>(a, t, sm, twt, sync);
@@ -427,11 +432,11 @@ template <typename V, class Plan> inline void plan_table(V* out)
             }
     }
 }
-// the table of the transform fft_geom runs with R elements per thread
-template <typename V, int N, int R> inline void transform_table(V* out)
+// the table of the transform fft_geom runs in geometry G
+template <typename V, int N, class G> inline void transform_table(V* out)
 {
-    if constexpr (!LenKind<N>::SPLIT) {
-        plan_table<V, RadixPlan<N, R>>(out);
+    if constexpr (!G::SPLIT) {
+        plan_table<V, RadixPlan<N, G::R>>(out);
     } else {
         const long double two_pi = 6.283185307179586476925286766559005768L;
         constexpr int RA = SplitPlan<N>::RA, RB = SplitPlan<N>::RB;
@@ -504,9 +509,9 @@ template <typename V> struct SmemRow {
             return here > rest ? here : rest;
         }
     }
-    template <int N, int R> __host__ __device__ static constexpr int size()
+    template <int N, int R, bool SPLIT> __host__ __device__ static constexpr int size()
     {
-        if constexpr (LenKind<N>::SPLIT) {
+        if constexpr (SPLIT) {
             constexpr int A = SplitPlan<N>::RA, B = SplitPlan<N>::RB;
             constexpr int x = A * pitch(B), y = B * pitch(A);
             return x > y ? x : y;

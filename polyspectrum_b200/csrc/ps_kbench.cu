@@ -80,7 +80,7 @@ double time_pass_y(int reps, float2* data, int S, int ncols, int jband, int jout
 {
     using G = PencilGeom<float, M, RX>;
     std::vector<float2> hp(M);
-    transform_table<float2, M, G::R>(hp.data());
+    transform_table<float2, M, G>(hp.data());
     float2* tw;
     CK(cudaMalloc(&tw, M * 8));
     CK(cudaMemcpy(tw, hp.data(), M * 8, cudaMemcpyHostToDevice));
@@ -112,7 +112,7 @@ template <int M, int RX> float2* pair_row_table()
 {
     using G = RowGeom<float, M, RX>;
     std::vector<float2> hr(M / 2);
-    transform_table<float2, M / 2, G::R>(hr.data());
+    transform_table<float2, M / 2, G>(hr.data());
     float2* d;
     CK(cudaMalloc(&d, M / 2 * 8));
     CK(cudaMemcpy(d, hr.data(), M / 2 * 8, cudaMemcpyHostToDevice));
@@ -290,9 +290,9 @@ int main(int argc, char** argv)
 
     // Y pass variants (elements per thread: the default and twice it)
     time_pass_y<384, true, 0>(reps, wb, Sb, Sb, bb, M, "inv B");
-    time_pass_y<384, true, 24>(reps, wb, Sb, Sb, bb, M, "inv B");
+    time_pass_y<384, true, 12>(reps, wb, Sb, Sb, bb, M, "inv B");
     time_pass_y<384, false, 0>(reps, w3, S, S, M, bc, "fwd");
-    time_pass_y<384, false, 24>(reps, w3, S, S, M, bc, "fwd");
+    time_pass_y<384, false, 12>(reps, w3, S, S, M, bc, "fwd");
     time_pass_y<512, false, 0>(reps, spec, SN, 176, N, N, "field");
     time_pass_y<512, false, 32>(reps, spec, SN, 176, N, N, "field");
     time_pass_y<512, false, 8>(reps, spec, SN, 176, N, N, "field");

@@ -49,11 +49,10 @@ template <typename T, int N> struct PencilThreads {
     static constexpr int value = LenKind<N>::SPLIT ? split(SplitPlan<N>::RB)
                                : N / ((sizeof(T) == 4 && N == 512) ? 16 : DefaultRadix<N>::value);
 };
-// RX > 0 overrides the elements per thread of a register-plan pencil length
-// (pass variants with fewer, larger radix passes).
+// RX > 0 takes the register plan with RX elements per thread (pass variants).
 template <typename T, int N, int RX = 0> struct PencilGeom {
-    static constexpr bool SPLIT = LenKind<N>::SPLIT;
-    static constexpr int TPF = RX > 0 && !SPLIT ? N / RX : PencilThreads<T, N>::value;
+    static constexpr bool SPLIT = LenKind<N>::SPLIT && RX == 0;
+    static constexpr int TPF = RX > 0 ? N / RX : PencilThreads<T, N>::value;
     using SG = SplitGeom<SPLIT ? N : 600, TPF>;
     // slots of a thread going in and coming out, and what they hold: position
     // ip(t, e) where il(t, e), op and ol likewise (register plans: t + TPF e, all live)
@@ -77,12 +76,18 @@ template <typename T, int N, int RX = 0> struct PencilGeom {
     static constexpr size_t SMEM_DOT = SMEM + (DK_SMEM ? DK_BYTES : 0);
 };
 
-// The alternative pencil geometry of the FP32 Y pass for the larger
-// register-plan lengths: twice the elements per thread, half the threads per
-// pencil, one radix pass fewer (0: none).  Chosen per length by the plan
-// autotuner against the default.
+// The alternative pencil geometry of the FP32 Y and dot passes for the larger
+// lengths: twice the elements per thread, half the threads per pencil, one radix
+// pass fewer; for a split length its register plan, which needs fewer registers (0:
+// none).  Chosen per length by the plan autotuner against the default.
 template <typename T, int N> struct PencilAlt {
-    static constexpr int value = (sizeof(T) == 4 && !LenKind<N>::SPLIT && N >= 128 && N <= 512) ? 2 * PencilGeom<T, N>::R : 0;
+    static constexpr int odd = LenKind<N>::odd_of(N);
+    static constexpr int value = !(sizeof(T) == 4 && N >= 128 && N <= 512 && odd <= 5) ? 0
+                               : LenKind<N>::SPLIT ? DefaultRadix<N>::value : 2 * PencilGeom<T, N>::R;
+    // the dot pass without a timed choice: 0.136 against 0.155 ms at 384 points (the
+    // split plan's 24 elements and 16 sums per thread spill at two CTAs per SM), the
+    // split plan below
+    static constexpr int dot_default = N == 384 && value > 0 ? 1 : 0;
 };
 
 // Elements per thread of the row (contiguous-axis) transforms of length NH:
@@ -99,9 +104,9 @@ template <typename T, int NH> struct RowRadix {
 // (the pair kernel's variants).
 template <typename T, int N, int RX = 0> struct RowGeom {
     static constexpr int NH = N / 2;
-    static constexpr bool SPLIT = LenKind<NH>::SPLIT;
-    // split rows (30, 150, 300): a power of two of threads, so that rows pack warps
-    static constexpr int TPF = SPLIT ? (NH == 30 ? 8 : NH == 150 ? 16 : sizeof(T) == 4 ? 16 : 32)
+    static constexpr bool SPLIT = LenKind<NH>::SPLIT && RX == 0;
+    // split rows (30, 96, 150, 160, 192, 300): a power of two of threads, so that rows pack warps
+    static constexpr int TPF = SPLIT ? (NH == 30 || NH == 96 ? 8 : NH <= 192 || sizeof(T) == 4 ? 16 : 32)
                                      : NH / (RX > 0 ? RX : RowRadix<T, NH>::value);
     using SG = SplitGeom<SPLIT ? NH : 300, TPF>;
     // slots of a thread on the spectrum side (kp, kl: column k) and on the real side
@@ -122,9 +127,10 @@ template <typename T, int N, int RX = 0> struct RowGeom {
     static constexpr int SKEW = TPF < BLOCK ? (TPF < EPC ? EPC : TPF) : 0;
     // rows per CTA (tile): up to 256 threads and 32 rows, and as many as fit
     // in 227 KB of shared memory with two double-buffered full-length inputs
-    static constexpr int WZ0 = (256 / TPF) < 32 ? (256 / TPF) : 32;
+    // (FP64: 128 threads, whose smaller tiles leave less of an SM unused)
+    static constexpr int WZ0 = ((sizeof(T) == 8 ? 128 : 256) / TPF) < 32 ? ((sizeof(T) == 8 ? 128 : 256) / TPF) : 32;
     // exchange buffer of a row: its padded passes, rounded up to the skew
-    static constexpr int ROWBUF0 = (SmemRow<V2<T>>::template size<NH, R>() + EPC - 1) / EPC * EPC;
+    static constexpr int ROWBUF0 = (SmemRow<V2<T>>::template size<NH, R, SPLIT>() + EPC - 1) / EPC * EPC;
     static constexpr int ROWBUF = SKEW ? ROWBUF0 + (SKEW + BLOCK - ROWBUF0 % BLOCK) % BLOCK : ROWBUF0;
     // input stage pitch (elements) for rows of hv valid entries
     __host__ __device__ static constexpr int pitch(int hv)
@@ -850,7 +856,7 @@ template <typename T, int N> struct PairVariants {
 // alias: the exchange buffer of a row is its current stage buffer of A, whose pitch
 // is then at least ROWBUF (full-band legs: a third less shared memory per row).
 template <typename T, int N, int RX = 0, bool KEEP = false, bool REAL = false, bool TWO = true>
-__global__ void __launch_bounds__(RowGeom<T, N, RX>::THREADS, (sizeof(T) == 4 && LenKind<N / 2>::SPLIT) ? 2 : 0)
+__global__ void __launch_bounds__(RowGeom<T, N, RX>::THREADS, sizeof(T) == 8 ? 0 : !TWO && N <= 512 ? 3 : LenKind<N / 2>::SPLIT ? 2 : 0)
     k_pair_z(const __grid_constant__ Items<PairItem<T>> items, int nrows, int alias,
              const V2<T>* __restrict__ twr_g, const V2<T>* __restrict__ twpp_g)
 {

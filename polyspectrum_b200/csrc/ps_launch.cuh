@@ -75,6 +75,7 @@ template <typename T, int N> struct L3 {
     using RG = RowGeom<T, N>;
     static int pencil_width() { return PG::W; }
     static constexpr int ALT = PencilAlt<T, N>::value;
+    static constexpr int DOT_ALT = PencilAlt<T, N>::dot_default;
     // host copy of the alternative Y pass's table (false: no alternative)
     static bool host_alt_table(V* twp_alt);
     static constexpr int PAIR_RX2 = PairVariants<T, N>::ALT_RX;

@@ -11,7 +11,7 @@ bool L3<T, N>::host_alt_table(V* twp_alt)
 {
     if constexpr (ALT > 0) {
         static_assert(PencilGeom<T, N, ALT>::W == PG::W, "same pencil tile width");
-        transform_table<V, N, ALT>(twp_alt);
+        transform_table<V, N, PencilGeom<T, N, ALT>>(twp_alt);
         return true;
     } else {
         (void)twp_alt;
@@ -24,7 +24,7 @@ bool L3<T, N>::host_pair_alt_table(V* twr_alt)
 {
     if constexpr (PAIR_RX2 > 0) {
         using G2 = RowGeom<T, N, PAIR_RX2>;
-        transform_table<V, N / 2, G2::R>(twr_alt);
+        transform_table<V, N / 2, G2>(twr_alt);
         return true;
     } else {
         (void)twr_alt;
@@ -46,8 +46,8 @@ int L3<T, N>::pair_variants()
 template <typename T, int N>
 void L3<T, N>::host_tables(V* twp, V* twr)
 {
-    transform_table<V, N, PG::R>(twp);
-    transform_table<V, N / 2, RG::R>(twr);
+    transform_table<V, N, PG>(twp);
+    transform_table<V, N / 2, RG>(twr);
 }
 
 template <typename T, int N>
