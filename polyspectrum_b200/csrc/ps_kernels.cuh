@@ -686,8 +686,8 @@ __device__ __forceinline__ V2<T> load_pair(int kind, const unsigned char* ra, co
 //  * STAGED: the tile's input bytes (contiguous: WZ rows of N values per input
 //    array) are copied to shared memory by cp.async (16-byte, L2-only) and the
 //    loader reads its value pairs from there, so no register holds a load in
-//    flight; FP32 rows of 512 then run four 256-thread CTAs per SM with up to
-//    64 registers.  Needs 16-byte aligned inputs of 4- or 8-byte values.
+//    flight; the exchange buffers of the rows then take the stage's place, and FP32
+//    rows of 512 run five 256-thread CTAs per SM.  Needs 16-byte aligned inputs of 4- or 8-byte values.
 //    With BULK the tile arrives by one bulk copy per input array
 //    (cp.async.bulk through the TMA engine, completion counted on an mbarrier)
 //    instead of one 16-byte cp.async per thread and chunk.  The wait on the
@@ -720,7 +720,7 @@ __device__ __forceinline__ bool mbar_try_wait_parity(unsigned bar, unsigned pari
 
 template <typename T, int N, bool STAGED, bool BULK = false>
 __global__ void __launch_bounds__(RowGeom<T, N>::THREADS,
-                                  (sizeof(T) == 4 && N == 512) ? (STAGED ? 4 : 8) : 1)
+                                  (sizeof(T) == 4 && N == 512) ? (STAGED ? 5 : 8) : 1)
     k_fwd_z(int kind, const void* __restrict__ a_src, const void* __restrict__ b_src,
             V2<T>* __restrict__ dst, int dst_stride, int hout, int vec, const V2<T>* __restrict__ twr_g,
             const V2<T>* __restrict__ twpp_g, int* __restrict__ status = nullptr, int tx_extra = 0)
@@ -734,7 +734,7 @@ __global__ void __launch_bounds__(RowGeom<T, N>::THREADS,
     if constexpr (STAGED) {
         const int eb = (kind == SRC_F32 || kind == SRC_XHI_F32) ? 4 : 8;
         const size_t tile_bytes = (size_t)G::WZ * N * eb;
-        unsigned char* sa = smem_raw + G::STAGE_OFF;
+        unsigned char* sa = smem_raw + G::ROWBUF_OFF;  // the exchange buffers take its place later
         unsigned char* sb = sa + tile_bytes;
         const unsigned char* ga = reinterpret_cast<const unsigned char*>(a_src) + (size_t)blockIdx.x * tile_bytes;
         const unsigned char* gb =
@@ -787,6 +787,7 @@ __global__ void __launch_bounds__(RowGeom<T, N>::THREADS,
 #pragma unroll
         for (int e = 0; e < G::RT; e++)
             a[e] = G::tl(t0, e) ? load_pair<T>(kind, ra, rb, G::tp(t0, e)) : czero<V>();
+        __syncthreads();  // every row is in registers
         r2c_row<T, N>(a, rc, dst + row * dst_stride, hout);
     } else {
         if (kind == SRC_T) {

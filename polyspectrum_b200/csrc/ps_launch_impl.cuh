@@ -102,7 +102,8 @@ int L3<T, N>::fwd_z(cudaStream_t st, int kind, const void* a, const void* b, V* 
     const bool two = kind == SRC_XHI_F32 || kind == SRC_XHI_F64;
     const size_t eb = (kind == SRC_F32 || kind == SRC_XHI_F32) ? 4 : 8;
     const uintptr_t addr = (uintptr_t)a | (two ? (uintptr_t)b : 0);
-    const size_t smem_staged = RG::STAGE_OFF + (two ? 2 : 1) * (size_t)RG::WZ * N * eb;
+    const size_t smem_staged = RG::ROWBUF_OFF + std::max((two ? 2 : 1) * (size_t)RG::WZ * N * eb,
+                                                         (size_t)RG::WZ * RG::ROWBUF * sizeof(V));
     const bool can_stage = kind != SRC_T && addr % 16 == 0 && smem_staged <= 227 * 1024;
     const unsigned blocks = (unsigned)((nrows ? nrows : (size_t)N * N) / RG::WZ);
     if (blocks == 0) return PS_OK;
