@@ -394,26 +394,16 @@ bool grid_size_ok(int n)
 }
 double ref_pi() { return acos(-1.0); }  // filter.c:19
 
-// Pencil-tile width (complex elements per row segment) of the pencil kernels.
+// Columns every spectrum's row stride is a multiple of: the widest tile of a pencil
+// kernel; and the tile width of the summing X pass, whose blocks leave partial sums.
+// (One 128-byte segment but at 16 and 1024 points: L3 asserts it.)
+template <typename T> int dot_tile(int N)
+{
+    return N == 16 ? PencilGeom<T, 16>::W : N == 1024 ? PencilGeom<T, 1024>::W : PencilWidth<T>::value;
+}
 template <typename T> int pw(int N)
 {
-    switch (N) {
-    case 16: return PencilGeom<T, 16>::W;
-    case 32: return PencilGeom<T, 32>::W;
-    case 64: return PencilGeom<T, 64>::W;
-    case 128: return PencilGeom<T, 128>::W;
-    case 192: return PencilGeom<T, 192>::W;
-    case 256: return PencilGeom<T, 256>::W;
-    case 320: return PencilGeom<T, 320>::W;
-    case 384: return PencilGeom<T, 384>::W;
-    case 512: return PencilGeom<T, 512>::W;
-    case 48: return PencilGeom<T, 48>::W;
-    case 60: return PencilGeom<T, 60>::W;
-    case 96: return PencilGeom<T, 96>::W;
-    case 300: return PencilGeom<T, 300>::W;
-    case 600: return PencilGeom<T, 600>::W;
-    default: return PencilGeom<T, 1024>::W;
-    }
+    return N == 1024 ? std::max(StoreXGeom<T, 1024, 0>::type::W, dot_tile<T>(1024)) : dot_tile<T>(N);
 }
 
 template <typename T> int alloc_dev(T** p, size_t count)
@@ -957,7 +947,7 @@ int dot_pass(ps_gpu_ctx* c, V2<T>* data, int epi, int S, int hvalid, const Shell
     PS_TRY(tables_for<T>(c, N, &tb));
     for (int s0 = 0; s0 < ns; s0 += MAX_DOT_SHELLS) {
         const int cnt = std::min(MAX_DOT_SHELLS, ns - s0);
-        const size_t blocks = (size_t)N * (S / pw<T>(N));
+        const size_t blocks = (size_t)N * (S / dot_tile<T>(N));
         PS_TRY(ensure_partials(c, blocks * MAX_DOT_SHELLS));
         bool lut_ok = true;
         int lut_size = 0;
@@ -2201,7 +2191,7 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
     P->dsumA = sumA;
     P->dsumD = sumD;
     {
-        const size_t pen32 = (size_t)N * (c->f.S / pw<float>(N)), pen64 = (size_t)N * (c->d.S / pw<double>(N));
+        const size_t pen32 = (size_t)N * (c->f.S / dot_tile<float>(N)), pen64 = (size_t)N * (c->d.S / dot_tile<double>(N));
         const size_t np = std::max({(size_t)N * N, pen32 * MAX_DOT_SHELLS, pen64 * MAX_DOT_SHELLS,
                                     (size_t)148 * 8 * 2 * MAX_DOT_SHELLS,
                                     (size_t)p2_blocks * kP2Shells + iv.size() * kP2CountParts});
@@ -2325,7 +2315,7 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
     // dot passes, one launch each
     const auto sum_bytes = [&](size_t g, int M) {  // block sums of a group (twice with the condition numbers')
         const int Sp = round_up(info[g].hmax + 1, pw<float>(M));
-        return sizeof(double) * (size_t)M * (size_t)(Sp / pw<float>(M)) * info[g].gtable.size() * (kappa ? 2 : 1);
+        return sizeof(double) * (size_t)M * (size_t)(Sp / dot_tile<float>(M)) * info[g].gtable.size() * (kappa ? 2 : 1);
     };
     const auto group_bytes = [&](size_t g, int M) {  // spectra of a group
         const GroupInfo& I = info[g];
@@ -2409,7 +2399,7 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
                 it.interval = interval && it.nshell <= 2;
                 it.r2max = (int)std::min<long long>(r2max, 0x7fffffff);
                 it.weight = wD;
-                const int nblk = M * (Sp / w);
+                const int nblk = M * (Sp / dot_tile<float>(M));
                 for (int ab = 0; ab < (kappa ? 2 : 1); ab++) {
                     it.partials = part;
                     part += (size_t)nblk * it.nshell;
@@ -2496,7 +2486,7 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
     if (any_fft) {
         PS_TRY(ensure_pair_bufs(c, c->d));
         SideLane lane(c, true);  // the side lane's own scratch, profiling or not
-        PS_TRY(ensure_partials(c, std::max((size_t)N * N, (size_t)N * (c->d.S / pw<double>(N)) * MAX_DOT_SHELLS)));
+        PS_TRY(ensure_partials(c, std::max((size_t)N * N, (size_t)N * (c->d.S / dot_tile<double>(N)) * MAX_DOT_SHELLS)));
         PS_TRY(ensure_lut(c, (size_t)3 * (N / 2) * (N / 2) + 2));
     }
     auto fft_counts = [&](size_t g, int M) -> std::function<int()> {

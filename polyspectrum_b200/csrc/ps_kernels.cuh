@@ -50,7 +50,8 @@ template <typename T, int N> struct PencilThreads {
                                : N / ((sizeof(T) == 4 && N == 512) ? 16 : DefaultRadix<N>::value);
 };
 // RX > 0 takes the register plan with RX elements per thread (pass variants).
-template <typename T, int N, int RX = 0> struct PencilGeom {
+// MAXT: most threads of a CTA (the tile is then narrower than a 128-byte segment).
+template <typename T, int N, int RX = 0, int MAXT = 512> struct PencilGeom {
     static constexpr bool SPLIT = LenKind<N>::SPLIT && RX == 0;
     static constexpr int TPF = RX > 0 ? N / RX : PencilThreads<T, N>::value;
     using SG = SplitGeom<SPLIT ? N : 600, TPF>;
@@ -62,10 +63,10 @@ template <typename T, int N, int RX = 0> struct PencilGeom {
     __device__ static constexpr bool il(int t, int e) { return !SPLIT || SG::il(t, e); }
     __device__ static constexpr int op(int t, int e) { return SPLIT ? SG::op(t, e) : t + TPF * e; }
     __device__ static constexpr bool ol(int t, int e) { return !SPLIT || SG::ol(t, e); }
-    // one 128-byte segment per row, whole warps per CTA, at most 512 threads
-    // (so an epilogue keeps 16 FP64 accumulators in registers)
+    // one 128-byte segment per row, whole warps per CTA, at most MAXT threads
+    // (512: an epilogue keeps 16 FP64 accumulators in registers)
     static constexpr int W0 = PencilWidth<T>::value * TPF >= 32 ? PencilWidth<T>::value : 32 / TPF;
-    static constexpr int W = W0 * TPF > 512 ? 512 / TPF : W0;
+    static constexpr int W = W0 * TPF > MAXT ? MAXT / TPF : W0;
     static constexpr int THREADS = TPF * W;
     static constexpr size_t TW_BYTES = (size_t)N * sizeof(V2<T>);  // Stockham table (N-1 used)
     static constexpr size_t SMEM = TW_BYTES + (size_t)N * W * sizeof(V2<T>);
@@ -74,6 +75,19 @@ template <typename T, int N, int RX = 0> struct PencilGeom {
     static constexpr size_t DK_BYTES = (size_t)N * W * sizeof(V2<T>);
     static constexpr bool DK_SMEM = sizeof(T) == 4 && SMEM + DK_BYTES <= 227 * 1024;
     static constexpr size_t SMEM_DOT = SMEM + (DK_SMEM ? DK_BYTES : 0);
+};
+
+// Geometries of single passes at 1024 points in FP32.  The storing X pass, whose rows
+// lie 4 MB apart, takes whole 128-byte segments and one CTA of 1024 threads per SM
+// (2.43 against 2.92 ms for the 1024^3 field with 64-byte segments and two CTAs of
+// 512), the Y pass 32 elements per thread in two passes (1.91 against 2.11 ms).
+template <typename T, int N, int RX> struct StoreXGeom {
+    static constexpr bool WIDE = sizeof(T) == 4 && N == 1024 && RX == 0;
+    using type = PencilGeom<T, N, RX, WIDE ? 1024 : 512>;
+};
+template <typename T, int N, int RX> struct YGeom {
+    static constexpr bool LONG = sizeof(T) == 4 && N == 1024 && RX == 0;
+    using type = PencilGeom<T, N, LONG ? 32 : RX, LONG ? 256 : 512>;
 };
 
 // The alternative pencil geometry of the FP32 Y and dot passes for the larger
@@ -381,10 +395,10 @@ __global__ void __launch_bounds__(PencilGeom<T, N>::THREADS)
 
 // ------------------------------------------------------------------ Y pass
 template <typename T, int N, bool INV, int RX = 0>
-__global__ void __launch_bounds__(PencilGeom<T, N, RX>::THREADS)
+__global__ void __launch_bounds__(YGeom<T, N, RX>::type::THREADS)
     k_pass_y(const __grid_constant__ Items<YItem<T>> items, int quad_arg, const V2<T>* __restrict__ tw_g)
 {
-    using G = PencilGeom<T, N, RX>;
+    using G = typename YGeom<T, N, RX>::type;
     using V = V2<T>;
     const int quad = quad_arg;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -992,10 +1006,20 @@ __global__ void __launch_bounds__(RowGeom<T, N>::THREADS)
                 if constexpr (REAL) c2r_row_real<T, N>(reinterpret_cast<const T*>(z), it.hv[f], rc, a);
                 else c2r_row<T, N>(z, it.hv[f], rc, a);
                 const int p = it.power[f];
+                if (p == 2) {  // one branch for the row, not a loop per element
+#pragma unroll
+                    for (int e = 0; e < G::RT; e++) a[e] = V{a[e].x * a[e].x, a[e].y * a[e].y};
+                } else if (p == 3) {
+#pragma unroll
+                    for (int e = 0; e < G::RT; e++) a[e] = V{a[e].x * a[e].x * a[e].x, a[e].y * a[e].y * a[e].y};
+                } else if (p > 3) {
+#pragma unroll
+                    for (int e = 0; e < G::RT; e++) a[e] = V{ipow(a[e].x, p), ipow(a[e].y, p)};
+                }
                 double s = 0.0;
 #pragma unroll
                 for (int e = 0; e < G::RT; e++) {
-                    const T x0 = ipow(a[e].x, p), x1 = ipow(a[e].y, p);
+                    const T x0 = a[e].x, x1 = a[e].y;
                     if (!last) {
                         prod[e] = f == 0 ? V{x0, x1} : V{prod[e].x * x0, prod[e].y * x1};
                     } else if (G::tl(rc.t, e)) {
@@ -1041,15 +1065,17 @@ enum SpecEpi : int {
 // RX > 0 (FP32 dot passes, autotuned): the alternative pencil geometry of
 // PencilAlt, twice the elements per thread and one radix pass fewer.
 enum FwdKind : int { FWD_STORE = 0, FWD_SUMS = 1, FWD_MASK = 2 };
+template <typename T, int N, int KIND, int RX>
+using FwdXGeom = std::conditional_t<KIND == FWD_STORE, typename StoreXGeom<T, N, RX>::type, PencilGeom<T, N, RX>>;
 template <typename T, int N, int KIND, int RX = 0>
-__global__ void __launch_bounds__(PencilGeom<T, N, RX>::THREADS,
+__global__ void __launch_bounds__(FwdXGeom<T, N, KIND, RX>::THREADS,
                                   KIND == FWD_SUMS ? (((sizeof(T) == 4 && N <= 384) || PencilGeom<T, N, RX>::THREADS <= 256) ? 2 : 1)
-                                      : (sizeof(T) == 8 ? 1 : 2))
+                                      : (sizeof(T) == 8 || FwdXGeom<T, N, KIND, RX>::THREADS > 512 ? 1 : 2))
     k_fwd_x(const __grid_constant__ std::conditional_t<KIND == FWD_SUMS, Items<FwdXItem<T>>, FwdXItem<T>> items, int epi,
             V2<T>* out, int out_stride, const V2<T>* __restrict__ dk, int dk_stride, int ndk, int quad_arg, const V2<T>* __restrict__ tw_g,
             T* __restrict__ mod_out, int jband)
 {
-    using G = PencilGeom<T, N, RX>;
+    using G = FwdXGeom<T, N, KIND, RX>;
     using V = V2<T>;
     constexpr bool DOT = KIND == FWD_SUMS;
     const int quad = DOT && sizeof(T) == 8 ? quad_arg : 0;  // FP64 counts only

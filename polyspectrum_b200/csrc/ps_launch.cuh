@@ -73,10 +73,11 @@ template <typename T, int N> struct L3 {
     using V = V2<T>;
     using PG = PencilGeom<T, N>;
     using RG = RowGeom<T, N>;
-    static int pencil_width() { return PG::W; }
+    static_assert(N == 16 || N == 1024 || PG::W == PencilWidth<T>::value, "tiles of one 128-byte segment");
     static constexpr int ALT = PencilAlt<T, N>::value;
     static constexpr int DOT_ALT = PencilAlt<T, N>::dot_default;
-    // host copy of the alternative Y pass's table (false: no alternative)
+    // host copy of the alternative pencil table, or of the Y pass's where it has a
+    // geometry of its own (false: neither)
     static bool host_alt_table(V* twp_alt);
     static constexpr int PAIR_RX2 = PairVariants<T, N>::ALT_RX;
     // host copy of the row table of pair kernel variant 2 (false: no such variant)

@@ -13,6 +13,9 @@ bool L3<T, N>::host_alt_table(V* twp_alt)
         static_assert(PencilGeom<T, N, ALT>::W == PG::W, "same pencil tile width");
         transform_table<V, N, PencilGeom<T, N, ALT>>(twp_alt);
         return true;
+    } else if constexpr (YGeom<T, N, 0>::LONG) {  // the Y pass's own geometry
+        transform_table<V, N, typename YGeom<T, N, 0>::type>(twp_alt);
+        return true;
     } else {
         (void)twp_alt;
         return false;
@@ -65,7 +68,8 @@ template <typename T, int N>
 int L3<T, N>::pass_y_b(cudaStream_t st, const YItem<T>* items, int nitems, int ncols, bool inv,
                        const Tables<T>& tb, int quad, int alt)
 {
-    const dim3 grid((unsigned)((quad ? N / 2 + 1 : N) * (ncols / PG::W)), (unsigned)nitems);
+    using YG = typename YGeom<T, N, 0>::type;  // (the alternative geometries have the default's tile width)
+    const dim3 grid((unsigned)((quad ? N / 2 + 1 : N) * (ncols / YG::W)), (unsigned)nitems);
     auto go = [&](auto kernel, int threads, size_t smem, const V* tw) -> int {
         PS_LTRY(set_smem(kernel, smem));
         kernel<<<grid, threads, smem, st>>>(pack(items, nitems), quad, tw);
@@ -77,8 +81,8 @@ int L3<T, N>::pass_y_b(cudaStream_t st, const YItem<T>* items, int nitems, int n
             return inv ? go(k_pass_y<T, N, true, ALT>, PA::THREADS, PA::SMEM, tb.twp_alt)
                        : go(k_pass_y<T, N, false, ALT>, PA::THREADS, PA::SMEM, tb.twp_alt);
     }
-    return inv ? go(k_pass_y<T, N, true>, PG::THREADS, PG::SMEM, tb.twp)
-               : go(k_pass_y<T, N, false>, PG::THREADS, PG::SMEM, tb.twp);
+    const V* tw = YGeom<T, N, 0>::LONG ? tb.twp_alt : tb.twp;
+    return inv ? go(k_pass_y<T, N, true>, YG::THREADS, YG::SMEM, tw) : go(k_pass_y<T, N, false>, YG::THREADS, YG::SMEM, tw);
 }
 
 template <typename T, int N>
@@ -199,7 +203,9 @@ int L3<T, N>::fwd_x(cudaStream_t st, const FwdXItem<T>* items, int nitems, int n
                     V* out, int ostride, const V* dk, int dks, const Tables<T>& tb, int* nblocks, int quad, int ndk,
                     T* mod_out, int jband, int alt)
 {
-    const dim3 grid((unsigned)((quad ? N / 2 + 1 : N) * (ncols / PG::W)), (unsigned)nitems);
+    using SG = typename StoreXGeom<T, N, 0>::type;
+    const bool store = epi == SPEC_STORE || epi == SPEC_STORE_PHASE;
+    const dim3 grid((unsigned)((quad ? N / 2 + 1 : N) * (ncols / (store ? SG::W : PG::W))), (unsigned)nitems);
     const bool dot = epi == SPEC_DOT || epi == SPEC_COUNT || epi == SPEC_DOT_ABS;
     if (nblocks) *nblocks = (int)grid.x;
     auto go = [&](auto batch, auto kernel, int threads, size_t smem, const V* tw) -> int {
@@ -219,7 +225,7 @@ int L3<T, N>::fwd_x(cudaStream_t st, const FwdXItem<T>* items, int nitems, int n
     }
     if (dot) return go(std::true_type{}, k_fwd_x<T, N, FWD_SUMS>, PG::THREADS, PG::SMEM_DOT, tb.twp);
     return epi == SPEC_MASK_ADD ? go(std::false_type{}, k_fwd_x<T, N, FWD_MASK>, PG::THREADS, PG::SMEM, tb.twp)
-                                : go(std::false_type{}, k_fwd_x<T, N, FWD_STORE>, PG::THREADS, PG::SMEM, tb.twp);
+                                : go(std::false_type{}, k_fwd_x<T, N, FWD_STORE>, SG::THREADS, SG::SMEM, tb.twp);
 }
 
 }  // namespace ps
