@@ -261,10 +261,55 @@ struct PlanArena {
     unsigned char* dev = nullptr;
     unsigned char* host = nullptr;
     size_t cap = 0, used = 0, flushed = 0;
+    size_t host_cap = 0;  // the mirror's own size, at least cap
 };
 constexpr size_t kArenaBytes = (size_t)1 << 20;  // smallest arena
+
+// Page-locked host blocks of closed contexts' arenas, kept for the process's next ones
+// (allocating 1 MB page-locked takes 1 to 3 ms, more than a first evaluation): at most
+// kHostBlocks of them, at most kSpareBytes in all; any thread may take and give.
+constexpr size_t kHostBlocks = 8;
+struct HostBlocks {
+    std::mutex m;
+    std::vector<std::pair<unsigned char*, size_t>> kept;
+    size_t bytes = 0;
+    static HostBlocks& get()
+    {
+        static HostBlocks* pool = new HostBlocks();  // (never destroyed: the runtime may be gone by then)
+        return *pool;
+    }
+    // a kept block of at least n bytes, the smallest; its size in *cap (NULL: none)
+    unsigned char* take(size_t n, size_t* cap)
+    {
+        std::lock_guard<std::mutex> lk(m);
+        size_t best = kept.size();
+        for (size_t q = 0; q < kept.size(); q++)
+            if (kept[q].second >= n && (best == kept.size() || kept[q].second < kept[best].second)) best = q;
+        if (best == kept.size()) return nullptr;
+        unsigned char* p = kept[best].first;
+        *cap = kept[best].second;
+        bytes -= *cap;
+        kept.erase(kept.begin() + (long)best);
+        return p;
+    }
+    void give(unsigned char* p, size_t cap);
+};
 constexpr size_t kSpareArenas = 4;
 constexpr size_t kSpareBytes = (size_t)64 << 20;  // larger arenas are given back at once
+
+void HostBlocks::give(unsigned char* p, size_t cap)
+{
+    if (!p) return;
+    {
+        std::lock_guard<std::mutex> lk(m);
+        if (kept.size() < kHostBlocks && bytes + cap <= kSpareBytes) {
+            kept.push_back({p, cap});
+            bytes += cap;
+            return;
+        }
+    }
+    cudaFreeHost(p);
+}
 
 struct ps_gpu_ctx {
     int N = 0;
@@ -1418,10 +1463,12 @@ int arena_take(ps_gpu_plan* P, size_t bytes, void** dev, void** host)
             const size_t prev = P->arenas.empty() ? 0 : P->arenas.back().cap;
             const size_t cap = std::max({bytes, kArenaBytes, std::min(2 * prev, kSpareBytes)});
             PS_TRY(alloc_dev(&a.dev, cap));
-            if (fault_hit(FAULT_ALLOC) || cudaHostAlloc((void**)&a.host, cap, cudaHostAllocDefault) != cudaSuccess) {
+            a.host = HostBlocks::get().take(cap, &a.host_cap);
+            if (!a.host && (fault_hit(FAULT_ALLOC) || cudaHostAlloc((void**)&a.host, cap, cudaHostAllocPortable) != cudaSuccess)) {
                 cudaFree(a.dev);
                 return fail(PS_ERR_OOM, "page-locked plan tables of %zu bytes", cap);
             }
+            a.host_cap = std::max(a.host_cap, cap);
             a.cap = cap;
         }
         a.used = a.flushed = 0;
@@ -2716,13 +2763,14 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
                     const int share = std::max(1, (int)(small ? ceil(part) : part));
                     const int nmc = std::max(1, (it.nb + threads * kCountBPT - 1) / (threads * kCountBPT));
                     const int nrs = std::max(1, std::min(it.nrep, ((small ? 2 : 8) * share + nmc - 1) / nmc));
-                    it.rep_slice = std::min(kCountRepChunk, std::max(8, (it.nrep + nrs - 1) / nrs));
+                    it.rep_slice = std::min(cl == 0 ? kOneRepChunk : kCountRepChunk, std::max(8, (it.nrep + nrs - 1) / nrs));
                     const int nitems = nmc * ((it.nrep + it.rep_slice - 1) / it.rep_slice);
                     it.cta0 = cta;
                     it.nctas = std::max(1, std::min(nitems, share));
                     cta += it.nctas;
                 }
-                Launch L{nullptr, (int)items.size(), cta, kCountStageBytes + (size_t)nb_max * sizeof(unsigned int), wrap != 0, cl};
+                Launch L{nullptr, (int)items.size(), cta,
+                         cl == 0 ? 0 : kCountStageBytes + (size_t)nb_max * sizeof(unsigned int), wrap != 0, cl};
                 PS_TRY(plan_upload(P, &L.items, items));
                 launches.push_back(L);
             }
@@ -2743,8 +2791,8 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
                     const auto go = [&](auto kernel, int threads) {
                         kernel<<<L.grid, threads, L.smem, c->stream>>>(L.items, L.n, N);
                     };
-                    if (L.cl == 0 && L.wrap) go(k_pair_counts<true, kCountBPT, kCountSmallThreads, true>, kCountSmallThreads);
-                    else if (L.cl == 0) go(k_pair_counts<false, kCountBPT, kCountSmallThreads, true>, kCountSmallThreads);
+                    if (L.cl == 0 && L.wrap) go(k_pair_counts_one<true>, kOneThreads);
+                    else if (L.cl == 0) go(k_pair_counts_one<false>, kOneThreads);
                     else if (L.cl == 1 && L.wrap) go(k_pair_counts<true, kCountBPT, kCountSmallThreads>, kCountSmallThreads);
                     else if (L.cl == 1) go(k_pair_counts<false, kCountBPT, kCountSmallThreads>, kCountSmallThreads);
                     else if (L.wrap) go(k_pair_counts<true>, kCountThreads);
@@ -3047,7 +3095,7 @@ void plan_release(ps_gpu_plan* P, bool keep)
                 c->spare_arenas.push_back(a);
             } else {
                 cudaFree(a.dev);
-                cudaFreeHost(a.host);
+                HostBlocks::get().give(a.host, a.host_cap);
             }
         }
         P->arenas.clear();
@@ -4379,7 +4427,7 @@ void ps_gpu_finalize(ps_gpu_ctx* c)
     c->plans.clear();
     for (PlanArena& a : c->spare_arenas) {
         cudaFree(a.dev);
-        cudaFreeHost(a.host);
+        HostBlocks::get().give(a.host, a.host_cap);
     }
     for (PlanArena& a : c->spare_device) cudaFree(a.dev);
     free_prec(c->f);

@@ -39,13 +39,9 @@ namespace ps {
 // 0.24 ms for the 2.2e8 wrapping pairs of 64 equilateral triangles at 128^3).
 constexpr int kCountBPT = 4;
 constexpr int kCountThreads = 1024;  // one CTA per SM: 32 warps to hide the atomics' latency
-// Lists of groups with one closing shell each (equilateral and single triangles)
-// need no histogram: a pair inside the shell's interval adds its weight in a
-// register (ONE), about seven instructions a pair without a branch or an atomic.
-// They and short histograms hold no SM's shared memory, and such a list is cut
-// finer: CTAs of 256 threads, six per SM in all, so that no group's last CTA is
-// left over.  64 equilateral triangles at 128^3: 0.42 ms with histograms and CTAs of
-// 1024 threads.
+// Short histograms hold no SM's shared memory, and a list of such groups is cut
+// finer: CTAs of 256 threads, six per SM in all, so that no group's last CTA is left
+// over.
 constexpr int kCountSmallBins = 2048, kCountSmallThreads = 256;
 constexpr int kCountRepChunk = 512;  // largest rep_slice
 constexpr size_t kCountStageBytes = kCountRepChunk * 2 * sizeof(int4);
@@ -61,7 +57,7 @@ struct CountItem {
     int nrep, nb, s_lo, nbins, rep_slice, ncl;
     int cta0, nctas;
 };
-template <bool WRAP, int BPT = kCountBPT, int THREADS = kCountThreads, bool ONE = false>
+template <bool WRAP, int BPT = kCountBPT, int THREADS = kCountThreads>
 __global__ void __launch_bounds__(THREADS, THREADS == kCountSmallThreads ? 6 : 1)
     k_pair_counts(const CountItem* __restrict__ items, int ngroups, int n)
 {
@@ -80,19 +76,9 @@ __global__ void __launch_bounds__(THREADS, THREADS == kCountSmallThreads ? 6 : 1
     int rep_slice = it.rep_slice;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     int4* srep = reinterpret_cast<int4*>(smem_raw);
-    int4* sedge = srep + kCountRepChunk;  // -2 n a (WRAP), |a|^2 - base
+    int4* sedge = srep + kCountRepChunk;  // -2 n a (WRAP), |a|^2 - s_lo
     unsigned int* hist = reinterpret_cast<unsigned int*>(smem_raw + kCountStageBytes);
-    int one_lo = 0;
-    unsigned one_span = 0u;
-    unsigned long long inside = 0ull;
-    if constexpr (ONE) {  // the interval, empty as one no value falls into
-        const int lo = closing[0].r2lo, hi = closing[0].r2hi;
-        one_lo = hi >= lo ? lo : 0x7fffffff;
-        one_span = hi >= lo ? (unsigned)(hi - lo) : 0u;
-    } else {
-        for (int i = threadIdx.x; i < nbins; i += blockDim.x) hist[i] = 0u;
-    }
-    const int base = ONE ? one_lo : s_lo;  // bins count from here
+    for (int i = threadIdx.x; i < nbins; i += blockDim.x) hist[i] = 0u;
     constexpr int kChunk = THREADS * BPT;
     rep_slice = max(1, min(rep_slice, kCountRepChunk));  // the staging buffer's size
     const int nmc = (nb + kChunk - 1) / kChunk, nrs = (nrep + rep_slice - 1) / rep_slice;
@@ -120,10 +106,9 @@ __global__ void __launch_bounds__(THREADS, THREADS == kCountSmallThreads ? 6 : 1
         for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
             const int4 a = reps[r0 + i];
             srep[i] = int4{2 * a.x, 2 * a.y, 2 * a.z, a.w};
-            sedge[i] = int4{-2 * n * a.x, -2 * n * a.y, -2 * n * a.z, a.x * a.x + a.y * a.y + a.z * a.z - base};
+            sedge[i] = int4{-2 * n * a.x, -2 * n * a.y, -2 * n * a.z, a.x * a.x + a.y * a.y + a.z * a.z - s_lo};
         }
         __syncthreads();
-        unsigned here = 0u;  // ONE: at most rep_slice BPT 48
 #pragma unroll 2
         for (int r = 0; r < cnt; r++) {
             const int4 a = srep[r];
@@ -133,17 +118,9 @@ __global__ void __launch_bounds__(THREADS, THREADS == kCountSmallThreads ? 6 : 1
                 int sb = d.w + bn[u] + a.x * bx[u] + a.y * by[u] + a.z * bz[u];
                 if constexpr (WRAP)
                     sb += __viaddmin_s32(d.x, ex[u], 0) + __viaddmin_s32(d.y, ey[u], 0) + __viaddmin_s32(d.z, ez[u], 0);
-                if constexpr (ONE) here += (unsigned)sb <= one_span ? (unsigned)a.w : 0u;
-                else if ((unsigned)sb < (unsigned)nbins) atomicAdd(&hist[sb], (unsigned)a.w);
+                if ((unsigned)sb < (unsigned)nbins) atomicAdd(&hist[sb], (unsigned)a.w);
             }
         }
-        inside += here;
-    }
-    if constexpr (ONE) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) inside += __shfl_xor_sync(0xffffffffu, inside, o);
-        if ((threadIdx.x & 31) == 0 && inside) atomicAdd(&counts[0], inside);
-        return;
     }
     __syncthreads();
     // closing shell c: the bins of its interval (clamped to the histogram)
@@ -157,6 +134,121 @@ __global__ void __launch_bounds__(THREADS, THREADS == kCountSmallThreads ? 6 : 1
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
         if (lane == 0 && v) atomicAdd(&counts[c], v);
     }
+}
+
+// The same for groups with one closing shell each (equilateral and single triangles),
+// without a histogram: a pair inside the shell's interval adds its weight in a
+// register.  The norms are computed in FP32, where every value is an integer or a half
+// below 2^23 (WRAP: doubled, below 2^24) and so exact, two modes per packed
+// instruction: about four instructions a pair, nine with WRAP, where
+// min(0, x) = (x - |x|) / 2 leaves one packed sum and an |x| operand per component.
+// (In integers, whose multiply-adds and minima issue at half rate, the 2.4e8 pairs of 64
+// equilateral triangles at 128^3 took 0.197 instead of 0.156 ms, with histograms 0.42 ms.)
+constexpr int kOneThreads = 256, kOneBPT = 4, kOneRepChunk = 256;
+
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
+{
+    float2 r;
+    asm("{\n\t.reg .b64 pa, pb, pc, pd;\n\tmov.b64 pa, {%2, %3};\n\tmov.b64 pb, {%4, %5};\n\tmov.b64 pc, {%6, %7};\n\t"
+        "fma.rn.f32x2 pd, pa, pb, pc;\n\tmov.b64 {%0, %1}, pd;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return r;
+}
+
+template <bool WRAP>
+__global__ void __launch_bounds__(kOneThreads, 4)
+    k_pair_counts_one(const CountItem* __restrict__ items, int ngroups, int n)
+{
+    int gi = 0;  // the group of this CTA
+    for (int e = ngroups; gi + 1 < e;) {
+        const int mid = (gi + e) >> 1;
+        if (items[mid].cta0 <= (int)blockIdx.x) gi = mid;
+        else e = mid;
+    }
+    const CountItem it = items[gi];
+    // representatives, each value twice (packed operands): f (a, c), f a = 2 a (WRAP: 4 a),
+    // c the constant part; WRAP: -2 n a
+    __shared__ float2 sa[kOneRepChunk][4], su[WRAP ? kOneRepChunk : 1][4];
+    __shared__ unsigned sw[kOneRepChunk];
+    const int lo = it.closing[0].r2lo, hi = it.closing[0].r2hi;
+    const float f = WRAP ? 2.f : 1.f, fn = (float)n;
+    const float mid = 0.5f * f * ((float)lo + (float)hi);
+    const float hw = hi >= lo ? 0.5f * f * ((float)hi - (float)lo) : -1.f;  // no value is within -1
+    constexpr int kChunk = kOneThreads * kOneBPT, NP = kOneBPT / 2;
+    const int rep_slice = max(1, min(it.rep_slice, kOneRepChunk));
+    const int nmc = (it.nb + kChunk - 1) / kChunk, nrs = (it.nrep + rep_slice - 1) / rep_slice;
+    unsigned long long inside = 0ull;
+    for (int item = (int)blockIdx.x - it.cta0; item < nmc * nrs; item += it.nctas) {
+        const int mc = item % nmc, r0 = (item / nmc) * rep_slice;
+        const int cnt = min(rep_slice, it.nrep - r0);
+        float2 bx[NP], by[NP], bz[NP], bc[NP], ex[NP], ey[NP], ez[NP];
+#pragma unroll
+        for (int p = 0; p < NP; p++)
+#pragma unroll
+            for (int l = 0; l < 2; l++) {
+                const int idx = mc * kChunk + (2 * p + l) * kOneThreads + (int)threadIdx.x;
+                const bool valid = idx < it.nb;
+                const short4 m = valid ? it.modes[idx] : short4{0, 0, 0, 0};
+                const float x = (float)m.x, y = (float)m.y, z = (float)m.z;
+                const float qx = fn * (fn - 2.f * x), qy = fn * (fn - 2.f * y), qz = fn * (fn - 2.f * z);
+                float c = f * (x * x + y * y + z * z);
+                if (WRAP) c += qx + qy + qz;
+                if (!valid) c = 1e30f;  // never inside
+                (l ? bx[p].y : bx[p].x) = x;
+                (l ? by[p].y : by[p].x) = y;
+                (l ? bz[p].y : bz[p].x) = z;
+                (l ? bc[p].y : bc[p].x) = c;
+                (l ? ex[p].y : ex[p].x) = qx;
+                (l ? ey[p].y : ey[p].x) = qy;
+                (l ? ez[p].y : ez[p].x) = qz;
+            }
+        __syncthreads();  // the previous item's representatives are no longer read
+        for (int i = threadIdx.x; i < cnt; i += kOneThreads) {
+            const int4 a = it.reps[r0 + i];
+            const float x = (float)a.x, y = (float)a.y, z = (float)a.z;
+            const float ux = -2.f * fn * x, uy = -2.f * fn * y, uz = -2.f * fn * z;
+            float c = f * (x * x + y * y + z * z) - mid;
+            if (WRAP) c += ux + uy + uz;
+            sa[i][0] = float2{2.f * f * x, 2.f * f * x};
+            sa[i][1] = float2{2.f * f * y, 2.f * f * y};
+            sa[i][2] = float2{2.f * f * z, 2.f * f * z};
+            sa[i][3] = float2{c, c};
+            if constexpr (WRAP) {
+                su[i][0] = float2{ux, ux};
+                su[i][1] = float2{uy, uy};
+                su[i][2] = float2{uz, uz};
+            }
+            sw[i] = (unsigned)a.w;
+        }
+        __syncthreads();
+        unsigned here = 0u;  // at most rep_slice BPT 48
+#pragma unroll 2
+        for (int r = 0; r < cnt; r++) {
+            const float4 a01 = *reinterpret_cast<const float4*>(sa[r]), a23 = *reinterpret_cast<const float4*>(sa[r] + 2);
+            const unsigned w = sw[r];
+#pragma unroll
+            for (int p = 0; p < NP; p++) {
+                float2 v = cadd(float2{a23.z, a23.w}, bc[p]);
+                v = fma2(float2{a01.x, a01.y}, bx[p], v);
+                v = fma2(float2{a01.z, a01.w}, by[p], v);
+                v = fma2(float2{a23.x, a23.y}, bz[p], v);
+                if constexpr (WRAP) {
+                    const float4 u01 = *reinterpret_cast<const float4*>(su[r]);
+                    const float2 tx = cadd(float2{u01.x, u01.y}, ex[p]), ty = cadd(float2{u01.z, u01.w}, ey[p]),
+                                 tz = cadd(su[r][2], ez[p]);
+                    v.x = ((v.x - fabsf(tx.x)) - fabsf(ty.x)) - fabsf(tz.x);
+                    v.y = ((v.y - fabsf(tx.y)) - fabsf(ty.y)) - fabsf(tz.y);
+                }
+                if (fabsf(v.x) <= hw) here += w;
+                if (fabsf(v.y) <= hw) here += w;
+            }
+        }
+        inside += here;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) inside += __shfl_xor_sync(0xffffffffu, inside, o);
+    if ((threadIdx.x & 31) == 0 && inside) atomicAdd(&it.counts[0], inside);
 }
 
 // sumI[idx[c]] = counts[c] (exact integers, below 2^53)
@@ -250,7 +342,8 @@ inline bool pair_count_lists(const Shell& sa, const Shell& sb, int N, int c_lo, 
     L->reps = interval_orbits(*pa, N);
     if (48.0 * (double)L->reps.size() * 4.19 * std::max(volume(*pb), 1.0) / 48.0 > 1.2e10) return false;
     L->modes = interval_modes(*pb, N);
-    // about 5 (wrapping 1.2) pairs in a nanosecond; the transforms take 1.5 ms at 600 points
+    // a single closing shell takes about 1.5 wrapping pairs in a nanosecond (0.14 ms of
+    // the 128^3 sweep's), the transforms of a group at 600 points 1.5 ms
     const bool wraps = std::min(sa.band, N / 2) + std::min(sb.band, N / 2) >= N / 2;
     if ((double)L->reps.size() * (double)L->modes.size() > (wraps ? 1.5e9 : 4e9)) return false;
     const int bmax_a = std::min(sa.band, N / 2), bmax_b = std::min(sb.band, N / 2);

@@ -77,17 +77,18 @@ template <typename T, int N, int RX = 0, int MAXT = 512> struct PencilGeom {
     static constexpr size_t SMEM_DOT = SMEM + (DK_SMEM ? DK_BYTES : 0);
 };
 
-// Geometries of single passes at 1024 points in FP32.  The storing X pass, whose rows
+// Geometries of single passes at 512 and 1024 points in FP32.  The storing X pass, whose rows
 // lie 4 MB apart, takes whole 128-byte segments and one CTA of 1024 threads per SM
 // (2.43 against 2.92 ms for the 1024^3 field with 64-byte segments and two CTAs of
-// 512), the Y pass 32 elements per thread in two passes (1.91 against 2.11 ms).
+// 512), the Y pass 32 elements per thread in two passes (1.91 against 2.11 ms; at 512
+// points 0.146 against 0.156 ms).
 template <typename T, int N, int RX> struct StoreXGeom {
     static constexpr bool WIDE = sizeof(T) == 4 && N == 1024 && RX == 0;
     using type = PencilGeom<T, N, RX, WIDE ? 1024 : 512>;
 };
 template <typename T, int N, int RX> struct YGeom {
-    static constexpr bool LONG = sizeof(T) == 4 && N == 1024 && RX == 0;
-    using type = PencilGeom<T, N, LONG ? 32 : RX, LONG ? 256 : 512>;
+    static constexpr bool LONG = sizeof(T) == 4 && (N == 512 || N == 1024) && RX == 0;
+    using type = PencilGeom<T, N, LONG ? 32 : RX, LONG && N == 1024 ? 256 : 512>;
 };
 
 // The alternative pencil geometry of the FP32 Y and dot passes for the larger
@@ -135,8 +136,7 @@ template <typename T, int N, int RX = 0> struct RowGeom {
     // Rows shorter than a 128-byte block of threads share a warp: their buffers are
     // set apart by SKEW elements modulo a block, so that the rows of a warp fall on
     // different banks (rows of 4 threads at 96 points: two of three shared-memory
-    // accesses were conflicts, pair kernel of 13 equilateral groups at 128 points
-    // 0.134 -> @@ ms).
+    // accesses were conflicts; pair kernel of a batch there 0.031 -> 0.015 ms).
     static constexpr int BLOCK = 128 / (int)sizeof(V2<T>);
     static constexpr int SKEW = TPF < BLOCK ? (TPF < EPC ? EPC : TPF) : 0;
     // rows per CTA (tile): up to 256 threads and 32 rows, and as many as fit
