@@ -795,38 +795,63 @@ int sum_partials(ps_gpu_ctx* c, int nblocks, int ncols, double* out, int out_str
     return PS_OK;
 }
 
-// Inverse X and Y passes of a shell-filtered spectrum into dst, band-limited to
-// the shell: h < hb = min(band, N/2) + 1 columns, row stride *S_out.
-// mode: LOAD_MASKED (F * field spectrum) or LOAD_UNIT (F).  M > 0 runs the
-// transform on an M-grid (M < N, the shell's band below M/2): the same
-// spectrum sampled on a coarser real-space grid.
-template <typename T>
-int c2r_xy(ps_gpu_ctx* c, int mode, const Shell* dshell, int band, V2<T>* dst, int* S_out, int* hb_out,
-           int quad = 0, int M = 0)
+// Inverse X and Y passes of up to kItems shell-filtered spectra, each into its dst,
+// band-limited to its shell: h < hb = min(band, N/2) + 1 columns, row stride S (both
+// set here), one launch per pass.  mode: LOAD_MASKED (F * field spectrum) or LOAD_UNIT
+// (F, on the quadrant).  M > 0 runs the transforms on an M-grid (M < N, the shells'
+// bands below M/2): the same spectra sampled on a coarser real-space grid.
+template <typename T> struct XyLeg {
+    const Shell* dshell;
+    int band;
+    V2<T>* dst;
+    int S, hb;
+};
+template <typename T> void size_leg(XyLeg<T>& l, int M, int quad)
+{
+    l.hb = std::min(l.band, M / 2) + 1;
+    l.S = round_up(quad ? (l.hb + 1) / 2 : l.hb, pw<T>(M));  // quad: two columns per element
+}
+template <typename T> int c2r_xy_n(ps_gpu_ctx* c, int mode, XyLeg<T>* legs, int n, int quad = 0, int M = 0)
 {
     PrecBufs<T>& B = bufs<T>(c);
     const int N = M > 0 ? M : c->N;
     Tables<T> tb;
     PS_TRY(tables_for<T>(c, N, &tb));
-    const int hb = std::min(band, N / 2) + 1;
-    const int S = round_up(quad ? (hb + 1) / 2 : hb, pw<T>(N));  // quad: two columns per element
-    const double V = sizeof(V2<T>), NN2 = (double)N * N;
-    {
-        Prof pf(c);
-        PS_SWITCH_N(N, PS_TRY((L3<T, NN>::inv_x(c->stream, B.spec, B.S, dst, S, mode, dshell, N / 2 + 1, tb, quad,
-                                                c->N, 1))));
-        const double q = quad ? (double)(N / 2 + 1) * (N / 2 + 1) / NN2 : 1.0;
-        pf.end(fam<T>(KF_INV_X), q * NN2 * S * V + (mode == LOAD_MASKED ? NN2 * hb * V : 0.0), N);
+    const double V = sizeof(V2<T>), NN2 = (double)N * N, q = quad ? (double)(N / 2 + 1) * (N / 2 + 1) / NN2 : 1.0;
+    std::vector<XItem<T>> xi;
+    std::vector<YItem<T>> yi;
+    int Smax = 0;
+    double bx = 0.0, by = 0.0;
+    for (int x = 0; x < n; x++) {
+        XyLeg<T>& l = legs[x];
+        size_leg(l, N, quad);
+        xi.push_back(XItem<T>{l.dst, l.S, N / 2 + 1, l.dshell, 0});
+        yi.push_back(YItem<T>{l.dst, l.S, l.S, std::min(l.band, N / 2), N});
+        Smax = std::max(Smax, l.S);
+        bx += q * NN2 * l.S * V + (mode == LOAD_MASKED ? NN2 * l.hb * V : 0.0);
+        by += 2.0 * q * NN2 * l.S * V;
     }
     {
         Prof pf(c);
-        PS_SWITCH_N(N, PS_TRY((L3<T, NN>::pass_y(c->stream, dst, S, true, tb, quad, std::min(band, N / 2), 0, NN,
-                                                 pencil_alt_of<T>(c, N)))));
-        const double q = quad ? (double)(N / 2 + 1) * (N / 2 + 1) / NN2 : 1.0;
-        pf.end(fam<T>(KF_PASS_Y), 2.0 * q * NN2 * S * V, N);
+        PS_SWITCH_N(N, PS_TRY((L3<T, NN>::inv_x_b(c->stream, B.spec, B.S, xi.data(), n, Smax, mode, tb, quad, c->N, 1))));
+        pf.end(fam<T>(KF_INV_X), bx, N);
     }
-    *S_out = S;
-    *hb_out = hb;
+    {
+        Prof pf(c);
+        PS_SWITCH_N(N, PS_TRY((L3<T, NN>::pass_y_b(c->stream, yi.data(), n, Smax, true, tb, quad, pencil_alt_of<T>(c, N)))));
+        pf.end(fam<T>(KF_PASS_Y), by, N);
+    }
+    return PS_OK;
+}
+
+// One spectrum on the context's own grid.
+template <typename T>
+int c2r_xy(ps_gpu_ctx* c, int mode, const Shell* dshell, int band, V2<T>* dst, int* S_out, int* hb_out)
+{
+    XyLeg<T> l{dshell, band, dst, 0, 0};
+    PS_TRY(c2r_xy_n<T>(c, mode, &l, 1));
+    *S_out = l.S;
+    *hb_out = l.hb;
     return PS_OK;
 }
 
@@ -2544,11 +2569,12 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
         const int hmax = info[g].hmax;
         const int hout = info[g].hmax + 1, go = gofs[g], io = gidx_ofs[g];
         return [=]() {
-            int Sa = 0, ha = 0, Sb = 0, hbb = 0, S = 0;
-            PS_TRY(c2r_xy<double>(c, LOAD_UNIT, dtable + G.a, sa.band, c->d.work, &Sa, &ha, 1, M));
-            if (G.a != G.b)
-                PS_TRY(c2r_xy<double>(c, LOAD_UNIT, dtable + G.b, sb.band, c->d.work2, &Sb, &hbb, 1, M));
-            PS_TRY(pair_spectrum<double>(c, c->d.work, Sa, ha, G.a != G.b ? c->d.work2 : nullptr, Sb, hbb, hout, &S, 1, M));
+            XyLeg<double> l[2] = {{dtable + G.a, sa.band, c->d.work, 0, 0}, {dtable + G.b, sb.band, c->d.work2, 0, 0}};
+            const bool two = G.a != G.b;
+            int S = 0;
+            PS_TRY(c2r_xy_n<double>(c, LOAD_UNIT, l, two ? 2 : 1, 1, M));
+            PS_TRY(pair_spectrum<double>(c, l[0].dst, l[0].S, l[0].hb, two ? l[1].dst : nullptr, l[1].S, l[1].hb, hout, &S,
+                                         1, M));
             PS_TRY(dot_pass<double>(c, c->d.work3, SPEC_COUNT, S, hout, dtable + go, gtable.data(), (int)gtable.size(), sumI,
                                     1, M, 1.0, didx + io, &vol, hmax));
             return PS_OK;
@@ -3305,7 +3331,6 @@ int grad_impl(ps_gpu_ctx* c, int n, const std::vector<Shell>& legs, double scale
     const int N = c->N;
     const size_t nspec = (size_t)N * N * B.S;
     const size_t n3 = (size_t)N * N * N;
-    PS_TRY(ensure_pair_bufs(c, B));
     PS_TRY(alloc_dev(&B.hacc, nspec));
     PS_TRY(ensure_shells(c, PS_MAX_LEGS));
     PS_CK(cudaMemcpyAsync(c->dshells, legs.data(), sizeof(Shell) * n, cudaMemcpyHostToDevice, c->stream));
@@ -3349,26 +3374,97 @@ int grad_impl(ps_gpu_ctx* c, int n, const std::vector<Shell>& legs, double scale
             }
             if (!found) terms.push_back({key, 1});
         }
-        for (const auto& term : terms) {
-            const int li = term.first[0], la = term.first[1], lb = term.first[2];
-            const bool same = same_shell(legs[la], legs[lb]);
-            int Sa = 0, ha = 0, Sb = 0, hbb = 0, S = 0;
-            PS_TRY(c2r_xy<T>(c, LOAD_MASKED, c->dshells + la, legs[la].band, B.work, &Sa, &ha, 0, M));
-            if (!same) PS_TRY(c2r_xy<T>(c, LOAD_MASKED, c->dshells + lb, legs[lb].band, B.work2, &Sb, &hbb, 0, M));
-            const int hout = std::min(legs[li].band, N / 2) + 1;
-            PS_TRY(pair_spectrum<T>(c, B.work, Sa, ha, same ? nullptr : B.work2, Sb, hbb, hout, &S, 0, M));
-            const int N = M;  // PS_SWITCH_N's subject
-            Prof pf(c);
+        // the distinct legs, and where each leg's transform is
+        std::vector<XyLeg<T>> lx;
+        int at[3];
+        for (int l = 0; l < 3; l++) {
+            at[l] = -1;
+            for (int p = 0; p < l && at[l] < 0; p++)
+                if (same_shell(legs[p], legs[l])) at[l] = at[p];
+            if (at[l] < 0) {
+                at[l] = (int)lx.size();
+                lx.push_back(XyLeg<T>{c->dshells + l, legs[l].band, nullptr, 0, 0});
+            }
+        }
+        // all legs and products side by side when they fit the work spectrum (any M up to
+        // about N/2): one launch per pass for all terms.  Else term by term through the
+        // three work spectra.
+        const size_t rows = (size_t)M * M;
+        size_t need = 0;
+        for (auto& l : lx) {
+            size_leg(l, M, 0);
+            need += rows * (size_t)l.S;
+        }
+        for (const auto& term : terms) need += rows * (size_t)round_up(std::min(legs[term.first[0]].band, N / 2) + 1, pw<T>(M));
+        const bool side_by_side = need <= nspec;
+        if (!side_by_side) PS_TRY(ensure_pair_bufs(c, B));
+        const auto add = [&](V2<T>* data, int S, int li, double weight) -> int {  // hacc += weight F_li FFT_x[data]
             FwdXItem<T> it{};
-            it.data = B.work3;
+            it.data = data;
             it.stride = it.ncols = S;
-            it.hvalid = hout;
+            it.hvalid = std::min(legs[li].band, c->N / 2) + 1;
             it.shells = c->dshells + li;
             it.nshell = 1;
-            it.weight = up * (double)term.second;
+            it.weight = weight;
+            const int N = M;  // PS_SWITCH_N's subject
+            Prof pf(c);
             PS_SWITCH_N(N, PS_TRY((L3<T, NN>::fwd_x(c->stream, &it, 1, S, SPEC_MASK_ADD, B.hacc, B.S, nullptr, 0, tm,
                                                     nullptr, 0, c->N))));
             pf.end(fam<T>(KF_GRAD), 3.0 * N * N * S * sizeof(V2<T>), N);
+            return PS_OK;
+        };
+        if (side_by_side) {
+            V2<T>* p = B.work;
+            for (auto& l : lx) {
+                l.dst = p;
+                p += rows * (size_t)l.S;
+            }
+            PS_TRY(c2r_xy_n<T>(c, LOAD_MASKED, lx.data(), (int)lx.size(), 0, M));
+            std::vector<PairItem<T>> two, one;  // products of two legs, squares
+            std::vector<YItem<T>> yf;
+            std::vector<V2<T>*> prod;
+            int Pmax = 0, ha = 0, hb2 = 0;
+            for (const auto& term : terms) {
+                const XyLeg<T>&la = lx[at[term.first[1]]], &lb = lx[at[term.first[2]]];
+                const bool same = at[term.first[1]] == at[term.first[2]];
+                const int hout = std::min(legs[term.first[0]].band, N / 2) + 1, S = round_up(hout, pw<T>(M));
+                (same ? one : two).push_back(PairItem<T>{la.dst, same ? nullptr : lb.dst, p, la.S, la.hb, lb.S, lb.hb, S, hout});
+                yf.push_back(YItem<T>{p, S, S, M, hout - 1});
+                prod.push_back(p);
+                p += rows * (size_t)S;
+                Pmax = std::max(Pmax, S);
+                ha = std::max(ha, la.hb);
+                hb2 = std::max(hb2, lb.hb);
+            }
+            const int nt = (int)terms.size();
+            {
+                const int N = M;
+                for (const auto* v : {&two, &one}) {
+                    if (v->empty()) continue;
+                    Prof pf(c);
+                    PS_SWITCH_N(N, PS_TRY((L3<T, NN>::pair_z_b(c->stream, v->data(), (int)v->size(), v == &two ? 2 : 1, ha, hb2,
+                                                               tm, 0, pair_var_of<T>(c, M)))));
+                    pf.end(fam<T>(KF_PAIR_Z), (double)rows * 3.0 * Pmax * sizeof(V2<T>) * v->size(), M);
+                }
+                Prof pf(c);
+                PS_SWITCH_N(N, PS_TRY((L3<T, NN>::pass_y_b(c->stream, yf.data(), nt, Pmax, false, tm, 0,
+                                                           pencil_alt_of<T>(c, M)))));
+                pf.end(fam<T>(KF_PASS_Y), 2.0 * rows * Pmax * sizeof(V2<T>) * nt, M);
+            }
+            for (int q = 0; q < nt; q++) PS_TRY(add(prod[q], yf[q].stride, terms[q].first[0], up * (double)terms[q].second));
+        } else {
+            for (const auto& term : terms) {
+                const int li = term.first[0];
+                XyLeg<T> l[2] = {lx[at[term.first[1]]], lx[at[term.first[2]]]};
+                const bool same = at[term.first[1]] == at[term.first[2]];
+                l[0].dst = B.work;
+                l[1].dst = B.work2;
+                int S = 0;
+                PS_TRY(c2r_xy_n<T>(c, LOAD_MASKED, l, same ? 1 : 2, 0, M));
+                PS_TRY(pair_spectrum<T>(c, l[0].dst, l[0].S, l[0].hb, same ? nullptr : l[1].dst, l[1].S, l[1].hb,
+                                        std::min(legs[li].band, N / 2) + 1, &S, 0, M));
+                PS_TRY(add(B.work3, S, li, up * (double)term.second));
+            }
         }
     }
     if (c->use_only_phase == 1) {  // the field entered through z/|z|
