@@ -1013,9 +1013,19 @@ __global__ void __launch_bounds__(RowGeom<T, N>::THREADS)
 #pragma unroll
                     for (int e = 0; e < G::RT; e++) a[e] = V{a[e].x * a[e].x * a[e].x, a[e].y * a[e].y * a[e].y};
                 } else if (p > 3) {
+                    // the last factor's power in two halves, whose product the sum takes in
+                    // double: the eighth power of 6e4 is above FP32's range
+                    const int q = last ? p - p / 2 : p;
 #pragma unroll
-                    for (int e = 0; e < G::RT; e++) a[e] = V{ipow(a[e].x, p), ipow(a[e].y, p)};
+                    for (int e = 0; e < G::RT; e++) {
+                        if (last) {
+                            const V h{ipow(a[e].x, p / 2), ipow(a[e].y, p / 2)};
+                            prod[e] = f == 0 ? h : V{prod[e].x * h.x, prod[e].y * h.y};
+                        }
+                        a[e] = V{ipow(a[e].x, q), ipow(a[e].y, q)};
+                    }
                 }
+                const bool alone = f == 0 && p <= 3;
                 double s = 0.0;
 #pragma unroll
                 for (int e = 0; e < G::RT; e++) {
@@ -1023,8 +1033,8 @@ __global__ void __launch_bounds__(RowGeom<T, N>::THREADS)
                     if (!last) {
                         prod[e] = f == 0 ? V{x0, x1} : V{prod[e].x * x0, prod[e].y * x1};
                     } else if (G::tl(rc.t, e)) {
-                        const double y0 = f == 0 ? (double)x0 : (double)prod[e].x * (double)x0;
-                        const double y1 = f == 0 ? (double)x1 : (double)prod[e].y * (double)x1;
+                        const double y0 = alone ? (double)x0 : (double)prod[e].x * (double)x0;
+                        const double y1 = alone ? (double)x1 : (double)prod[e].y * (double)x1;
                         s += abs_terms ? fabs(y0) + fabs(y1) : y0 + y1;
                     }
                 }
