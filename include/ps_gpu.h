@@ -151,14 +151,13 @@ int ps_gpu_polyspectrum_batch(ps_gpu_ctx *ctx, int method, int nconf, ps_cfg *cf
  * PS_PLAN_GRAPH the first execution captures it into a CUDA graph that later
  * executions replay.  A plan belongs to the context it was created on and
  * uses the field most recently loaded into it.  PS_PLAN_KAPPA adds the
- * condition-number passes.  PS_FP64_PLAIN plans evaluate their configurations
- * one by one (no graph). */
+ * condition-number passes.  PS_FP64_PLAIN plans run eagerly (no graph). */
 #define PS_PLAN_GRAPH 1
 #define PS_PLAN_KAPPA 2
 /* PS_PLAN_AUTOTUNE: each pair group (configurations sharing two legs) runs its
  * transforms on an alias-free sub-grid; by default the smallest one, with this
  * flag the fastest of the smallest and up to two larger supported sizes, timed
- * at plan creation; the flag also times, per FP32 transform size the groups
+ * at plan creation (not for groups whose smallest size is below 96); the flag also times, per FP32 transform size the groups
  * use, the Y pass with its default thread layout against one with twice the
  * elements per thread (one radix pass fewer) and keeps the faster, and the
  * pair kernel (the per-row product of two inverse transforms, transformed
@@ -174,7 +173,9 @@ int ps_gpu_polyspectrum_batch(ps_gpu_ctx *ctx, int method, int nconf, ps_cfg *cf
  * GIVEN and DERIVED binning) are counted exactly in integers by default:
  * every leg pair (m_a, m_b), S_a reduced to orbit representatives under the
  * 48 axis permutations and sign flips, histogrammed by |m_a + m_b|^2 (wrapped
- * on the grid as the reference's cyclic sums wrap).  PS_PLAN_FFT_COUNTS
+ * on the grid as the reference's cyclic sums wrap), or compared with the
+ * interval of the one closing shell; groups of more than 4e9 pairs (1.5e9
+ * when they wrap) are counted with transforms.  PS_PLAN_FFT_COUNTS
  * counts with FP64 transforms of the unit shells instead (the reference's
  * dataflow; WATKINSON shells always do).  Both give the same integers. */
 #define PS_PLAN_FFT_COUNTS 8
@@ -265,11 +266,12 @@ int ps_gpu_plan_results_device(ps_gpu_ctx *ctx, ps_gpu_plan *plan, double *dst);
 
 /* The context's autotuned choices as text, one "grid N b_a b_b b_c M" line per
  * pair-group signature, one "pencil M alt" line (alt 0 or 1) per transform
- * size whose Y pass layout was timed and one "pair M v" line per FP32
+ * size whose Y pass layout was timed (alt 1: twice the elements per thread, or
+ * the register plan where the default is the two-pass split transform) and one "pair M v" line per FP32
  * transform size whose pair kernel variant was timed (v 0: the default, 1: one
  * row transform live in registers, 2: twice the elements per thread, one
- * radix pass fewer) and one "dot M alt" line per FP32 transform size whose
- * dot pass geometry was timed (alt 1: twice the elements per thread): writes
+ * radix pass fewer; a length without variant v runs the default) and one "dot M alt" line per FP32 transform size whose
+ * dot pass geometry was timed (alt as for the Y pass): writes
  * at most buflen bytes (NUL-terminated) and
  * returns the length of the whole text, or a negative status.  Import adds
  * the lines of such a text to the context's choices (unknown or malformed
