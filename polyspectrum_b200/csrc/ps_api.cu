@@ -795,6 +795,23 @@ int sum_partials(ps_gpu_ctx* c, int nblocks, int ncols, double* out, int out_str
     return PS_OK;
 }
 
+// The disc of pencils passes may confine themselves to for these shells on the M-grid
+// (XItem::r2): their largest |m|^2, 0 for none.  Interval shells only; DERIVED ones
+// carry the host bound of their interval, which the device checks.  From 192 points
+// on: inverse X pass at 600 points FP32 1.15 -> 0.95, FP64 quadrants 0.86 -> 0.72 ms over
+// the 600^3 triangles (17.07 -> 16.81 ms in all), at 384 points 0.051 -> 0.046 ms; the Y
+// passes, bound by their exchanges, gain little.  At 128 points sixteen columns are too
+// coarse a step for a shell of 20 to 60 modes (64 triangles FP64 0.856 -> 0.860 ms).
+int cut_r2(const Shell* sh, int n, int M)
+{
+    int r2 = 0;
+    for (int q = 0; q < n; q++) {
+        if (sh[q].kind > SHELL_RANGE || M < kCutFrom) return 0;
+        r2 = std::max(r2, sh[q].r2hi);
+    }
+    return r2;
+}
+
 // Inverse X and Y passes of up to kItems shell-filtered spectra, each into its dst,
 // band-limited to its shell: h < hb = min(band, N/2) + 1 columns, row stride S (both
 // set here), one launch per pass.  mode: LOAD_MASKED (F * field spectrum) or LOAD_UNIT
@@ -805,6 +822,7 @@ template <typename T> struct XyLeg {
     int band;
     V2<T>* dst;
     int S, hb;
+    int r2 = 0;  // cut_r2 of the shell
 };
 template <typename T> void size_leg(XyLeg<T>& l, int M, int quad)
 {
@@ -825,8 +843,8 @@ template <typename T> int c2r_xy_n(ps_gpu_ctx* c, int mode, XyLeg<T>* legs, int 
     for (int x = 0; x < n; x++) {
         XyLeg<T>& l = legs[x];
         size_leg(l, N, quad);
-        xi.push_back(XItem<T>{l.dst, l.S, N / 2 + 1, l.dshell, 0});
-        yi.push_back(YItem<T>{l.dst, l.S, l.S, std::min(l.band, N / 2), N});
+        xi.push_back(XItem<T>{l.dst, l.S, N / 2 + 1, l.dshell, 0, l.r2});
+        yi.push_back(YItem<T>{l.dst, l.S, l.S, std::min(l.band, N / 2), N, l.r2});
         Smax = std::max(Smax, l.S);
         bx += q * NN2 * l.S * V + (mode == LOAD_MASKED ? NN2 * l.hb * V : 0.0);
         by += 2.0 * q * NN2 * l.S * V;
@@ -884,10 +902,11 @@ int c2r_shell(ps_gpu_ctx* c, int mode, const Shell* dshell, int band, T* out, co
 
 // Spectrum of the real product of two band-limited inverse transforms (B may be
 // NULL: square of A), rows kept to h < hout, forward Y pass done; into B.work3.
-// M > 0: the inputs are M-grid transforms (c2r_xy with the same M).
+// M > 0: the inputs are M-grid transforms (c2r_xy with the same M).  r2: cut_r2 of
+// the shells the spectrum is read with.
 template <typename T>
 int pair_spectrum(ps_gpu_ctx* c, const V2<T>* A, int Sa, int hba, const V2<T>* Bq, int Sb, int hbb, int hout,
-                  int* S_out, int quad = 0, int M = 0)
+                  int* S_out, int quad = 0, int M = 0, int r2 = 0)
 {
     PrecBufs<T>& B = bufs<T>(c);
     const int N = M > 0 ? M : c->N;
@@ -906,7 +925,7 @@ int pair_spectrum(ps_gpu_ctx* c, const V2<T>* A, int Sa, int hba, const V2<T>* B
         Prof pf(c);
         // rows |my| >= hout lie outside every shell the product is dotted with
         PS_SWITCH_N(N, PS_TRY((L3<T, NN>::pass_y(c->stream, B.work3, S, false, tb, quad, NN, 0, hout - 1,
-                                                 pencil_alt_of<T>(c, N)))));
+                                                 pencil_alt_of<T>(c, N), r2))));
         pf.end(fam<T>(KF_PASS_Y), 2.0 * q * NN2 * S * V, N);
     }
     *S_out = S;
@@ -1899,8 +1918,9 @@ int prod_ops(ps_gpu_ctx* c, const std::vector<Shell>& host, const Shell* dtable,
             const Shell& sh = host[b.shells[q]];
             const int band = std::min(sh.band, M / 2), hb = band + 1, S = round_up(unit ? (hb + 1) / 2 : hb, pw<T>(M));
             V2<T>* dst = (V2<T>*)(base + b.at[q]);
-            xi.push_back(XItem<T>{dst, S, M / 2 + 1, dtable + b.shells[q], 0});
-            yi.push_back(YItem<T>{dst, S, S, band, M});
+            const int r2 = cut_r2(&sh, 1, M);
+            xi.push_back(XItem<T>{dst, S, M / 2 + 1, dtable + b.shells[q], 0, r2});
+            yi.push_back(YItem<T>{dst, S, S, band, M, r2});
             where[b.shells[q]] = {dst, {S, hb}};
             Smax = std::max(Smax, S);
             bx += rows * S * V + (unit ? 0.0 : rows * hb * V);
@@ -2428,8 +2448,9 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
                 *h = band + 1;
                 *S = round_up(*h, w);
                 V2<float>* dst = (V2<float>*)carve(rows * (size_t)*S * sizeof(V2<float>));
-                xi.push_back(XItem<float>{dst, *S, M / 2 + 1, dtable + shell, 0});
-                yi.push_back(YItem<float>{dst, *S, *S, band, M});
+                const int r2 = cut_r2(&sh, 1, M);
+                xi.push_back(XItem<float>{dst, *S, M / 2 + 1, dtable + shell, 0, r2});
+                yi.push_back(YItem<float>{dst, *S, *S, band, M, r2});
                 Smax = std::max(Smax, *S);
                 bx += NN2 * (*S + *h) * V;
                 by += 2.0 * NN2 * *S * V;
@@ -2441,7 +2462,7 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
             const int hout = I.hmax + 1, Sp = round_up(hout, w);
             V2<float>* D = (V2<float>*)carve(rows * (size_t)Sp * sizeof(V2<float>));
             (B ? pi_ : sq).push_back(PairItem<float>{A, B, D, Sa, ha, Sb, hb, Sp, hout});
-            yf.push_back(YItem<float>{D, Sp, Sp, M, hout - 1});
+            yf.push_back(YItem<float>{D, Sp, Sp, M, hout - 1, cut_r2(I.gtable.data(), (int)I.gtable.size(), M)});
             ha_max = std::max(ha_max, ha);
             hb_max = std::max(hb_max, hb);
             Pmax = std::max(Pmax, Sp);
@@ -2569,12 +2590,13 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
         const int hmax = info[g].hmax;
         const int hout = info[g].hmax + 1, go = gofs[g], io = gidx_ofs[g];
         return [=]() {
-            XyLeg<double> l[2] = {{dtable + G.a, sa.band, c->d.work, 0, 0}, {dtable + G.b, sb.band, c->d.work2, 0, 0}};
+            XyLeg<double> l[2] = {{dtable + G.a, sa.band, c->d.work, 0, 0, cut_r2(&sa, 1, M)},
+                                  {dtable + G.b, sb.band, c->d.work2, 0, 0, cut_r2(&sb, 1, M)}};
             const bool two = G.a != G.b;
             int S = 0;
             PS_TRY(c2r_xy_n<double>(c, LOAD_UNIT, l, two ? 2 : 1, 1, M));
             PS_TRY(pair_spectrum<double>(c, l[0].dst, l[0].S, l[0].hb, two ? l[1].dst : nullptr, l[1].S, l[1].hb, hout, &S,
-                                         1, M));
+                                         1, M, cut_r2(gtable.data(), (int)gtable.size(), M)));
             PS_TRY(dot_pass<double>(c, c->d.work3, SPEC_COUNT, S, hout, dtable + go, gtable.data(), (int)gtable.size(), sumI,
                                     1, M, 1.0, didx + io, &vol, hmax));
             return PS_OK;
@@ -3383,7 +3405,7 @@ int grad_impl(ps_gpu_ctx* c, int n, const std::vector<Shell>& legs, double scale
                 if (same_shell(legs[p], legs[l])) at[l] = at[p];
             if (at[l] < 0) {
                 at[l] = (int)lx.size();
-                lx.push_back(XyLeg<T>{c->dshells + l, legs[l].band, nullptr, 0, 0});
+                lx.push_back(XyLeg<T>{c->dshells + l, legs[l].band, nullptr, 0, 0, cut_r2(&legs[l], 1, M)});
             }
         }
         // all legs and products side by side when they fit the work spectrum (any M up to

@@ -265,11 +265,13 @@ template <typename T> struct XItem {  // inverse X
     int hvalid;
     const Shell* shell;  // NULL for plain loads
     int band;            // plain loads: components above it are zero and not read
+    int r2;              // > 0: no mode with |m|^2 > r2 (skip_dead leaves those tiles unwritten)
 };
 template <typename T> struct YItem {  // Y pass
     V2<T>* data;
     int stride, ncols;  // columns h < ncols, a multiple of the pencil width
     int jband, jout;
+    int r2;             // > 0: as XItem's, of the input rows (inverse) or of the rows to store (forward)
 };
 template <typename T> struct PairItem {  // pair kernel
     const V2<T>* A;
@@ -293,6 +295,13 @@ template <typename T> struct FwdXItem {  // forward X
     double* partials;           // [nshell][blocks]
 };
 
+// The pencils (my, h) that can hold a mode of a spectrum with |m|^2 <= r2 are those
+// with my^2 + h^2 <= r2: a disc, which a shell's X and Y passes leave out a fifth of
+// the band's square for.  Decided per 16 columns (per tile at most), so that passes of
+// different tile widths agree: the first real column of the 16 that element h is in.
+__device__ __forceinline__ int cut_column(int h, int quad) { return (h & ~15) * (quad ? 2 : 1); }
+constexpr int kCutFrom = 192;  // points: below, the kernels have no such test (the items' r2 is 0)
+
 // ------------------------------------------------------------------ inverse X
 enum InvLoad : int { LOAD_PLAIN = 0, LOAD_MASKED = 1, LOAD_UNIT = 2 };  // LOAD_UNIT: quad only
 
@@ -311,11 +320,18 @@ __global__ void __launch_bounds__(PencilGeom<T, N>::THREADS)
     const Shell* __restrict__ shell_p = it.shell;
     const int tiles_per_row = dst_stride / G::W;
     if ((int)blockIdx.x >= (quad ? N / 2 + 1 : N) * tiles_per_row) return;
-    // skip_dead: a filtered tile whose |my| exceeds the shell's band holds only
-    // zeros and is not written (the inverse Y pass then treats those rows as
-    // zero, its jband)
-    if (skip_dead && abs(lattice_freq((int)(blockIdx.x / tiles_per_row), N)) > (mode == LOAD_PLAIN ? it.band : shell_p->band))
-        return;
+    // skip_dead: a filtered tile whose |my| exceeds the shell's band, or that lies
+    // outside the disc of its r2, holds only zeros and is not written (the inverse Y
+    // pass then treats those rows as zero, its jband and r2)
+    static_assert(N == 16 || 16 % G::W == 0, "cut_column");
+    if (skip_dead) {
+        const int my = lattice_freq((int)(blockIdx.x / tiles_per_row), N);
+        if (abs(my) > (mode == LOAD_PLAIN ? it.band : shell_p->band)) return;
+        if constexpr (N >= kCutFrom) {
+            const int hc = cut_column((int)(blockIdx.x % tiles_per_row) * G::W, quad);
+            if (it.r2 > 0 && my * my + hc * hc > it.r2) return;
+        }
+    }
     const V* tw = stage_table<V>(smem_raw, tw_g, N);
     __syncthreads();
     SmemInterleaved<V, G::W> sm{reinterpret_cast<V*>(smem_raw + G::TW_BYTES), (int)(threadIdx.x % G::W)};
@@ -404,10 +420,21 @@ __global__ void __launch_bounds__(YGeom<T, N, RX>::type::THREADS)
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const YItem<T>& it = items.at[blockIdx.y];
     V* __restrict__ data = it.data;
-    const int stride = it.stride, ncols = it.ncols, jband = it.jband, jout = it.jout;
+    const int stride = it.stride, ncols = it.ncols;
+    const int jband = it.jband, jout = it.jout;
     if ((int)blockIdx.x >= (quad ? N / 2 + 1 : N) * (ncols / G::W)) return;
     const int w = threadIdx.x % G::W, t = threadIdx.x / G::W;
     const int tiles_per_plane = ncols / G::W;  // columns h < ncols of rows of stride `stride`
+    static_assert(N == 16 || 16 % G::W == 0, "cut_column");
+    int cut = 0x7fffffff;  // rows my^2 > cut: zero, or not to be stored
+    if constexpr (N >= kCutFrom) {
+        const int hc = cut_column((int)(blockIdx.x % tiles_per_plane) * G::W, quad);
+        if (it.r2 > 0) cut = it.r2 - hc * hc;
+        if (!INV && cut < 0) return;
+    }
+    const auto inside = [&](int my, int band) {
+        return (band >= N / 2 || abs(my) <= band) && (N < kCutFrom || my * my <= cut);
+    };
     // quad: planes i <= N/2, rows j <= N/2 stored, row N-j read as row j
     // (data even in y)
     const int nj = quad ? N / 2 + 1 : N;
@@ -421,8 +448,8 @@ __global__ void __launch_bounds__(YGeom<T, N, RX>::type::THREADS)
     for (int e = 0; e < G::RI; e++) {
         const int j = G::ip(t, e);
         const int jr = quad && j > N / 2 ? N - j : j;
-        a[e] = G::il(t, e) && (jband >= N / 2 || abs(lattice_freq(j, N)) <= jband) ? base[(size_t)jr * stride]
-                                                                                  : czero<V>();
+        const bool in = INV ? inside(lattice_freq(j, N), jband) : jband >= N / 2 || abs(lattice_freq(j, N)) <= jband;
+        a[e] = G::il(t, e) && in ? base[(size_t)jr * stride] : czero<V>();
     }
     const V* tw = stage_table<V>(smem_raw, tw_g, N);
     __syncthreads();
@@ -432,7 +459,8 @@ __global__ void __launch_bounds__(YGeom<T, N, RX>::type::THREADS)
     for (int e = 0; e < G::RO; e++) {
         const int j = G::op(t, e);
         // jout < N/2: rows with |my| > jout are read by no later pass and not stored
-        if (G::ol(t, e) && (!quad || j <= N / 2) && (jout >= N / 2 || abs(lattice_freq(j, N)) <= jout))
+        const bool in = INV ? jout >= N / 2 || abs(lattice_freq(j, N)) <= jout : inside(lattice_freq(j, N), jout);
+        if (G::ol(t, e) && (!quad || j <= N / 2) && in)
             base[(size_t)j * stride] = a[e];
     }
 }
@@ -1012,6 +1040,9 @@ __global__ void __launch_bounds__(RowGeom<T, N>::THREADS)
                 } else if (p == 3) {
 #pragma unroll
                     for (int e = 0; e < G::RT; e++) a[e] = V{a[e].x * a[e].x * a[e].x, a[e].y * a[e].y * a[e].y};
+                } else if (p > 3 && sizeof(T) == 8) {
+#pragma unroll
+                    for (int e = 0; e < G::RT; e++) a[e] = V{ipow(a[e].x, p), ipow(a[e].y, p)};
                 } else if (p > 3) {
                     // the last factor's power in two halves, whose product the sum takes in
                     // double: the eighth power of 6e4 is above FP32's range
@@ -1025,7 +1056,7 @@ __global__ void __launch_bounds__(RowGeom<T, N>::THREADS)
                         a[e] = V{ipow(a[e].x, q), ipow(a[e].y, q)};
                     }
                 }
-                const bool alone = f == 0 && p <= 3;
+                const bool alone = f == 0 && (sizeof(T) == 8 || p <= 3);
                 double s = 0.0;
 #pragma unroll
                 for (int e = 0; e < G::RT; e++) {

@@ -94,7 +94,7 @@ template <typename T, int N> struct L3 {
     static int inv_x(cudaStream_t st, const V* src, int ss, V* dst, int ds, int mode, const Shell* sh,
                      int hvalid, const Tables<T>& tb, int quad = 0, int nsrc = 0, int skip_dead = 0, int band = N)
     {
-        const XItem<T> it{dst, ds, hvalid, sh, band};
+        const XItem<T> it{dst, ds, hvalid, sh, band, 0};
         return inv_x_b(st, src, ss, &it, 1, ds, mode, tb, quad, nsrc, skip_dead);
     }
     // The batched forms take nitems <= kItems descriptions (copied into the launch);
@@ -106,10 +106,10 @@ template <typename T, int N> struct L3 {
     // jout < N/2: output rows with |my| > jout are not stored
     // alt: the alternative geometry (PencilAlt) when this length has one
     static int pass_y(cudaStream_t st, V* data, int stride, bool inv, const Tables<T>& tb, int quad = 0,
-                      int jband = N, int ncols = 0, int jout = N, int alt = 0)
+                      int jband = N, int ncols = 0, int jout = N, int alt = 0, int r2 = 0)
     {
         const int nc = ncols > 0 ? ncols : stride;
-        const YItem<T> it{data, stride, nc, jband, jout};
+        const YItem<T> it{data, stride, nc, jband, jout, r2};
         return pass_y_b(st, &it, 1, nc, inv, tb, quad, alt);
     }
     static int pass_y_b(cudaStream_t st, const YItem<T>* items, int nitems, int ncols, bool inv,
