@@ -158,8 +158,8 @@ template <typename T, int N> struct L3 {
 
 // Grid sizes.  Powers of two 16..1024, the 3 2^k / 5 2^k sizes of the
 // alias-free sub-grids of pair groups (192, 320, 384), and further grid sizes
-// 2^a 3^b 5^c a context may run on (48, 96: register plans; 60, 300, 600:
-// shared-memory passes) - instantiated in four translation units per precision.
+// 2^a 3^b 5^c a context may run on (48, 60, 96, 300, 600), instantiated in three
+// translation units per precision.
 #define PS_INSTANTIATE_L3_A(T)        \
     template struct L3<T, 16>;        \
     template struct L3<T, 32>;        \
