@@ -943,38 +943,40 @@ __global__ void __launch_bounds__(RowGeom<T, N, RX>::THREADS, sizeof(T) == 8 ? 0
         cp_async_wait_prev();
         __syncthreads();
         const size_t row = (size_t)tile * G::WZ + rc.w;
-        if (row >= (size_t)nrows) {  // whole row group idle in the last tile
-            __syncthreads();
-            continue;
-        }
-        if (alias) rc.rowbuf = stA + st * G::WZ * PA + rc.w * PA;
-        V a[G::R];
-        c2r(stA + st * G::WZ * PA + rc.w * PA, it.hva, a);
-        if constexpr (two) {
-            if constexpr (KEEP) {
+        // A row group past the quadrant's last row idles; every thread reaches the one
+        // barrier below (rows of a warp on different barriers is what the hardware's
+        // CTA barrier does not allow).  The N^2 rows of a full grid are whole tiles.
+        static_assert(REAL || N * N % G::WZ == 0, "whole tiles");
+        if (!REAL || row < (size_t)nrows) {
+            if (alias) rc.rowbuf = stA + st * G::WZ * PA + rc.w * PA;
+            V a[G::R];
+            c2r(stA + st * G::WZ * PA + rc.w * PA, it.hva, a);
+            if constexpr (two) {
+                if constexpr (KEEP) {
 #pragma unroll
-                for (int e = 0; e < G::RT; e++)
-                    if (G::tl(rc.t, e)) keep[G::tp(rc.t, e)] = a[e];
-                c2r(stB + st * G::WZ * PB + rc.w * PB, it.hvb, a);
+                    for (int e = 0; e < G::RT; e++)
+                        if (G::tl(rc.t, e)) keep[G::tp(rc.t, e)] = a[e];
+                    c2r(stB + st * G::WZ * PB + rc.w * PB, it.hvb, a);
 #pragma unroll
-                for (int e = 0; e < G::RT; e++) {
-                    const V q = G::tl(rc.t, e) ? keep[G::tp(rc.t, e)] : czero<V>();
-                    a[e] = V{a[e].x * q.x, a[e].y * q.y};
+                    for (int e = 0; e < G::RT; e++) {
+                        const V q = G::tl(rc.t, e) ? keep[G::tp(rc.t, e)] : czero<V>();
+                        a[e] = V{a[e].x * q.x, a[e].y * q.y};
+                    }
+                } else {
+                    V b[G::R];
+                    c2r(stB + st * G::WZ * PB + rc.w * PB, it.hvb, b);
+#pragma unroll
+                    for (int e = 0; e < G::RT; e++) a[e] = V{a[e].x * b[e].x, a[e].y * b[e].y};
                 }
             } else {
-                V b[G::R];
-                c2r(stB + st * G::WZ * PB + rc.w * PB, it.hvb, b);
 #pragma unroll
-                for (int e = 0; e < G::RT; e++) a[e] = V{a[e].x * b[e].x, a[e].y * b[e].y};
+                for (int e = 0; e < G::RT; e++) a[e] = V{a[e].x * a[e].x, a[e].y * a[e].y};
             }
-        } else {
-#pragma unroll
-            for (int e = 0; e < G::RT; e++) a[e] = V{a[e].x * a[e].x, a[e].y * a[e].y};
+            // the products sit in canonical layout as (x[2n], x[2n+1]): r2c input as is
+            if constexpr (REAL) r2c_row<T, N, RX, true>(a, rc, reinterpret_cast<T*>(dst + row * ds), hout);
+            else r2c_row<T, N, RX>(a, rc, dst + row * ds, hout);
         }
-        // the products sit in canonical layout as (x[2n], x[2n+1]): r2c input as is
-        if constexpr (REAL) r2c_row<T, N, RX, true>(a, rc, reinterpret_cast<T*>(dst + row * ds), hout);
-        else r2c_row<T, N, RX>(a, rc, dst + row * ds, hout);
-        __syncthreads();
+        __syncthreads();  // this stage is refilled two tiles later
     }
 }
 

@@ -142,7 +142,7 @@ int L3<T, N>::pair_z_v(cudaStream_t st, const PairItem<T>* items, int nitems, in
     const bool alias = PGm::smem(ninputs, ea, eb, true) < PGm::smem(ninputs, ea, eb, false);
     const size_t smem = PGm::smem(ninputs, ea, eb, alias);
     PS_LTRY(set_smem(k_pair_z<T, N, RX, KEEP, REAL, TWO>, PGm::smem(2, N / 2 + 1, N / 2 + 1)));
-    const int nrows = quad ? (N / 2 + 1) * (N / 2 + 1) : N * N;
+    const int nrows = REAL ? (N / 2 + 1) * (N / 2 + 1) : N * N;
     const int tiles = (nrows + G::WZ - 1) / G::WZ;
     int grid = 0;  // resident CTAs, shared out among the items
     PS_LTRY(persistent_grid(k_pair_z<T, N, RX, KEEP, REAL, TWO>, G::THREADS, smem, tiles * nitems, &grid));
