@@ -53,9 +53,18 @@ __global__ void k_fill_real(float* p, size_t n, unsigned seed)
         p[i] = (h & 0xffff) / 65536.0f;
     }
 }
+// Device copy of a host table.
+float2* to_device(const std::vector<float2>& h)
+{
+    float2* d;
+    CK(cudaMalloc(&d, h.size() * sizeof(float2)));
+    CK(cudaMemcpy(d, h.data(), h.size() * sizeof(float2), cudaMemcpyHostToDevice));
+    return d;
+}
+// Every table an M-point launch may read, the alternative ones where M has them.
 template <int M> Tables<float> make_tables()
 {
-    std::vector<float2> hp(M), hr(M / 2), h(M);
+    std::vector<float2> hp(M), hr(M / 2), h(M), ha(M), hr2(M / 2);
     L3<float, M>::host_tables(hp.data(), hr.data());
     const long double two_pi = 6.283185307179586476925286766559005768L;
     for (int m = 0; m < M; m++) {
@@ -63,12 +72,10 @@ template <int M> Tables<float> make_tables()
         h[m].x = (float)cosl(a);
         h[m].y = (float)(-sinl(a));
     }
-    float2 *a, *b, *c;
-    CK(cudaMalloc(&a, M * 8)); CK(cudaMalloc(&b, M / 2 * 8)); CK(cudaMalloc(&c, M * 8));
-    CK(cudaMemcpy(a, hp.data(), M * 8, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(b, hr.data(), M / 2 * 8, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(c, h.data(), M * 8, cudaMemcpyHostToDevice));
-    return Tables<float>{a, b, c};
+    Tables<float> t{to_device(hp), to_device(hr), to_device(h)};
+    if (L3<float, M>::host_alt_table(ha.data())) t.twp_alt = to_device(ha);
+    if (L3<float, M>::host_pair_alt_table(hr2.data())) t.twr_alt = to_device(hr2);
+    return t;
 }
 static int rup(int a, int b) { return (a + b - 1) / b * b; }
 

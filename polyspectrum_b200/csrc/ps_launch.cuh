@@ -32,6 +32,10 @@ double host_norm_coef(double L, int N, int n);
         if (e_ != cudaSuccess) return launch_fail(e_, #x); \
     } while (0)
 
+// A kernel reads its transform's table without a test: a launch without one is refused here.
+#define PS_NEED_TABLE(p) \
+    if (!(p)) return launch_fail(cudaErrorInvalidValue, "twiddle table " #p " of this transform is missing")
+
 template <typename K> int set_smem(K kernel, size_t bytes)
 {
     if (bytes > 48 * 1024)
@@ -60,12 +64,13 @@ template <class I> inline Items<I> pack(const I* items, int n)
 
 // Twiddle tables of one precision: twp = Stockham table of the pencil
 // transforms (length N), twr = of the row transforms (length N/2), twpp =
-// W_N^k for the r2c / c2r pre- and post-processing (k < N).
+// W_N^k for the r2c / c2r pre- and post-processing (k < N).  twp_alt is not optional
+// where the Y pass's default geometry is not the pencils' (host_alt_table says so).
 template <typename T> struct Tables {
     const V2<T>* twp;
     const V2<T>* twr;
     const V2<T>* twpp;
-    const V2<T>* twp_alt = nullptr;  // Stockham table of the alternative Y pass (PencilAlt), if any
+    const V2<T>* twp_alt = nullptr;  // Stockham table of the alternative pencil geometry or the Y pass's own, if any
     const V2<T>* twr_alt = nullptr;  // row table of pair kernel variant 2 (PairVariants::ALT_RX), if any
 };
 

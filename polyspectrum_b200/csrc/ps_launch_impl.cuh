@@ -57,6 +57,7 @@ template <typename T, int N>
 int L3<T, N>::inv_x_b(cudaStream_t st, const V* src, int ss, const XItem<T>* items, int nitems,
                       int ds, int mode, const Tables<T>& tb, int quad, int nsrc, int skip_dead)
 {
+    PS_NEED_TABLE(tb.twp);
     PS_LTRY(set_smem(k_inv_x<T, N>, PG::SMEM));
     const int nj = quad ? N / 2 + 1 : N;
     k_inv_x<T, N><<<dim3((unsigned)(nj * (ds / PG::W)), (unsigned)nitems), PG::THREADS, PG::SMEM, st>>>(
@@ -71,6 +72,7 @@ int L3<T, N>::pass_y_b(cudaStream_t st, const YItem<T>* items, int nitems, int n
     using YG = typename YGeom<T, N, 0>::type;  // (the alternative geometries have the default's tile width)
     const dim3 grid((unsigned)((quad ? N / 2 + 1 : N) * (ncols / YG::W)), (unsigned)nitems);
     auto go = [&](auto kernel, int threads, size_t smem, const V* tw) -> int {
+        PS_NEED_TABLE(tw);
         PS_LTRY(set_smem(kernel, smem));
         kernel<<<grid, threads, smem, st>>>(pack(items, nitems), quad, tw);
         return PS_OK;
@@ -89,6 +91,8 @@ template <typename T, int N>
 int L3<T, N>::inv_z(cudaStream_t st, const V* src, int ss, int hvalid, T* out, const T* aux, int epi,
                  int power, double* partials, const Tables<T>& tb, int* nblocks, double scale)
 {
+    PS_NEED_TABLE(tb.twr);
+    PS_NEED_TABLE(tb.twpp);
     const size_t smem = RG::smem(1, hvalid, 0);
     PS_LTRY(set_smem(k_inv_z<T, N>, RG::smem(1, N / 2 + 1, 0)));
     int grid = 0;
@@ -103,6 +107,8 @@ template <typename T, int N>
 int L3<T, N>::fwd_z(cudaStream_t st, int kind, const void* a, const void* b, V* dst, int ds, int hout,
                  const Tables<T>& tb, int stage, size_t nrows, int* status, int tx_extra)
 {
+    PS_NEED_TABLE(tb.twr);
+    PS_NEED_TABLE(tb.twpp);
     const bool two = kind == SRC_XHI_F32 || kind == SRC_XHI_F64;
     const size_t eb = (kind == SRC_F32 || kind == SRC_XHI_F32) ? 4 : 8;
     const uintptr_t addr = (uintptr_t)a | (two ? (uintptr_t)b : 0);
@@ -136,6 +142,8 @@ template <int RX, bool KEEP, bool REAL, bool TWO>
 int L3<T, N>::pair_z_v(cudaStream_t st, const PairItem<T>* items, int nitems, int ninputs,
                        int hva, int hvb, const V* twr, const V* twpp, int quad)
 {
+    PS_NEED_TABLE(twr);
+    PS_NEED_TABLE(twpp);
     using G = RowGeom<T, N, RX>;
     using PGm = PairGeom<T, N, RX, KEEP>;
     const int ea = REAL ? (hva + 1) / 2 : hva, eb = REAL ? (hvb + 1) / 2 : hvb;
@@ -178,6 +186,8 @@ template <typename T, int N>
 int L3<T, N>::prod_z(cudaStream_t st, const ProdItem<T>* items, int nitems, int hv, bool real, int abs_terms,
                      const Tables<T>& tb, int* nblocks)
 {
+    PS_NEED_TABLE(tb.twr);
+    PS_NEED_TABLE(tb.twpp);
     const int P0 = RG::pitch(real ? (hv + 1) / 2 : hv);
     const bool alias = 2 * std::max(P0, RG::ROWBUF) < 2 * P0 + RG::ROWBUF;  // rows' exchange buffers in their stages
     const int P = alias ? std::max(P0, RG::ROWBUF) : P0;
@@ -209,6 +219,7 @@ int L3<T, N>::fwd_x(cudaStream_t st, const FwdXItem<T>* items, int nitems, int n
     const bool dot = epi == SPEC_DOT || epi == SPEC_COUNT || epi == SPEC_DOT_ABS;
     if (nblocks) *nblocks = (int)grid.x;
     auto go = [&](auto batch, auto kernel, int threads, size_t smem, const V* tw) -> int {
+        PS_NEED_TABLE(tw);
         PS_LTRY(set_smem(kernel, smem));
         if constexpr (std::is_same_v<decltype(batch), std::true_type>)
             kernel<<<grid, threads, smem, st>>>(pack(items, nitems), epi, out, ostride, dk, dks, ndk > 0 ? ndk : N, quad,
