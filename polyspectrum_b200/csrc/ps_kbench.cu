@@ -85,12 +85,10 @@ static int rup(int a, int b) { return (a + b - 1) / b * b; }
 template <int M, bool INV, int RX>
 double time_pass_y(int reps, float2* data, int S, int ncols, int jband, int jout, const char* what)
 {
-    using G = PencilGeom<float, M, RX>;
+    using G = typename YGeom<float, M, RX>::type;  // the kernel's own
     std::vector<float2> hp(M);
     transform_table<float2, M, G>(hp.data());
-    float2* tw;
-    CK(cudaMalloc(&tw, M * 8));
-    CK(cudaMemcpy(tw, hp.data(), M * 8, cudaMemcpyHostToDevice));
+    float2* tw = to_device(hp);
     auto kern = k_pass_y<float, M, INV, RX>;
     CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM));
     int per_sm = 0;
@@ -120,10 +118,7 @@ template <int M, int RX> float2* pair_row_table()
     using G = RowGeom<float, M, RX>;
     std::vector<float2> hr(M / 2);
     transform_table<float2, M / 2, G>(hr.data());
-    float2* d;
-    CK(cudaMalloc(&d, M / 2 * 8));
-    CK(cudaMemcpy(d, hr.data(), M / 2 * 8, cudaMemcpyHostToDevice));
-    return d;
+    return to_device(hr);
 }
 
 // Mean time of `reps` launches of the pair kernel variant <M, RX, KEEP> on
