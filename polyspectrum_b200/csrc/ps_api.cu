@@ -327,6 +327,7 @@ struct ps_gpu_ctx {
     unsigned short* side_lut = nullptr;
     size_t side_lut_cap = 0;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    bool side_fp64 = false;  // FP64 counts have been prepared on it (join_side)
     // field lanes: the batches of pair groups of a plan split over two streams
     // (0 the main one, 1 lane2_stream), each with its own workspace (leg and
     // product spectra, block sums), so the kernels of different batches overlap;
@@ -644,10 +645,23 @@ struct Lane2 {
     }
 };
 
+// Counts by FP64 transforms (PART_COUNTS) write d.work, d.work2 and d.work3.  Prepared
+// ones (ps_gpu_plan_prepare) run on the side stream until their plan's next execution,
+// beside whatever the context does meanwhile: work on the main stream that uses one of
+// these spectra (products, FP64 gradients, counts there) waits for them here first.
+// Never inside a capture: a graph's launch is what has to wait.
+int join_side(ps_gpu_ctx* c)
+{
+    if (!c->side_fp64) return PS_OK;
+    PS_CK(cudaEventRecord(c->ev_join, c->side_stream));
+    PS_CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
+    return PS_OK;
+}
+
 // Workspace of a field lane, at least `bytes`.  A buffer of the context that nothing
 // else uses while the lane works serves as long as it is large enough: lane 0 the FP32
 // work spectrum, lane 1 an FP32 real grid, the products (2) the FP64 work spectrum
-// (FP64 counts use it on the side lane, which is joined first).  A replaced own one is
+// (after join_side).  A replaced own one is
 // retired: a captured graph or a plan's launches may still point at it.
 int ensure_lane_work(ps_gpu_ctx* c, int lane, size_t bytes)
 {
@@ -1460,6 +1474,7 @@ struct ps_gpu_plan {
     std::vector<std::function<int()>> ops_groups;  // the pair groups' field parts (main or second lane)
     std::vector<std::function<int()>> ops_tail;    // n = 2 and leg-by-leg configurations, finalisation
     bool has_groups = false, two_lanes = false;
+    bool fft_counts = false, products = false;  // its counts, its tail use the FP64 work spectra
     std::vector<PlanArena> arenas;          // this plan's device tables and their host mirrors
     std::vector<PlanArena> device_only;     // tables made on the device (no mirror)
     std::vector<std::function<int()>> ops_once;  // their launches, after the next flush
@@ -2576,6 +2591,8 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
         if (I.enum_counts) I.enum_counts = pair_count_lists(I.sa, I.sb, N, c_lo, c_hi, I.gtable.size() == 1, &I.lists);
         any_fft = any_fft || !I.enum_counts;
     }
+    P->fft_counts = any_fft;
+    P->products = !direct.empty();
     if (any_fft) {
         PS_TRY(ensure_pair_bufs(c, c->d));
         SideLane lane(c, true);  // the side lane's own scratch, profiling or not
@@ -2648,6 +2665,7 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
                     if (q != M && (q >= 2 * M || most > ((size_t)1 << 30))) break;
                 }
             PS_TRY(ensure_lane_work(c, 0, most));
+            if (!I.enum_counts) PS_TRY(join_side(c));
             PS_TRY(tune_grid(c, group_op, M, &M, [&]() { return plan_flush(P); }));
             c->tune_grid[key] = M;
         }
@@ -2996,6 +3014,7 @@ int plan_enqueue(ps_gpu_ctx* c, ps_gpu_plan* P)
         PS_CK(cudaStreamWaitEvent(c->stream, P->ev_counts, 0));
         P->prepared = false;
     }
+    if (!c->capturing && (P->fft_counts || P->products)) PS_TRY(join_side(c));  // of other plans
     PS_TRY(enqueue_part(c, P, PART_DERIVED));
     if (P->has_groups) {  // fork the side lane after the DERIVED chain the counts read
         PS_CK(cudaEventRecord(c->ev_fork, c->stream));
@@ -3217,9 +3236,11 @@ int plan_run(ps_gpu_ctx* c, ps_gpu_plan* P)
         PS_CK(cudaStreamWaitEvent(c->stream, P->ev_derived, 0));
         PS_TRY(run_part(c, P, PART_GROUPS));
         PS_CK(cudaStreamWaitEvent(c->stream, P->ev_counts, 0));
+        if (P->products) PS_TRY(join_side(c));  // counts of other plans prepared since
         return run_part(c, P, PART_TAIL);
     }
     if (!(P->flags & PS_PLAN_GRAPH)) return plan_enqueue(c, P);
+    if (P->fft_counts || P->products) PS_TRY(join_side(c));
     return capture_launch(c, &P->graph, &P->exec, &P->graph_launches, [=]() { return plan_enqueue(c, P); });
 }
 
@@ -3234,6 +3255,7 @@ int plan_prepare(ps_gpu_ctx* c, ps_gpu_plan* P)
     PS_CK(cudaStreamWaitEvent(c->side_stream, P->ev_prep, 0));
     SideLane lane(c, true);
     PS_TRY(run_part(c, P, PART_DERIVED));
+    c->side_fp64 = c->side_fp64 || P->fft_counts;
     PS_CK(cudaEventRecord(P->ev_derived, c->stream));
     PS_TRY(run_part(c, P, PART_COUNTS));
     PS_CK(cudaEventRecord(P->ev_counts, c->stream));
@@ -3287,9 +3309,7 @@ int plain_batch(ps_gpu_ctx* c, int nconf, ps_cfg* cfgs, double* B, double* Np, d
         PS_TRY(arena_take(&tmp, sizeof(double) * 4 * (size_t)nconf, &dh, &hh));
         double* h = (double*)hh;  // B, Npoly | sum D | sum |D|
         PS_TRY(plan_flush(&tmp));
-        // the counts of a prepared plan may still use the FP64 work spectrum
-        PS_CK(cudaEventRecord(c->ev_join, c->side_stream));
-        PS_CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
+        PS_TRY(join_side(c));
         double *sD = sums, *sI = sums + nconf, *sA = sums + 2 * (size_t)nconf;
         std::vector<ProdCfg> fit, large;
         for (const ProdCfg& g : prods) (prod_fits<double>(table, g, N, false) ? fit : large).push_back(g);
@@ -3353,6 +3373,7 @@ int grad_impl(ps_gpu_ctx* c, int n, const std::vector<Shell>& legs, double scale
     const int N = c->N;
     const size_t nspec = (size_t)N * N * B.S;
     const size_t n3 = (size_t)N * N * N;
+    if (sizeof(T) == 8) PS_TRY(join_side(c));
     PS_TRY(alloc_dev(&B.hacc, nspec));
     PS_TRY(ensure_shells(c, PS_MAX_LEGS));
     PS_CK(cudaMemcpyAsync(c->dshells, legs.data(), sizeof(Shell) * n, cudaMemcpyHostToDevice, c->stream));
