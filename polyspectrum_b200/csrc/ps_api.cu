@@ -13,6 +13,7 @@
 #include <atomic>
 #include <functional>
 #include <map>
+#include <memory>
 #include <set>
 #include <string>
 #include <condition_variable>
@@ -295,6 +296,10 @@ struct HostBlocks {
     void give(unsigned char* p, size_t cap);
 };
 constexpr size_t kSpareArenas = 4;
+// A configuration's legs must all be in memory at once; above this (two or more
+// full-band legs at 1024 points in FP64) they are taken one by one with the running
+// product on a real grid, which needs one spectrum however many legs there are.
+constexpr size_t kProdMost = (size_t)16 << 30;
 constexpr size_t kSpareBytes = (size_t)64 << 20;  // larger arenas are given back at once
 
 void HostBlocks::give(unsigned char* p, size_t cap)
@@ -310,6 +315,21 @@ void HostBlocks::give(unsigned char* p, size_t cap)
     }
     cudaFreeHost(p);
 }
+
+// Device memory of a field lane's workspace: a buffer of the context, or its own.  A
+// plan holds the blocks its launches have addresses in; a block the context has
+// replaced is freed when the last such plan is gone.
+struct WorkBlock {
+    unsigned char* p;
+    size_t cap;  // bytes
+    bool own;
+    WorkBlock(unsigned char* q, size_t n, bool o) : p(q), cap(n), own(o) {}
+    WorkBlock(const WorkBlock&) = delete;
+    ~WorkBlock()
+    {
+        if (own) cudaFree(p);
+    }
+};
 
 struct ps_gpu_ctx {
     int N = 0;
@@ -333,9 +353,7 @@ struct ps_gpu_ctx {
     // product spectra, block sums), so the kernels of different batches overlap;
     // workspace 2 is the products' (prod_ops)
     cudaStream_t lane2_stream = nullptr;
-    unsigned char* lane_work[3] = {nullptr, nullptr, nullptr};
-    size_t lane_work_cap[3] = {0, 0, 0};  // bytes
-    bool lane_work_own[3] = {false, false, false};  // allocated for it (else one of the buffers below)
+    std::shared_ptr<WorkBlock> lane_work[3];
     cudaEvent_t ev_join2 = nullptr;
     // memory of destroyed plans kept for the next ones (at most kSpareArenas)
     std::vector<PlanArena> spare_arenas, spare_device;
@@ -585,6 +603,7 @@ template <typename T> int ensure_pair_bufs(ps_gpu_ctx* c, PrecBufs<T>& b)
 int ensure_partials(ps_gpu_ctx* c, size_t n)
 {
     if (n <= c->partials_cap) return PS_OK;
+    n = std::max(n, c->partials_cap + c->partials_cap / 2);  // (the replaced ones add up to twice the last)
     if (c->partials) c->retired.push_back(c->partials);
     c->partials = nullptr;
     c->partials_cap = 0;
@@ -661,27 +680,39 @@ int join_side(ps_gpu_ctx* c)
 // Workspace of a field lane, at least `bytes`.  A buffer of the context that nothing
 // else uses while the lane works serves as long as it is large enough: lane 0 the FP32
 // work spectrum, lane 1 an FP32 real grid, the products (2) the FP64 work spectrum
-// (after join_side).  A replaced own one is
-// retired: a captured graph or a plan's launches may still point at it.
+// (after join_side).  Above that the lane has a block of its own, which grows by half
+// at least, up to the most one configuration can ask for, so that a series of ever
+// larger calls allocates a few times only; the block it replaces is freed first unless
+// a plan's launches hold addresses in it.
 int ensure_lane_work(ps_gpu_ctx* c, int lane, size_t bytes)
 {
-    if (bytes <= c->lane_work_cap[lane]) return PS_OK;
+    std::shared_ptr<WorkBlock>& w = c->lane_work[lane];
+    if (w && bytes <= w->cap) return PS_OK;
     const size_t rows = (size_t)c->N * c->N;
     unsigned char* const base[3] = {(unsigned char*)c->f.work, (unsigned char*)c->f.ra, (unsigned char*)c->d.work};
     const size_t size[3] = {rows * (size_t)c->f.S * sizeof(V2<float>), rows * (size_t)c->N * sizeof(float),
                             rows * (size_t)c->d.S * sizeof(V2<double>)};
     if (base[lane] && bytes <= size[lane]) {
-        c->lane_work[lane] = base[lane];
-        c->lane_work_cap[lane] = size[lane];
+        w = std::make_shared<WorkBlock>(base[lane], size[lane], false);
         return PS_OK;
     }
-    if (c->lane_work_own[lane]) c->retired.push_back(c->lane_work[lane]);
-    c->lane_work[lane] = nullptr;
-    c->lane_work_cap[lane] = 0;
-    c->lane_work_own[lane] = false;
-    PS_TRY(alloc_dev(&c->lane_work[lane], bytes));
-    c->lane_work_cap[lane] = bytes;
-    c->lane_work_own[lane] = true;
+    if (fault_hit(FAULT_ALLOC)) return fail(PS_ERR_OOM, "workspace of %zu bytes: injected failure", bytes);
+    const size_t most = lane == 2 ? kProdMost : 3 * size[0];  // three full-band spectra
+    size_t want = w && w->own ? std::max(bytes, std::min(w->cap + w->cap / 2, most)) : bytes;
+    for (cudaStream_t st : {c->stream, c->lane2_stream}) cudaStreamSynchronize(st);  // nothing uses it any more
+    w.reset();
+    unsigned char* p = nullptr;
+    cudaError_t e = cudaMalloc((void**)&p, want);
+    if (e != cudaSuccess && want > bytes) {
+        cudaGetLastError();  // the refused size is no kernel's error
+        want = bytes;
+        e = cudaMalloc((void**)&p, want);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return fail(PS_ERR_OOM, "workspace of %zu bytes: %s", bytes, cudaGetErrorString(e));
+    }
+    w = std::make_shared<WorkBlock>(p, want, true);
     return PS_OK;
 }
 
@@ -1477,6 +1508,7 @@ struct ps_gpu_plan {
     bool fft_counts = false, products = false;  // its counts, its tail use the FP64 work spectra
     std::vector<PlanArena> arenas;          // this plan's device tables and their host mirrors
     std::vector<PlanArena> device_only;     // tables made on the device (no mirror)
+    std::vector<std::shared_ptr<WorkBlock>> work;  // workspaces its launches have addresses in
     std::vector<std::function<int()>> ops_once;  // their launches, after the next flush
     double* dres = nullptr;                 // B, Npoly per configuration
     double* dsumA = nullptr;                // sum |terms| (condition numbers)
@@ -1862,32 +1894,24 @@ template <typename T> size_t prod_spectrum_bytes(const Shell& sh, int M, bool un
     return (rows * (size_t)S * sizeof(V2<T>) + 255) / 256 * 256;
 }
 
-// A configuration's legs must all be in memory at once; above this (two or more
-// full-band legs at 1024 points in FP64) they are taken one by one with the running
-// product on a real grid, which needs one spectrum however many legs there are.
-constexpr size_t kProdMost = (size_t)16 << 30;
 constexpr size_t kProdBatch = (size_t)64 << 20;  // spectra of a batch: they stay in L2
 
-// Launch sequence of the grid sums of `cfgs` on the M-grid, `scale` times each into
-// out[cfg.out] (and of the terms' absolute values into out_abs, if not NULL).  unit:
-// sums of products of the shells themselves (T double).  The distinct shells of a
-// batch of configurations are transformed along X and Y once, in one launch each;
-// k_prod_z does the rows, the product and the sum.
+// Configurations whose distinct shells are transformed together, while the spectra
+// stay within kProdBatch (one configuration alone may exceed it).
+struct ProdBatch {
+    std::vector<int> shells;
+    std::vector<size_t> at;  // offsets of their spectra
+    std::vector<const ProdCfg*> cfgs;
+    size_t bytes = 0;
+};
 template <typename T>
-int prod_ops(ps_gpu_ctx* c, const std::vector<Shell>& host, const Shell* dtable, const std::vector<ProdCfg>& cfgs, int M,
-             bool unit, double scale, double* out, double* out_abs, std::vector<std::function<int()>>* ops)
+std::vector<ProdBatch> prod_batches(const std::vector<Shell>& host, const std::vector<ProdCfg>& cfgs, int M, bool unit)
 {
-    struct Batch {
-        std::vector<int> shells;
-        std::vector<size_t> at;  // offsets of their spectra
-        std::vector<const ProdCfg*> cfgs;
-        size_t bytes = 0;
-    };
-    std::vector<Batch> batches;
+    std::vector<ProdBatch> batches;
     for (const ProdCfg& g : cfgs) {
         size_t more = 0;
         std::vector<int> add;
-        const auto missing = [&](const Batch* b) {
+        const auto missing = [&](const ProdBatch* b) {
             more = 0;
             add.clear();
             for (const auto& f : g.f)
@@ -1902,7 +1926,7 @@ int prod_ops(ps_gpu_ctx* c, const std::vector<Shell>& host, const Shell* dtable,
             batches.emplace_back();
             missing(nullptr);
         }
-        Batch& b = batches.back();
+        ProdBatch& b = batches.back();
         for (int sidx : add) {
             b.shells.push_back(sidx);
             b.at.push_back(b.bytes);
@@ -1910,19 +1934,57 @@ int prod_ops(ps_gpu_ctx* c, const std::vector<Shell>& host, const Shell* dtable,
         }
         b.cfgs.push_back(&g);
     }
-    int most = 0;  // partial sums of a product
+    return batches;
+}
+
+// Partial sums of a product at most: its blocks are resident ones (32 per SM).
+template <typename T> int prod_sums(ps_gpu_ctx* c, int M, bool unit, int* most)
+{
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+    const int N = M;
+    PS_SWITCH_N(N, (*most = std::min(L3<T, NN>::prod_blocks(unit), 32 * sms)));
+    return PS_OK;
+}
+
+// What the prod_ops of a call need: add<T>() once for each, then take() makes it
+// available to all of them (and the plan holds it).
+struct ProdRoom {
+    size_t spectra = 0, sums = 0;
+    template <typename T>
+    int add(ps_gpu_ctx* c, const std::vector<Shell>& host, const std::vector<ProdCfg>& cfgs, int M, bool unit)
     {
-        const int N = M;
-        PS_SWITCH_N(N, (most = L3<T, NN>::prod_blocks(unit)));
+        for (const ProdBatch& b : prod_batches<T>(host, cfgs, M, unit)) spectra = std::max(spectra, b.bytes);
+        int most = 0;
+        PS_TRY(prod_sums<T>(c, M, unit, &most));
+        sums = std::max(sums, (size_t)most * kItems);
+        return PS_OK;
     }
-    size_t spectra = 0;
-    for (const Batch& b : batches) spectra = std::max(spectra, b.bytes);
-    PS_TRY(ensure_lane_work(c, 2, spectra + sizeof(double) * (size_t)most * kItems));
+    int take(ps_gpu_ctx* c, ps_gpu_plan* P) const
+    {
+        PS_TRY(ensure_lane_work(c, 2, spectra));
+        PS_TRY(ensure_partials(c, sums));
+        P->work.push_back(c->lane_work[2]);
+        return PS_OK;
+    }
+};
+
+// Launch sequence of the grid sums of `cfgs` on the M-grid, `scale` times each into
+// out[cfg.out] (and of the terms' absolute values into out_abs, if not NULL).  unit:
+// sums of products of the shells themselves (T double).  The distinct shells of a
+// batch of configurations are transformed along X and Y once, in one launch each;
+// k_prod_z does the rows, the product and the sum.  Its memory: ProdRoom.
+template <typename T>
+int prod_ops(ps_gpu_ctx* c, const std::vector<Shell>& host, const Shell* dtable, const std::vector<ProdCfg>& cfgs, int M,
+             bool unit, double scale, double* out, double* out_abs, std::vector<std::function<int()>>* ops)
+{
+    const std::vector<ProdBatch> batches = prod_batches<T>(host, cfgs, M, unit);
+    int most = 0;
+    PS_TRY(prod_sums<T>(c, M, unit, &most));
     Tables<T> tb;
     PS_TRY(tables_for<T>(c, M, &tb));
-    unsigned char* base = c->lane_work[2];
-    double* partials = (double*)(base + spectra);
-    for (const Batch& b : batches) {
+    unsigned char* base = c->lane_work[2]->p;
+    for (const ProdBatch& b : batches) {
         std::vector<XItem<T>> xi;
         std::vector<YItem<T>> yi;
         std::map<int, std::pair<V2<T>*, std::pair<int, int>>> where;  // shell -> spectrum, stride, columns
@@ -1964,6 +2026,7 @@ int prod_ops(ps_gpu_ctx* c, const std::vector<Shell>& host, const Shell* dtable,
             const int N = M;  // PS_SWITCH_N's subject
             const int quad = unit ? 1 : 0, mode = unit ? LOAD_UNIT : LOAD_MASKED;
             const PrecBufs<T>& F = bufs<T>(c);
+            double* partials = c->partials;
             for (int q = 0; q < nx; q += kItems) {
                 const int n = std::min(kItems, nx - q);
                 Prof pf(c);
@@ -2439,8 +2502,8 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
                         std::function<int()>* op) -> int {
         const int w = pw<float>(M);
         const size_t rows = (size_t)M * M;
-        unsigned char* at = c->lane_work[lane] + spectra_at;
-        double* part = (double*)(c->lane_work[lane] + sums_at);
+        unsigned char* at = c->lane_work[lane]->p + spectra_at;
+        double* part = (double*)(c->lane_work[lane]->p + sums_at);
         auto carve = [&](size_t n) {
             unsigned char* p = at;
             at += (n + 255) / 256 * 256;
@@ -2734,7 +2797,9 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
         }
         for (int l = 0; l < 2; l++) {  // final size before any batch takes addresses
             nsums[l] = (nsums[l] + 255) / 256 * 256;
-            if (need[l]) PS_TRY(ensure_lane_work(c, l, nsums[l] + need[l]));
+            if (!need[l]) continue;
+            PS_TRY(ensure_lane_work(c, l, nsums[l] + need[l]));
+            P->work.push_back(c->lane_work[l]);
         }
         sums.clear();  // of the tuning's candidates
         for (size_t q = 0; q < batches.size(); q++) {
@@ -2940,6 +3005,13 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
             const int M = alias_free_grid_n(N, total, bmax);
             (prod_fits<float>(table, g, M, false) ? by_size[M] : large).push_back(g);
         }
+        ProdRoom room;
+        for (const auto& kv : by_size) {
+            PS_TRY(room.add<float>(c, table, kv.second, kv.first, false));
+            PS_TRY(room.add<double>(c, table, kv.second, kv.first, true));
+        }
+        if (!large.empty()) PS_TRY(room.add<double>(c, table, large, N, true));
+        PS_TRY(room.take(c, P));
         for (const auto& kv : by_size) {
             const double up = ((double)N / kv.first) * ((double)N / kv.first) * ((double)N / kv.first);
             PS_TRY(prod_ops<float>(c, table, dtable, kv.second, kv.first, false, up, sumD, kappa ? sumA : nullptr, &tail));
@@ -3172,6 +3244,7 @@ void plan_release(ps_gpu_plan* P, bool keep)
         }
         P->device_only.clear();
     }
+    P->work.clear();
     P->ops_once.clear();
     P->hres = nullptr;
 }
@@ -3313,6 +3386,10 @@ int plain_batch(ps_gpu_ctx* c, int nconf, ps_cfg* cfgs, double* B, double* Np, d
         double *sD = sums, *sI = sums + nconf, *sA = sums + 2 * (size_t)nconf;
         std::vector<ProdCfg> fit, large;
         for (const ProdCfg& g : prods) (prod_fits<double>(table, g, N, false) ? fit : large).push_back(g);
+        ProdRoom room;
+        if (!fit.empty()) PS_TRY(room.add<double>(c, table, fit, N, false));
+        PS_TRY(room.add<double>(c, table, prods, N, true));
+        PS_TRY(room.take(c, &tmp));
         std::vector<std::function<int()>> ops;
         if (!fit.empty()) PS_TRY(prod_ops<double>(c, table, dtable, fit, N, false, 1.0, sD, kappa ? sA : nullptr, &ops));
         PS_TRY(enqueue_ops(ops));
@@ -4602,8 +4679,7 @@ void ps_gpu_finalize(ps_gpu_ctx* c)
         cudaStreamSynchronize(c->lane2_stream);
         cudaStreamDestroy(c->lane2_stream);
     }
-    for (int l = 0; l < 3; l++)
-        if (c->lane_work_own[l]) cudaFree(c->lane_work[l]);
+    for (auto& w : c->lane_work) w.reset();
     if (c->ev_join2) cudaEventDestroy(c->ev_join2);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
