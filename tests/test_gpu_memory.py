@@ -67,16 +67,16 @@ def test_one_full_band_leg_fits_the_work_spectrum(gpu_lib):
         ctx.get_FT_field(ps.PS_FIELD_DENS, field())
         ctx.batch([triangle(ps, 20.0, 20.0, 20.0)], 1)
         before = used()
-        ctx.batch([triangle(ps, 127.6, 127.6, 127.6)], 1)  # band 128
+        ctx.batch([triangle(ps, 128.1, 128.1, 128.1)], 1)  # band 128
         assert used() - before <= 32 << 20
 
 
 def test_growing_shell_lists_keep_bounded_sums(gpu_lib):
     ps = gpu_lib
-    n = 32
+    n = 128
     with ps.Context(n, BOX, methods=2) as ctx:
         ctx.get_FT_field(ps.PS_FIELD_DENS, synth.lognormal_density(n, 2.0, 3))
-        ks = np.linspace(1.0, 15.0, 1600) * KF
+        ks = np.linspace(1.0, 63.0, 1600) * KF
         cfgs = [ps.make_cfg(2, [k, k], kbinwidth=1.0) for k in ks]
         ctx.batch(cfgs[:4], 2)
         before = used()
