@@ -110,3 +110,29 @@ def test_plans_keep_their_workspace(gpu_lib, graph):
         np.testing.assert_array_equal(Np, wantq[1])
         np.testing.assert_array_equal(B, wantq[0])
         q.close()
+
+
+def test_calls_after_running_out_of_memory(gpu_lib):
+    """A refused allocation is that call's error and no later one's."""
+    import torch
+    ps = gpu_lib
+    with ps.Context(N, BOX) as ctx:
+        ctx.get_FT_field(ps.PS_FIELD_DENS, field())
+        small, large = [triangle(ps, 20.0, 21.0, 25.0)], [triangle(ps, 100.0, 101.0, 127.4)]
+        want = ctx.batch(small, 2)
+        wantp = ctx.batch(small, 1)
+        torch.cuda.empty_cache()
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - (48 << 20), dtype=torch.uint8, device="cuda")
+        for refused in (lambda: ctx.batch(large, 2), lambda: ctx.batch(large, 1), lambda: ps.Context(N, BOX),
+                        lambda: ctx.grad(3, [20 * KF] * 3, [0.0] * 3, [0.0] * 3, 0.5, 0)):
+            with pytest.raises(ps.PsError) as err:
+                refused()
+            assert err.value.status == -2, err.value
+            for method, w in ((2, want), (1, wantp)):
+                B, Np, _, _ = ctx.batch(small, method)
+                np.testing.assert_array_equal(Np, w[1])
+                np.testing.assert_array_equal(B, w[0])
+        del hog
+        torch.cuda.empty_cache()
+        _, Np, _, _ = ctx.batch(large, 2)
+        assert Np[0] > 0
