@@ -1509,6 +1509,7 @@ struct ps_gpu_plan {
     std::vector<PlanArena> arenas;          // this plan's device tables and their host mirrors
     std::vector<PlanArena> device_only;     // tables made on the device (no mirror)
     std::vector<std::shared_ptr<WorkBlock>> work;  // workspaces its launches have addresses in
+    std::vector<cudaEvent_t> foreign;  // ends of its launches on callers' streams, oldest first
     std::vector<std::function<int()>> ops_once;  // their launches, after the next flush
     double* dres = nullptr;                 // B, Npoly per configuration
     double* dsumA = nullptr;                // sum |terms| (condition numbers)
@@ -3202,10 +3203,35 @@ int submit_slot(ps_gpu_ctx* c, size_t len, double** host, cudaEvent_t* ev)
     return PS_OK;
 }
 
+// Marks the end of a plan's launch on a caller's stream: the caller may give the context
+// another one, and destroy this one, before the launch is done.
+int mark_foreign(ps_gpu_ctx* c, ps_gpu_plan* P)
+{
+    if (c->stream == c->own_stream) return PS_OK;
+    size_t done = 0;
+    while (done < P->foreign.size() && cudaEventQuery(P->foreign[done]) == cudaSuccess) c->spare_events.push_back(P->foreign[done++]);
+    P->foreign.erase(P->foreign.begin(), P->foreign.begin() + (long)done);
+    cudaEvent_t ev = nullptr;
+    if (!c->spare_events.empty()) {
+        ev = c->spare_events.back();
+        c->spare_events.pop_back();
+    } else {
+        PS_CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    }
+    P->foreign.push_back(ev);
+    PS_CK(cudaEventRecord(ev, c->stream));
+    return PS_OK;
+}
+
 // Graphs and tables of a plan (the plan object itself stays); keep: its memory
 // goes back to the context for the next plan, else it is freed.
 void plan_release(ps_gpu_plan* P, bool keep)
 {
+    for (cudaEvent_t e : P->foreign) {
+        cudaEventSynchronize(e);
+        cudaEventDestroy(e);
+    }
+    P->foreign.clear();
     if (P->exec) cudaGraphExecDestroy(P->exec);
     if (P->graph) cudaGraphDestroy(P->graph);
     P->exec = nullptr;
@@ -3227,7 +3253,7 @@ void plan_release(ps_gpu_plan* P, bool keep)
     if (!P->arenas.empty()) {
         // nothing may still read the tables or their mirrors when the next plan writes them
         ps_gpu_ctx* c = P->ctx;
-        for (cudaStream_t st : {c->stream, c->side_stream, c->lane2_stream})
+        for (cudaStream_t st : {c->stream, c->own_stream, c->side_stream, c->lane2_stream})
             if (st) cudaStreamSynchronize(st);
         for (PlanArena& a : P->arenas) {
             if (keep && a.cap <= kSpareBytes && c->spare_arenas.size() < kSpareArenas) {
@@ -4426,8 +4452,9 @@ int ps_gpu_plan_launch(ps_gpu_ctx* c, ps_gpu_plan* P)
     if (!c->f.have_spec) return fail(PS_ERR_ARG, "FP32 spectrum not available");
     PS_TRY(check_band(c, P->band));
     PS_CK(cudaSetDevice(c->device));
-    if ((P->flags & PS_PLAN_GRAPH) && c->prof_on) return plan_enqueue(c, P);
-    return plan_run(c, P);
+    if ((P->flags & PS_PLAN_GRAPH) && c->prof_on) PS_TRY(plan_enqueue(c, P));
+    else PS_TRY(plan_run(c, P));
+    return mark_foreign(c, P);
 }
 
 int ps_gpu_plan_prepare(ps_gpu_ctx* c, ps_gpu_plan* P)
@@ -4464,7 +4491,7 @@ int ps_gpu_plan_results_device(ps_gpu_ctx* c, ps_gpu_plan* P, double* dst)
     const size_t n = (size_t)P->nconf;
     PS_CK(cudaMemcpyAsync(dst, P->dres, 16 * n, cudaMemcpyDeviceToDevice, c->stream));
     PS_CK(cudaMemcpyAsync(dst + 2 * n, P->dwb, 48 * n, cudaMemcpyDeviceToDevice, c->stream));
-    return PS_OK;
+    return mark_foreign(c, P);
 }
 
 int ps_gpu_synchronize(ps_gpu_ctx* c)

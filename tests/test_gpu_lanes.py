@@ -90,3 +90,36 @@ def test_tuning_between_prepare_and_execution(gpu_lib):
     with ps.Context(N, BOX, methods=ps.PS_FP32_BATCHED) as ctx:
         ctx.get_FT_field(ps.PS_FIELD_DENS, field)
         np.testing.assert_array_equal(ctx.batch(triangles(ps, ps.PS_BIN_WATKINSON, 4, 36.0, 7))[1], tuned)
+
+
+def test_plan_destroyed_while_a_callers_stream_still_runs_it(gpu_lib):
+    """A launch and its result copy queued on a caller's stream, the context given back to
+    its own stream, the plan destroyed and others made in its memory: the copy still
+    brings the first plan's results."""
+    import torch
+    ps = gpu_lib
+    field = torch.from_numpy(synth.lognormal_density(N, 2.0, 3)).cuda()
+    first, other = triangles(ps, 0, 6, 30.0, 1), triangles(ps, 0, 9, 20.0, 2)
+    s = torch.cuda.Stream()
+    with ps.Context(N, BOX, methods=ps.PS_FP32_BATCHED) as ctx:
+        ctx.get_FT_field(ps.PS_FIELD_DENS, field)
+        for graph in (False, True):
+            p = ctx.plan(first, graph=graph)
+            B, Np, _, _ = p.execute()
+            out = torch.zeros(8 * len(first), dtype=torch.float64, device="cuda")
+            torch.cuda.synchronize()
+            with torch.cuda.stream(s):
+                torch.cuda._sleep(100_000_000)  # some 50 ms ahead of the launch
+            ctx.set_stream(s.cuda_stream)
+            p.launch()
+            p.results_to_device(out.data_ptr())
+            ctx.set_stream(None)
+            p.close()
+            for _ in range(4):
+                q = ctx.plan(other, graph=graph)
+                q.execute()
+                q.close()
+            torch.cuda.synchronize()
+            got = out.cpu().numpy()[:2 * len(first)].reshape(-1, 2)
+            np.testing.assert_array_equal(got[:, 0], B)
+            np.testing.assert_array_equal(got[:, 1], Np)
