@@ -145,6 +145,11 @@ __global__ void __launch_bounds__(THREADS, THREADS == kCountSmallThreads ? 6 : 1
 // (In integers, whose multiply-adds and minima issue at half rate, the 2.4e8 pairs of 64
 // equilateral triangles at 128^3 took 0.197 instead of 0.156 ms, with histograms 0.42 ms.)
 constexpr int kOneThreads = 256, kOneBPT = 4, kOneRepChunk = 256;
+struct __align__(16) OneRep {  // a staged representative, read as two float4
+    float2 v[4];
+    __device__ __forceinline__ float4 pair(int q) const { return reinterpret_cast<const float4*>(v)[q]; }
+};
+static_assert(alignof(OneRep) == alignof(float4) && sizeof(OneRep) == 2 * sizeof(float4), "vector reads of shared rows");
 
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
 {
@@ -169,7 +174,7 @@ __global__ void __launch_bounds__(kOneThreads, 4)
     const CountItem it = items[gi];
     // representatives, each value twice (packed operands): f (a, c), f a = 2 a (WRAP: 4 a),
     // c the constant part; WRAP: -2 n a
-    __shared__ float2 sa[kOneRepChunk][4], su[WRAP ? kOneRepChunk : 1][4];
+    __shared__ OneRep sa[kOneRepChunk], su[WRAP ? kOneRepChunk : 1];
     __shared__ unsigned sw[kOneRepChunk];
     const int lo = it.closing[0].r2lo, hi = it.closing[0].r2hi;
     const float f = WRAP ? 2.f : 1.f, fn = (float)n;
@@ -210,14 +215,14 @@ __global__ void __launch_bounds__(kOneThreads, 4)
             const float ux = -2.f * fn * x, uy = -2.f * fn * y, uz = -2.f * fn * z;
             float c = f * (x * x + y * y + z * z) - mid;
             if (WRAP) c += ux + uy + uz;
-            sa[i][0] = float2{2.f * f * x, 2.f * f * x};
-            sa[i][1] = float2{2.f * f * y, 2.f * f * y};
-            sa[i][2] = float2{2.f * f * z, 2.f * f * z};
-            sa[i][3] = float2{c, c};
+            sa[i].v[0] = float2{2.f * f * x, 2.f * f * x};
+            sa[i].v[1] = float2{2.f * f * y, 2.f * f * y};
+            sa[i].v[2] = float2{2.f * f * z, 2.f * f * z};
+            sa[i].v[3] = float2{c, c};
             if constexpr (WRAP) {
-                su[i][0] = float2{ux, ux};
-                su[i][1] = float2{uy, uy};
-                su[i][2] = float2{uz, uz};
+                su[i].v[0] = float2{ux, ux};
+                su[i].v[1] = float2{uy, uy};
+                su[i].v[2] = float2{uz, uz};
             }
             sw[i] = (unsigned)a.w;
         }
@@ -225,7 +230,7 @@ __global__ void __launch_bounds__(kOneThreads, 4)
         unsigned here = 0u;  // at most rep_slice BPT 48
 #pragma unroll 2
         for (int r = 0; r < cnt; r++) {
-            const float4 a01 = *reinterpret_cast<const float4*>(sa[r]), a23 = *reinterpret_cast<const float4*>(sa[r] + 2);
+            const float4 a01 = sa[r].pair(0), a23 = sa[r].pair(1);
             const unsigned w = sw[r];
 #pragma unroll
             for (int p = 0; p < NP; p++) {
@@ -234,9 +239,9 @@ __global__ void __launch_bounds__(kOneThreads, 4)
                 v = fma2(float2{a01.z, a01.w}, by[p], v);
                 v = fma2(float2{a23.x, a23.y}, bz[p], v);
                 if constexpr (WRAP) {
-                    const float4 u01 = *reinterpret_cast<const float4*>(su[r]);
+                    const float4 u01 = su[r].pair(0);
                     const float2 tx = cadd(float2{u01.x, u01.y}, ex[p]), ty = cadd(float2{u01.z, u01.w}, ey[p]),
-                                 tz = cadd(su[r][2], ez[p]);
+                                 tz = cadd(su[r].v[2], ez[p]);
                     v.x = ((v.x - fabsf(tx.x)) - fabsf(ty.x)) - fabsf(tz.x);
                     v.y = ((v.y - fabsf(tx.y)) - fabsf(ty.y)) - fabsf(tz.y);
                 }
