@@ -49,10 +49,34 @@ def _deps() -> list[str]:
             + glob.glob(os.path.join(ROOT, "include", "*.h")))
 
 
-def _stale(obj: str) -> bool:
-    """Whether an object is older than a file it was compiled from (nvcc's own dependency list)."""
+def _compile_cmd(src: str, obj: str) -> list[str]:
+    return [nvcc(), *FLAGS, "-MD", "-MF", obj + ".d", "-c", os.path.join(CSRC, src), "-o", obj]
+
+
+def _signature(cmd: list[str]) -> str:
+    """What an object's or the library's code depends on besides its files: the compiler and its options."""
+    version = subprocess.run([cmd[0], "--version"], capture_output=True, text=True).stdout
+    return "\n".join([*(a.replace(ROOT, ".") for a in cmd), version])  # (the same wherever the tree lies)
+
+
+def _recorded(path: str, cmd: list[str]) -> bool:
+    """Whether `path` was made by this command (kept beside it when it was made)."""
+    if not os.path.exists(path + ".cmd"):
+        return False
+    with open(path + ".cmd") as f:
+        return f.read() == _signature(cmd)
+
+
+def _record(path: str, cmd: list[str]) -> None:
+    with open(path + ".cmd", "w") as f:
+        f.write(_signature(cmd))
+
+
+def _stale(obj: str, cmd: list[str]) -> bool:
+    """Whether an object is older than a file it was compiled from (nvcc's own
+    dependency list), or was compiled by another command."""
     dep = obj + ".d"
-    if not os.path.exists(obj) or not os.path.exists(dep):
+    if not os.path.exists(obj) or not os.path.exists(dep) or not _recorded(obj, cmd):
         return True
     with open(dep) as f:
         files = f.read().split(":", 1)[1].replace("\\\n", " ").split()
@@ -64,7 +88,10 @@ def up_to_date() -> bool:
     if not os.path.exists(LIB):
         return False
     t = os.path.getmtime(LIB)
-    return all(os.path.getmtime(p) <= t for p in _deps())
+    if any(os.path.getmtime(p) > t for p in _deps()):
+        return False
+    objs = [os.path.join(OUT_DIR, src.replace(".cu", ".o")) for src in SOURCES]
+    return all(_recorded(obj, _compile_cmd(src, obj)) for src, obj in zip(SOURCES, objs))
 
 
 def build_driver(force: bool = False) -> str:
@@ -102,20 +129,23 @@ def build(force: bool = False, ptxas_verbose: bool = False, quiet: bool = False)
     for src in SOURCES:
         obj = os.path.join(OUT_DIR, src.replace(".cu", ".o"))
         objs.append(obj)
-        if not force and not ptxas_verbose and not _stale(obj):
+        cmd = _compile_cmd(src, obj)
+        if not force and not ptxas_verbose and not _stale(obj, cmd):
             continue
-        cmd = [exe, *FLAGS, "-MD", "-MF", obj + ".d", "-c", os.path.join(CSRC, src), "-o", obj]
-        if ptxas_verbose:
-            cmd += ["-Xptxas", "-v"]
-        procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT,
-                                            text=True)))
+        extra = ["-Xptxas", "-v"] if ptxas_verbose else []
+        if os.path.exists(obj + ".cmd"):
+            os.remove(obj + ".cmd")
+        procs.append((src, obj, cmd, subprocess.Popen(cmd + extra, stdout=subprocess.PIPE, stderr=subprocess.STDOUT,
+                                                      text=True)))
     failed = False
-    for src, p in procs:
+    for src, obj, cmd, p in procs:
         out, _ = p.communicate()
         if p.returncode != 0:
             failed = True
             sys.stderr.write(f"nvcc failed for {src}:\n{out}\n")
-        elif out and (ptxas_verbose or not quiet):
+            continue
+        _record(obj, cmd)
+        if out and (ptxas_verbose or not quiet):
             lines = [ln for ln in out.splitlines() if "Wno-deprecated" not in ln]
             if lines:
                 sys.stdout.write("\n".join(lines) + "\n")
