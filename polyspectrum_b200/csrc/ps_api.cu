@@ -336,6 +336,7 @@ struct ps_gpu_ctx {
     double L = 0.0;  // (double)(float) box size, grid.h:9
     int methods = 0;
     int device = 0;
+    int sms = 148;
     cudaStream_t stream = nullptr;
     cudaStream_t own_stream = nullptr;
     // side lane: the count (FP64) parts of pair groups run on their own stream
@@ -1902,7 +1903,7 @@ constexpr size_t kProdBatch = (size_t)64 << 20;  // spectra of a batch: they sta
 struct ProdBatch {
     std::vector<int> shells;
     std::vector<size_t> at;  // offsets of their spectra
-    std::vector<const ProdCfg*> cfgs;
+    std::vector<const ProdCfg*> cfgs;  // (of the list they were made from)
     size_t bytes = 0;
 };
 template <typename T>
@@ -1938,27 +1939,34 @@ std::vector<ProdBatch> prod_batches(const std::vector<Shell>& host, const std::v
     return batches;
 }
 
-// Partial sums of a product at most: its blocks are resident ones (32 per SM).
-template <typename T> int prod_sums(ps_gpu_ctx* c, int M, bool unit, int* most)
-{
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-    const int N = M;
-    PS_SWITCH_N(N, (*most = std::min(L3<T, NN>::prod_blocks(unit), 32 * sms)));
-    return PS_OK;
-}
+// The grid sums of `cfgs` on the M-grid, `scale` times each into out[cfg.out] (and of
+// the terms' absolute values into out_abs, if not NULL).  unit: sums of products of the
+// shells themselves (T double).
+struct ProdCall {
+    const std::vector<ProdCfg>* cfgs;
+    int M;
+    bool unit;
+    double scale;
+    double *out, *out_abs;
+    std::vector<ProdBatch> batches;
+    int most = 0;  // partial sums of a product at most: its blocks are resident ones (32 per SM)
+};
 
-// What the prod_ops of a call need: add<T>() once for each, then take() makes it
-// available to all of them (and the plan holds it).
-struct ProdRoom {
+// The calls of an evaluation, made with one workspace for all of them: add() each, take()
+// once (the plan then holds the memory), then prod_ops() each.
+struct ProdCalls {
+    std::vector<ProdCall> calls;
     size_t spectra = 0, sums = 0;
     template <typename T>
-    int add(ps_gpu_ctx* c, const std::vector<Shell>& host, const std::vector<ProdCfg>& cfgs, int M, bool unit)
+    int add(ps_gpu_ctx* c, const std::vector<Shell>& host, const std::vector<ProdCfg>& cfgs, int M, bool unit, double scale,
+            double* out, double* out_abs)
     {
-        for (const ProdBatch& b : prod_batches<T>(host, cfgs, M, unit)) spectra = std::max(spectra, b.bytes);
-        int most = 0;
-        PS_TRY(prod_sums<T>(c, M, unit, &most));
-        sums = std::max(sums, (size_t)most * kItems);
+        calls.push_back(ProdCall{&cfgs, M, unit, scale, out, out_abs, prod_batches<T>(host, cfgs, M, unit), 0});
+        ProdCall& k = calls.back();
+        for (const ProdBatch& b : k.batches) spectra = std::max(spectra, b.bytes);
+        const int N = M;
+        PS_SWITCH_N(N, (k.most = std::min(L3<T, NN>::prod_blocks(unit), 32 * c->sms)));
+        sums = std::max(sums, (size_t)k.most * kItems);
         return PS_OK;
     }
     int take(ps_gpu_ctx* c, ps_gpu_plan* P) const
@@ -1970,22 +1978,21 @@ struct ProdRoom {
     }
 };
 
-// Launch sequence of the grid sums of `cfgs` on the M-grid, `scale` times each into
-// out[cfg.out] (and of the terms' absolute values into out_abs, if not NULL).  unit:
-// sums of products of the shells themselves (T double).  The distinct shells of a
-// batch of configurations are transformed along X and Y once, in one launch each;
-// k_prod_z does the rows, the product and the sum.  Its memory: ProdRoom.
+// Launch sequence of one call.  The distinct shells of a batch of configurations are
+// transformed along X and Y once, in one launch each; k_prod_z does the rows, the
+// product and the sum.
 template <typename T>
-int prod_ops(ps_gpu_ctx* c, const std::vector<Shell>& host, const Shell* dtable, const std::vector<ProdCfg>& cfgs, int M,
-             bool unit, double scale, double* out, double* out_abs, std::vector<std::function<int()>>* ops)
+int prod_ops(ps_gpu_ctx* c, const std::vector<Shell>& host, const Shell* dtable, const ProdCall& call,
+             std::vector<std::function<int()>>* ops)
 {
-    const std::vector<ProdBatch> batches = prod_batches<T>(host, cfgs, M, unit);
-    int most = 0;
-    PS_TRY(prod_sums<T>(c, M, unit, &most));
+    const int M = call.M, most = call.most;
+    const bool unit = call.unit;
+    const double scale = call.scale;
+    double *const out = call.out, *const out_abs = call.out_abs;
     Tables<T> tb;
     PS_TRY(tables_for<T>(c, M, &tb));
     unsigned char* base = c->lane_work[2]->p;
-    for (const ProdBatch& b : batches) {
+    for (const ProdBatch& b : call.batches) {
         std::vector<XItem<T>> xi;
         std::vector<YItem<T>> yi;
         std::map<int, std::pair<V2<T>*, std::pair<int, int>>> where;  // shell -> spectrum, stride, columns
@@ -2846,8 +2853,7 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
             if (info[g].enum_counts) total += info[g].gtable.size();
         unsigned long long* dcounts = nullptr;
         if (total) PS_TRY(plan_alloc(P, &dcounts, total));
-        int sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+        const int sms = c->sms;
         constexpr int kClass[4] = {0, kCountSmallBins, 12 * 1024, kCountMaxBins};  // bins (0: one closing shell)
         for (int wrap = 0; wrap < 2; wrap++)
             for (int cl = 0; cl < 4; cl++) {
@@ -3006,20 +3012,17 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
             const int M = alias_free_grid_n(N, total, bmax);
             (prod_fits<float>(table, g, M, false) ? by_size[M] : large).push_back(g);
         }
-        ProdRoom room;
-        for (const auto& kv : by_size) {
-            PS_TRY(room.add<float>(c, table, kv.second, kv.first, false));
-            PS_TRY(room.add<double>(c, table, kv.second, kv.first, true));
-        }
-        if (!large.empty()) PS_TRY(room.add<double>(c, table, large, N, true));
-        PS_TRY(room.take(c, P));
+        ProdCalls prods;
         for (const auto& kv : by_size) {
             const double up = ((double)N / kv.first) * ((double)N / kv.first) * ((double)N / kv.first);
-            PS_TRY(prod_ops<float>(c, table, dtable, kv.second, kv.first, false, up, sumD, kappa ? sumA : nullptr, &tail));
-            PS_TRY(prod_ops<double>(c, table, dtable, kv.second, kv.first, true, up, sumI, nullptr, &tail));
+            PS_TRY(prods.add<float>(c, table, kv.second, kv.first, false, up, sumD, kappa ? sumA : nullptr));
+            PS_TRY(prods.add<double>(c, table, kv.second, kv.first, true, up, sumI, nullptr));
         }
+        if (!large.empty()) PS_TRY(prods.add<double>(c, table, large, N, true, 1.0, sumI, nullptr));
+        PS_TRY(prods.take(c, P));
+        for (const ProdCall& k : prods.calls)
+            PS_TRY(k.unit ? prod_ops<double>(c, table, dtable, k, &tail) : prod_ops<float>(c, table, dtable, k, &tail));
         if (!large.empty()) {
-            PS_TRY(prod_ops<double>(c, table, dtable, large, N, true, 1.0, sumI, nullptr, &tail));
             const std::vector<Shell> host = table;
             tail.push_back([=]() {
                 for (const ProdCfg& g : large)
@@ -3253,7 +3256,8 @@ void plan_release(ps_gpu_plan* P, bool keep)
     if (!P->arenas.empty()) {
         // nothing may still read the tables or their mirrors when the next plan writes them
         ps_gpu_ctx* c = P->ctx;
-        for (cudaStream_t st : {c->stream, c->own_stream, c->side_stream, c->lane2_stream})
+        if (c->own_stream && c->own_stream != c->stream) cudaStreamSynchronize(c->own_stream);
+        for (cudaStream_t st : {c->stream, c->side_stream, c->lane2_stream})
             if (st) cudaStreamSynchronize(st);
         for (PlanArena& a : P->arenas) {
             if (keep && a.cap <= kSpareBytes && c->spare_arenas.size() < kSpareArenas) {
@@ -3412,16 +3416,17 @@ int plain_batch(ps_gpu_ctx* c, int nconf, ps_cfg* cfgs, double* B, double* Np, d
         double *sD = sums, *sI = sums + nconf, *sA = sums + 2 * (size_t)nconf;
         std::vector<ProdCfg> fit, large;
         for (const ProdCfg& g : prods) (prod_fits<double>(table, g, N, false) ? fit : large).push_back(g);
-        ProdRoom room;
-        if (!fit.empty()) PS_TRY(room.add<double>(c, table, fit, N, false));
-        PS_TRY(room.add<double>(c, table, prods, N, true));
-        PS_TRY(room.take(c, &tmp));
-        std::vector<std::function<int()>> ops;
-        if (!fit.empty()) PS_TRY(prod_ops<double>(c, table, dtable, fit, N, false, 1.0, sD, kappa ? sA : nullptr, &ops));
-        PS_TRY(enqueue_ops(ops));
-        ops.clear();
-        PS_TRY(prod_ops<double>(c, table, dtable, prods, N, true, 1.0, sI, nullptr, &ops));
-        PS_TRY(enqueue_ops(ops));
+        // one after the other, so that the shells' products are planned while the fields' run
+        const auto sums_of = [&](const std::vector<ProdCfg>& list, bool unit, double* out, double* out_abs) -> int {
+            ProdCalls call;
+            std::vector<std::function<int()>> ops;
+            PS_TRY(call.add<double>(c, table, list, N, unit, 1.0, out, out_abs));
+            PS_TRY(call.take(c, &tmp));
+            PS_TRY(prod_ops<double>(c, table, dtable, call.calls[0], &ops));
+            return enqueue_ops(ops);
+        };
+        if (!fit.empty()) PS_TRY(sums_of(fit, false, sD, kappa ? sA : nullptr));
+        PS_TRY(sums_of(prods, true, sI, nullptr));
         for (const ProdCfg& g : large) PS_TRY(legwise_sum<double>(c, table, dtable, g, sD + g.out, kappa ? sA + g.out : nullptr));
         {
             Prof pf(c);
@@ -3984,6 +3989,7 @@ int ps_gpu_create(ps_gpu_ctx** out, int nbins, double boxsize, int methods, int 
     c->L = boxsize;
     c->methods = methods;
     cudaGetDevice(&c->device);
+    cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device);
     int rc = PS_OK;
     do {
         if (cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking) != cudaSuccess) {
