@@ -1723,7 +1723,7 @@ int tune_pencil(ps_gpu_ctx* c, int M)
     bool has_alt = false;
     {
         const int N = M;
-        PS_SWITCH_N(N, (has_alt = L3<float, NN>::ALT > 0));
+        PS_SWITCH_N(N, (has_alt = L3<float, NN>::Y_ALT > 0));
     }
     if (!has_alt || !c->f.work) {
         c->pencil_alt[M] = 0;

@@ -296,7 +296,6 @@ int main(int argc, char** argv)
     time_pass_y<384, false, 0>(reps, w3, S, S, M, bc, "fwd");
     time_pass_y<384, false, 12>(reps, w3, S, S, M, bc, "fwd");
     time_pass_y<512, false, 0>(reps, spec, SN, 176, N, N, "field");
-    time_pass_y<512, false, 32>(reps, spec, SN, 176, N, N, "field");
     time_pass_y<512, false, 8>(reps, spec, SN, 176, N, N, "field");
 
     // pair kernel variants: the 384-point group above, and a 320-point group

@@ -94,7 +94,8 @@ template <typename T, int N, int RX> struct YGeom {
 // The alternative pencil geometry of the FP32 Y and dot passes for the larger
 // lengths: twice the elements per thread, half the threads per pencil, one radix
 // pass fewer; for a split length its register plan, which needs fewer registers (0:
-// none).  Chosen per length by the plan autotuner against the default.
+// none).  Chosen per length by the plan autotuner against the default; the 512-point Y
+// pass has this geometry anyway (YGeom).
 template <typename T, int N> struct PencilAlt {
     static constexpr int odd = LenKind<N>::odd_of(N);
     static constexpr int value = !(sizeof(T) == 4 && N >= 128 && N <= 512 && odd <= 5) ? 0

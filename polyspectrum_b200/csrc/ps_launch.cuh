@@ -80,6 +80,8 @@ template <typename T, int N> struct L3 {
     using RG = RowGeom<T, N>;
     static_assert(N == 16 || N == 1024 || PG::W == PencilWidth<T>::value, "tiles of one 128-byte segment");
     static constexpr int ALT = PencilAlt<T, N>::value;
+    // the Y pass's alternative geometry (0: none, or its default already is that one)
+    static constexpr int Y_ALT = YGeom<T, N, 0>::LONG ? 0 : ALT;
     static constexpr int DOT_ALT = PencilAlt<T, N>::dot_default;
     // host copy of the alternative pencil table, or of the Y pass's where it has a
     // geometry of its own (false: neither)

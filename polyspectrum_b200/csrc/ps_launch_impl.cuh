@@ -77,7 +77,7 @@ int L3<T, N>::pass_y_b(cudaStream_t st, const YItem<T>* items, int nitems, int n
         kernel<<<grid, threads, smem, st>>>(pack(items, nitems), quad, tw);
         return PS_OK;
     };
-    if constexpr (ALT > 0) {
+    if constexpr (Y_ALT > 0) {
         using PA = PencilGeom<T, N, ALT>;
         if (alt && tb.twp_alt)
             return inv ? go(k_pass_y<T, N, true, ALT>, PA::THREADS, PA::SMEM, tb.twp_alt)
