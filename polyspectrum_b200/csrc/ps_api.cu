@@ -669,10 +669,16 @@ struct Lane2 {
 // ones (ps_gpu_plan_prepare) run on the side stream until their plan's next execution,
 // beside whatever the context does meanwhile: work on the main stream that uses one of
 // these spectra (products, FP64 gradients, counts there) waits for them here first.
-// Never inside a capture: a graph's launch is what has to wait.
+// Never inside a capture, the context's or the caller's: a graph's launch is what has
+// to wait.
+bool stream_captured(cudaStream_t st)
+{
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &s) == cudaSuccess && s != cudaStreamCaptureStatusNone;
+}
 int join_side(ps_gpu_ctx* c)
 {
-    if (!c->side_fp64) return PS_OK;
+    if (!c->side_fp64 || stream_captured(c->stream)) return PS_OK;
     PS_CK(cudaEventRecord(c->ev_join, c->side_stream));
     PS_CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
     return PS_OK;
@@ -3210,7 +3216,7 @@ int submit_slot(ps_gpu_ctx* c, size_t len, double** host, cudaEvent_t* ev)
 // another one, and destroy this one, before the launch is done.
 int mark_foreign(ps_gpu_ctx* c, ps_gpu_plan* P)
 {
-    if (c->stream == c->own_stream) return PS_OK;
+    if (c->stream == c->own_stream || stream_captured(c->stream)) return PS_OK;
     size_t done = 0;
     while (done < P->foreign.size() && cudaEventQuery(P->foreign[done]) == cudaSuccess) c->spare_events.push_back(P->foreign[done++]);
     P->foreign.erase(P->foreign.begin(), P->foreign.begin() + (long)done);

@@ -123,3 +123,34 @@ def test_plan_destroyed_while_a_callers_stream_still_runs_it(gpu_lib):
             got = out.cpu().numpy()[:2 * len(first)].reshape(-1, 2)
             np.testing.assert_array_equal(got[:, 0], B)
             np.testing.assert_array_equal(got[:, 1], Np)
+
+
+def test_launch_inside_a_callers_graph(gpu_lib):
+    """An eager plan launched on a caller's stream that captures: the caller's graph
+    replays it on the field loaded last."""
+    import torch
+    ps = gpu_lib
+    fields = [torch.from_numpy(synth.lognormal_density(N, 2.0, seed)).cuda() for seed in (3, 4)]
+    cfgs = triangles(ps, 0, 6, 30.0, 1) + triangles(ps, ps.PS_BIN_WATKINSON, 2, 12.0, 2) + quads(ps)
+    with ps.Context(N, BOX, methods=ps.PS_FP32_BATCHED) as ctx:
+        p = ctx.plan(cfgs, graph=False)
+        want = []
+        for f in fields:
+            ctx.get_FT_field(ps.PS_FIELD_DENS, f)
+            want.append(p.execute()[:2])
+        p.prepare()  # counts by transforms have been on the side stream of this context
+        p.execute()
+        s = torch.cuda.Stream()
+        ctx.set_stream(s.cuda_stream)
+        p.launch()  # one launch outside: the capture below finds everything made
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            p.launch()
+        ctx.set_stream(None)
+        for f, w in zip(fields, want):
+            ctx.get_FT_field(ps.PS_FIELD_DENS, f)
+            g.replay()
+            torch.cuda.synchronize()
+            same(p.results()[:2], w)
+        p.close()
