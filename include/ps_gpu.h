@@ -136,8 +136,10 @@ int ps_gpu_init(ps_gpu_ctx **ctx, int nbins, double boxsize, const void *field,
 int ps_gpu_polyspectrum(ps_gpu_ctx *ctx, int n, const double *k, double *kmin, double *kmax,
                         double kbinwidth, int kbinningCase, double *B, double *Npoly);
 
-/* nconf configurations with an explicit method (PS_FP64_PLAIN evaluates them
- * one by one; PS_FP32_BATCHED plans them together).  kappa_or_NULL receives a
+/* nconf configurations with an explicit method (PS_FP64_PLAIN takes every sum on
+ * the full grid in FP64, the distinct legs of a batch of configurations
+ * transformed together; PS_FP32_BATCHED plans them together on the smallest
+ * grids).  kappa_or_NULL receives a
  * condition number per configuration: sum |terms| / |sum terms| of the final
  * FP64 sum the method evaluates (grid sum or Parseval k-space sum). */
 int ps_gpu_polyspectrum_batch(ps_gpu_ctx *ctx, int method, int nconf, ps_cfg *cfgs, double *B,
@@ -159,7 +161,8 @@ int ps_gpu_polyspectrum_batch(ps_gpu_ctx *ctx, int method, int nconf, ps_cfg *cf
  * flag the fastest of the smallest and up to two larger supported sizes, timed
  * at plan creation (not for groups whose smallest size is below 96); the flag also times, per FP32 transform size the groups
  * use, the Y pass with its default thread layout against one with twice the
- * elements per thread (one radix pass fewer) and keeps the faster, and the
+ * elements per thread (one radix pass fewer; or, for split transforms, the
+ * register plan) and keeps the faster, and the
  * pair kernel (the per-row product of two inverse transforms, transformed
  * forward again) in its default layout, with one row transform live in
  * registers, and with twice the elements per thread, keeping the fastest,
@@ -323,7 +326,9 @@ int ps_make_configs(const ps_run_params *p, ps_cfg *cfgs, int max_cfg, double *k
                     double *theta_out);
 
 /* Use a caller-provided CUDA stream (cudaStream_t passed as void*); NULL
- * returns to the context's own stream. */
+ * returns to the context's own stream.  Work queued on different streams of one
+ * context shares its buffers: order them.  Destroying a plan waits for its
+ * launches on either. */
 int ps_gpu_set_stream(ps_gpu_ctx *ctx, void *stream);
 
 /* Device timing of the last ps_gpu_* compute call on the context, in ms
