@@ -2665,7 +2665,10 @@ int plan_batched(ps_gpu_ctx* c, ps_gpu_plan* P)
             c_lo = std::min(c_lo, uniq[G.third[q]].tag == 0 ? std::max(I.gtable[q].r2lo, 0) : 0);
             c_hi = std::max(c_hi, uniq[G.third[q]].tag == 0 ? I.gtable[q].r2hi : 0x7fffffff);
         }
-        if (I.enum_counts) I.enum_counts = pair_count_lists(I.sa, I.sb, N, c_lo, c_hi, I.gtable.size() == 1, &I.lists);
+        if (I.enum_counts) {
+            const int M = alias_free_grid(N, std::min(I.sa.band, N / 2), std::min(I.sb.band, N / 2), I.hmax);
+            I.enum_counts = pair_count_lists(I.sa, I.sb, N, M, c_lo, c_hi, I.gtable.size() == 1, &I.lists);
+        }
         any_fft = any_fft || !I.enum_counts;
     }
     P->fft_counts = any_fft;

@@ -273,36 +273,6 @@ struct PairCountLists {
     bool wrap = false;
 };
 
-// Modes of an interval shell on the N-grid (lattice frequencies [-N/2, N/2)):
-// per (x, y) column the z with r2lo <= x^2 + y^2 + z^2 <= r2hi.
-inline std::vector<short4> interval_modes(const Shell& sh, int N)
-{
-    std::vector<short4> out;
-    const int b = std::min(sh.band, N / 2);
-    const int top = std::min(b, N / 2 - 1);
-    if (sh.r2hi < 0 || sh.r2lo > sh.r2hi) return out;
-    for (int x = -b; x <= top; x++)
-        for (int y = -b; y <= top; y++) {
-            const long long rest_hi = (long long)sh.r2hi - x * x - y * y;
-            if (rest_hi < 0) continue;
-            const long long rest_lo = (long long)sh.r2lo - x * x - y * y;
-            int zmax = (int)sqrt((double)rest_hi);
-            while ((long long)zmax * zmax > rest_hi) zmax--;
-            while ((long long)(zmax + 1) * (zmax + 1) <= rest_hi) zmax++;
-            int zmin = 0;
-            if (rest_lo > 0) {
-                zmin = (int)sqrt((double)rest_lo);
-                while ((long long)zmin * zmin < rest_lo) zmin++;
-                while (zmin > 0 && (long long)(zmin - 1) * (zmin - 1) >= rest_lo) zmin--;
-            }
-            for (int az = zmin; az <= zmax; az++) {
-                if (az <= top) out.push_back(short4{(short)x, (short)y, (short)az, 0});
-                if (az > 0 && az <= b) out.push_back(short4{(short)x, (short)y, (short)-az, 0});
-            }
-        }
-    return out;
-}
-
 // Representatives 0 <= x <= y <= z (N/2 stands for -N/2, which is the same index) of the
 // orbits of an interval shell's modes under the 48 axis permutations and sign
 // flips, with the orbit sizes: 6, 3 or 1 permutations, two signs per component
@@ -330,29 +300,71 @@ inline std::vector<int4> interval_orbits(const Shell& sh, int N)
     return out;
 }
 
-// The lists of a group with interval legs a, b on an N-grid, the histogram over
-// the squared radii [c_lo, c_hi] its closing shells may hold (one: a single closing
-// shell, no histogram); false when the
-// enumeration does not apply (histogram too large for shared memory, or more
-// pairs than the FP64 transforms of the shells would cost).
-inline bool pair_count_lists(const Shell& sa, const Shell& sb, int N, int c_lo, int c_hi, bool one, PairCountLists* L)
+inline size_t orbit_total(const std::vector<int4>& reps)
 {
-    // host work O(b^2 + |S|); the enumeration itself |S_a| |S_b| / 48 pairs
+    size_t n = 0;
+    for (const int4& a : reps) n += (size_t)a.w;
+    return n;
+}
+
+// The modes of a shell from its orbits (lattice frequencies [-N/2, N/2)): one pass over
+// the representatives per permutation and signs, so that neighbours in the list are
+// neighbours on the shell.  About 2 ns a mode; a walk over all (x, y) columns with their
+// square roots took 8.5.
+template <int A, int B, int C>  // component A takes x, B takes y, C takes z
+inline void orbit_images(const std::vector<int4>& reps, int N, short4*& out)
+{
+    constexpr bool xy = B < A, yz = C < B;  // equal components in one order only
+    for (int signs = 0; signs < 8; signs++) {
+        // no -0, and N/2 as -N/2 only: the value that a sign leaves out
+        const int sx = signs & 1 ? -1 : 1, sy = signs & 2 ? -1 : 1, sz = signs & 4 ? -1 : 1;
+        const int ox = sx < 0 ? 0 : N / 2, oy = sy < 0 ? 0 : N / 2, oz = sz < 0 ? 0 : N / 2;
+        for (const int4& a : reps) {
+            if ((a.x == ox) | (a.y == oy) | (a.z == oz) | (xy & (a.x == a.y)) | (yz & (a.y == a.z))) continue;
+            const short x = (short)(sx * a.x), y = (short)(sy * a.y), z = (short)(sz * a.z);
+            *out++ = short4{A == 0 ? x : B == 0 ? y : z, A == 1 ? x : B == 1 ? y : z, A == 2 ? x : B == 2 ? y : z, 0};
+        }
+    }
+}
+inline std::vector<short4> orbit_modes(const std::vector<int4>& reps, int N)
+{
+    std::vector<short4> modes(orbit_total(reps));
+    short4* out = modes.data();
+    orbit_images<0, 1, 2>(reps, N, out);
+    orbit_images<0, 2, 1>(reps, N, out);
+    orbit_images<1, 0, 2>(reps, N, out);
+    orbit_images<1, 2, 0>(reps, N, out);
+    orbit_images<2, 0, 1>(reps, N, out);
+    orbit_images<2, 1, 0>(reps, N, out);
+    return modes;
+}
+
+// Pairs up to which the counts of a group with one closing shell are enumerated; beyond,
+// the FP64 transforms of the unit shells on the group's M-grid are the cheaper.  A group's
+// transforms take about 60 us and 7 ps a cell (96 points 65 us, 256 points 180 us, 600
+// points 1.57 ms), the enumeration 1 ps a pair where components wrap, 0.37 ps where none
+// can, beside the field's part.  Lone triangles at 128 points: 4.9e7 pairs 107 us against
+// 94 us by transforms, 5.9e8 pairs 356 against 107; at 320 points 2.8e8 pairs 491 against
+// 501, 1.1e9 pairs 849 against 501.  Lists of many small groups, whose transforms are chains
+// of launches one after the other, are why the line is not lower at 128 points (64
+// equilateral triangles, up to 5.4e7 pairs each: 0.49 ms in all).
+inline double one_shell_pairs(int M, bool wrap) { return (60e6 + 7.0 * (double)M * M * M) * (wrap ? 1.0 : 2.67); }
+constexpr double kHistPairs = 4e9;  // the same with histograms (several closing shells share them)
+
+// The lists of a group with interval legs a, b on an N-grid whose transforms would run on
+// the M-grid, the histogram over the squared radii [c_lo, c_hi] its closing shells may
+// hold (one: a single closing shell, no histogram); false when the enumeration does not
+// apply (histogram too large for shared memory, or more pairs than the FP64 transforms of
+// the shells would cost).  Nothing is listed before that is known, but the orbits: listing
+// the modes of thick shells first took longer than all transforms (256^3, sides of 64 to 77
+// modes, 13 modes thick: 6.8 of 8.3 ms).
+inline bool pair_count_lists(const Shell& sa, const Shell& sb, int N, int M, int c_lo, int c_hi, bool one, PairCountLists* L)
+{
     const double est = 4.0 * 3.14159 * (double)std::max(sa.r2hi, 1) * 4.0 * 3.14159 * (double)std::max(sb.r2hi, 1);
     if (std::max(sa.band, sb.band) > 300 || est / 48.0 > 4e10) return false;
-    // representatives from the smaller shell
-    const Shell *pa = &sa, *pb = &sb;
-    const auto volume = [](const Shell& h) { return pow((double)std::max(h.r2hi, 0), 1.5) - pow((double)std::max(h.r2lo, 0), 1.5); };
-    if (volume(sa) > volume(sb)) std::swap(pa, pb);
-    L->reps = interval_orbits(*pa, N);
-    if (48.0 * (double)L->reps.size() * 4.19 * std::max(volume(*pb), 1.0) / 48.0 > 1.2e10) return false;
-    L->modes = interval_modes(*pb, N);
-    // a single closing shell takes about 1.5 wrapping pairs in a nanosecond (0.14 ms of
-    // the 128^3 sweep's), the transforms of a group at 600 points 1.5 ms
-    const bool wraps = std::min(sa.band, N / 2) + std::min(sb.band, N / 2) >= N / 2;
-    if ((double)L->reps.size() * (double)L->modes.size() > (wraps ? 1.5e9 : 4e9)) return false;
     const int bmax_a = std::min(sa.band, N / 2), bmax_b = std::min(sb.band, N / 2);
     L->wrap = bmax_a + bmax_b >= N / 2;
+    const double most = one ? one_shell_pairs(M, L->wrap) : kHistPairs;
     const double ra_hi = sqrt((double)std::max(sa.r2hi, 0)), rb_hi = sqrt((double)std::max(sb.r2hi, 0));
     const double ra_lo = sqrt((double)std::max(sa.r2lo, 0)), rb_lo = sqrt((double)std::max(sb.r2lo, 0));
     double smax = (ra_hi + rb_hi) * (ra_hi + rb_hi);
@@ -361,12 +373,24 @@ inline bool pair_count_lists(const Shell& sa, const Shell& sb, int N, int c_lo, 
     L->s_lo = std::max(0, (int)floor(dmin * dmin) - 1);
     L->s_lo = std::max(L->s_lo, c_lo);
     const long long s_hi = std::max<long long>(L->s_lo, std::min<long long>((long long)ceil(smax) + 1, c_hi));
-    if (one) {
-        L->nbins = 0;
-        return true;
-    }
-    if (s_hi - L->s_lo + 1 > kCountMaxBins) return false;
-    L->nbins = (int)(s_hi - L->s_lo + 1);
+    if (!one && s_hi - L->s_lo + 1 > kCountMaxBins) return false;
+    L->nbins = one ? 0 : (int)(s_hi - L->s_lo + 1);
+    const auto volume = [](const Shell& h) {
+        return 4.18879 * (pow((double)std::max(h.r2hi, 0), 1.5) - pow((double)std::max(h.r2lo, 0), 1.5));
+    };
+    // shells inside the grid's cube hold about their volume of modes: far too many are
+    // refused before their orbits are listed
+    const double inside = (double)(N / 2) * (N / 2);
+    if (sa.r2hi < inside && sb.r2hi < inside && volume(sa) * volume(sb) / 48.0 > 1.5 * most) return false;
+    // representatives from the smaller shell
+    const Shell *pa = &sa, *pb = &sb;
+    if (volume(sa) > volume(sb)) std::swap(pa, pb);
+    L->reps = interval_orbits(*pa, N);
+    const bool same = sa.r2lo == sb.r2lo && sa.r2hi == sb.r2hi && sa.band == sb.band;
+    const std::vector<int4> other = same ? std::vector<int4>() : interval_orbits(*pb, N);
+    const std::vector<int4>& orbits_b = same ? L->reps : other;
+    if ((double)L->reps.size() * (double)orbit_total(orbits_b) > most) return false;
+    L->modes = orbit_modes(orbits_b, N);
     return true;
 }
 

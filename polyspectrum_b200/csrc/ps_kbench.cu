@@ -347,7 +347,7 @@ int main(int argc, char** argv)
         std::vector<Shell> cl;
         for (int q = 0; q < 16; q++) cl.push_back(shell(32.0 + 8.0 * q, 32.0 + 8.0 * q + 16.0));
         PairCountLists L;
-        if (!pair_count_lists(sa, sb, NG, 0, 0x7fffffff, false, &L)) { fprintf(stderr, "count lists refused\n"); return 1; }
+        if (!pair_count_lists(sa, sb, NG, 384, 0, 0x7fffffff, false, &L)) { fprintf(stderr, "count lists refused\n"); return 1; }
         int4* dreps; short4* dmodes; Shell* dcl; unsigned long long* dcnt;
         CK(cudaMalloc(&dreps, L.reps.size() * sizeof(int4)));
         CK(cudaMalloc(&dmodes, L.modes.size() * sizeof(short4)));
