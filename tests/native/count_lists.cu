@@ -1,6 +1,5 @@
 // The lists of exact polygon counts on the host: modes of interval shells from their
 // orbits against a walk over the whole grid, and which pairs of shells are listed.
-#include <chrono>
 #include <cstdio>
 #include <set>
 #include <tuple>
@@ -63,12 +62,10 @@ int main()
     for (const auto& q : rule) {
         PairCountLists L;
         const Shell s = thick(q.r, q.w, q.n);
-        const auto t0 = std::chrono::steady_clock::now();
         const bool got = pair_count_lists(s, s, q.n, q.m, 0, 0x7fffffff, q.one != 0, &L);
-        const double us = std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t0).count();
         const double pairs = (double)L.reps.size() * (double)orbit_total(L.reps);
-        printf("rule n %d m %d r %.1f w %.1f one %d: %d want %d, reps %zu, pairs %.2e, modes %zu, %.0f us\n", q.n, q.m, q.r, q.w,
-               q.one, (int)got, q.want, L.reps.size(), pairs, L.modes.size(), us);
+        printf("rule n %d m %d r %.1f w %.1f one %d: %d want %d, reps %zu, pairs %.2e, modes %zu\n", q.n, q.m, q.r, q.w,
+               q.one, (int)got, q.want, L.reps.size(), pairs, L.modes.size());
     }
     return 0;
 }
