@@ -177,8 +177,8 @@ int ps_gpu_polyspectrum_batch(ps_gpu_ctx *ctx, int method, int nconf, ps_cfg *cf
  * every leg pair (m_a, m_b), S_a reduced to orbit representatives under the
  * 48 axis permutations and sign flips, histogrammed by |m_a + m_b|^2 (wrapped
  * on the grid as the reference's cyclic sums wrap), or compared with the
- * interval of the one closing shell; groups of more than 4e9 pairs (1.5e9
- * when they wrap) are counted with transforms.  PS_PLAN_FFT_COUNTS
+ * interval of the one closing shell; groups with so many pairs that the
+ * transforms cost less are counted with those.  PS_PLAN_FFT_COUNTS
  * counts with FP64 transforms of the unit shells instead (the reference's
  * dataflow; WATKINSON shells always do).  Both give the same integers. */
 #define PS_PLAN_FFT_COUNTS 8
